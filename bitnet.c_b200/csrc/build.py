@@ -47,6 +47,7 @@ SOURCES: Dict[str, str] = {
     "unit_norm": "unit_norm.cu",
     "mlstm": "mlstm.cu",
     "moe": "moe.cu",
+    "moe_few": "moe_few.cu",
     "rotary_pairs": "rotary_pairs.cu",
     "delta_rule": "delta_rule.cu",
     "streams": "streams.cu",

@@ -2135,7 +2135,8 @@ def moe_few_fits(width: int, top: int, ff: int) -> bool:
 def moe_experts_few(h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gate_up: torch.Tensor,
                     w_down: torch.Tensor, limit: float, slope: float, scale_input: bool,
                     add: Optional[torch.Tensor] = None, act: int = -1, add_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """The chosen experts of every token, streamed once per (token, expert): float32 ``[T, width]``, the sum over
+    """The chosen experts of every token (in bfloat16 each expert is read once for all tokens that chose it; else, and where rows
+    are not whole 16-byte pieces, once per (token, expert)): float32 ``[T, width]``, the sum over
     a token's experts plus ``add``.  The weight multiplies the expert's input (``scale_input``) or its output.
     ``act`` < 0: the clamped unit with ``limit`` and ``slope``; ACT_SILU / ACT_GELU_TANH: act(gate) * up; ACT_RELU2: no gate,
     the square of relu(up), and ``w_gate_up`` is ``[experts, ff, width]``.  Ids from the number of experts on are identity experts:
@@ -2163,17 +2164,43 @@ def moe_experts_few(h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w
         if add_scale.shape[0] != T:
             raise KernelError("moe_experts_few: add_scale does not fit")
     y = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
+    out = torch.empty((T, width), dtype=torch.float32, device=h.device)
+    per_call = min(MOE_FEW_TOKENS, MOE_FEW_ITEMS // top)
+    if (h.dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and E <= 1024 and per_call > 0
+            and (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0):
+        for t0 in range(0, T, per_call):
+            _moe_few_tokens(h, ids, weights, w_gate_up, w_down, limit, slope, scale_input, add, act, add_scale, y, out, t0,
+                            min(per_call, T - t0))
+        return out
     w_up = w_gate_up[:, ff:] if per == 2 else w_gate_up
     _check(_fn("moe", "bn_moe_gate_up_ex")(_ptr(h), int(_code(h)), int(T), int(width), _ptr(ids), _ptr(weights),
                                            int(bool(scale_input)), _ptr(w_gate_up if per == 2 else None), c_void_p(w_up.data_ptr()),
                                            ctypes.c_longlong(per * ff * width), int(ff), int(top), c_float(limit),
                                            c_float(slope), int(act), int(E), _ptr(y), _stream()), "moe_gate_up")
-    out = torch.empty((T, width), dtype=torch.float32, device=h.device)
     _check(_fn("moe", "bn_moe_down")(_ptr(y), int(_code(y)), int(T), int(ff), _ptr(ids), _ptr(weights),
                                      int(not scale_input), _ptr(w_down), int(width), int(top), _ptr(add),
                                      int(_code(add) if add is not None else 0), _ptr(add_scale), int(E), _ptr(h), _ptr(out), _stream()),
            "moe_down")
     return out
+
+
+MOE_FEW_ITEMS = 128  # (token, expert) items one launch of moe_few.cu takes (MF_MAX_ITEMS)
+MOE_FEW_TOKENS = 64  # and tokens: an expert's rows are then read once for all of them
+
+
+def _moe_few_tokens(h, ids, weights, w_gate_up, w_down, limit, slope, scale_input, add, act, add_scale, y, out, t0: int, n: int) -> None:
+    """``moe_experts_few`` for the tokens ``t0 .. t0 + n``: every chosen expert read once for all of them (bfloat16)."""
+    width, top, E, ff = h.shape[1], ids.shape[1], w_gate_up.shape[0], w_down.shape[2]
+    per = w_gate_up.shape[1] // ff
+    at = lambda t, rows: c_void_p(t.data_ptr() + rows * t.stride(0) * t.element_size() if t is not None else 0)
+    gate = w_gate_up.data_ptr()
+    _check(_fn("moe_few", "bn_moe_few")(
+        at(h, t0), int(n), int(width), at(ids, t0), at(weights, t0), int(bool(scale_input)), c_void_p(gate if per == 2 else 0),
+        c_void_p(gate + (per - 1) * ff * width * 2), ctypes.c_longlong(per * ff * width), int(ff), int(top), c_float(limit), c_float(slope),
+        int(act), int(E), at(y, t0 * top), _ptr(w_down), at(add, t0), int(_code(add) if add is not None else 0), at(add_scale, t0),
+        at(out, t0), _stream()), "moe_few")
+    global LAUNCHES
+    LAUNCHES += 1  # two kernels
 
 
 def moe_count(ids: torch.Tensor, n_experts: int) -> torch.Tensor:

@@ -26,12 +26,12 @@ class Moe(FeedForward):
     the input itself; ``activation`` "relu2": down(max(up x, 0)^2), no gate; ``shared_gate``: the shared expert's output times the
     logistic function of one number per token, a row of the router's product.
 
-    Few rows (a decode step): two kernels stream the chosen experts once per (token, expert), from
+    Few rows (a decode step): two kernels stream the chosen experts, in bfloat16 once for all the tokens that chose them, from
     device memory alone.  Many rows: the (token, expert) items are sorted by expert, and in bfloat16 all experts run as one
     grouped product each way, which reads the experts' row counts on the device.  Otherwise (float32, odd sizes) every
     expert's rows go through the ordinary products; the host then needs the counts, one copy per call."""
 
-    kernels = ("linear", "linear_mma", "linear_tc", "gemm_tc", "act", "moe")
+    kernels = ("linear", "linear_mma", "linear_tc", "gemm_tc", "act", "moe", "moe_few")
     graph_safe = True  # the steps that are recorded are decode steps, which take the path without the host
     FEW_ITEMS = 64  # up to so many (token, expert) items the streaming kernels run
     USE_GROUPED = True  # (tests and comparisons set it to False)
