@@ -1422,7 +1422,7 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: 
         # a matrix with few rows shares its inner dimension out over several blocks (a property of the matrix alone)
         n_splits = getattr(build.library("linear"), "bn_linear_skinny_splits")
         n_splits.restype = c_int
-        splits = n_splits(int(N), int(K))
+        splits = n_splits(int(N), int(K), int(_code(w)))
         partial = torch.empty((splits, M, N), dtype=torch.float32, device=x.device) if splits > 1 else None
         _check(_fn("linear", "bn_linear_skinny")(_ptr(x), _ptr(w), int(_code(w)), _ptr(out), int(_DT[out_dtype]),
                                                  int(M), int(N), int(K), int(N),

@@ -84,6 +84,24 @@ def test_linear_skinny(cuda_device, dtype, M, N, K):
     assert (y.double() - ref).abs().max().item() < 1e-4 * max(1.0, K / 256)
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 3, 8), (2, 37, 2048), (3, 5, 2056), (4, 4099, 4096), (5, 1203, 136), (8, 9473, 2176),
+                                   (9, 2371, 4104), (16, 33, 14336)])
+def test_linear_stream_float32(cuda_device, M, N, K):
+    """Streamed float32 products: columns that do not fill a warp's four, inner dimensions that end within a piece or a part of
+    2,048, more rows than one group; and a row's result is the same whatever rows are beside it."""
+    g = torch.Generator().manual_seed(M * 7919 + N)
+    x = torch.randn(M, K, generator=g).to(cuda_device)
+    w = (torch.randn(N, K, generator=g) * 0.05).to(cuda_device)
+    b = torch.randn(N, generator=g).to(cuda_device)
+    y = ops.linear(x, w, bias=b)
+    ref = x.double() @ w.double().t() + b.double()
+    # every partial sum is rounded once per addition: at most K / 32 in a lane, five in the tree, one per part and one for the bias
+    size = x.double().abs() @ w.double().abs().t() + b.double().abs()
+    assert ((y.double() - ref).abs() <= (K / 32 + 7 + K / 2048) * 2.0 ** -24 * size).all()
+    for m in {0, M - 1}:
+        assert torch.equal(ops.linear(x[m:m + 1], w, bias=b)[0], y[m])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_linear_many_rows_is_float32_exact(cuda_device, dtype):
     g = torch.Generator().manual_seed(5)
