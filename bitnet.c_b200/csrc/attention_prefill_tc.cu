@@ -109,12 +109,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
   unsigned char* k_smem = q_smem + Q_BYTES;                   // KS pages of keys
   unsigned char* v_smem = k_smem + KS * PAGE_BYTES;           // VS pages of values
   unsigned long long* bars = (unsigned long long*)(v_smem + VS * V_BYTES);
-  // barriers: q_full, k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], s_full[2], p_full[2], pv_done
+  // barriers: q_full, k_full[KS], k_empty[KS], v_full[VS], v_empty[VS], s_full[2], p_full[2], pv_done[2]
   const unsigned bar0 = smem_u32(bars);
   const unsigned q_full = bar0, k_full0 = bar0 + 8, k_empty0 = k_full0 + 8 * KS, v_full0 = k_empty0 + 8 * KS,
                  v_empty0 = v_full0 + 8 * VS, s_full0 = v_empty0 + 8 * VS,
-                 p_full0 = s_full0 + 16, pv_done = p_full0 + 16;
-  unsigned* tmem_slot = (unsigned*)(bars + 2 * KS + 2 * VS + 6);
+                 p_full0 = s_full0 + 16, pv_done0 = p_full0 + 16;
+  unsigned* tmem_slot = (unsigned*)(bars + 2 * KS + 2 * VS + 7);
   volatile int* failed = (volatile int*)(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -156,8 +156,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     for (int b = 0; b < 2; ++b) {
       mbar_init(s_full0 + 8 * b, 1);
       mbar_init(p_full0 + 8 * b, 4);  // one arrival per softmax warp
+      mbar_init(pv_done0 + 8 * b, 1);
     }
-    mbar_init(pv_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -253,7 +253,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
               umma_mma_ts(tbase + O_COL, tbase + b * PT_KEYS + PT_KEYS / 2 + kk * 8, umma_desc_mn(sv + kk * 2048, KV_BOX), IDESC_O, 1u);
           }
           umma_commit(v_empty0 + 8 * s);    // the value stage may be refilled
-          umma_commit(pv_done);             // O holds the pages up to i
+          umma_commit(pv_done0 + 8 * (i & 1));  // O holds the pages up to i
           BN_TRACE_ONLY(if (tr) a.trace[i * 12 + 8] = global_timer();)
         }
         __syncwarp();
@@ -274,6 +274,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       BN_TRACE_ONLY(const bool tr = a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && tid == 64 && j < PT_TRACE_TILES;)
       BN_TRACE_ONLY(if (tr) a.trace[j * 12 + 0] = global_timer();)
       if (!pt_wait(s_full0 + 8 * b, (unsigned)(j >> 1) & 1u, failed, a.status)) { ok = false; break; }
+      // The product of the page before the last is done too (its MMAs were issued before S_j's).  Even and odd pages have a barrier
+      // each and every warp takes each of their phases in turn, so a parity always means the phase that is asked for: with
+      // one barrier for all pages a warp that came to the epilogue after both last products were done waited for the next
+      // phase, which never came.
+      if (j >= 2 && !pt_wait(pv_done0 + 8 * b, (unsigned)((j >> 1) - 1) & 1u, failed, a.status)) { ok = false; break; }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       BN_TRACE_ONLY(if (tr) a.trace[j * 12 + 1] = global_timer();)
       float s[PT_KEYS];
@@ -297,7 +302,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       else need = m_tile > m_ref + PT_RESCALE;
       if (__any_sync(0xffffffffu, need)) {
         // O of the pages before this one must be complete before it is rescaled (j >= 1 here)
-        if (!pt_wait(pv_done, (unsigned)(j - 1) & 1u, failed, a.status)) { ok = false; break; }
+        if (!pt_wait(pv_done0 + 8 * ((j - 1) & 1), (unsigned)((j - 1) >> 1) & 1u, failed, a.status)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const float alpha = need ? exp2f(m_ref - m_tile) : 1.0f;
         if (need) { m_ref = m_tile; l_run *= alpha; }
@@ -360,11 +365,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       BN_TRACE_ONLY(if (tr) a.trace[j * 12 + 5] = global_timer();)
     }
     // ---- epilogue: O / sum -> out
-    // A warp may be here while the others still owe their share of P for the page before the last: the last scores were
-    // issued ahead of that page's product.  pv_done is asked for both pages in turn, since its parity alone would not tell
-    // the last page from the one two before it.
-    if (ok && n_tiles > 1) ok = pt_wait(pv_done, (unsigned)n_tiles & 1u, failed, a.status);
-    if (ok && pt_wait(pv_done, (unsigned)(n_tiles - 1) & 1u, failed, a.status)) {
+    // (a warp may be here while the others still owe their share of P for the page before the last: both pages in turn)
+    if (ok && n_tiles > 1) ok = pt_wait(pv_done0 + 8 * ((n_tiles - 2) & 1), (unsigned)((n_tiles - 2) >> 1) & 1u, failed, a.status);
+    if (ok && pt_wait(pv_done0 + 8 * ((n_tiles - 1) & 1), (unsigned)((n_tiles - 1) >> 1) & 1u, failed, a.status)) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       float inv = 1.0f / l_run;
       if (a.sink) {  // 1 / (sum + 2^(sink - m)), also when the sink exceeds every score
@@ -429,7 +432,7 @@ extern "C" int bn_attention_prefill_tc_trace_read(unsigned long long* host) {
 template <int HD, int VD, int KS, int VS, bool PRECISE>
 static int launch_pt(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const PtArgs& a, int n_tiles,
                      cudaStream_t stream) {
-  size_t smem = (size_t)PT_ROWS * HD * 2 + (size_t)(KS * HD + VS * VD) * PT_KEYS * 2 + (2 * KS + 2 * VS + 6) * 8 + 16;
+  size_t smem = (size_t)PT_ROWS * HD * 2 + (size_t)(KS * HD + VS * VD) * PT_KEYS * 2 + (2 * KS + 2 * VS + 7) * 8 + 16;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<HD, VD, KS, VS, PRECISE>,

@@ -669,3 +669,32 @@ def test_linear_takes_the_own_gemm_when_asked(cuda_device, monkeypatch):
     monkeypatch.setattr(ops, "gemm_tc", lambda *p, **k: (calls.append(1), real(*p, **k))[1])
     b = ops.linear(x, w, out_dtype=torch.float32)
     assert calls and (a - b).abs().max().item() < 1e-4
+
+
+@pytest.mark.parametrize("hd,precise", [(64, False), (128, False), (128, True)])
+def test_attention_prefill_tc_warps_apart_at_the_end(cuda_device, hd, precise):
+    """Many sequences of every length from one page on, launched again and again: however far the softmax warps of a block are
+    apart when the last pages' products complete, each takes every page's signal in turn (a warp that came late to one barrier
+    shared by all pages missed the last but one, waited for two seconds and gave up).  The results are the same every time and
+    no wait gave up."""
+    H, KV = 4, 2
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    lens = [1 + (i * 37) % 700 for i in range(64)]
+    n, pages = sum(lens), [(m + 63) // 64 for m in lens]
+    q = torch.randn((n, H * hd), device="cuda", generator=g).bfloat16()
+    kc, vc = (torch.randn((sum(pages) + 1, KV, 64, hd), device="cuda", generator=g).bfloat16() for _ in range(2))
+    ints = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")
+    table, at = torch.zeros((64, max(pages)), dtype=torch.int32, device="cuda"), 1
+    for i, p in enumerate(pages):
+        table[i, :p] = torch.arange(at, at + p, device="cuda")
+        at += p
+    tiles = [(i, r) for i, c in enumerate(lens) for r in range(0, c, 128)]
+    start = ints(np.concatenate([[0], np.cumsum(lens)]))
+    args = (ints(i for i, _ in tiles), ints(r for _, r in tiles), start, ints([0] * 64), ints(range(64)), table, kc, vc)
+    first = None
+    for _ in range(20):
+        out = torch.empty((n, H * hd), dtype=torch.bfloat16, device="cuda")
+        ops.attention_prefill_tc(q, q.shape[1], out, H, KV, hd, hd ** -0.5, 0, *args, precise=precise)
+        first = out if first is None else first
+        assert torch.equal(out, first)
+    ops.check_tc_status(torch.device("cuda:0"))
