@@ -17,7 +17,8 @@
 
 __device__ __forceinline__ float dr_softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
-// One block per token.  proj [T, stride] (type T): the channels of q, k, v at q_off, k_off, v_off
+// A block per token and part of its channels (blockIdx.y of gridDim.y: a share of the q and k heads, of v's channels and of the
+// decays; one block per token took 46 us for the 6,144 channels of a single token, each thread 24 of them in turn).  proj [T, stride] (type T): the channels of q, k, v at q_off, k_off, v_off
 // (n_qk = kv_heads * dim wide twice, n_v = heads * vdim).  conv_w: the three tap tables [channels, taps]
 // one after another (q, k, v; type W).  The heads' beta pre-activations lie at b_off in proj's rows;
 // a_raw [T, a_stride] float32 holds the decays' pre-activations in its first heads * dim columns.
@@ -33,13 +34,18 @@ __global__ void delta_prepare_kernel(const T* __restrict__ proj, int stride, int
                                      float* __restrict__ beta) {
   pdl_launch_dependents();
   pdl_wait();
-  extern __shared__ float ch[];  // the q and k channels after convolution and SiLU
+  extern __shared__ float ch[];  // this part's q and k channels after convolution and SiLU
   const int t = blockIdx.x;
   const int s = tok_seq[t];
   const int r = t - seq_start[s];  // the token's place among the new tokens of its sequence
   const int n_qk = kv_heads * dim, n_v = heads * vdim, n_ch = 2 * n_qk + n_v;
   const float* tail = state + (size_t)slots[s] * state_stride + tail_off;
-  for (int c = threadIdx.x; c < n_ch; c += blockDim.x) {
+  const int part = blockIdx.y, parts = gridDim.y;
+  auto share = [&](int n, int p) { return (int)((long long)n * p / parts); };
+  const int item0 = share(2 * kv_heads, part), items = share(2 * kv_heads, part + 1) - item0;  // q heads, then k heads
+  const int v0 = share(n_v, part), own_qk = items * dim, own = own_qk + share(n_v, part + 1) - v0;
+  for (int i = threadIdx.x; i < own; i += blockDim.x) {
+    const int c = i < own_qk ? item0 * dim + i : 2 * n_qk + v0 + (i - own_qk);
     const int col = c < n_qk ? q_off + c : (c < 2 * n_qk ? k_off + c - n_qk : v_off + c - 2 * n_qk);
     float acc = 0.f;
     for (int j = 0; j < taps; ++j) {
@@ -50,27 +56,31 @@ __global__ void delta_prepare_kernel(const T* __restrict__ proj, int stride, int
       acc = fmaf(to_f32<W>(conv_w[(size_t)c * taps + j]), xin, acc);
     }
     const float y = acc / (1.0f + expf(-acc));
-    if (c < 2 * n_qk) ch[c] = y;
+    if (i < own_qk) ch[i] = y;
     else vc[(size_t)t * n_v + c - 2 * n_qk] = y;
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-  for (int item = warp; item < 2 * kv_heads; item += n_warps) {  // q heads, then k heads
-    const float* v = ch + (size_t)item * dim;
+  for (int i = warp; i < items; i += n_warps) {
+    const int item = item0 + i;
+    const float* v = ch + (size_t)i * dim;
     float ss = 0.f;
-    for (int i = lane; i < dim; i += 32) ss = fmaf(v[i], v[i], ss);
+    for (int e = lane; e < dim; e += 32) ss = fmaf(v[e], v[e], ss);
     ss = warp_sum(ss);
     const bool is_q = item < kv_heads;
     const float scale = (1.0f / sqrtf(ss + 1e-6f)) * (is_q ? q_scale : 1.0f);
     float* dst = (is_q ? qn : kn) + (size_t)t * n_qk + (size_t)(is_q ? item : item - kv_heads) * dim;
-    for (int i = lane; i < dim; i += 32) dst[i] = v[i] * scale;
+    for (int e = lane; e < dim; e += 32) dst[e] = v[e] * scale;
   }
-  for (int e = threadIdx.x; e < heads * dim; e += blockDim.x) {
+  const int e1 = share(heads * dim, part + 1);
+  for (int e = share(heads * dim, part) + threadIdx.x; e < e1; e += blockDim.x) {
     const int h = e / dim;
     const float dt = dr_softplus(a_raw[(size_t)t * a_stride + e] + to_f32<W>(dt_bias[e]));
     decay[(size_t)t * heads * dim + e] = expf(-expf(to_f32<W>(a_log[h])) * dt);
   }
-  for (int h = threadIdx.x; h < heads; h += blockDim.x) beta[(size_t)t * heads + h] = 1.0f / (1.0f + expf(-to_f32<T>(proj[(size_t)t * stride + b_off + h])));
+  const int h1 = share(heads, part + 1);
+  for (int h = share(heads, part) + threadIdx.x; h < h1; h += blockDim.x)
+    beta[(size_t)t * heads + h] = 1.0f / (1.0f + expf(-to_f32<T>(proj[(size_t)t * stride + b_off + h])));
 }
 
 // After the step's convolutions: the last taps - 1 inputs of every sequence, old ones kept where the
@@ -229,7 +239,11 @@ extern "C" int bn_delta_prepare(const void* proj, int dtype, int n_tokens, int s
       !beta || q_off < 0 || k_off < 0 || v_off < 0 || q_off + n_qk > stride || k_off + n_qk > stride || v_off + n_v > stride ||
       (size_t)2 * n_qk * sizeof(float) > 160 * 1024)
     return BN_ERR_BAD_ARG;
-  const size_t smem = (size_t)2 * n_qk * sizeof(float);
+  // parts of a token: four channels per thread, or one where there are few tokens; at most one per q or k head
+  const int channels = 2 * n_qk + n_v, per_part = n_tokens <= 64 ? 256 : 1024;
+  int parts = (channels + per_part - 1) / per_part;
+  if (parts > 2 * kv_heads) parts = 2 * kv_heads;
+  const size_t smem = (size_t)((2 * kv_heads + parts - 1) / parts) * dim * sizeof(float);
 #define DR_PREP(TT, WW)                                                                                                    \
   do {                                                                                                                     \
     if (smem > 48 * 1024) {                                                                                                \
@@ -240,7 +254,7 @@ extern "C" int bn_delta_prepare(const void* proj, int dtype, int n_tokens, int s
         granted = smem;                                                                                                    \
       }                                                                                                                    \
     }                                                                                                                      \
-    BN_LAUNCH((delta_prepare_kernel<TT, WW>), n_tokens, 256, smem, stream, (const TT*)proj, stride, q_off, k_off, v_off,  \
+    BN_LAUNCH((delta_prepare_kernel<TT, WW>), dim3(n_tokens, parts), 256, smem, stream, (const TT*)proj, stride, q_off, k_off, v_off,  \
               kv_heads, heads, dim, vdim, taps, (const WW*)conv_w, (const float*)state, (size_t)state_stride,             \
               (size_t)tail_off, tok_seq, seq_start, slots, b_off, a_raw, a_stride, (const WW*)dt_bias, (const WW*)a_log, q_scale,   \
               qn, kn, vc, decay, beta);                                                                                    \
