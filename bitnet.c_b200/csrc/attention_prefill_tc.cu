@@ -24,7 +24,7 @@
 // contiguous (MN-major); K and Q are K-major.
 // With PRECISE the weights enter the second product as two bfloat16 terms, P = P_hi + P_lo (16 bits of mantissa): P_lo
 // takes the second half of the columns S_j came from, and O += P_lo V_j follows O += P_hi V_j.  Value rows may have a
-// width of their own (VD), and a sink, a score per head without a key or a value, may enlarge the rows' sums at the end.
+// width of their own (VD), several key heads may read one value head, the result may be left in float32, and a sink, a score per head without a key or a value, may enlarge the rows' sums at the end.
 // The new tokens' own keys and values must already be in the cache, so the same kernel serves
 // whole prompts, pieces of prompts and ragged batches (a table gives each block its sequence and
 // first row).  Head sizes in steps of 16 up to 192 run on the instantiation for 64, 128 or 192: columns
@@ -49,8 +49,9 @@
 #define PT_ERR_WAIT 5
 
 struct PtArgs {
-  __nv_bfloat16* out;
-  int out_stride;
+  void* out;  // bfloat16, or float32 with out_wide
+  int out_stride, out_wide;
+  int v_share;  // so many key heads, neighbours, read one value head
   int n_heads, n_kv_heads, head_dim, v_dim;
   const float* sink;  // [n_heads] or null
   const __nv_bfloat16* gate;  // [n_tokens, gate_stride]: a number per head whose logistic function multiplies its output, or null
@@ -189,7 +190,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         mbar_expect_tx(bar, values ? V_BYTES : PAGE_BYTES);
 #pragma unroll
         for (int bx = 0; bx < (BOXES > V_BOXES ? BOXES : V_BOXES); ++bx)
-          if (bx < (values ? V_BOXES : BOXES)) tma_load_3d(dst + bx * KV_BOX, values ? &map_v : &map_k, bar, bx * 64, kvh * BN_PAGE, page);
+          if (bx < (values ? V_BOXES : BOXES)) tma_load_3d(dst + bx * KV_BOX, values ? &map_v : &map_k, bar, bx * 64, (values ? kvh / a.v_share : kvh) * BN_PAGE, page);
         return true;
       };
       bool ok = true;
@@ -376,7 +377,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       }
       if (a.gate && r < rows_here) inv *= 1.0f / (1.0f + expf(-__bfloat162float(a.gate[(size_t)(start + row0 + r) * a.gate_stride + h])));
       inv *= a.out_scale;
-      __nv_bfloat16* orow = a.out + (size_t)(start + row0 + r) * a.out_stride + (size_t)h * a.v_dim;
+      const size_t at = (size_t)(start + row0 + r) * a.out_stride + (size_t)h * a.v_dim;
 #pragma unroll
       for (int c = 0; c < VD; c += 32) {
         float o[32];
@@ -384,10 +385,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         if (r < rows_here) {
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
-            if (c + g * 8 < a.v_dim) {  // head sizes are multiples of 16: groups of 8 are whole
+            if (c + g * 8 >= a.v_dim) continue;  // head sizes are multiples of 16: groups of 8 are whole
+            if (a.out_wide) {
+              float4* o4 = reinterpret_cast<float4*>((float*)a.out + at + c + g * 8);
+              o4[0] = make_float4(o[g * 8] * inv, o[g * 8 + 1] * inv, o[g * 8 + 2] * inv, o[g * 8 + 3] * inv);
+              o4[1] = make_float4(o[g * 8 + 4] * inv, o[g * 8 + 5] * inv, o[g * 8 + 6] * inv, o[g * 8 + 7] * inv);
+            } else {
               uint4 w = make_uint4(pack_bf16x2(o[g * 8] * inv, o[g * 8 + 1] * inv), pack_bf16x2(o[g * 8 + 2] * inv, o[g * 8 + 3] * inv),
                                    pack_bf16x2(o[g * 8 + 4] * inv, o[g * 8 + 5] * inv), pack_bf16x2(o[g * 8 + 6] * inv, o[g * 8 + 7] * inv));
-              *reinterpret_cast<uint4*>(orow + c + g * 8) = w;
+              *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + at + c + g * 8) = w;
             }
           }
         }
@@ -457,14 +463,16 @@ static int launch_pt(const CUtensorMap& mq, const CUtensorMap& mk, const CUtenso
 // The values' cache is [n_cache_pages, n_kv_heads, 64, v_dim] with v_dim a multiple of 16 up to 128.  precise: the weights
 // enter the value product with 16 bits of mantissa.  sink: [n_heads] float32 scores that stand in the sums only, or null.
 // gate [n_tokens, gate_stride]: a number per token and head whose logistic function multiplies the head's output, or null;
-// out_scale: a factor on all of the output.
+// out_scale: a factor on all of the output.  v_share: so many key heads, neighbours, read one value head (the values' cache then has
+// n_kv_heads / v_share heads).  out_wide: the output is float32.
 extern "C" int bn_attention_prefill_tc_ex(const void* q, int q_stride, int n_tokens, void* out, int out_stride, int n_tiles,
                                           int n_heads, int n_kv_heads, int head_dim, int v_dim, float scale, int window, int precise,
-                                          const float* sink, const void* gate, int gate_stride, float out_scale, const int* tile_seq, const int* tile_row0, const int* seq_start,
-                                          const int* seq_pos0, const int* slots, const int* page_table, int pt_stride,
+                                          const float* sink, const void* gate, int gate_stride, float out_scale, int v_share, int out_wide,
+                                          const int* tile_seq, const int* tile_row0, const int* seq_start, const int* seq_pos0, const int* slots, const int* page_table, int pt_stride,
                                           const void* k_cache, const void* v_cache, int n_cache_pages, int* status,
                                           cudaStream_t stream) {
   if (n_tiles <= 0) return BN_OK;
+  if (v_share <= 0 || n_kv_heads <= 0 || n_kv_heads % v_share) return BN_ERR_BAD_ARG;
   if (head_dim <= 0 || head_dim % 16 || head_dim > 192 || v_dim <= 0 || v_dim % 16 || v_dim > 128 || !(scale > 0.f) || n_kv_heads <= 0 || n_heads % n_kv_heads || window < 0 ||
       n_heads > 65535 || (q_stride % 8) || (out_stride % 8) || n_tokens <= 0 || n_cache_pages <= 0 || !status ||
       (((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15))
@@ -473,10 +481,10 @@ extern "C" int bn_attention_prefill_tc_ex(const void* q, int q_stride, int n_tok
   if (!tma_map_bf16_strided(&mq, q, (unsigned long long)n_tokens, (unsigned long long)n_heads * head_dim,
                             (unsigned long long)q_stride, PT_ROWS) ||
       !tma_map_bf16_pages(&mk, k_cache, n_cache_pages, (unsigned long long)n_kv_heads * BN_PAGE, head_dim, BN_PAGE) ||
-      !tma_map_bf16_pages(&mv, v_cache, n_cache_pages, (unsigned long long)n_kv_heads * BN_PAGE, v_dim, BN_PAGE))
+      !tma_map_bf16_pages(&mv, v_cache, n_cache_pages, (unsigned long long)(n_kv_heads / v_share) * BN_PAGE, v_dim, BN_PAGE))
     return BN_ERR_BAD_ARG;
   PtArgs a = {};
-  a.out = (__nv_bfloat16*)out; a.out_stride = out_stride; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
+  a.out = out; a.out_stride = out_stride; a.out_wide = out_wide; a.v_share = v_share; a.n_heads = n_heads; a.n_kv_heads = n_kv_heads;
   a.head_dim = head_dim; a.v_dim = v_dim; a.sink = sink; a.gate = (const __nv_bfloat16*)gate;
   a.gate_stride = gate_stride; a.out_scale = out_scale; a.scale_log2e = scale * 1.4426950408889634f; a.window = window; a.tile_seq = tile_seq;
   a.tile_row0 = tile_row0; a.seq_start = seq_start; a.seq_pos0 = seq_pos0; a.slots = slots; a.page_table = page_table;
@@ -505,6 +513,6 @@ extern "C" int bn_attention_prefill_tc(const void* q, int q_stride, int n_tokens
                                        const void* k_cache, const void* v_cache, int n_cache_pages, int* status,
                                        cudaStream_t stream) {
   return bn_attention_prefill_tc_ex(q, q_stride, n_tokens, out, out_stride, n_tiles, n_heads, n_kv_heads, head_dim, head_dim, scale,
-                                    window, 0, nullptr, nullptr, 0, 1.0f, tile_seq, tile_row0, seq_start, seq_pos0, slots, page_table, pt_stride,
+                                    window, 0, nullptr, nullptr, 0, 1.0f, 1, 0, tile_seq, tile_row0, seq_start, seq_pos0, slots, page_table, pt_stride,
                                     k_cache, v_cache, n_cache_pages, status, stream);
 }

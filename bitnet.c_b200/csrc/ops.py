@@ -758,15 +758,20 @@ def attention_prefill_tc(q: torch.Tensor, q_stride: int, out: torch.Tensor, n_he
                          seq_start: torch.Tensor, seq_pos0: torch.Tensor, slots: torch.Tensor, page_table: torch.Tensor,
                          k_cache: torch.Tensor, v_cache: torch.Tensor, *, precise: bool = False,
                          sink: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None, gate_stride: int = 0,
-                         out_scale: float = 1.0) -> torch.Tensor:
+                         out_scale: float = 1.0, v_share: int = 1) -> torch.Tensor:
     """bfloat16 causal attention of runs of new tokens on tcgen05 tensor cores with TMA-fed operands;
     block i handles up to 128 new tokens of sequence tile_seq[i] from its row tile_row0[i] on.
     Key widths up to 192 and value widths up to 128 (a value head has the width of ``v_cache``'s rows).  ``precise``: the softmax weights
-    enter the value product with 16 bits of mantissa instead of 8; ``sink``, ``gate``, an ``out`` of columns and ``out_scale`` as for
-    ``attention_general``."""
+    enter the value product with 16 bits of mantissa instead of 8; ``sink``, ``gate``, ``v_share``, a float32 ``out``, an ``out`` of columns and ``out_scale``
+    as for ``attention_general``."""
     if not q.is_cuda or q.dim() != 2 or q.stride(-1) != 1 or q.stride(0) != q_stride or q.dtype != torch.bfloat16:
         raise KernelError("attention_prefill_tc: q must be a bfloat16 CUDA matrix with unit inner stride")
-    _need_rows(out, "out", torch.bfloat16)
+    _need_rows(out, "out")
+    wide = out.dtype == torch.float32
+    if out.dtype not in (torch.bfloat16, torch.float32):
+        raise KernelError("attention_prefill_tc: out must be bfloat16 or float32")
+    if v_share < 1 or n_kv_heads % v_share:
+        raise KernelError(f"attention_prefill_tc: {n_kv_heads} key heads cannot share values {v_share} at a time")
     if gate is not None and (not gate.is_cuda or gate.dtype != torch.bfloat16 or gate.stride(-1) != 1
                              or gate.shape[-1] < n_heads or gate_stride <= 0):
         raise KernelError("attention_prefill_tc: gate must be a bfloat16 CUDA view with unit inner stride and one number per head")
@@ -777,7 +782,7 @@ def attention_prefill_tc(q: torch.Tensor, q_stride: int, out: torch.Tensor, n_he
     _need(k_cache, "k_cache", torch.bfloat16, 4)
     _need(v_cache, "v_cache", torch.bfloat16, 4)
     v_dim = v_cache.shape[3]
-    if tuple(k_cache.shape[1:]) != (n_kv_heads, PAGE, head_dim) or k_cache.shape[:3] != v_cache.shape[:3]:
+    if tuple(k_cache.shape[1:]) != (n_kv_heads, PAGE, head_dim) or tuple(v_cache.shape[:3]) != (k_cache.shape[0], n_kv_heads // v_share, PAGE):
         raise KernelError(f"attention_prefill_tc: cache {tuple(k_cache.shape)} / {tuple(v_cache.shape)} is not "
                           f"[pages, {n_kv_heads}, {PAGE}, {head_dim} / value width]")
     if head_dim % 16 or head_dim > 192 or v_dim % 16 or v_dim > 128 or n_heads % n_kv_heads:
@@ -788,11 +793,11 @@ def attention_prefill_tc(q: torch.Tensor, q_stride: int, out: torch.Tensor, n_he
             raise KernelError(f"attention_prefill_tc: {sink.shape[0]} sink scores for {n_heads} heads")
     if out.shape[1] < n_heads * v_dim or q_stride % 8 or n_heads * head_dim > q_stride or out.shape[0] < q.shape[0]:
         raise KernelError("attention_prefill_tc: out or q_stride does not fit")
-    if precise or sink is not None or v_dim != head_dim or gate is not None or out_scale != 1.0:
+    if precise or sink is not None or v_dim != head_dim or gate is not None or out_scale != 1.0 or v_share > 1 or wide:
         _check(_fn("attention_prefill_tc", "bn_attention_prefill_tc_ex")(
             _ptr(q), int(q_stride), int(q.shape[0]), _ptr(out), int(out.stride(0)), int(tile_seq.shape[0]), int(n_heads),
             int(n_kv_heads), int(head_dim), int(v_dim), c_float(scale), int(window), int(bool(precise)), _ptr(sink), _ptr(gate),
-            int(gate_stride), c_float(out_scale), _ptr(tile_seq), _ptr(tile_row0), _ptr(seq_start), _ptr(seq_pos0), _ptr(slots), _ptr(page_table), int(page_table.shape[1]), _ptr(k_cache),
+            int(gate_stride), c_float(out_scale), int(v_share), int(wide), _ptr(tile_seq), _ptr(tile_row0), _ptr(seq_start), _ptr(seq_pos0), _ptr(slots), _ptr(page_table), int(page_table.shape[1]), _ptr(k_cache),
             _ptr(v_cache), int(k_cache.shape[0]), _ptr(tc_status(q.device)), _stream()), "attention_prefill_tc")
         return out
     _check(_fn("attention_prefill_tc", "bn_attention_prefill_tc")(

@@ -27,7 +27,7 @@ class NormedAttention(Mixer):
     times 1 - diff.  The rows of the query projection are reordered when the weights are bound so that the maps
     of the heads that share a key head lie side by side, [group][map][head in group]."""
 
-    kernels = ("linear", "linear_mma", "linear_tc", "gemm_tc", "attention", "attention_prefill", "unit_norm")
+    kernels = ("linear", "linear_mma", "linear_tc", "gemm_tc", "attention", "attention_prefill", "attention_prefill_tc", "unit_norm")
     TILED_MIN_TOKENS = 16  # runs of new tokens from this many on take the tensor-core kernel (bfloat16)
     graph_safe = True
 
@@ -159,10 +159,16 @@ class NormedAttention(Mixer):
         # two maps leave their sums unrounded for the difference that follows
         out = torch.empty((n, H * s.v_head_dim), dtype=torch.float32 if s.maps == 2 else dt, device=dev)
         gate = proj[:, self.g_off:] if s.head_gate else None
-        if (dt == torch.bfloat16 and not ctx.decode and ctx.tile_seq is not None and ctx.max_new >= self.TILED_MIN_TOKENS
-                and s.v_head_dim % 16 == 0 and s.head_dim % 16 == 0 and s.head_dim <= 256 and s.v_head_dim <= 256):
-            # runs of new tokens: 64 tokens of a sequence and a head per block on the tensor cores, the
-            # softmax weights with 16 bits of mantissa
+        runs = dt == torch.bfloat16 and not ctx.decode and ctx.max_new >= self.TILED_MIN_TOKENS
+        if (runs and ops.USE_TCGEN05_ATTENTION and ctx.wide_tile_seq is not None and s.scale > 0 and s.head_dim % 16 == 0
+                and s.head_dim <= 192 and s.v_head_dim % 16 == 0 and s.v_head_dim <= 128):
+            # runs of new tokens on tcgen05: 128 tokens of a sequence and a head per block, the softmax weights with 16 bits of
+            # mantissa (two prompts of up to 4,000 tokens, three such layers at 32 heads: 5.5 ms on the kernel below, 2.1 here)
+            ops.attention_prefill_tc(proj, self.row, out, H, G, s.head_dim, s.scale, s.window, ctx.wide_tile_seq, ctx.wide_tile_row0,
+                                     ctx.seq_start, ctx.seq_pos0, ctx.slots, kv.page_table, kv.k, kv.v, precise=True, sink=self.sink,
+                                     gate=gate, gate_stride=self.row, v_share=s.maps)
+        elif (runs and ctx.tile_seq is not None and s.v_head_dim % 16 == 0 and s.head_dim % 16 == 0 and s.head_dim <= 256 and s.v_head_dim <= 256):
+            # the same on mma.sync, 64 tokens per block: wide heads
             ops.attention_prefill(proj, self.row, out, H, G, s.head_dim, s.scale, s.window, ctx.tile_seq, ctx.tile_row0,
                                   ctx.seq_start, ctx.seq_pos0, ctx.slots, kv.page_table, kv.k, kv.v, gate=gate,
                                   gate_stride=self.row, precise=True, sink=self.sink, v_share=s.maps)

@@ -203,6 +203,41 @@ def test_attention_with_a_sink_and_shared_values_over_the_pages(cuda_device, dty
             check(out, f"runs of tokens, float32 out {wide}")
 
 
+@pytest.mark.parametrize("H,G,d,dv,share,window,gated", [(8, 4, 64, 128, 2, 0, False), (4, 2, 16, 48, 2, 100, False), (6, 6, 128, 64, 3, 0, True),
+                                                         (4, 4, 176, 128, 4, 70, False), (4, 2, 128, 128, 1, 0, True)])
+@pytest.mark.parametrize("wide", [False, True])
+def test_shared_values_and_float32_results_on_tcgen05(cuda_device, H, G, d, dv, share, window, gated, wide):
+    """Several key heads over one value head and results left in float32, pieces behind cached tokens and unequal runs, against
+    the general kernel in float32."""
+    from bitnet_c_b200.csrc import ops
+    lens, new = [300, 131, 17], [300, 70, 17]
+    g = torch.Generator(device="cuda").manual_seed(H * d + dv)
+    n, pages = sum(new), [(m + 63) // 64 for m in lens]
+    q = torch.randn((n, H * d + H + 8 - H % 8), device="cuda", generator=g).bfloat16() * 2
+    kc = torch.randn((sum(pages) + 1, G, 64, d), device="cuda", generator=g).bfloat16()
+    vc = torch.randn((sum(pages) + 1, G // share, 64, dv), device="cuda", generator=g).bfloat16()
+    table, at = torch.zeros((3, max(pages)), dtype=torch.int32, device="cuda"), 1
+    for i, p in enumerate(pages):
+        table[i, :p] = torch.arange(at, at + p, device="cuda")
+        at += p
+    start, slots = ints(np.concatenate([[0], np.cumsum(new)])), ints(range(3))
+    pos0 = ints(a - b for a, b in zip(lens, new))
+    tok_seq = ints(np.concatenate([np.full(c, i) for i, c in enumerate(new)]))
+    tok_pos = ints(np.concatenate([np.arange(m - c, m) for m, c in zip(lens, new)]))
+    tiles = [(i, r) for i, c in enumerate(new) for r in range(0, c, 128)]
+    sink, gate = torch.zeros(H, device="cuda"), q[:, H * d:] if gated else None
+    got = torch.full((n, H * dv), float("nan"), dtype=torch.float32 if wide else torch.bfloat16, device="cuda")
+    ops.attention_prefill_tc(q, q.shape[1], got, H, G, d, d ** -0.5, window, ints(i for i, _ in tiles), ints(r for _, r in tiles), start, pos0,
+                             slots, table, kc, vc, precise=True, sink=sink, gate=gate, gate_stride=q.shape[1], v_share=share)
+    ref = torch.empty((n, H * dv), dtype=torch.float32, device="cuda")
+    qf = q.float().contiguous()
+    ops.attention_general(qf, q.shape[1], ref, n, H, G, d, d ** -0.5, window, tok_seq, tok_pos, slots, table, kc.float(), vc.float(), sink=sink,
+                          gate=qf[:, H * d:] if gated else None, gate_stride=q.shape[1], v_share=share)
+    # weights of 16 bits of mantissa over values of size up to about 5, and the result's own rounding to bfloat16
+    assert bool(((got.float() - ref).abs() <= 5 * 2.0 ** -15 + (0 if wide else 2.0 ** -8) * ref.abs()).all())
+    ops.check_tc_status(torch.device("cuda:0"))
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_two_maps_combined_gates_on_rows_experts_by_table_and_the_rotation_of_halves(cuda_device, dtype):
     from bitnet_c_b200.csrc import ops
