@@ -210,13 +210,22 @@ class Cache:
                 self.states[i] = torch.zeros((n_slots,) + tuple(r.shape), dtype=r.dtype, device=device)
                 if isinstance(i, tuple):
                     self._named.setdefault(i[0], {})[i[1]] = self.states[i]
+        self._state_rows = None  # where the states lie, for zeroing a slot of all of them in one launch
+        if self.states and torch.device(device).type == "cuda":
+            from ..csrc import ops
+            self._state_rows = ops.slot_rows(self.states.values())
 
     # ---- slots ----------------------------------------------------------------------------
     def open(self) -> int:
         """A free slot for a new sequence: length 0, no pages, state zero."""
         slot = self.slots.open()
-        for t in self.states.values():
-            t[slot].zero_()
+        if self._state_rows is not None:
+            from ..csrc import ops
+            with torch.cuda.device(self.device):
+                ops.zero_slot(self._state_rows, slot)
+        else:
+            for t in self.states.values():
+                t[slot].zero_()
         return slot
 
     def close(self, slot: int) -> None:

@@ -30,6 +30,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 # family name -> source file
 SOURCES: Dict[str, str] = {
     "embed": "embed.cu",
+    "cache_rows": "cache_rows.cu",
     "norm": "norm.cu",
     "rope": "rope.cu",
     "act": "act.cu",

@@ -1456,6 +1456,23 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: 
     return out
 
 
+# ---- state --------------------------------------------------------------------------------
+def slot_rows(tensors) -> Optional[torch.Tensor]:
+    """What ``zero_slot`` needs of tensors ``[slots, ...]``: int64 ``[n, 2]`` on the device, each one's address and bytes per slot.
+    None if there are none, or where they are not contiguous on a CUDA device."""
+    tensors = list(tensors)
+    if not tensors or not all(t.is_cuda and t.is_contiguous() for t in tensors):
+        return None
+    rows = [[t.data_ptr(), t.stride(0) * t.element_size()] for t in tensors]
+    return torch.tensor(rows, dtype=torch.int64, device=tensors[0].device)
+
+
+def zero_slot(rows: torch.Tensor, slot: int) -> None:
+    """Slot ``slot`` of all tensors that ``rows`` (of ``slot_rows``) was made from is set to zero, in one launch."""
+    _need(rows, "rows", torch.int64, 2)
+    _check(_fn("cache_rows", "bn_zero_slot")(_ptr(rows), int(rows.shape[0]), int(slot), _stream()), "zero_slot")
+
+
 # ---- mLSTM ----------------------------------------------------------------------------------
 def mlstm_gates(h: torch.Tensor, w: torch.Tensor, bias: torch.Tensor, n_heads: int, cap: float) -> torch.Tensor:
     """float32 ``[T, 2 * heads]``: per head the soft-capped log input gate, then the log forget gate

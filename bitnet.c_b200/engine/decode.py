@@ -102,6 +102,7 @@ class DecodeRunner:
                     self._body()
                 ops.LAUNCHES = before  # recording launches nothing
                 self.graphs[self.ctx.max_len] = g
+            self.model.note_pass()
             g.replay()
             ops.LAUNCHES += self.launches_per_step  # the replay launches every recorded kernel
         self.host_pos = [p + 1 for p in positions]

@@ -9,6 +9,7 @@ src/transformer/prefill.c:2494) and one token (bn_transformer_forward, src/trans
 """
 from __future__ import annotations
 
+import itertools
 from typing import Any, Dict, List, Optional, Sequence
 
 import torch
@@ -61,6 +62,10 @@ class Model:
         self.embedding: Optional[torch.Tensor] = None
         self.head: Optional[torch.Tensor] = None
         self._bad_token: Optional[torch.Tensor] = None
+        # a number of its own for every forward pass and every replay of one: who looked at the kernels' status since the last of
+        # them need not look again
+        self._passes = itertools.count(1)
+        self.last_pass = 0
         self.diagnostics = None  # engine/diagnostics.py: tensor dumps, top logits, kernel timers
         self._owners: Dict[str, tuple] = {}
         for i, blk in enumerate(self.blocks):
@@ -243,8 +248,13 @@ class Model:
             cache.advance(s.slot, len(s.tokens))
         return logits
 
+    def note_pass(self) -> None:
+        """A pass is about to be launched (a forward, or the replay of a recorded one)."""
+        self.last_pass = next(self._passes)
+
     def forward(self, cache: Cache, ctx: StepContext) -> Optional[torch.Tensor]:
         """Embedding, every scheduled run, final norm and head at the wanted rows."""
+        self.note_pass()
         streams = getattr(self.spec, "streams", 1)
         x = torch.empty((ctx.n_tokens, streams * self.spec.width), dtype=torch.float32, device=self.device)
         sched = self.spec.schedule
