@@ -393,26 +393,331 @@ __global__ void attention_merge_kernel(const float* __restrict__ part, int n_spl
                                        const float* __restrict__ sink, int out_wide, float out_scale) {
   pdl_launch_dependents();
   pdl_wait();
+  // Bound by latency: the parts' maxima and sums are one load per lane, their weights are worked out once, and a thread's numbers
+  // are asked for eight at a time.
+  __shared__ float weight[64];  // at most 64 splits
+  __shared__ float s_inv;
   const int t = blockIdx.x, h = blockIdx.y;
   const float* p = part + ((size_t)t * n_heads + h) * n_splits * (v_dim + 2);
-  float M = -INFINITY;
-  for (int z = 0; z < n_splits; ++z) M = fmaxf(M, p[(size_t)z * (v_dim + 2)]);
-  float L = 0.f;
-  for (int z = 0; z < n_splits; ++z) {
-    float m = p[(size_t)z * (v_dim + 2)];
-    if (m != -INFINITY) L += expf(m - M) * p[(size_t)z * (v_dim + 2) + 1];
+  if (threadIdx.x < 32) {
+    float m[2], l[2], M = -INFINITY, L = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int z = threadIdx.x + 32 * i;
+      m[i] = z < n_splits ? p[(size_t)z * (v_dim + 2)] : -INFINITY;
+      l[i] = z < n_splits ? p[(size_t)z * (v_dim + 2) + 1] : 0.f;
+      M = fmaxf(M, m[i]);
+    }
+    M = warp_max(M);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float w = m[i] != -INFINITY ? expf(m[i] - M) : 0.f;  // (a part without keys holds nothing)
+      if (m[i] != -INFINITY) L += w * l[i];
+      weight[threadIdx.x + 32 * i] = w;
+    }
+    L = warp_sum(L);
+    if (threadIdx.x == 0) {
+      float inv = sink ? sink_inverse(M, L, sink[h]) : 1.0f / L;
+      if (gate) inv *= 1.0f / (1.0f + expf(-to_f32<T>(gate[(size_t)t * gate_stride + h])));
+      s_inv = inv * out_scale;
+    }
   }
-  float inv = sink ? sink_inverse(M, L, sink[h]) : 1.0f / L;
-  if (gate) inv *= 1.0f / (1.0f + expf(-to_f32<T>(gate[(size_t)t * gate_stride + h])));
-  inv *= out_scale;
+  __syncthreads();
+  const float inv = s_inv;
   for (int d = threadIdx.x; d < v_dim; d += blockDim.x) {
     float a = 0.f;
-    for (int z = 0; z < n_splits; ++z) {
-      float m = p[(size_t)z * (v_dim + 2)];
-      if (m != -INFINITY) a = fmaf(expf(m - M), p[(size_t)z * (v_dim + 2) + 2 + d], a);
+    for (int z0 = 0; z0 < n_splits; z0 += 8) {
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = z0 + i < n_splits ? p[(size_t)(z0 + i) * (v_dim + 2) + 2 + d] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float w = z0 + i < n_splits ? weight[z0 + i] : 0.f;
+        if (w != 0.f) a = fmaf(w, v[i], a);
+      }
     }
     store_result<T>(out, out_wide, (size_t)t * out_stride + (size_t)h * v_dim + d, a * inv);
   }
+}
+
+// ---- few tokens in bfloat16 on the tensor cores ---------------------------------------------------
+// A block takes one token, up to 16 query heads of one key/value head and, of every n_splits x 64 visible keys, 64.  Their key and
+// value rows are copied into shared memory (two stages where both fit), every row once for all the heads; four warps take 16 keys
+// each for the scores (mma.sync m16n8k16, heads as the 16 rows; the inner dimension is taken in the order in which 16-byte pieces
+// lie in a lane, the same for both operands) and a quarter of the value width each for the weighted sum.  The weights enter that
+// product as three bfloat16 terms, 24 bits of mantissa, so nothing is rounded that float32 would not round; values inside the key
+// rows are read from the same copy.
+// Bound by latency: a token's keys are few kilobytes per block.  The kernel above spends 4,300 instructions per warp on 128 keys
+// of 128 numbers, this one some 300.  Measured with the merge, us, before and after (tokens, heads, key/value heads, head size, visible keys):
+// 4, 16, 4, 128, 1024: 16.6 / 10.1;  2, 32, 8, 128, 4000: 35 / 25;  64, 32, 8, 128, 2000: 534 / 270;  key rows of 256 that hold values
+// of 192, 8, 16, 1, 1000: 33 / 13;  of 576 and 512, 2, 32, 1, 1024: 45 / 24.
+#define AM_THREADS 128
+#define AM_KEYS 64
+#define AM_P_PITCH 144  // bytes of 64 weights, padded: no bank conflicts between rows
+struct AmArgs {
+  const __nv_bfloat16* q;
+  int q_stride;
+  void* out;
+  int out_stride, n_heads, n_kv_heads, head_dim, v_dim;
+  float scale;
+  int window, keep_first, chunk, v_row;
+  const float* rel;
+  int n_rel;
+  const __nv_bfloat16* gate;
+  int gate_stride;
+  const int *tok_seq, *tok_pos, *slots, *page_table;
+  int pt_stride;
+  const __nv_bfloat16 *k_cache, *v_cache;
+  float* part;
+  int n_splits;
+  const float* sink;
+  int v_share, out_wide;
+  float out_scale;
+  int tiles_per_group;  // blocks of 16 heads per key/value head
+  int shared_rows;      // the values are a part of the key rows
+  int stages;
+  int q_pitch, k_pitch, v_pitch;  // bytes of a row in shared memory
+};
+__device__ __forceinline__ void am_copy(unsigned dst, const __nv_bfloat16* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ uint4 am_piece(unsigned addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void am_mma(float* c, unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int NT>  // tiles of 8 value dimensions per warp
+__global__ void __launch_bounds__(AM_THREADS) attention_few_mma_kernel(AmArgs a) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char am_smem[];
+  __shared__ int s_row[2][AM_KEYS];         // page x 64 + row of a stage's keys, -1: none
+  __shared__ float s_m[4][16], s_l[4][16];  // per warp and head
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, quad = lane & 3;
+  const int t = blockIdx.x, kvh = blockIdx.y / a.tiles_per_group, z = blockIdx.z;
+  const int gq = a.n_heads / a.n_kv_heads, first_head = (blockIdx.y % a.tiles_per_group) * 16;
+  const int h0 = kvh * gq + first_head, rows = min(16, gq - first_head);
+  const int vh = kvh / a.v_share, n_v_heads = a.n_kv_heads / a.v_share;
+  const int pos = a.tok_pos[t];
+  const int* pt = a.page_table + (size_t)a.slots[a.tok_seq[t]] * a.pt_stride;
+  const int lo = a.chunk > 0 ? (pos / a.chunk) * a.chunk : (a.window > 0 ? max(0, pos - a.window + 1) : 0);
+  const int n_first = min(a.keep_first, lo), n_keys = n_first + pos - lo + 1;
+  const int pieces = a.head_dim / 8, q_pieces = (a.head_dim + 31) / 32 * 4, v_pieces = a.v_dim / 8;
+
+  const unsigned base = (unsigned)__cvta_generic_to_shared(am_smem);
+  const unsigned qs = base, ps = qs + 16 * a.q_pitch, ks0 = ps + 3 * 16 * AM_P_PITCH;
+  const unsigned stage_bytes = AM_KEYS * (a.k_pitch + a.v_pitch);  // v_pitch 0: values in the key rows
+  auto position = [&](int u) { return u < n_first ? u : lo + (u - n_first); };
+  auto fill = [&](int it) {
+    const int u0 = (it * a.n_splits + z) * AM_KEYS, st = it % a.stages;
+    if (tid < AM_KEYS) {
+      const int u = u0 + tid, p = position(u);
+      s_row[st][tid] = u < n_keys ? pt[p / BN_PAGE] * BN_PAGE + p % BN_PAGE : -1;
+    }
+    __syncthreads();
+    const unsigned kd = ks0 + st * stage_bytes, vd = kd + AM_KEYS * a.k_pitch;
+    for (int i = tid; i < AM_KEYS * q_pieces; i += AM_THREADS) {  // (pieces past the head size are zeros)
+      const int r = i / q_pieces, c = i - r * q_pieces, at = s_row[st][r];
+      const bool live = at >= 0 && c < pieces;
+      am_copy(kd + r * a.k_pitch + c * 16,
+              live ? a.k_cache + (((size_t)(at / BN_PAGE) * a.n_kv_heads + kvh) * BN_PAGE + at % BN_PAGE) * a.head_dim + c * 8 : a.k_cache, live);
+    }
+    if (!a.shared_rows)
+      for (int i = tid; i < AM_KEYS * v_pieces; i += AM_THREADS) {
+        const int r = i / v_pieces, c = i - r * v_pieces, at = s_row[st][r];
+        am_copy(vd + r * a.v_pitch + c * 16,
+                at >= 0 ? a.v_cache + (((size_t)(at / BN_PAGE) * n_v_heads + vh) * BN_PAGE + at % BN_PAGE) * a.v_row + c * 8 : a.v_cache, at >= 0);
+      }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = tid; i < 16 * q_pieces; i += AM_THREADS) {
+    const int r = i / q_pieces, c = i - r * q_pieces;
+    const bool live = r < rows && c < pieces;
+    am_copy(qs + r * a.q_pitch + c * 16, live ? a.q + (size_t)t * a.q_stride + (size_t)(h0 + r) * a.head_dim + c * 8 : a.q, live);
+  }
+  const int span = a.n_splits * AM_KEYS;
+  const int turns = n_keys > z * AM_KEYS ? (n_keys - z * AM_KEYS + span - 1) / span : 0;
+  if (turns > 0) fill(0);
+
+  float o[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};  // heads g and g + 8; the sums of this lane's keys
+  for (int it = 0; it < turns; ++it) {
+    if (a.stages == 2 && it + 1 < turns) {
+      fill(it + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const int u0 = (it * a.n_splits + z) * AM_KEYS, st = it % a.stages;
+    const unsigned kd = ks0 + st * stage_bytes;
+    const unsigned vd = a.shared_rows ? kd : kd + AM_KEYS * a.k_pitch, v_pitch = a.shared_rows ? a.k_pitch : a.v_pitch;
+    // scores of this warp's 16 keys
+    float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    const unsigned xa = qs + g * a.q_pitch + quad * 16, ka = kd + (warp * 16 + g) * a.k_pitch + quad * 16;
+#pragma unroll 4
+    for (int c = 0; c < q_pieces; c += 4) {
+      const uint4 x0 = am_piece(xa + c * 16);
+      const uint4 x1 = rows > 8 ? am_piece(xa + 8 * a.q_pitch + c * 16) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        const uint4 k = am_piece(ka + n * 8 * a.k_pitch + c * 16);
+        am_mma(s[n], x0.x, x1.x, x0.y, x1.y, k.x, k.y);
+        am_mma(s[n], x0.z, x1.z, x0.w, x1.w, k.z, k.w);
+      }
+    }
+    float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int u = u0 + warp * 16 + n * 8 + quad * 2 + (e & 1), head = g + (e >> 1) * 8;
+        float v = -INFINITY;
+        if (u < n_keys) {
+          v = s[n][e] * a.scale;
+          if (a.rel && head < rows) v += a.rel[(size_t)min(pos - position(u), a.n_rel - 1) * a.n_heads + h0 + head];
+        }
+        s[n][e] = v;
+        mx[e >> 1] = fmaxf(mx[e >> 1], v);
+      }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
+      if (quad == 0) s_m[warp][g + 8 * i] = mx[i];
+    }
+    __syncthreads();
+    float alpha[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float m = m_run[i];
+#pragma unroll
+      for (int w = 0; w < 4; ++w) m = fmaxf(m, s_m[w][g + 8 * i]);
+      alpha[i] = m_run[i] == -INFINITY ? 0.f : expf(m_run[i] - m);
+      m_run[i] = m;
+      l_run[i] *= alpha[i];
+    }
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[j][e] *= alpha[e >> 1];
+    // the weights, as three bfloat16 terms each
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        float w0 = s[n][2 * i] == -INFINITY ? 0.f : expf(s[n][2 * i] - m_run[i]);
+        float w1 = s[n][2 * i + 1] == -INFINITY ? 0.f : expf(s[n][2 * i + 1] - m_run[i]);
+        l_run[i] += w0 + w1;
+        const unsigned dst = ps + (g + 8 * i) * AM_P_PITCH + (warp * 16 + n * 8 + quad * 2) * 2;
+#pragma unroll
+        for (int term = 0; term < 3; ++term) {
+          const __nv_bfloat162 both = __floats2bfloat162_rn(w0, w1);
+          asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + term * 16 * AM_P_PITCH), "r"(*reinterpret_cast<const unsigned*>(&both)) : "memory");
+          w0 -= __low2float(both);
+          w1 -= __high2float(both);
+        }
+      }
+    __syncthreads();
+    // this warp's share of the value dimensions
+#pragma unroll
+    for (int kk = 0; kk < AM_KEYS / 16; ++kk) {
+      unsigned p[3][4];
+#pragma unroll
+      for (int term = 0; term < 3; ++term)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(p[term][0]), "=r"(p[term][1]), "=r"(p[term][2]), "=r"(p[term][3])
+                     : "r"(ps + (term * 16 + (lane & 15)) * AM_P_PITCH + (kk * 16 + (lane >> 4) * 8) * 2) : "memory");
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const int tile = warp * NT + j;
+        if (tile >= v_pieces) continue;  // the same for the whole warp
+        unsigned b0, b1;
+        asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
+                     : "=r"(b0), "=r"(b1) : "r"(vd + (kk * 16 + (lane & 15)) * v_pitch + tile * 16) : "memory");
+#pragma unroll
+        for (int term = 0; term < 3; ++term) am_mma(o[j], p[term][0], p[term][1], p[term][2], p[term][3], b0, b1);
+      }
+    }
+    __syncthreads();  // keys, values and weights have been used
+    if (a.stages == 1 && it + 1 < turns) fill(it + 1);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
+    l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
+    if (quad == 0) s_l[warp][g + 8 * i] = l_run[i];
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");  // (q's copy, where there was no key)
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int head = g + 8 * i;
+    if (head >= rows) continue;
+    const int h = h0 + head;
+    const float l = (s_l[0][head] + s_l[1][head]) + (s_l[2][head] + s_l[3][head]);
+    if (a.part) {
+      float* prow = a.part + (((size_t)t * a.n_heads + h) * a.n_splits + z) * (a.v_dim + 2);
+      if (warp == 0 && quad == 0) { prow[0] = m_run[i]; prow[1] = l; }
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const int d = (warp * NT + j) * 8 + quad * 2;
+        if (d < a.v_dim) { prow[2 + d] = o[j][2 * i]; prow[3 + d] = o[j][2 * i + 1]; }
+      }
+    } else {
+      float inv = a.sink ? sink_inverse(m_run[i], l, a.sink[h]) : 1.0f / l;
+      if (a.gate) inv *= 1.0f / (1.0f + expf(-__bfloat162float(a.gate[(size_t)t * a.gate_stride + h])));
+      inv *= a.out_scale;
+      const size_t orow = (size_t)t * a.out_stride + (size_t)h * a.v_dim;
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const int d = (warp * NT + j) * 8 + quad * 2;
+        if (d < a.v_dim) {
+          store_result<__nv_bfloat16>((__nv_bfloat16*)a.out, a.out_wide, orow + d, o[j][2 * i] * inv);
+          store_result<__nv_bfloat16>((__nv_bfloat16*)a.out, a.out_wide, orow + d + 1, o[j][2 * i + 1] * inv);
+        }
+      }
+    }
+  }
+}
+
+#define AM_MAX_V_DIM 512
+#define AM_SMEM_MAX (200 * 1024)
+// Shared memory of the kernel above; fills in pitches and stages.
+static size_t am_layout(AmArgs* a) {
+  const int q_bytes = (a->head_dim + 31) / 32 * 64;
+  a->q_pitch = q_bytes % 128 ? q_bytes : q_bytes + 64;  // eight lanes read two rows' pieces without a conflict
+  a->k_pitch = a->shared_rows ? (q_bytes + 127) / 128 * 128 + 16 : a->q_pitch;  // ldmatrix reads eight rows
+  a->v_pitch = a->shared_rows ? 0 : (a->v_dim * 2 + 127) / 128 * 128 + 16;
+  const size_t fixed = (size_t)16 * a->q_pitch + 3 * 16 * AM_P_PITCH, stage = (size_t)AM_KEYS * (a->k_pitch + a->v_pitch);
+  a->stages = fixed + 2 * stage <= 112 * 1024 ? 2 : 1;
+  return fixed + a->stages * stage;
+}
+// Whether few tokens of these sizes run on it (bfloat16; 16-byte pieces everywhere).
+static bool am_fits(const AmArgs& a, int n_tokens) {
+  AmArgs b = a;
+  return n_tokens <= 256 && a.head_dim % 8 == 0 && a.v_dim % 8 == 0 && a.v_row % 8 == 0 && a.q_stride % 8 == 0 && a.v_dim <= AM_MAX_V_DIM &&
+         (((uintptr_t)a.q | (uintptr_t)a.k_cache | (uintptr_t)a.v_cache) & 15) == 0 && am_layout(&b) <= AM_SMEM_MAX;
+}
+template <int NT>
+static int am_launch(const AmArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
+  static bool granted = false;
+  if (!granted) {
+    cudaError_t e = cudaFuncSetAttribute(attention_few_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, AM_SMEM_MAX);
+    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
+    granted = true;
+  }
+  BN_LAUNCH(attention_few_mma_kernel<NT>, grid, AM_THREADS, smem, stream, a);
+  return BN_OK;
 }
 
 // q: [n_tokens, q_stride] with head h at element h*head_dim; out [n_tokens, out_stride] with head h at
@@ -437,6 +742,30 @@ extern "C" int bn_attention_general_ex(const void* q, int q_stride, void* out, i
       (!wide && v_dim > 8 * ATT_THREADS) || (rel && n_rel <= 0))
     return BN_ERR_BAD_ARG;
   if (n_heads > 65535) return BN_ERR_BAD_ARG;
+  if (dtype == BN_BF16) {
+    AmArgs am = {};
+    am.q = (const __nv_bfloat16*)q; am.q_stride = q_stride; am.out = out; am.out_stride = out_stride; am.n_heads = n_heads;
+    am.n_kv_heads = n_kv_heads; am.head_dim = head_dim; am.v_dim = v_dim; am.scale = scale; am.window = window; am.keep_first = keep_first;
+    am.chunk = chunk; am.v_row = v_row; am.rel = rel; am.n_rel = n_rel; am.gate = (const __nv_bfloat16*)gate; am.gate_stride = gate_stride;
+    am.tok_seq = tok_seq; am.tok_pos = tok_pos; am.slots = slots; am.page_table = page_table; am.pt_stride = pt_stride;
+    am.k_cache = (const __nv_bfloat16*)k_cache; am.v_cache = (const __nv_bfloat16*)v_cache; am.part = part; am.n_splits = n_splits;
+    am.sink = sink; am.v_share = v_share; am.out_wide = out_wide; am.out_scale = out_scale;
+    am.tiles_per_group = (n_heads / n_kv_heads + 15) / 16;
+    am.shared_rows = v_cache == k_cache && v_row == head_dim && v_share == 1 && v_dim <= head_dim;
+    if (am_fits(am, n_tokens)) {
+      const size_t smem = am_layout(&am);
+      const dim3 agrid(n_tokens, n_kv_heads * am.tiles_per_group, n_splits);
+      const int rc = v_dim <= 32 ? am_launch<1>(am, agrid, smem, stream) : v_dim <= 64 ? am_launch<2>(am, agrid, smem, stream) :
+                     v_dim <= 128 ? am_launch<4>(am, agrid, smem, stream) : v_dim <= 256 ? am_launch<8>(am, agrid, smem, stream) :
+                     am_launch<16>(am, agrid, smem, stream);
+      if (rc != BN_OK) return rc;
+      if (part)
+        BN_LAUNCH((attention_merge_kernel<__nv_bfloat16>), dim3(n_tokens, n_heads), 128, 0, stream, (const float*)part, n_splits, n_heads, v_dim,
+                  (const __nv_bfloat16*)gate, gate_stride, (__nv_bfloat16*)out, out_stride, sink, out_wide, out_scale);
+      BN_CHECK_LAUNCH();
+      return BN_OK;
+    }
+  }
   // few tokens whose heads share rows: the heads of a key/value head four (or two) at a time, rows read once for them
   const int gq = n_heads / n_kv_heads;
   const int R = (gq % 4 == 0) ? 4 : ((gq % 2 == 0) ? 2 : 1);

@@ -698,3 +698,51 @@ def test_attention_prefill_tc_warps_apart_at_the_end(cuda_device, hd, precise):
         first = out if first is None else first
         assert torch.equal(out, first)
     ops.check_tc_status(torch.device("cuda:0"))
+
+
+@pytest.mark.parametrize("H,KV,hd,dv,n_keys,window,keep,max_keys,extra", [
+    (4, 4, 8, 8, [1, 2, 64], 0, 0, 0, ""),                    # a head of its own each; one piece; one key; whole turns
+    (6, 2, 40, 72, [65, 128, 129], 0, 0, 0, "gate"),          # three heads a group, inner size that ends within 32, tiles for some warps only
+    (16, 1, 128, 128, [700, 63, 1], 0, 0, 1000, "sink"),      # a full tile of heads, splits without keys
+    (34, 2, 64, 136, [300, 5, 64], 0, 0, 0, "rel"),           # 17 heads a group: two blocks
+    (8, 2, 128, 256, [900, 100, 90], 70, 6, 76, "rel gate"),  # a window behind kept first positions, split
+    (12, 1, 576, 512, [200, 64, 3], 0, 0, 300, "latent"),     # values inside wide key rows
+    (5, 1, 96, 48, [200, 64, 3], 0, 0, 0, "latent"),
+    (8, 4, 64, 96, [2100, 40, 1], 0, 0, 2100, "share"),       # two turns per split
+])
+@pytest.mark.parametrize("wide", [False, True])
+def test_attention_of_few_tokens_on_tensor_cores(cuda_device, H, KV, hd, dv, n_keys, window, keep, max_keys, extra, wide):
+    """bfloat16, one token per sequence, against the kernel for float32 on the same numbers: scores and weights are float32 in
+    both (the weights as three bfloat16 terms), so a float32 result differs by rounding only."""
+    g = torch.Generator(device="cuda").manual_seed(hd + dv)
+    share = 2 if extra == "share" else 1
+    pages = [(n + 63) // 64 for n in n_keys]
+    kc = torch.randn((sum(pages) + 1, KV, 64, hd), device="cuda", generator=g).bfloat16()
+    vc = None if extra == "latent" else torch.randn((sum(pages) + 1, KV // share, 64, dv), device="cuda", generator=g).bfloat16()
+    table, at = torch.zeros((3, max(pages)), dtype=torch.int32, device="cuda"), 1
+    for i, p in enumerate(pages):
+        table[i, :p] = torch.arange(at, at + p, device="cuda")
+        at += p
+        for c in (kc, vc):  # what lies behind a sequence's last position is never read
+            if c is not None:
+                c[table[i, p - 1].long(), :, (n_keys[i] - 1) % 64 + 1:] = float("nan")
+    q = torch.randn((3, H * hd + H + 8 - H % 8), device="cuda", generator=g).bfloat16() * 2
+    ints = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")
+    more = {}
+    if "gate" in extra:
+        more.update(gate_stride=q.shape[1])
+    if "rel" in extra:
+        more.update(rel=torch.randn((50, H), device="cuda", generator=g))
+    if "sink" in extra:
+        more.update(sink=torch.randn(H, device="cuda", generator=g))
+    if extra == "latent":
+        more.update(v_dim=dv)
+
+    def run(x, k, v, out):
+        gate = {"gate": x[:, H * hd:]} if "gate" in extra else {}
+        return ops.attention_general(x, x.shape[1], out, 3, H, KV, hd, hd ** -0.5, window, ints(range(3)), ints(n - 1 for n in n_keys), ints(range(3)),
+                                     table, k, v, keep_first=keep, v_share=share, max_keys=max_keys, out_scale=0.7, **gate, **more)
+    got = run(q, kc, vc, torch.full((3, H * dv), float("nan"), dtype=torch.float32 if wide else torch.bfloat16, device="cuda"))
+    ref = run(q.float().contiguous(), kc.float(), vc.float() if vc is not None else None, torch.empty((3, H * dv), device="cuda"))
+    # scores of up to about 2 hd^(1/2) sums of hd products, their exponentials and the weighted sums: some 2^-18 of values up to 5
+    assert bool(((got.float() - ref).abs() <= 5 * 2.0 ** -18 + (0 if wide else 2.0 ** -8) * ref.abs()).all())
