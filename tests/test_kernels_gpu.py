@@ -276,6 +276,32 @@ def test_sample_topp_follows_the_reference_nucleus(cuda_device, V, topp, temp):
         assert differ <= 2
 
 
+@pytest.mark.parametrize("candidates", [1, 2, 1025, 16383, 16384, 16385])
+@pytest.mark.parametrize("levels", [0, 40])
+def test_sample_topp_lists_of_candidates(cuda_device, candidates, levels):
+    """Around the number of candidates that the kernel keeps in shared memory (16384), with distinct logits and with ties (``levels``
+    different ones), a vocabulary of more than one window, rows that are not 16-byte aligned, against sums in 64 bits: the token drawn
+    is the first in falling order, lower ids first, whose running sum exceeds the draw."""
+    V, rows = 140001, 4
+    g = torch.Generator().manual_seed(candidates + levels)
+    logits = torch.full((rows, V), -60.0)
+    for r in range(rows):
+        x = torch.rand(candidates, generator=g) * 1.5
+        logits[r, torch.randperm(V, generator=g)[:candidates]] = torch.round(x * levels) / levels if levels else x
+    seeds = [3, 14, 159, 2653]
+    state = torch.tensor(seeds, dtype=torch.int64, device=cuda_device)
+    got = ops.sample_topp(logits.to(cuda_device), 0.9, 0.95, state).cpu().tolist()
+    for r in range(rows):
+        p = torch.softmax(logits[r].double() / np.float32(0.9).item(), 0)
+        order = torch.argsort(-p, stable=True)
+        cum = torch.cumsum(p[order], 0)
+        cut = int((cum > np.float32(0.95).item()).nonzero()[0])
+        draw = float(plain_llama.Xorshift64Star(seeds[r]).next_float()) * cum[cut].item()
+        at = (order == got[r]).nonzero().item()
+        # float32 probabilities: each within 2^-21 of its own size (quotient, exponential, sum, division), sums of them too
+        assert at <= cut + 1 and cum[at] >= draw - 1e-6 and (cum[at - 1] if at else 0.0) <= draw + 1e-6
+
+
 def test_repeat_penalty(cuda_device):
     logits = torch.tensor([[1.0, -2.0, 3.0, 4.0, -5.0], [1.0, 1.0, 1.0, 1.0, 1.0]], device=cuda_device)
     recent = torch.tensor([[2, 4, 2, 9, 0], [1, 1, 1, 1, 1]], dtype=torch.int32, device=cuda_device)
