@@ -84,6 +84,15 @@ def test_linear_skinny(cuda_device, dtype, M, N, K):
     assert (y.double() - ref).abs().max().item() < 1e-4 * max(1.0, K / 256)
 
 
+def test_a_slot_of_every_state_is_zeroed(cuda_device):
+    """One launch for tensors of any size and type, rows of whole 16-byte pieces or not; other slots keep what they hold."""
+    states = [torch.full((3,) + shape, 7.0, dtype=t, device=cuda_device) for shape, t in
+              (((5,), torch.bfloat16), ((3, 4, 8), torch.float32), ((1,), torch.float32), ((4099,), torch.bfloat16), ((300, 256), torch.float32))]
+    ops.zero_slot(ops.slot_rows(states), 1)
+    for s in states:
+        assert (s[1] == 0).all() and (s[0] == 7).all() and (s[2] == 7).all()
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 3, 8), (2, 37, 2048), (3, 5, 2056), (4, 4099, 4096), (5, 1203, 136), (8, 9473, 2176),
                                    (9, 2371, 4104), (16, 33, 14336)])
 def test_linear_stream_float32(cuda_device, M, N, K):

@@ -206,6 +206,29 @@ def test_norms_over_whole_projections_the_blend_and_the_cache_in_one_launch(cuda
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("tokens,H,G,d,dv", [(2, 4, 2, 16, 24), (256, 9, 1, 512, 8), (257, 9, 3, 512, 40)])
+def test_norms_in_whole_pieces_are_those_number_by_number(cuda_device, dtype, tokens, H, G, d, dv):
+    """Rows whose slices lie at 16-byte boundaries, a block per slice or one for all three, slices longer than a thread keeps:
+    the same numbers as rows that lie elsewhere."""
+    from bitnet_c_b200.csrc import ops
+    g = torch.Generator(device="cuda").manual_seed(tokens + d)
+    t = DT[dtype]
+    nq, nk, nv = H * d, G * d, G * dv
+    x = torch.randn((tokens, nq + nk + nv), device="cuda", generator=g).to(t) * 3
+    wq, wk = (1 + 0.3 * torch.randn(n, device="cuda", generator=g).to(t) for n in (nq, nk))
+    other = torch.randn((tokens, nv), device="cuda", generator=g).to(t)
+    got = []
+    for pad in (0, 1):
+        rows = torch.cat([x, torch.zeros((tokens, pad), dtype=t, device="cuda")], dim=1).contiguous()
+        kc, vc = (torch.full((-(-tokens // 64), G, 64, n), 9.0, dtype=t, device="cuda") for n in (d, dv))
+        ops.slice_norm_append(rows, nq, wq, nq, wk, nq + nk, G, d, dv, 1e-5, v_other=other, blend=0.25, tok_seq=ints([0] * tokens),
+                              tok_pos=ints(range(tokens)), slots=ints([0]), page_table=ints(range(-(-tokens // 64)))[None].contiguous(), k_cache=kc, v_cache=vc)
+        got.append((rows[:, : nq + nk + nv].float(), kc.float(), vc.float()))
+    for a, b in zip(*got):  # the sums of squares differ in their order
+        assert bool(((a - b).abs() <= (1e-5 if dtype == "float32" else 2.0 ** -7) * b.abs() + 1e-6).all())
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_the_clamped_unit_and_the_routers_softmax_scores(cuda_device, dtype):
     from bitnet_c_b200.csrc import ops
     rng = np.random.default_rng(8)
@@ -253,6 +276,11 @@ def test_the_sum_of_the_deltas_and_the_next_blocks_two_norms_in_one_pass(cuda_de
         assert (h2 is None) == (not second)
         if second:
             assert np.abs(h2.float().cpu().numpy() - pm.rms_norm(want, w2, 1e-5)).max() < tol * 4
+
+
+@pytest.mark.parametrize("width", [4100, 8192])
+def test_the_sum_of_the_deltas_and_two_norms_of_long_rows(cuda_device, width):
+    test_the_sum_of_the_deltas_and_the_next_blocks_two_norms_in_one_pass(cuda_device, "bfloat16", width)
 
 
 # ---- whole models ------------------------------------------------------------------------------------

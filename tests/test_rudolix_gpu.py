@@ -81,6 +81,17 @@ def test_streams_are_updated_read_and_normed_in_one_pass(cuda_device, streams, w
         assert np.abs(h.cpu().numpy() - pr.layer_norm(xs[0] + y, w, b, eps)).max() < 3e-4
 
 
+@pytest.mark.parametrize("streams,width", [(1, 2056), (2, 4104), (16, 2056)])
+def test_streams_of_long_rows(cuda_device, streams, width):
+    """Rows long enough for a cluster of blocks where there are few of them."""
+    test_streams_are_updated_read_and_normed_in_one_pass(cuda_device, streams, width)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_the_input_convolution_of_long_rows(cuda_device, dtype):
+    test_the_input_convolution_however_the_tokens_are_cut(cuda_device, 4, dtype, 2056)
+
+
 @pytest.mark.parametrize("taps", [1, 2, 3, 4, 9, 16])
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width", [50, 64, 1024])
