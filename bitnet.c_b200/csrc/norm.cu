@@ -300,9 +300,7 @@ extern "C" int bn_residual_add(float* x, const void* a, int a_dtype, const void*
 
 // x += a (+ b) as above, then the norms that read the stream next, in the same pass: out1 = x * rsqrt(mean(x^2) + eps) * w1
 // and, if w2 is given, out2 = the same rows times w2 (two norms of one stream share their statistics).  One block
-// per row; float32 sums and statistics; out1 / out2 in the compute type.  VEC: rows of whole 16-byte pieces at aligned addresses are
-// read and written four numbers at a time, a row's loads together (number by number took 10 us for 8 rows of 4,096).
-template <bool VEC>
+// per row; float32 sums and statistics; out1 / out2 in the compute type.
 __global__ void residual_add_norms_kernel(float* __restrict__ x, const void* __restrict__ a, int a_dtype, const void* __restrict__ b,
                                           int b_dtype, const void* __restrict__ w1, const void* __restrict__ w2, int w_dtype,
                                           float eps, void* __restrict__ out1, void* __restrict__ out2, int out_dtype, int width) {
@@ -313,36 +311,6 @@ __global__ void residual_add_norms_kernel(float* __restrict__ x, const void* __r
   const size_t row = blockIdx.x;
   float* xr = x + row * width;
   float ss = 0.f;
-  if (VEC) {
-    const int n4 = width >> 2;
-    const size_t r4 = row * n4;
-    float4* x4 = reinterpret_cast<float4*>(xr);
-    float4* v4 = reinterpret_cast<float4*>(v);
-    for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-      float4 t = x4[i], d = load4_as_f32(a, a_dtype, (r4 + i) * 4);
-      if (b) {
-        const float4 e = load4_as_f32(b, b_dtype, (r4 + i) * 4);
-        d.x += e.x; d.y += e.y; d.z += e.z; d.w += e.w;
-      }
-      t.x += d.x; t.y += d.y; t.z += d.z; t.w += d.w;
-      x4[i] = t;
-      v4[i] = t;
-      ss += t.x * t.x + t.y * t.y + t.z * t.z + t.w * t.w;
-    }
-    ss = block_sum(ss, scratch);
-    const float scale = 1.0f / sqrtf(ss / (float)width + eps);
-    for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-      float4 t = v4[i];
-      t.x *= scale; t.y *= scale; t.z *= scale; t.w *= scale;
-      const float4 g = load4_as_f32(w1, w_dtype, (size_t)i * 4);
-      store4_from_f32(out1, out_dtype, (r4 + i) * 4, make_float4(t.x * g.x, t.y * g.y, t.z * g.z, t.w * g.w));
-      if (w2) {
-        const float4 g2 = load4_as_f32(w2, w_dtype, (size_t)i * 4);
-        store4_from_f32(out2, out_dtype, (r4 + i) * 4, make_float4(t.x * g2.x, t.y * g2.y, t.z * g2.z, t.w * g2.w));
-      }
-    }
-    return;
-  }
   for (int i = threadIdx.x; i < width; i += blockDim.x) {
     float d = load_as_f32(a, a_dtype, row * width + i);
     if (b) d += load_as_f32(b, b_dtype, row * width + i);  // the sublayers' sum first, then onto the stream
@@ -367,18 +335,17 @@ extern "C" int bn_residual_add_norms(float* x, const void* a, int a_dtype, const
   if (width <= 0 || !(eps > 0.f) || !x || !a || !w1 || !out1 || (w2 && !out2)) return BN_ERR_BAD_ARG;
   size_t smem = ((size_t)width + 32) * sizeof(float);
   if (smem > 200 * 1024) return BN_ERR_BAD_ARG;
-  const bool vec = width % 4 == 0 && (((uintptr_t)x | (uintptr_t)a | (uintptr_t)b | (uintptr_t)w1 | (uintptr_t)w2 | (uintptr_t)out1 | (uintptr_t)out2) & 15) == 0;
-  auto kernel = vec ? residual_add_norms_kernel<true> : residual_add_norms_kernel<false>;
   if (smem > 48 * 1024) {
-    static size_t granted[2] = {0, 0};
-    if (smem > granted[vec]) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static size_t granted = 0;
+    if (smem > granted) {
+      cudaError_t e = cudaFuncSetAttribute(residual_add_norms_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
-      granted[vec] = smem;
+      granted = smem;
     }
   }
-  int threads = width >= 4096 && vec && n_rows <= 256 ? 1024 : (width >= 2048 ? 512 : (width >= 512 ? 256 : 128));
-  BN_LAUNCH(kernel, n_rows, threads, smem, stream, x, a, a_dtype, b, b_dtype, w1, w2, w_dtype, eps, out1, out2, out_dtype, width);
+  int threads = width >= 2048 ? 512 : (width >= 512 ? 256 : 128);
+  BN_LAUNCH(residual_add_norms_kernel, n_rows, threads, smem, stream, x, a, a_dtype, b, b_dtype, w1, w2, w_dtype, eps, out1, out2,
+            out_dtype, width);
   BN_CHECK_LAUNCH();
   return BN_OK;
 }

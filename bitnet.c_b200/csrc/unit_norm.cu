@@ -71,71 +71,15 @@ extern "C" int bn_unit_norm_append(void* x, int dtype, int n_tokens, int row_str
   return BN_OK;
 }
 
-// One slice of a token's row, normed in place (no gain: left as it is), every piece of V numbers handed on as it is stored.  A thread
-// keeps its first KEEP pieces in registers between the sum and the norm.
-template <typename T, int V>
-struct alignas(V * sizeof(T)) SlicePiece {
-  T v[V];
-};
-template <typename T, int V>
-__device__ __forceinline__ SlicePiece<T, V> load_piece(const T* p) {
-  SlicePiece<T, V> r;
-  if (V * sizeof(T) == 16) *reinterpret_cast<uint4*>(r.v) = *reinterpret_cast<const uint4*>(p);
-  else r.v[0] = *p;
-  return r;
-}
-template <typename T, int V>
-__device__ __forceinline__ void store_piece(T* p, const SlicePiece<T, V>& r) {
-  if (V * sizeof(T) == 16) *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(r.v);
-  else *p = r.v[0];
-}
-template <typename T, int V, class F>
-__device__ __forceinline__ void slice_norm_part(T* __restrict__ p, int n, const void* __restrict__ w, int w_dtype, float eps, float* scratch, F place) {
-  constexpr int KEEP = V > 1 ? 2 : 8;
-  SlicePiece<T, V> kept[KEEP];
-  float s = 0.f;
-  auto add = [&](const SlicePiece<T, V>& r) {
-#pragma unroll
-    for (int e = 0; e < V; ++e) s = fmaf(to_f32<T>(r.v[e]), to_f32<T>(r.v[e]), s);
-  };
-#pragma unroll
-  for (int k = 0; k < KEEP; ++k) {
-    const int i = ((int)threadIdx.x + k * UN_THREADS) * V;
-    if (i < n) kept[k] = load_piece<T, V>(p + i);
-  }
-#pragma unroll
-  for (int k = 0; k < KEEP; ++k)
-    if (((int)threadIdx.x + k * UN_THREADS) * V < n) add(kept[k]);
-  for (int i = ((int)threadIdx.x + KEEP * UN_THREADS) * V; i < n; i += UN_THREADS * V) add(load_piece<T, V>(p + i));
-  s = block_sum(s, scratch);
-  const float scale = n > 0 && w ? 1.0f / sqrtf(s / (float)n + eps) : 1.0f;
-  auto finish = [&](int i, SlicePiece<T, V> r) {
-    if (w) {
-#pragma unroll
-      for (int e = 0; e < V; ++e) r.v[e] = from_f32<T>(to_f32<T>(r.v[e]) * scale * load_as_f32(w, w_dtype, i + e));
-      store_piece<T, V>(p + i, r);
-    }
-    place(i, r);
-  };
-#pragma unroll
-  for (int k = 0; k < KEEP; ++k) {
-    const int i = ((int)threadIdx.x + k * UN_THREADS) * V;
-    if (i < n) finish(i, kept[k]);
-  }
-  for (int i = ((int)threadIdx.x + KEEP * UN_THREADS) * V; i < n; i += UN_THREADS * V) finish(i, load_piece<T, V>(p + i));
-}
-
 // RMS norms over whole slices of a row (all query heads of a token at once, and all key heads), each with a
 // gain; values optionally blended with another tensor's rows; keys and values written into the paged cache.
 //
 //   q <- q / sqrt(mean(q^2) + eps) * wq   over q_len numbers at q_off;   k likewise over k_len at k_off
 //   v <- (1 - blend) v + blend v_other    when v_other is given (row t of v_other lies at v_other + t * other_stride)
 //
-// Statistics and the blend are float32; what the cache gets is what the row then holds.
-// Without a cache only the row is rewritten.  Bound by latency with few tokens, by the rows' bytes with many.  A block each for a token's
-// queries, keys and values where there are few, rows read once in 16-byte pieces (4,096 + 2 x 1,024 bfloat16, before, with one block
-// and number by number, and now: 8 tokens 17 / 3.6 us, 2,400 tokens 51 / 36 us).
-template <typename T, int V>  // V numbers at a time: 16 bytes where slices, heads and addresses allow it
+// One block per token.  Statistics and the blend are float32; what the cache gets is what the row then holds.
+// Without a cache only the row is rewritten.
+template <typename T>
 __global__ void slice_norm_append_kernel(T* __restrict__ x, int row_stride, int q_off, int q_len, const void* __restrict__ wq,
                                          int k_off, int k_len, const void* __restrict__ wk, int w_dtype, float eps, int v_off,
                                          const T* __restrict__ v_other, int other_stride, float blend, int n_kv_heads,
@@ -147,33 +91,43 @@ __global__ void slice_norm_append_kernel(T* __restrict__ x, int row_stride, int 
   __shared__ float scratch[32];
   const int t = blockIdx.x;
   T* row = x + (size_t)t * row_stride;
+  float sq = 0.f, sk = 0.f;
+  for (int i = threadIdx.x; i < q_len; i += blockDim.x) {
+    float a = to_f32<T>(row[q_off + i]);
+    sq += a * a;
+  }
+  for (int i = threadIdx.x; i < k_len; i += blockDim.x) {
+    float a = to_f32<T>(row[k_off + i]);
+    sk += a * a;
+  }
+  sq = block_sum(sq, scratch);
+  sk = block_sum(sk, scratch);
   const int pos = k_cache ? tok_pos[t] : 0;
   const int* pt = k_cache ? page_table + (size_t)slots[tok_seq[t]] * pt_stride : nullptr;
-  for (int part = blockIdx.y; part < 3; part += gridDim.y) {
-    if (part == 0) {
-      slice_norm_part<T, V>(row + q_off, q_len, wq, w_dtype, eps, scratch, [](int, const SlicePiece<T, V>&) {});
-    } else if (part == 1) {
-      slice_norm_part<T, V>(row + k_off, k_len, wk, w_dtype, eps, scratch, [&](int i, const SlicePiece<T, V>& y) {
-        if (!k_cache) return;
-        const int kvh = i / head_dim, d = i - kvh * head_dim;
-        store_piece<T, V>(k_cache + cache_row_offset(pt, pos, n_kv_heads, kvh, head_dim) + d, y);
-      });
-    } else {
-      for (int i = threadIdx.x * V; i < n_kv_heads * v_dim; i += blockDim.x * V) {
-        SlicePiece<T, V> y = load_piece<T, V>(row + v_off + i);
-        if (v_other) {
-          const SlicePiece<T, V> o = load_piece<T, V>(v_other + (size_t)t * other_stride + i);
-#pragma unroll
-          for (int e = 0; e < V; ++e) y.v[e] = from_f32<T>((1.0f - blend) * to_f32<T>(y.v[e]) + blend * to_f32<T>(o.v[e]));
-          store_piece<T, V>(row + v_off + i, y);
-        }
-        if (v_cache) {
-          const int kvh = i / v_dim, d = i - kvh * v_dim;
-          store_piece<T, V>(v_cache + cache_row_offset(pt, pos, n_kv_heads, kvh, v_dim) + d, y);
-        }
-      }
+  if (q_len > 0) {
+    const float scale = 1.0f / sqrtf(sq / (float)q_len + eps);
+    for (int i = threadIdx.x; i < q_len; i += blockDim.x)
+      row[q_off + i] = from_f32<T>(to_f32<T>(row[q_off + i]) * scale * load_as_f32(wq, w_dtype, i));
+  }
+  const float kscale = k_len > 0 && wk ? 1.0f / sqrtf(sk / (float)k_len + eps) : 1.0f;
+  for (int i = threadIdx.x; i < k_len; i += blockDim.x) {
+    T y = wk ? from_f32<T>(to_f32<T>(row[k_off + i]) * kscale * load_as_f32(wk, w_dtype, i)) : row[k_off + i];
+    row[k_off + i] = y;
+    if (k_cache) {
+      const int kvh = i / head_dim, d = i - kvh * head_dim;
+      k_cache[cache_row_offset(pt, pos, n_kv_heads, kvh, head_dim) + d] = y;
     }
-    __syncthreads();  // (one block for all three: slices that overlap are taken in turn)
+  }
+  for (int i = threadIdx.x; i < n_kv_heads * v_dim; i += blockDim.x) {
+    T y = row[v_off + i];
+    if (v_other) {
+      y = from_f32<T>((1.0f - blend) * to_f32<T>(y) + blend * to_f32<T>(v_other[(size_t)t * other_stride + i]));
+      row[v_off + i] = y;
+    }
+    if (v_cache) {
+      const int kvh = i / v_dim, d = i - kvh * v_dim;
+      v_cache[cache_row_offset(pt, pos, n_kv_heads, kvh, v_dim) + d] = y;
+    }
   }
 }
 
@@ -187,27 +141,16 @@ extern "C" int bn_slice_norm_append(void* x, int dtype, int n_tokens, int row_st
       !(eps > 0.f) || (k_cache && (!v_cache || !tok_seq || !tok_pos || !slots || !page_table)) ||
       (w_dtype != BN_F32 && w_dtype != BN_BF16))
     return BN_ERR_BAD_ARG;
-  const int v_len = n_kv_heads * v_dim;
-  auto apart = [](int a, int n, int b, int m) { return a + n <= b || b + m <= a; };
-  // with many tokens one block for all three keeps as much under way; slices that overlap are taken in turn
-  const int parts = n_tokens <= 256 && apart(q_off, q_len, k_off, k_len) && apart(q_off, q_len, v_off, v_len) && apart(k_off, k_len, v_off, v_len) ? 3 : 1;
-  const int piece = dtype == BN_F32 ? 4 : 8;
-  const bool vec = ((row_stride | q_off | q_len | k_off | v_off | head_dim | v_dim | (v_other ? other_stride : 0)) % piece) == 0 &&
-                   (((uintptr_t)x | (uintptr_t)v_other | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0;
-#define UN_SLICE(TT, V)                                                                                                        \
-  BN_LAUNCH((slice_norm_append_kernel<TT, V>), dim3(n_tokens, parts), UN_THREADS, 0, stream, (TT*)x, row_stride, q_off, q_len, wq, \
-            k_off, k_len, wk, w_dtype, eps, v_off, (const TT*)v_other, other_stride, blend, n_kv_heads, head_dim, v_dim, tok_seq, \
-            tok_pos, slots, page_table, pt_stride, (TT*)k_cache, (TT*)v_cache)
-  if (dtype == BN_F32) {
-    if (vec) UN_SLICE(float, 4);
-    else UN_SLICE(float, 1);
-  } else if (dtype == BN_BF16) {
-    if (vec) UN_SLICE(__nv_bfloat16, 8);
-    else UN_SLICE(__nv_bfloat16, 1);
-  } else {
+  if (dtype == BN_F32)
+    BN_LAUNCH(slice_norm_append_kernel<float>, n_tokens, UN_THREADS, 0, stream, (float*)x, row_stride, q_off, q_len, wq, k_off, k_len,
+              wk, w_dtype, eps, v_off, (const float*)v_other, other_stride, blend, n_kv_heads, head_dim, v_dim, tok_seq, tok_pos,
+              slots, page_table, pt_stride, (float*)k_cache, (float*)v_cache);
+  else if (dtype == BN_BF16)
+    BN_LAUNCH(slice_norm_append_kernel<__nv_bfloat16>, n_tokens, UN_THREADS, 0, stream, (__nv_bfloat16*)x, row_stride, q_off, q_len,
+              wq, k_off, k_len, wk, w_dtype, eps, v_off, (const __nv_bfloat16*)v_other, other_stride, blend, n_kv_heads, head_dim,
+              v_dim, tok_seq, tok_pos, slots, page_table, pt_stride, (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache);
+  else
     return BN_ERR_BAD_ARG;
-  }
-#undef UN_SLICE
   BN_CHECK_LAUNCH();
   return BN_OK;
 }
