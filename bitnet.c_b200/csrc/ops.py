@@ -2162,8 +2162,9 @@ def moe_few_fits(width: int, top: int, ff: int) -> bool:
 
 def moe_experts_few(h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w_gate_up: torch.Tensor,
                     w_down: torch.Tensor, limit: float, slope: float, scale_input: bool,
-                    add: Optional[torch.Tensor] = None, act: int = -1, add_scale: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """The chosen experts of every token (in bfloat16 each expert is read once for all tokens that chose it; else, and where rows
+                    add: Optional[torch.Tensor] = None, act: int = -1, add_scale: Optional[torch.Tensor] = None,
+                    read_once: bool = True) -> torch.Tensor:
+    """The chosen experts of every token (with ``read_once``, in bfloat16, each expert is read once for all tokens that chose it; else, and where rows
     are not whole 16-byte pieces, once per (token, expert)): float32 ``[T, width]``, the sum over
     a token's experts plus ``add``.  The weight multiplies the expert's input (``scale_input``) or its output.
     ``act`` < 0: the clamped unit with ``limit`` and ``slope``; ACT_SILU / ACT_GELU_TANH: act(gate) * up; ACT_RELU2: no gate,
@@ -2194,7 +2195,7 @@ def moe_experts_few(h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w
     y = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
     out = torch.empty((T, width), dtype=torch.float32, device=h.device)
     per_call = min(MOE_FEW_TOKENS, MOE_FEW_ITEMS // top)
-    if (h.dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and E <= 1024 and per_call > 0
+    if (read_once and h.dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and E <= 1024 and per_call > 0
             and (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0):
         for t0 in range(0, T, per_call):
             _moe_few_tokens(h, ids, weights, w_gate_up, w_down, limit, slope, scale_input, add, act, add_scale, y, out, t0,

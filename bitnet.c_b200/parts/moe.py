@@ -26,7 +26,7 @@ class Moe(FeedForward):
     the input itself; ``activation`` "relu2": down(max(up x, 0)^2), no gate; ``shared_gate``: the shared expert's output times the
     logistic function of one number per token, a row of the router's product.
 
-    Few rows (a decode step): two kernels stream the chosen experts, in bfloat16 once for all the tokens that chose them, from
+    Few rows (a decode step): two kernels stream the chosen experts (``read_once``: in bfloat16 once for all the tokens that chose them) from
     device memory alone.  Many rows: the (token, expert) items are sorted by expert, and in bfloat16 all experts run as one
     grouped product each way, which reads the experts' row counts on the device.  Otherwise (float32, odd sizes) every
     expert's rows go through the ordinary products; the host then needs the counts, one copy per call."""
@@ -148,7 +148,7 @@ class Moe(FeedForward):
             ctx.tap("moe_ids", lambda: ids.float())
         if self.few_fits and (ctx.decode or T * s.top <= self.FEW_ITEMS):
             return ops.moe_experts_few(h, ids, weights, self.w_gate_up, self.w_down, s.expert_limit, s.slope,
-                                       s.weight_on_input, add=shared, act=self.act, add_scale=shared_scale)
+                                       s.weight_on_input, add=shared, act=self.act, add_scale=shared_scale, read_once=s.read_once)
         rest = dict(add_scale=shared_scale, h=h if s.identity else None)
         if self.USE_GROUPED and h.dtype == torch.bfloat16 and ops.grouped_fits(self.w_gate_up) and ops.grouped_fits(self.w_down):
             x_sorted, place, offsets = ops.moe_sort(h, ids, weights, None, s.weight_on_input, n_experts=s.n_experts)
