@@ -352,6 +352,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
       if (tile * PT_KEYS + PT_KEYS - 1 > seq_last) {
         // the page holds rows behind the sequence's last position: their weights are zero, but zero
         // times anything must be zero, so clear those value rows (warp w takes every fourth row)
+        // once their copy has landed: the scores only say that the keys have, and a copy that comes later would bring the rows
+        // back (the stage is not refilled before these warps have signalled, so its phase stands)
+        if (!pt_wait(v_full0 + 8 * (j % VS), (unsigned)(j / VS) & 1u, failed, a.status)) { ok = false; break; }
         unsigned char* sv = v_smem + (j % VS) * V_BYTES;
         const int first = max(0, seq_last + 1 - tile * PT_KEYS);
         for (int e = (warp - 2) * 32 + lane; e < (PT_KEYS - first) * (VD / 8); e += 128) {

@@ -735,6 +735,37 @@ def test_attention_prefill_tc_warps_apart_at_the_end(cuda_device, hd, precise):
     ops.check_tc_status(torch.device("cuda:0"))
 
 
+@pytest.mark.parametrize("hd,vd", [(64, 64), (128, 128), (192, 128)])
+def test_attention_prefill_tc_rows_behind_the_last_position(cuda_device, hd, vd):
+    """What a page holds behind a sequence's last position does not matter, not-a-number neither: with keys and values of another
+    memory for every sequence, as many as keep the copies under way, the results are those of pages that hold zeros there, bit by
+    bit.  (The rows were cleared without a look at whether their copy had landed.)"""
+    H, n_seqs = 16, 96
+    g = torch.Generator(device="cuda").manual_seed(hd + vd)
+    lens = [1 + (i * 29) % 330 for i in range(n_seqs)]
+    n, pages = sum(lens), [(m + 63) // 64 for m in lens]
+    q = torch.randn((n, H * hd), device="cuda", generator=g).bfloat16()
+    kc, vc = (torch.randn((sum(pages), H, 64, d), device="cuda", generator=g).bfloat16() for d in (hd, vd))
+    ints = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")
+    table, at = torch.zeros((n_seqs, max(pages)), dtype=torch.int32, device="cuda"), 0
+    behind = torch.zeros((sum(pages), 1, 64, 1), dtype=torch.bool, device="cuda")
+    for i, p in enumerate(pages):
+        table[i, :p] = torch.arange(at, at + p, device="cuda")
+        at += p
+        behind[at - 1, 0, (lens[i] - 1) % 64 + 1:] = True
+    tiles = [(i, r) for i, c in enumerate(lens) for r in range(0, c, 128)]
+    rest = (ints(i for i, _ in tiles), ints(r for _, r in tiles), ints(np.concatenate([[0], np.cumsum(lens)])), ints([0] * n_seqs),
+            ints(range(n_seqs)), table)
+    outs = []
+    for fill in (0.0, float("nan")):
+        k, v = kc.masked_fill(behind, fill), vc.masked_fill(behind, fill)
+        for _ in range(10):
+            outs.append(torch.empty((n, H * vd), dtype=torch.bfloat16, device="cuda"))
+            ops.attention_prefill_tc(q, q.shape[1], outs[-1], H, H, hd, hd ** -0.5, 0, *rest, k, v, precise=True)
+    ops.check_tc_status(torch.device("cuda:0"))
+    assert bool(outs[0].isfinite().all()) and all(torch.equal(o, outs[0]) for o in outs)
+
+
 @pytest.mark.parametrize("H,KV,hd,dv,n_keys,window,keep,max_keys,extra", [
     (4, 4, 8, 8, [1, 2, 64], 0, 0, 0, ""),                    # a head of its own each; one piece; one key; whole turns
     (6, 2, 40, 72, [65, 128, 129], 0, 0, 0, "gate"),          # three heads a group, inner size that ends within 32, tiles for some warps only
