@@ -535,14 +535,16 @@ __global__ void __launch_bounds__(AM_THREADS) attention_few_mma_kernel(AmArgs a)
       }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int i = tid; i < 16 * q_pieces; i += AM_THREADS) {
-    const int r = i / q_pieces, c = i - r * q_pieces;
-    const bool live = r < rows && c < pieces;
-    am_copy(qs + r * a.q_pitch + c * 16, live ? a.q + (size_t)t * a.q_stride + (size_t)(h0 + r) * a.head_dim + c * 8 : a.q, live);
-  }
   const int span = a.n_splits * AM_KEYS;
   const int turns = n_keys > z * AM_KEYS ? (n_keys - z * AM_KEYS + span - 1) / span : 0;
-  if (turns > 0) fill(0);
+  if (turns > 0) {  // a part without keys copies nothing: what it leaves does not depend on q, and nothing would wait for the copy
+    for (int i = tid; i < 16 * q_pieces; i += AM_THREADS) {
+      const int r = i / q_pieces, c = i - r * q_pieces;
+      const bool live = r < rows && c < pieces;
+      am_copy(qs + r * a.q_pitch + c * 16, live ? a.q + (size_t)t * a.q_stride + (size_t)(h0 + r) * a.head_dim + c * 8 : a.q, live);
+    }
+    fill(0);  // (q's copy is in the first stage's group)
+  }
 
   float o[NT][4];
 #pragma unroll
@@ -657,8 +659,7 @@ __global__ void __launch_bounds__(AM_THREADS) attention_few_mma_kernel(AmArgs a)
     l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
     if (quad == 0) s_l[warp][g + 8 * i] = l_run[i];
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");  // (q's copy, where there was no key)
-  __syncthreads();
+  __syncthreads();  // (the last turn has waited for every copy)
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int head = g + 8 * i;

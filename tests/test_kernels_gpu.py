@@ -812,3 +812,29 @@ def test_attention_of_few_tokens_on_tensor_cores(cuda_device, H, KV, hd, dv, n_k
     ref = run(q.float().contiguous(), kc.float(), vc.float() if vc is not None else None, torch.empty((3, H * dv), device="cuda"))
     # scores of up to about 2 hd^(1/2) sums of hd products, their exponentials and the weighted sums: some 2^-18 of values up to 5
     assert bool(((got.float() - ref).abs() <= 5 * 2.0 ** -18 + (0 if wide else 2.0 ** -8) * ref.abs()).all())
+
+
+@pytest.mark.parametrize("hd,latent", [(64, 0), (128, 0), (576, 512)])
+def test_attention_of_few_tokens_with_parts_without_keys(cuda_device, hd, latent):
+    """One long sequence among short ones: most blocks of the short ones have no key.  They leave nothing in flight when they end
+    (their copy of q once was: nothing waited for it), so launches right behind one another give the same bits and the results are
+    those of the float32 kernel."""
+    H, n_seqs, n_keys = 16, 24, [2000] + [1 + (i * 11) % 64 for i in range(1, 24)]
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    pages = [(n + 63) // 64 for n in n_keys]
+    kc = torch.randn((sum(pages), 1, 64, hd), device="cuda", generator=g).bfloat16()
+    vc = None if latent else torch.randn((sum(pages), 1, 64, hd), device="cuda", generator=g).bfloat16()
+    table, at = torch.zeros((n_seqs, max(pages)), dtype=torch.int32, device="cuda"), 0
+    for i, p in enumerate(pages):
+        table[i, :p] = torch.arange(at, at + p, device="cuda")
+        at += p
+    q = torch.randn((n_seqs, H * hd), device="cuda", generator=g).bfloat16()
+    ints = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")
+    rest = (ints(range(n_seqs)), ints(n - 1 for n in n_keys), ints(range(n_seqs)), table)
+    dv = latent or hd
+    run = lambda x, k, v, dtype: ops.attention_general(x, H * hd, torch.empty((n_seqs, H * dv), dtype=dtype, device="cuda"), n_seqs, H, 1, hd,
+                                                       hd ** -0.5, 0, *rest, k, v, max_keys=2000, v_dim=latent)
+    outs = [run(q, kc, vc, torch.float32) for _ in range(20)]
+    ref = run(q.float(), kc.float(), None if latent else vc.float(), torch.float32)
+    # scores, exponentials and weighted sums in float32: some 2^-18 of values up to 5, as above
+    assert bool(((outs[0] - ref).abs() <= 5 * 2.0 ** -18).all()) and all(torch.equal(o, outs[0]) for o in outs)
