@@ -447,10 +447,13 @@ __global__ void attention_merge_kernel(const float* __restrict__ part, int n_spl
 // lie in a lane, the same for both operands) and a quarter of the value width each for the weighted sum.  The weights enter that
 // product as three bfloat16 terms, 24 bits of mantissa, so nothing is rounded that float32 would not round; values inside the key
 // rows are read from the same copy.
+// Scores are summed over 32 numbers of the inner dimension and weighted rows over 16 keys on the tensor cores, from zero each time; the
+// rest is float32 additions.  The tensor cores cut their sums off where an addition rounds: left in their accumulators, the results
+// were 1.2 (16 keys) to 18 times (4,000) as far from 64 bits as sums in float32, now 0.3 to 1.04 times, for 3 to 8 % of the time.
 // Bound by latency: a token's keys are few kilobytes per block.  The kernel above spends 4,300 instructions per warp on 128 keys
-// of 128 numbers, this one some 300.  Measured with the merge, us, before and after (tokens, heads, key/value heads, head size, visible keys):
-// 4, 16, 4, 128, 1024: 16.6 / 10.1;  2, 32, 8, 128, 4000: 35 / 25;  64, 32, 8, 128, 2000: 534 / 270;  key rows of 256 that hold values
-// of 192, 8, 16, 1, 1000: 33 / 13;  of 576 and 512, 2, 32, 1, 1024: 45 / 24.
+// of 128 numbers, this one some 300.  Measured with the merge, us, that kernel and this (tokens, heads, key/value heads, head size, visible keys):
+// 4, 16, 4, 128, 1024: 16.0 / 10.6;  1, 32, 8, 128, 4000: 25.6 / 16.6;  64, 32, 8, 128, 2000: 534 / 297;  key rows of 256 that hold values
+// of 192, 8, 16, 1, 1000: 31.9 / 13.4;  of 576 and 512, 2, 32, 1, 1024: 42.6 / 25.8.
 #define AM_THREADS 128
 #define AM_KEYS 64
 #define AM_P_PITCH 144  // bytes of 64 weights, padded: no bank conflicts between rows
@@ -573,8 +576,11 @@ __global__ void __launch_bounds__(AM_THREADS) attention_few_mma_kernel(AmArgs a)
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         const uint4 k = am_piece(ka + n * 8 * a.k_pitch + c * 16);
-        am_mma(s[n], x0.x, x1.x, x0.y, x1.y, k.x, k.y);
-        am_mma(s[n], x0.z, x1.z, x0.w, x1.w, k.z, k.w);
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        am_mma(d, x0.x, x1.x, x0.y, x1.y, k.x, k.y);
+        am_mma(d, x0.z, x1.z, x0.w, x1.w, k.z, k.w);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[n][e] += d[e];
       }
     }
     float mx[2] = {-INFINITY, -INFINITY};
@@ -646,8 +652,11 @@ __global__ void __launch_bounds__(AM_THREADS) attention_few_mma_kernel(AmArgs a)
         unsigned b0, b1;
         asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
                      : "=r"(b0), "=r"(b1) : "r"(vd + (kk * 16 + (lane & 15)) * v_pitch + tile * 16) : "memory");
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int term = 0; term < 3; ++term) am_mma(o[j], p[term][0], p[term][1], p[term][2], p[term][3], b0, b1);
+        for (int term = 2; term >= 0; --term) am_mma(d, p[term][0], p[term][1], p[term][2], p[term][3], b0, b1);  // the small ones first
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[j][e] += d[e];
       }
     }
     __syncthreads();  // keys, values and weights have been used

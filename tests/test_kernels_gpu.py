@@ -838,3 +838,27 @@ def test_attention_of_few_tokens_with_parts_without_keys(cuda_device, hd, latent
     ref = run(q.float(), kc.float(), None if latent else vc.float(), torch.float32)
     # scores, exponentials and weighted sums in float32: some 2^-18 of values up to 5, as above
     assert bool(((outs[0] - ref).abs() <= 5 * 2.0 ** -18).all()) and all(torch.equal(o, outs[0]) for o in outs)
+
+
+@pytest.mark.parametrize("H,KV,hd,dv,n", [(8, 8, 64, 64, 1000), (32, 8, 128, 128, 2000), (16, 1, 576, 512, 300)])
+def test_attention_of_few_tokens_is_as_exact_as_float32(cuda_device, H, KV, hd, dv, n):
+    """Products on the tensor cores, unrounded results: no further from 64 bits than the kernel that multiplies and adds in float32 (sums
+    that stay in the tensor cores' accumulators, which cut off instead of rounding, were 2 to 18 times as far)."""
+    S = 64
+    g = torch.Generator(device="cuda").manual_seed(n)
+    pages = (n + 63) // 64
+    kc = torch.randn((S * pages, KV, 64, hd), device="cuda", generator=g).bfloat16()
+    vc = torch.randn((S * pages, KV, 64, dv), device="cuda", generator=g).bfloat16() if dv == hd else None
+    q = torch.randn((S, H * hd), device="cuda", generator=g).bfloat16() * 2
+    ints = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")
+    rest = (ints(range(S)), ints([n - 1] * S), ints(range(S)), torch.arange(S * pages, device="cuda").int().view(S, pages).contiguous())
+
+    def run(x, k, v):
+        out = torch.empty((S, H * dv), dtype=torch.float32, device="cuda")
+        return ops.attention_general(x, H * hd, out, S, H, KV, hd, hd ** -0.5, 0, *rest, k, v, v_dim=0 if v is not None else dv, max_keys=n)
+    rows = lambda c, d: c.view(S, pages, KV, 64, -1).transpose(2, 3).reshape(S, pages * 64, KV, -1)[:, :n, :, :d].double()
+    k64, v64 = rows(kc, hd), rows(kc if vc is None else vc, dv)
+    p = torch.softmax(torch.einsum("skgd,snkd->skgn", q.view(S, KV, H // KV, hd).double(), k64) * hd ** -0.5, -1)
+    ref = torch.einsum("skgn,snkd->skgd", p, v64).reshape(S, -1)
+    err = [float((o.double() - ref).norm()) for o in (run(q, kc, vc), run(q.float(), kc.float(), vc.float() if vc is not None else None))]
+    assert err[0] <= 1.2 * err[1]  # (a fifth for chance: the orders of the sums differ)
