@@ -65,12 +65,29 @@ __device__ __forceinline__ uint4 mf_slot(unsigned addr) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
   return v;
 }
-// Both halves of a group of 32 of the inner dimension: tokens' pieces x0 (rows g), x1 (rows g + 8), weights' piece w.
+// The sums of a group of 32 of the inner dimension, added to c: tokens' pieces x0 (rows g), x1 (rows g + 8), weights' piece w.  Each
+// half is a product of its own from zero, and float32 additions do the rest: the tensor cores cut their sums off where an addition
+// rounds, which along an inner dimension of 7,168 made the error against 64 bits 7 times that of float32 sums.
 __device__ __forceinline__ void mf_mma(float* c, const uint4& x0, const uint4& x1, const uint4& w) {
+  float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(x0.x), "r"(x1.x), "r"(x0.y), "r"(x1.y), "r"(w.x), "r"(w.y));
+               : "+f"(d[0][0]), "+f"(d[0][1]), "+f"(d[0][2]), "+f"(d[0][3]) : "r"(x0.x), "r"(x1.x), "r"(x0.y), "r"(x1.y), "r"(w.x), "r"(w.y));
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(x0.z), "r"(x1.z), "r"(x0.w), "r"(x1.w), "r"(w.z), "r"(w.w));
+               : "+f"(d[1][0]), "+f"(d[1][1]), "+f"(d[1][2]), "+f"(d[1][3]) : "r"(x0.z), "r"(x1.z), "r"(x0.w), "r"(x1.w), "r"(w.z), "r"(w.w));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) c[i] += d[0][i] + d[1][i];
+}
+// part(0) + ... + part(MF_WARPS - 1), neighbours first
+template <class Part>
+__device__ __forceinline__ float mf_sum_of_warps(Part part) {
+  float v[MF_WARPS];
+#pragma unroll
+  for (int w = 0; w < MF_WARPS; ++w) v[w] = part(w);
+#pragma unroll
+  for (int n = MF_WARPS / 2; n > 0; n >>= 1)
+#pragma unroll
+    for (int w = 0; w < n; ++w) v[w] = v[2 * w] + v[2 * w + 1];
+  return v[0];
 }
 // Eight bfloat16 times a number, rounded to bfloat16 again (the expert's input as the path that sorts tokens stores it)
 __device__ __forceinline__ uint4 mf_scaled(uint4 v, float s) {
@@ -316,9 +333,7 @@ __global__ void __launch_bounds__(MF_THREADS, 2) moe_few_gate_up_kernel(MfArgs a
           float sum[G];
 #pragma unroll
           for (int m = 0; m < G; ++m) {
-            sum[m] = 0.f;
-#pragma unroll
-            for (int w = 0; w < MF_WARPS; ++w) sum[m] += part[((w * 8 * XR + r) * S + m * R) * 8 + j];
+            sum[m] = mf_sum_of_warps([&](int w) { return part[((w * 8 * XR + r) * S + m * R) * 8 + j]; });
           }
           // the products' results pass through bfloat16, as they do on the sorted path
           const float up = to_f32<__nv_bfloat16>(from_f32<__nv_bfloat16>(sum[G - 1]));
@@ -390,8 +405,7 @@ __global__ void __launch_bounds__(MF_THREADS, 2) moe_few_down_kernel(MfArgs a) {
       if (e >= a.n_real) {
         d = to_f32<__nv_bfloat16>(a.h[(size_t)t * a.rows + c0 + r]);
       } else if (e >= 0) {
-#pragma unroll
-        for (int q = 0; q < MF_WARPS; ++q) d += parts[((size_t)q * a.n_items + item) * 8 * R + r];
+        d = mf_sum_of_warps([&](int q) { return parts[((size_t)q * a.n_items + item) * 8 * R + r]; });
       }
       total += d * (a.scale_output ? a.weights[item] : 1.0f);
     }
