@@ -205,9 +205,9 @@ linear_stream_f32_kernel(const float* __restrict__ x, const float* __restrict__ 
                        : "=f"(v[c].x), "=f"(v[c].y), "=f"(v[c].z), "=f"(v[c].w) : "r"(ring + src * STAGE + c * SLOT) : "memory");
         src = src + 1 == D ? 0 : src + 1;
         const int k = p * 128 + lane * 4;
-        if (k < kn) {
+        auto add_rows = [&](auto rows) {
 #pragma unroll
-          for (int i = 0; i < MT; ++i) {
+          for (int i = 0; i < decltype(rows)::value; ++i) {
             const float4 u = *reinterpret_cast<const float4*>(xs + i * SF_KC + k);
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
@@ -216,6 +216,10 @@ linear_stream_f32_kernel(const float* __restrict__ x, const float* __restrict__ 
               acc[i * COLS + c] = FOURS ? acc[i * COLS + c] + t : t;
             }
           }
+        };
+        if (k < kn) {  // half of the rows where there are no more: the last ones of 9 to 12
+          if (MT == 8 && mt <= 4) add_rows(std::integral_constant<int, MT / 2>());
+          else add_rows(std::integral_constant<int, MT>());
         }
       }
       float v;
