@@ -411,7 +411,7 @@ __global__ void attention_merge_kernel(const float* __restrict__ part, int n_spl
     M = warp_max(M);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const float w = m[i] != -INFINITY ? expf(m[i] - M) : 0.f;  // (a part without keys holds nothing)
+      const float w = m[i] != -INFINITY ? expf(m[i] - M) : -1.f;  // (a part without keys holds nothing and is passed over)
       if (m[i] != -INFINITY) L += w * l[i];
       weight[threadIdx.x + 32 * i] = w;
     }
@@ -432,8 +432,8 @@ __global__ void attention_merge_kernel(const float* __restrict__ part, int n_spl
       for (int i = 0; i < 8; ++i) v[i] = z0 + i < n_splits ? p[(size_t)(z0 + i) * (v_dim + 2) + 2 + d] : 0.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float w = z0 + i < n_splits ? weight[z0 + i] : 0.f;
-        if (w != 0.f) a = fmaf(w, v[i], a);
+        const float w = z0 + i < n_splits ? weight[z0 + i] : -1.f;
+        if (!(w < 0.f)) a = fmaf(w, v[i], a);  // also with a weight of zero: times not a number it is none
       }
     }
     store_result<T>(out, out_wide, (size_t)t * out_stride + (size_t)h * v_dim + d, a * inv);

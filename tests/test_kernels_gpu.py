@@ -884,3 +884,30 @@ def test_linear_stream_float32_is_as_exact_as_shorter_parts(cuda_device, M, N, K
         short = short + lanes[:, :, part, 0]
     err = [float((o.double() - ref).norm()) for o in (ops.linear(x, w)[:, some], short)]
     assert err[0] <= 1.1 * err[1]
+
+
+def _few_tokens(n_keys, KV, hd, dv, seed):
+    """Caches and tables of sequences of n_keys keys with one new token each."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    pages = [(n + 63) // 64 for n in n_keys]
+    kc, vc = (torch.randn((sum(pages), KV, 64, d), device="cuda", generator=g).bfloat16() for d in (hd, dv))
+    table, at = torch.zeros((len(n_keys), max(pages)), dtype=torch.int32, device="cuda"), 0
+    for i, p in enumerate(pages):
+        table[i, :p] = torch.arange(at, at + p, device="cuda")
+        at += p
+    ints = lambda v: torch.tensor(list(v), dtype=torch.int32, device="cuda")
+    return g, kc, vc, (ints(range(len(n_keys))), ints(n - 1 for n in n_keys), ints(range(len(n_keys))), table)
+
+
+def test_attention_merge_keeps_what_is_not_a_number(cuda_device):
+    """A part whose weight has become zero beside the others still makes the result not a number if it is not one; a part without
+    keys does nothing."""
+    n_keys = [300, 20]
+    g, kc, vc, rest = _few_tokens(n_keys, 1, 64, 64, 5)
+    kc[rest[3][0, 0].long(), 0, :, 0] = -200.0  # the first 64 keys' scores: some 100 times what still leaves a weight
+    q = torch.randn((2, 16 * 64), device="cuda", generator=g).bfloat16().view(2, 16, 64)
+    q[:, :, 0] = 30.0
+    vc[rest[3][0, 0].long(), 0, 5, 9] = float("nan")
+    out = ops.attention_general(q.reshape(2, -1), 1024, torch.empty((2, 1024), dtype=torch.float32, device="cuda"), 2, 16, 1, 64, 0.125, 0, *rest, kc, vc,
+                                max_keys=300).view(2, 16, 64)
+    assert out[0, :, 9].isnan().all() and out[1].isfinite().all() and int(out[0].isnan().sum()) == 16
