@@ -667,14 +667,27 @@ __global__ void __launch_bounds__(AM_THREADS) attention_few_mma_kernel(AmArgs a)
     l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 1);
     l_run[i] += __shfl_xor_sync(0xffffffffu, l_run[i], 2);
     if (quad == 0) s_l[warp][g + 8 * i] = l_run[i];
+    if (quad == 0 && warp == 0) s_m[0][g + 8 * i] = m_run[i];  // (the same for every warp)
   }
-  __syncthreads();  // (the last turn has waited for every copy)
+  float zero = 0.f;  // not a number where a sum is not finite
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) zero = fmaf(0.f, o[j][e], zero);
+  const bool all_finite = !__syncthreads_or(zero != 0.f);  // (the last turn has waited for every copy)
+  auto sum_of = [&](int head) { return (s_l[0][head] + s_l[1][head]) + (s_l[2][head] + s_l[3][head]); };
+  auto factor = [&](int head, float m, float l) {
+    const int h = h0 + head;
+    float inv = a.sink ? sink_inverse(m, l, a.sink[h]) : 1.0f / l;
+    if (a.gate) inv *= 1.0f / (1.0f + expf(-__bfloat162float(a.gate[(size_t)t * a.gate_stride + h])));
+    return inv * a.out_scale;
+  };
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int head = g + 8 * i;
     if (head >= rows) continue;
     const int h = h0 + head;
-    const float l = (s_l[0][head] + s_l[1][head]) + (s_l[2][head] + s_l[3][head]);
+    const float l = sum_of(head);
     if (a.part) {
       float* prow = a.part + (((size_t)t * a.n_heads + h) * a.n_splits + z) * (a.v_dim + 2);
       if (warp == 0 && quad == 0) { prow[0] = m_run[i]; prow[1] = l; }
@@ -684,9 +697,7 @@ __global__ void __launch_bounds__(AM_THREADS) attention_few_mma_kernel(AmArgs a)
         if (d < a.v_dim) { prow[2 + d] = o[j][2 * i]; prow[3 + d] = o[j][2 * i + 1]; }
       }
     } else {
-      float inv = a.sink ? sink_inverse(m_run[i], l, a.sink[h]) : 1.0f / l;
-      if (a.gate) inv *= 1.0f / (1.0f + expf(-__bfloat162float(a.gate[(size_t)t * a.gate_stride + h])));
-      inv *= a.out_scale;
+      const float inv = factor(head, m_run[i], l);
       const size_t orow = (size_t)t * a.out_stride + (size_t)h * a.v_dim;
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
@@ -697,6 +708,32 @@ __global__ void __launch_bounds__(AM_THREADS) attention_few_mma_kernel(AmArgs a)
         }
       }
     }
+  }
+  if (all_finite) return;
+  // A value of infinity times the lower terms of its weight, which may be zero or of the other sign, made a sum that is not a number,
+  // where one in float32 is infinite.  Looked for only in sums that are not finite; a value or a weight that is not a number, and
+  // infinities of both signs, leave them as they are.
+  __syncthreads();  // the block's results have been written
+  for (int i = tid; i < rows * a.v_dim; i += AM_THREADS) {
+    const int head = i / a.v_dim, d = i - head * a.v_dim;
+    float* p = a.part ? a.part + (((size_t)t * a.n_heads + h0 + head) * a.n_splits + z) * (a.v_dim + 2) + 2 + d : nullptr;
+    const size_t at = (size_t)t * a.out_stride + (size_t)(h0 + head) * a.v_dim + d;
+    const float is = p ? *p : load_as_f32(a.out, a.out_wide ? BN_F32 : BN_BF16, at), l = sum_of(head);
+    bool up = false, down = false, none = l != l;
+    if (fabsf(is) < INFINITY || none) continue;
+    for (int u0 = z * AM_KEYS; u0 < n_keys; u0 += span)
+      for (int u = u0; u < min(u0 + AM_KEYS, n_keys); ++u) {
+        const int pos_u = position(u);
+        const float v = __bfloat162float(
+            a.v_cache[(((size_t)pt[pos_u / BN_PAGE] * n_v_heads + vh) * BN_PAGE + pos_u % BN_PAGE) * a.v_row + d]);
+        up |= v == INFINITY;
+        down |= v == -INFINITY;
+        none |= v != v;
+      }
+    if (none || up == down) continue;
+    const float o = up ? INFINITY : -INFINITY;
+    if (p) *p = o;
+    else store_result<__nv_bfloat16>((__nv_bfloat16*)a.out, a.out_wide, at, o * factor(head, s_m[0][head], l));
   }
 }
 

@@ -911,3 +911,31 @@ def test_attention_merge_keeps_what_is_not_a_number(cuda_device):
     out = ops.attention_general(q.reshape(2, -1), 1024, torch.empty((2, 1024), dtype=torch.float32, device="cuda"), 2, 16, 1, 64, 0.125, 0, *rest, kc, vc,
                                 max_keys=300).view(2, 16, 64)
     assert out[0, :, 9].isnan().all() and out[1].isfinite().all() and int(out[0].isnan().sum()) == 16
+
+
+@pytest.mark.parametrize("H,KV,hd,dv,max_keys", [(16, 4, 64, 72, 0), (8, 1, 128, 128, 300), (5, 1, 32, 16, 300)])
+@pytest.mark.parametrize("wide", [False, True])
+def test_attention_of_few_tokens_with_values_that_are_not_finite(cuda_device, H, KV, hd, dv, max_keys, wide):
+    """An infinite value makes its column infinite, both signs or a value that is not a number make it not a number, as in float32
+    (the lower terms of a weight turned infinities into something that is no number); the other columns are as with finite values."""
+    n_keys = [300, 64, 7]
+    g, kc, vc, rest = _few_tokens(n_keys, KV, hd, dv, hd + dv)
+    q = torch.randn((3, H * hd), device="cuda", generator=g).bfloat16()
+    run = lambda x, k, v, dtype: ops.attention_general(x, H * hd, torch.empty((3, H * dv), dtype=dtype, device="cuda"), 3, H, KV, hd, hd ** -0.5, 0,
+                                                       *rest, k, v, max_keys=max_keys, out_scale=-0.5)
+    dtype = torch.float32 if wide else torch.bfloat16
+    plain = run(q, kc, vc, dtype).float().view(3, H, dv)
+    for s, n in enumerate(n_keys):
+        row = lambda p: vc[rest[3][s, p // 64].long(), KV - 1, p % 64]
+        row(n - 1)[0] = row(0)[1] = float("inf")
+        row(n // 2)[2] = float("-inf")
+        row(0)[3], row(n - 1)[3] = float("inf"), float("-inf")
+        row(n - 1)[4] = float("nan")
+        row(0)[5], row(n - 1)[5] = float("inf"), float("nan")
+        row(n // 2)[dv - 1] = float("-inf")
+    got = run(q, kc, vc, dtype).float().view(3, H, dv)
+    ref = run(q.float(), kc.float(), vc.float(), torch.float32).view(3, H, dv)
+    heads = slice(H - H // KV, H)
+    assert ref[:, heads, [0, 1]].eq(float("-inf")).all() and ref[:, heads, [2, dv - 1]].eq(float("inf")).all() and ref[:, heads, 3:6].isnan().all()
+    odd = ~ref.isfinite()
+    assert torch.equal(got[odd].nan_to_num(nan=1.0), ref[odd].nan_to_num(nan=1.0)) and torch.equal(got[~odd], plain[~odd])
