@@ -749,11 +749,12 @@ static size_t am_layout(AmArgs* a) {
   a->stages = fixed + 2 * stage <= 112 * 1024 ? 2 : 1;
   return fixed + a->stages * stage;
 }
-// Whether few tokens of these sizes run on it (bfloat16; 16-byte pieces everywhere).
-static bool am_fits(const AmArgs& a, int n_tokens) {
-  AmArgs b = a;
-  return n_tokens <= 256 && a.head_dim % 8 == 0 && a.v_dim % 8 == 0 && a.v_row % 8 == 0 && a.q_stride % 8 == 0 && a.v_dim <= AM_MAX_V_DIM &&
-         (((uintptr_t)a.q | (uintptr_t)a.k_cache | (uintptr_t)a.v_cache) & 15) == 0 && am_layout(&b) <= AM_SMEM_MAX;
+// Whether the kernel above is built for these sizes: whole 16-byte pieces, value rows and shared memory that fit.
+extern "C" int bn_attention_few_fits(int head_dim, int v_dim, int v_row, int q_stride, int shared_rows) {
+  AmArgs a = {};
+  a.head_dim = head_dim; a.v_dim = v_dim; a.shared_rows = shared_rows;
+  return head_dim > 0 && v_dim > 0 && head_dim % 8 == 0 && v_dim % 8 == 0 && v_row % 8 == 0 && q_stride % 8 == 0 && v_dim <= AM_MAX_V_DIM &&
+         am_layout(&a) <= AM_SMEM_MAX;
 }
 template <int NT>
 static int am_launch(const AmArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
@@ -768,14 +769,15 @@ static int am_launch(const AmArgs& a, dim3 grid, size_t smem, cudaStream_t strea
 }
 
 // q: [n_tokens, q_stride] with head h at element h*head_dim; out [n_tokens, out_stride] with head h at
-// element h*v_dim.  The keys and values of the new tokens must already be in the cache.
+// element h*v_dim.  The keys and values of the new tokens must already be in the cache.  few: on the tensor cores, a block per token
+// (bfloat16 of sizes that bn_attention_few_fits, q and the caches 16-byte aligned; n_splits then deals out 64 keys at a time).
 extern "C" int bn_attention_general_ex(const void* q, int q_stride, void* out, int out_stride, int dtype,
                                        int n_tokens, int n_heads, int n_kv_heads, int head_dim, int v_dim, float scale,
                                        int window, int keep_first, int chunk, int v_row, const float* rel, int n_rel,
                                        const void* gate, int gate_stride, const int* tok_seq, const int* tok_pos, const int* slots,
                                        const int* page_table, int pt_stride,
                                        const void* k_cache, const void* v_cache, float* part, int n_splits,
-                                       const float* sink, int v_share, int out_wide, float out_scale, cudaStream_t stream) {
+                                       const float* sink, int v_share, int out_wide, float out_scale, int few, cudaStream_t stream) {
   if (n_tokens <= 0) return BN_OK;
   if (v_share < 1 || n_kv_heads % v_share || (v_share > 1 && v_row > 0)) return BN_ERR_BAD_ARG;
   if (n_splits < 1 || n_splits > 64 || (n_splits > 1 && !part)) return BN_ERR_BAD_ARG;
@@ -789,7 +791,7 @@ extern "C" int bn_attention_general_ex(const void* q, int q_stride, void* out, i
       (!wide && v_dim > 8 * ATT_THREADS) || (rel && n_rel <= 0))
     return BN_ERR_BAD_ARG;
   if (n_heads > 65535) return BN_ERR_BAD_ARG;
-  if (dtype == BN_BF16) {
+  if (few) {
     AmArgs am = {};
     am.q = (const __nv_bfloat16*)q; am.q_stride = q_stride; am.out = out; am.out_stride = out_stride; am.n_heads = n_heads;
     am.n_kv_heads = n_kv_heads; am.head_dim = head_dim; am.v_dim = v_dim; am.scale = scale; am.window = window; am.keep_first = keep_first;
@@ -799,19 +801,20 @@ extern "C" int bn_attention_general_ex(const void* q, int q_stride, void* out, i
     am.sink = sink; am.v_share = v_share; am.out_wide = out_wide; am.out_scale = out_scale;
     am.tiles_per_group = (n_heads / n_kv_heads + 15) / 16;
     am.shared_rows = v_cache == k_cache && v_row == head_dim && v_share == 1 && v_dim <= head_dim;
-    if (am_fits(am, n_tokens)) {
-      const size_t smem = am_layout(&am);
-      const dim3 agrid(n_tokens, n_kv_heads * am.tiles_per_group, n_splits);
-      const int rc = v_dim <= 32 ? am_launch<1>(am, agrid, smem, stream) : v_dim <= 64 ? am_launch<2>(am, agrid, smem, stream) :
-                     v_dim <= 128 ? am_launch<4>(am, agrid, smem, stream) : v_dim <= 256 ? am_launch<8>(am, agrid, smem, stream) :
-                     am_launch<16>(am, agrid, smem, stream);
-      if (rc != BN_OK) return rc;
-      if (part)
-        BN_LAUNCH((attention_merge_kernel<__nv_bfloat16>), dim3(n_tokens, n_heads), 128, 0, stream, (const float*)part, n_splits, n_heads, v_dim,
-                  (const __nv_bfloat16*)gate, gate_stride, (__nv_bfloat16*)out, out_stride, sink, out_wide, out_scale);
-      BN_CHECK_LAUNCH();
-      return BN_OK;
-    }
+    if (dtype != BN_BF16 || !bn_attention_few_fits(head_dim, v_dim, v_row, q_stride, am.shared_rows) ||
+        (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15))
+      return BN_ERR_BAD_ARG;
+    const size_t smem = am_layout(&am);
+    const dim3 agrid(n_tokens, n_kv_heads * am.tiles_per_group, n_splits);
+    const int rc = v_dim <= 32 ? am_launch<1>(am, agrid, smem, stream) : v_dim <= 64 ? am_launch<2>(am, agrid, smem, stream) :
+                   v_dim <= 128 ? am_launch<4>(am, agrid, smem, stream) : v_dim <= 256 ? am_launch<8>(am, agrid, smem, stream) :
+                   am_launch<16>(am, agrid, smem, stream);
+    if (rc != BN_OK) return rc;
+    if (part)
+      BN_LAUNCH((attention_merge_kernel<__nv_bfloat16>), dim3(n_tokens, n_heads), 128, 0, stream, (const float*)part, n_splits, n_heads, v_dim,
+                (const __nv_bfloat16*)gate, gate_stride, (__nv_bfloat16*)out, out_stride, sink, out_wide, out_scale);
+    BN_CHECK_LAUNCH();
+    return BN_OK;
   }
   // few tokens whose heads share rows: the heads of a key/value head four (or two) at a time, rows read once for them
   const int gq = n_heads / n_kv_heads;
@@ -886,5 +889,5 @@ extern "C" int bn_attention_general(const void* q, int q_stride, void* out, int 
                                     const void* k_cache, const void* v_cache, cudaStream_t stream) {
   return bn_attention_general_ex(q, q_stride, out, out_stride, dtype, n_tokens, n_heads, n_kv_heads, head_dim, head_dim,
                                  scale, window, 0, 0, 0, nullptr, 0, nullptr, 0, tok_seq, tok_pos, slots, page_table,
-                                 pt_stride, k_cache, v_cache, nullptr, 1, nullptr, 1, 0, 1.0f, stream);
+                                 pt_stride, k_cache, v_cache, nullptr, 1, nullptr, 1, 0, 1.0f, 0, stream);
 }

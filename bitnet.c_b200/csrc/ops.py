@@ -8,6 +8,7 @@ back to the CPU: tensors that are not on a CUDA device are refused.
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_float, c_int, c_void_p
 from typing import Optional
 
@@ -575,6 +576,37 @@ def sigmoid_attention(q: torch.Tensor, q_stride: int, out: torch.Tensor, n_token
     return out
 
 
+@functools.lru_cache(maxsize=1024)
+def _attention_few_fits(head_dim: int, v_dim: int, v_row: int, q_stride: int, shared_rows: bool) -> bool:
+    return bool(build.library("attention").bn_attention_few_fits(head_dim, v_dim, v_row, q_stride, int(shared_rows)))
+
+
+def attention_few_pays(blocks: int, heads: int, head_dim: int, max_keys: int, sms: int) -> bool:
+    """Whether few tokens run on the kernel with tensor cores (``blocks``: tokens times key/value heads; ``heads`` that share one).
+    It copies 64 keys at a time for 16 places of heads, so with one or two heads it gains only what its splits and copies in flight
+    gain; the other kernels take 128 keys at a time, more of them beside each other on an SM.  Time of the other kernel over this
+    one's, merge and all, bfloat16, 4 to 2,048 blocks, 16 to 1,024 keys:
+    4 or more heads 1.0 to 3.9;  3 heads beyond 128 keys 0.95 to 2.7, up to 128 keys and 64 blocks 0.66 to 1.0, more blocks 0.7 to 2.0;
+    2 heads of 64 0.95 to 1.6 (from 65 to 128 keys 0.88 to 0.97), of 32 up to 64 keys 1.0 to 1.4, beyond 128 keys and 32 blocks 0.66 to 1.1,
+    of 96 and more up to 2 blocks an SM 0.9 to 2.6 (of 96 beyond 256 keys and 32 blocks 0.78 to 0.88), beyond 0.53 to 1.2;
+    1 head up to 128 keys 0.3 to 1.2 (1.7 in 256 blocks of heads of 256), beyond: of 32 0.44 to 1.0, of 64 and 256 up to 4 blocks an SM
+    0.9 to 2.1, of 96 up to 16 blocks 0.98 to 1.5 and above 0.54 to 1.5, of 128 and 192 up to 64 blocks 0.93 to 1.9 and above 0.5 to 1.7."""
+    up_to = lambda keys: 0 < max_keys <= keys  # (0: not known)
+    if heads >= 4:
+        return True
+    if heads == 3:
+        return not up_to(128) or blocks > 64
+    if heads == 2:
+        if head_dim < 64:
+            return up_to(64) or (not up_to(128) and blocks <= 32)
+        if head_dim < 96:
+            return up_to(64) or not up_to(128)
+        return blocks <= (32 if head_dim < 128 and not up_to(256) else 2 * sms)
+    if head_dim < 64 or up_to(128):
+        return False
+    return blocks <= (4 * sms if head_dim < 96 or head_dim >= 256 else 16 if head_dim < 128 else 64)
+
+
 def attention_general(q: torch.Tensor, q_stride: int, out: torch.Tensor, n_tokens: int, n_heads: int,
                       n_kv_heads: int, head_dim: int, scale: float, window: int, tok_seq: torch.Tensor,
                       tok_pos: torch.Tensor, slots: torch.Tensor, page_table: torch.Tensor,
@@ -644,24 +676,29 @@ def attention_general(q: torch.Tensor, q_stride: int, out: torch.Tensor, n_token
         if not gate.is_cuda or gate.dtype != q.dtype or gate.stride(-1) != 1 or gate.shape[-1] < n_heads or gate_stride <= 0:
             raise KernelError("attention: gate must be a CUDA view of q's type with unit inner stride and one number per head")
     splits = 1
-    piece = 4 if q.dtype == torch.float32 else 8
-    pieces = head_dim % piece == 0 and v_dim % piece == 0 and (v_row or v_dim) % piece == 0
     gq = n_heads // n_kv_heads
-    if q.dtype == torch.bfloat16 and n_tokens <= 256 and pieces and q_stride % 8 == 0 and v_dim <= 512 and head_dim <= 640:
-        # few tokens on the tensor cores: a block per token and 16 heads of a key/value head takes 64 keys at a time, and a second
-        # turn costs it half as much again as the first (a split costs the merge a load)
+    few = (q.dtype == torch.bfloat16 and n_tokens <= 256
+           and (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0
+           and _attention_few_fits(head_dim, v_dim, v_row or v_dim, int(q_stride),
+                                   v_cache.data_ptr() == k_cache.data_ptr() and (v_row or v_dim) == head_dim and v_share == 1)
+           and attention_few_pays(n_tokens * n_kv_heads, gq, head_dim, max_keys, n_sms(q.device)))
+    if few:
+        # a block per token and 16 heads of a key/value head takes 64 keys at a time, and a second turn costs it half as much again as
+        # the first (a split costs the merge a load)
         blocks, keys, most = n_tokens * n_kv_heads * ((gq + 15) // 16), 64, 32
     else:
         # a block per token and head, or per token and group of heads where the kernel takes the heads of a key/value head four or two
         # at a time (few tokens, rows of whole 16-byte pieces)
         per_block = 1
-        if n_tokens <= 256 and pieces and v_dim // piece <= 128:
+        piece = 4 if q.dtype == torch.float32 else 8
+        if (n_tokens <= 256 and head_dim % piece == 0 and v_dim % piece == 0 and (v_row or v_dim) % piece == 0
+                and v_dim // piece <= 128):
             per_block = 4 if gq % 4 == 0 else (2 if gq % 2 == 0 else 1)
         blocks, keys, most = n_tokens * n_heads // per_block, DECODE_CHUNK, 16
     if max_keys > 2 * keys and blocks < 2 * n_sms(q.device):
         splits = min(most, (max_keys + keys - 1) // keys, max(1, 4 * n_sms(q.device) // blocks))
     if (keep_first or rel is not None or gate is not None or v_dim != head_dim or splits > 1 or chunk or v_row
-            or sink is not None or v_share > 1 or out_wide or out_scale != 1.0):
+            or sink is not None or v_share > 1 or out_wide or out_scale != 1.0 or few):
         part = None
         if splits > 1:
             part = torch.empty(n_tokens * n_heads * splits * (v_dim + 2), dtype=torch.float32, device=q.device)
@@ -672,7 +709,7 @@ def attention_general(q: torch.Tensor, q_stride: int, out: torch.Tensor, n_token
             int(n_kv_heads), int(head_dim), int(v_dim), c_float(scale), int(window), int(keep_first), int(chunk), int(v_row),
             _ptr(rel), int(n_rel), _ptr(gate), int(gate_stride), _ptr(tok_seq), _ptr(tok_pos), _ptr(slots), _ptr(page_table),
             int(page_table.shape[1]), _ptr(k_cache), _ptr(v_cache), _ptr(part), int(splits), _ptr(sink), int(v_share),
-            int(out_wide), c_float(out_scale), _stream()), "attention_general")
+            int(out_wide), c_float(out_scale), int(few), _stream()), "attention_general")
         return out
     _check(_fn("attention", "bn_attention_general")(
         _ptr(q), int(q_stride), _ptr(out), int(out.stride(0)), int(_code(q)), int(n_tokens), int(n_heads),

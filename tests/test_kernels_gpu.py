@@ -939,3 +939,20 @@ def test_attention_of_few_tokens_with_values_that_are_not_finite(cuda_device, H,
     assert ref[:, heads, [0, 1]].eq(float("-inf")).all() and ref[:, heads, [2, dv - 1]].eq(float("inf")).all() and ref[:, heads, 3:6].isnan().all()
     odd = ~ref.isfinite()
     assert torch.equal(got[odd].nan_to_num(nan=1.0), ref[odd].nan_to_num(nan=1.0)) and torch.equal(got[~odd], plain[~odd])
+
+
+@pytest.mark.parametrize("H,KV,hd,dv,n,max_keys", [(4, 4, 8, 8, 60, 0), (8, 8, 64, 40, 129, 129), (4, 2, 32, 32, 64, 64), (4, 2, 96, 96, 300, 300),
+                                                   (6, 2, 40, 72, 128, 128), (6, 2, 128, 64, 700, 700), (4, 4, 704, 64, 70, 0), (8, 1, 1024, 128, 70, 0)])
+@pytest.mark.parametrize("S", [1, 3, 64])
+def test_both_kernels_for_few_tokens_agree(cuda_device, monkeypatch, H, KV, hd, dv, n, max_keys, S):
+    """The kernels between which sizes choose, for every number of heads that share rows, with and without splits; heads wider than
+    the one with tensor cores has shared memory for run on the other."""
+    g, kc, vc, rest = _few_tokens([n] * S, KV, hd, dv, n + hd)
+    q = torch.randn((S, H * hd), device="cuda", generator=g).bfloat16()
+    outs = []
+    for pays in (True, False):
+        monkeypatch.setattr(ops, "attention_few_pays", lambda *a: pays)
+        outs.append(ops.attention_general(q, H * hd, torch.empty((S, H * dv), dtype=torch.float32, device="cuda"), S, H, KV, hd, hd ** -0.5, 0, *rest, kc, vc,
+                                          max_keys=max_keys))
+    # scores, exponentials and weighted sums in float32: some 2^-18 of values up to 5
+    assert bool(((outs[0] - outs[1]).abs() <= 5 * 2.0 ** -18).all())
