@@ -2233,6 +2233,7 @@ def moe_experts_few(h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w
     out = torch.empty((T, width), dtype=torch.float32, device=h.device)
     per_call = min(MOE_FEW_TOKENS, MOE_FEW_ITEMS // top)
     if (read_once and h.dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and E <= 1024 and per_call > 0
+            and moe_once_pays(width, ff, E, top, T * top, -(-T // per_call))
             and (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0):
         for t0 in range(0, T, per_call):
             _moe_few_tokens(h, ids, weights, w_gate_up, w_down, limit, slope, scale_input, add, act, add_scale, y, out, t0,
@@ -2248,6 +2249,22 @@ def moe_experts_few(h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w
                                      int(_code(add) if add is not None else 0), _ptr(add_scale), int(E), _ptr(h), _ptr(out), _stream()),
            "moe_down")
     return out
+
+
+def moe_once_pays(width: int, ff: int, experts: int, top: int, items: int, launches: int) -> bool:
+    """Whether few bfloat16 tokens gain from reading each chosen expert once for all of them (``items``: tokens times ``top``).  They do
+    unless experts are small or so many that hardly two items meet: then the kernel that reads an expert per item finds it in the L2
+    again and has more blocks.  Its time over this one's, up to 1,024 items: experts of 512 x 256: 8 of them 0.86 to 2.3, 32 0.56 to 1.3 (with
+    up to two items 1.1 to 1.4, with 8 per token in one launch 1.15 to 1.5); of 1024 x 512 and more, up to 32 of them 0.93 to 3.8; 64 of
+    2048 x 1408 in one launch 1.0 to 3.2, in two 1.0 to 1.15 if both are full and 0.9 if not, in more 0.82 to 0.94; 128 of
+    2048 x 768 up to 32 items 1.0 to 2.3, beyond 0.57 to 1.0."""
+    if width * ff < 1 << 19:
+        return items <= 2 or experts * width * ff <= 1 << 21 or (top >= 8 and launches == 1)
+    if experts <= MOE_FEW_ITEMS // 3:
+        return True
+    if experts <= MOE_FEW_ITEMS // 2:
+        return launches == 1 or (launches == 2 and items > MOE_FEW_ITEMS)
+    return items <= 32
 
 
 MOE_FEW_ITEMS = 128  # (token, expert) items one launch of moe_few.cu takes (MF_MAX_ITEMS)

@@ -105,3 +105,20 @@ def test_moe_experts_few_is_as_exact_as_float32(tokens, width, ff, experts, top)
     err = [float((ops.moe_experts_few(h, ids, weights, up, down, 0.0, 0.0, False, act=ops.ACT_RELU2, read_once=once).double() - want).norm())
            for once in (True, False)]
     assert err[0] <= 1.1 * err[1]
+
+
+@pytest.mark.parametrize("tokens,width,ff,experts,top", [(2, 512, 256, 32, 1), (3, 512, 256, 32, 1), (3, 512, 256, 17, 1), (16, 512, 256, 32, 8), (17, 512, 256, 32, 8),
+                                                         (43, 1024, 512, 42, 4), (33, 1024, 512, 43, 4), (65, 1024, 512, 64, 2), (65, 1024, 512, 64, 1),
+                                                         (32, 1024, 512, 65, 1), (33, 1024, 512, 65, 1)])
+def test_moe_experts_few_on_both_sides_of_the_choice(monkeypatch, tokens, width, ff, experts, top):
+    """Whichever kernels the sizes choose (each expert once for all tokens, or per token), the results agree."""
+    h, ids, weights, up, down = _case(tokens, width, ff, experts, top, 0, 0, seed=tokens + experts)
+    run = lambda: ops.moe_experts_few(h, ids, weights, up, down, 0.0, 0.0, False, act=0)
+    got = run()
+    want, size = _expected(h, ids, weights, up, down, 0.0, 0.0, False, None, 0, None)
+    for chosen in (None, True, False):
+        if chosen is not None:
+            monkeypatch.setattr(ops, "moe_once_pays", lambda *a: chosen)
+        assert ((run().double() - want).abs() <= (4 * 2.0 ** -8) * size + 1e-6).all()  # as above
+    monkeypatch.undo()
+    assert torch.equal(run(), got)
