@@ -457,9 +457,20 @@ __device__ int nucleus_first_exceeding(const float* p, int n, unsigned cutoff_bi
 // The same where the candidates are few, as they are in use: they are kept in shared memory with their ids, in any order.  Both
 // thresholds are found by halving the range of probabilities (as bits), adding the masses of the upper half of what is left: some 28
 // rounds over at most 16 numbers per thread, which rest in registers.  Searching the whole row passes over it eight times, adding 64-bit
-// masses to few bins: 64 rows of 128,256 logits, us, before and after: 279 / 83 in a served batch of the 1B configuration, 183 / 83
-// and 220 / 207 with normal logits of deviation 5 and 3 at temperature 0.7; flat rows keep the search over the row (867 / 875).
-#define NUC_LIST (16 * SAMPLE_THREADS)  // the most candidates; with more the whole row is searched
+// masses to bins, which takes long where they meet in few of them.  The list's time goes by the candidates, the row's by its length.  us,
+// row and list (candidates in brackets): of 128,256 logits 178 / 57 (under 200), 310 / 312 (35,000); 32,000: 62 / 34 (under 200), 72 / 70 (2,600),
+// 98 / 138 (9,000); 16,000: 43 / 32 (200), 48 / 50 (1,000), 61 / 94 (4,200), 111 / 191 (15,400); 4,096: 30 / 29 (under 100), 35 / 44 (1,000),
+// 48 / 68 (3,800); 256: 27 / 29.  So candidates are listed where the first 4,096 logits promise no more than an eleventh of the row
+// less 300 (more may come and are listed too; a list given up costs what its pass over the row took), and none of shorter rows.  Except
+// in rows so flat that the average token has more than 0.28 of the largest probability: 16,000 527 / 195,
+// 4,096 145 / 68, 1,000 52 / 38, 256 36 / 29 (beyond NUC_LIST they keep the search over the row: 128,256 867 / 875).
+#define NUC_LIST (16 * SAMPLE_THREADS)  // the most candidates
+#define NUC_LIST_ROW 4096  // the shortest row of which some are listed that is not flat
+__host__ __device__ __forceinline__ int nuc_list_room(int vocab) { return vocab < NUC_LIST ? vocab : NUC_LIST; }
+__device__ __forceinline__ int nuc_list_most(int vocab, float s) {  // s: the probabilities' sum over the largest one
+  if (s > 0.28f * (float)vocab) return nuc_list_room(vocab);
+  return vocab < NUC_LIST_ROW ? 0 : min(NUC_LIST, vocab / 11 - 300);
+}
 #define NUC_WINDOW (32 * SAMPLE_THREADS)  // logits looked at between two scans
 
 // The sum of v over the first `threads` threads of the block, to each of them; `turn` alternates between calls, so that one barrier is
@@ -561,7 +572,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_topp_kernel(const float
                                    float* __restrict__ probs, int* __restrict__ out) {
   pdl_launch_dependents();  // the next kernel in the stream may begin its prologue
   pdl_wait();               // the kernels before this one have completed and their writes are visible
-  extern __shared__ unsigned long long list[];  // [NUC_LIST]
+  extern __shared__ unsigned long long list[];  // [nuc_list_room(vocab)]
   __shared__ float scratch[32];
   __shared__ int iscratch[32];
   __shared__ float r_shared;
@@ -589,15 +600,31 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_topp_kernel(const float
   }
   const float cutoff = (1.0f - topp) / (float)(vocab - 1);
   const unsigned cutoff_bits = __float_as_uint(fmaxf(cutoff, 0.f));
-  // A token well below this logit cannot reach the cut-off: x / T - m < log(cutoff * s), less what rounding in the quotient, the
-  // difference, the exponential and the division can amount to.  (Not a number: every token is looked at.)
-  const double edge = (double)m + log((double)cutoff * (double)s);
-  const float below = (float)((double)temperature * (edge - 1e-4 - 1e-6 * (fabs((double)m) + fabs(edge))));
   // The candidates' places in the list: counted per thread, then shared out by a scan (one counter for all, 7,000 additions to one
   // address, took longer than the passes over the logits).  A thread marks what it found among its 32 numbers of a window.
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool aligned = ((((uintptr_t)l) & 15) == 0);
-  bool fits = true;
+  const int most = nuc_list_most(vocab, s), room = nuc_list_room(vocab);
+  bool fits = most > 0;
+  float below = 0.f;
+  if (fits) {
+    // A token well below this logit cannot reach the cut-off: x / T - m < log(cutoff * s), less what rounding in the quotient, the
+    // difference, the exponential and the division can amount to.  (Not a number: every token is looked at.)
+    const double edge = (double)m + log((double)cutoff * (double)s);
+    below = (float)((double)temperature * (edge - 1e-4 - 1e-6 * (fabs((double)m) + fabs(edge))));
+    if (most < vocab / 4) {  // (a row that is not flat; it has 4 logits per thread)
+      int mine = 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) mine += !(l[threadIdx.x + e * SAMPLE_THREADS] < below);
+      mine = __reduce_add_sync(0xffffffffu, mine);
+      if (lane == 0) iscratch[warp] = mine;
+      __syncthreads();
+      int all = 0;
+      for (int w = 0; w < SAMPLE_THREADS / 32; ++w) all += iscratch[w];
+      fits = (double)all * vocab <= most * (4.0 * SAMPLE_THREADS);
+      __syncthreads();  // iscratch is written again
+    }
+  }
   for (int base = 0; base < vocab && fits; base += NUC_WINDOW) {
     const int end = min(vocab, base + NUC_WINDOW);
     unsigned marks = 0u;
@@ -639,7 +666,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_topp_kernel(const float
     __syncthreads();  // everyone has read them
     if (threadIdx.x == 0) found = all;
     // where the list is full, or will be if the rest of the row is like this, the whole row is searched
-    fits = all <= NUC_LIST && (double)all * vocab <= 1.25 * NUC_LIST * (double)end;
+    fits = all <= room && (double)all * vocab <= 1.25 * room * (double)end;
     if (fits)
       for (unsigned left = marks; left; left &= left - 1, ++at) {
         const int i = place(__ffs(left) - 1);
@@ -669,10 +696,10 @@ extern "C" int bn_sample_topp(const float* logits, int ld, int n_rows, int vocab
                               cudaStream_t stream) {
   if (n_rows <= 0) return BN_OK;
   if (vocab <= 0 || !(temperature > 0.f) || !(topp > 0.f && topp < 1.f) || !probs) return BN_ERR_BAD_ARG;
-  const size_t smem = NUC_LIST * sizeof(unsigned long long);
+  const size_t smem = nuc_list_room(vocab) * sizeof(unsigned long long);
   static bool granted = false;
   if (!granted) {
-    cudaError_t e = cudaFuncSetAttribute(sample_topp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(sample_topp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NUC_LIST * (int)sizeof(unsigned long long));
     if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
     granted = true;
   }

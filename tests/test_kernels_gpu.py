@@ -956,3 +956,33 @@ def test_both_kernels_for_few_tokens_agree(cuda_device, monkeypatch, H, KV, hd, 
                                           max_keys=max_keys))
     # scores, exponentials and weighted sums in float32: some 2^-18 of values up to 5
     assert bool(((outs[0] - outs[1]).abs() <= 5 * 2.0 ** -18).all())
+
+
+@pytest.mark.parametrize("V,candidates,where,spread", [
+    (140001, 12427, "any", 8.0), (140001, 13000, "any", 8.0),  # about as many as are listed
+    (4095, 60, "any", 8.0), (4096, 60, "any", 8.0), (4096, 200, "any", 8.0),  # about the shortest row of which some are listed
+    (140001, 16384, "back", 8.0), (140001, 16385, "back", 8.0),  # a list promised to be short that is full, or would be more than that
+    (30000, 2000, "front", 8.0), (30000, 9000, "back", 8.0),   # the first logits promise more than there are, or fewer
+    (300, 300, "any", 0.2), (4096, 4096, "any", 0.2), (16384, 16384, "any", 0.2), (16385, 16385, "any", 0.2),  # flat rows
+    (70001, 70001, "any", 0.2), (20000, 12000, "any", 0.2),
+])
+def test_sample_topp_list_or_row(cuda_device, V, candidates, where, spread):
+    """On both sides of every line between the search in a list and over the row, against sums in 64 bits: the token drawn is the first in
+    falling order, lower ids first, whose running sum exceeds the draw."""
+    g = torch.Generator().manual_seed(V + candidates)
+    rows = 3
+    logits = torch.full((rows, V), -60.0)
+    for r in range(rows):
+        at = torch.randperm(V, generator=g)[:candidates] if where == "any" else torch.arange(V)[:candidates] if where == "front" else torch.arange(V)[-candidates:]
+        logits[r, at] = torch.rand(candidates, generator=g) * spread
+    seeds = [3, 14, 159]
+    got = ops.sample_topp(logits.to(cuda_device), 0.9, 0.95, torch.tensor(seeds, dtype=torch.int64, device=cuda_device)).cpu().tolist()
+    for r in range(rows):
+        p = torch.softmax(logits[r].double() / np.float32(0.9).item(), 0)
+        order = torch.argsort(-p, stable=True)
+        cum = torch.cumsum(p[order], 0)
+        cut = int((cum > np.float32(0.95).item()).nonzero()[0])
+        draw = float(plain_llama.Xorshift64Star(seeds[r]).next_float()) * cum[cut].item()
+        at = (order == got[r]).nonzero().item()
+        # float32 probabilities, each within 2^-21 of its own size, and sums of them too
+        assert at <= cut + 1 and cum[at] >= draw - 1e-6 and (cum[at - 1] if at else 0.0) <= draw + 1e-6
