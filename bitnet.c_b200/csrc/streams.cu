@@ -210,8 +210,9 @@ static int launch_streams(const StreamsArgs& args, int n_rows, cudaStream_t stre
   StreamsArgs a = args;
   // A cluster per row only where a row is long and there are few: its three barriers cost more than it saves otherwise (two streams, us,
   // a cluster and one block: 16 rows of 1,024 5.7 / 4.5, of 2,048 5.9 / 4.8, of 4,096 6.2 / 7.4, of 8,192 6.8 / 12.7; 64 rows of 4,096
-  // 7.4 / 8.2; 256 rows of 1,024 12.3 / 5.3, of 4,096 20.4 / 9.2).
-  const bool cluster = V == 4 && n_rows <= 64 && a.width > 2048;
+  // 7.4 / 8.2; 256 rows of 1,024 12.3 / 5.3, of 4,096 20.4 / 9.2; 65 rows of 4,096 5.8 / 4.7).  More than four streams take a block
+  // longer (eight, 80 rows of 4,096 7.5 / 10.8, of 2,056 7.0 / 7.5; 96 rows of 4,096 12.3 / 10.8).
+  const bool cluster = V == 4 && n_rows <= (MS > 4 ? 80 : 64) && a.width > 2048;
   a.cols = cluster ? ((a.width + ST_CLUSTER - 1) / ST_CLUSTER + 3) / 4 * 4 : a.width;
   const size_t smem = (((size_t)a.cols + 3) / 4 * 4) * sizeof(float);
   if (smem > 200 * 1024) return BN_ERR_BAD_ARG;

@@ -47,13 +47,13 @@ def ints(a):
 # ---- kernels alone -----------------------------------------------------------------------------------
 @pytest.mark.parametrize("streams", [1, 2, 3, 4, 7, 16])
 @pytest.mark.parametrize("width", [50, 96, 1032, 2048])
-def test_streams_are_updated_read_and_normed_in_one_pass(cuda_device, streams, width):
+def test_streams_are_updated_read_and_normed_in_one_pass(cuda_device, streams, width, counts=((5, "float32"), (300, "bfloat16"), (7, "bfloat16"))):
     """With and without an update, a layer scale, a bias; every row, or some rows with the streams left alone; a mean far
     from zero; rows of whole 16-byte pieces or not, few rows of wide models (clusters of blocks) or many."""
     from bitnet_c_b200.csrc import ops
     rng = np.random.default_rng(streams * 10000 + width)
     S, W, m, eps = streams, width, 0.7, 1e-5
-    for n, dtype in ((5, "float32"), (300, "bfloat16"), (7, "bfloat16")):
+    for n, dtype in counts:
         t = DT[dtype]
         xs = f32(rng.standard_normal((S, n, W)) + 20.0)  # the mean dwarfs the spread
         y, ls = bf(rng.standard_normal((n, W))), f32(1 + 0.3 * rng.standard_normal(W))
@@ -81,10 +81,16 @@ def test_streams_are_updated_read_and_normed_in_one_pass(cuda_device, streams, w
         assert np.abs(h.cpu().numpy() - pr.layer_norm(xs[0] + y, w, b, eps)).max() < 3e-4
 
 
-@pytest.mark.parametrize("streams,width", [(1, 2056), (2, 4104), (16, 2056)])
+@pytest.mark.parametrize("streams,width", [(1, 2056), (2, 4104), (3, 2056), (4, 4104), (7, 2056), (16, 2056)])
 def test_streams_of_long_rows(cuda_device, streams, width):
-    """Rows long enough for a cluster of blocks where there are few of them."""
+    """Rows long enough for a cluster of blocks where there are few of them (of up to eight streams; more take one block)."""
     test_streams_are_updated_read_and_normed_in_one_pass(cuda_device, streams, width)
+
+
+@pytest.mark.parametrize("streams,width", [(2, 2056), (4, 2056), (8, 2056)])
+def test_streams_of_long_rows_from_clusters_to_blocks(cuda_device, streams, width):
+    """The most rows that clusters take, and one more, for up to four streams and for up to eight."""
+    test_streams_are_updated_read_and_normed_in_one_pass(cuda_device, streams, width, [(n, "float32") for n in (64, 65, 80, 81)])
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
