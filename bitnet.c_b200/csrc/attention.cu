@@ -758,12 +758,9 @@ extern "C" int bn_attention_few_fits(int head_dim, int v_dim, int v_row, int q_s
 }
 template <int NT>
 static int am_launch(const AmArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-  static bool granted = false;
-  if (!granted) {
-    cudaError_t e = cudaFuncSetAttribute(attention_few_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, AM_SMEM_MAX);
-    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
-    granted = true;
-  }
+  static BnGrant grant;
+  cudaError_t e = grant.ask((const void*)attention_few_mma_kernel<NT>, smem, 2048);
+  if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
   BN_LAUNCH(attention_few_mma_kernel<NT>, grid, AM_THREADS, smem, stream, a);
   return BN_OK;
 }

@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "grant.h"
 
 #define BN_F32 0
 #define BN_BF16 1

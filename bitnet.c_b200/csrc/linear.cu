@@ -307,12 +307,9 @@ extern "C" int bn_linear_skinny(const void* x, const void* w, int dtype, void* o
     const bool fours = K > SF_KC / 2 && (N + 15) / 16 <= 4 * sk_sm_count();
 #define SF_LAUNCH(MT, COLS, FOURS)                                                                                            \
   do {                                                                                                                        \
-    static bool granted = false;                                                                                              \
-    if (!granted) {                                                                                                           \
-      cudaError_t e = cudaFuncSetAttribute(linear_stream_f32_kernel<MT, COLS, FOURS>, cudaFuncAttributeMaxDynamicSharedMemorySize, sf_smem(MT)); \
-      if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;                                                                    \
-      granted = true;                                                                                                         \
-    }                                                                                                                         \
+    static BnGrant grant;                                                                                                     \
+    cudaError_t e = grant.ask((const void*)linear_stream_f32_kernel<MT, COLS, FOURS>, sf_smem(MT), 0);                        \
+    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;                                                                      \
     BN_LAUNCH((linear_stream_f32_kernel<MT, COLS, FOURS>), grid, SF_THREADS, sf_smem(MT), stream, (const float*)x, (const float*)w,  \
               out, out_dtype, M, N, K, ldo, partial, bias);                                                                   \
   } while (0)

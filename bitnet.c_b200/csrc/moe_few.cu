@@ -426,16 +426,6 @@ static int mf_sm_count() {
 static size_t mf_list_bytes(const MfArgs& a) { return (size_t)(3 * a.n_real + 1 + a.n_items) * sizeof(int); }
 
 #define MF_SMEM_MAX (180 * 1024)
-template <typename K>
-static int mf_grant(K kernel, bool* granted) {
-  if (!*granted) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MF_SMEM_MAX);
-    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
-    *granted = true;
-  }
-  return BN_OK;
-}
-
 // The most items (tokens times experts per token) of one call.
 extern "C" int bn_moe_few_max_items() { return MF_MAX_ITEMS; }
 
@@ -467,9 +457,10 @@ extern "C" int bn_moe_few(const void* h, int n_tokens, int width, const int* ids
 #define MF_UP(G, R, XR, SCALED)                                                                                                 \
   do {                                                                                                                          \
     const size_t smem = mf_ring_bytes(G * R, XR) + mf_part_turns(G * R, XR) * mf_part_floats(G * R, XR) * sizeof(float) + mf_list_bytes(a); \
-    static bool granted = false;                                                                                                \
+    static BnGrant grant;                                                                                                       \
     if (smem > MF_SMEM_MAX) return BN_ERR_BAD_ARG;                                                                              \
-    if (int rc = mf_grant(moe_few_gate_up_kernel<G, R, XR, SCALED>, &granted)) return rc;                                       \
+    cudaError_t e = grant.ask((const void*)moe_few_gate_up_kernel<G, R, XR, SCALED>, smem, 1024);                               \
+    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;                                                                        \
     BN_LAUNCH((moe_few_gate_up_kernel<G, R, XR, SCALED>), grid, MF_THREADS, smem, stream, a);                                   \
   } while (0)
 #define MF_UP_ROWS(G, SCALED)                              \
@@ -491,9 +482,10 @@ extern "C" int bn_moe_few(const void* h, int n_tokens, int width, const int* ids
 #define MF_DOWN(R, XR)                                                                                                          \
   do {                                                                                                                          \
     const size_t smem = mf_ring_bytes(R, XR) + (size_t)MF_WARPS * a.n_items * 8 * R * sizeof(float) + mf_list_bytes(a);         \
-    static bool granted = false;                                                                                                \
+    static BnGrant grant;                                                                                                       \
     if (smem > MF_SMEM_MAX) return BN_ERR_BAD_ARG;                                                                              \
-    if (int rc = mf_grant(moe_few_down_kernel<R, XR>, &granted)) return rc;                                                     \
+    cudaError_t e = grant.ask((const void*)moe_few_down_kernel<R, XR>, smem, 1024);                                             \
+    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;                                                                        \
     BN_LAUNCH((moe_few_down_kernel<R, XR>), (unsigned)(width / (8 * R)), MF_THREADS, smem, stream, a);                          \
   } while (0)
   if (xr == 1 && wide) MF_DOWN(2, 1);

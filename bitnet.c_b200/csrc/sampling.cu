@@ -697,12 +697,9 @@ extern "C" int bn_sample_topp(const float* logits, int ld, int n_rows, int vocab
   if (n_rows <= 0) return BN_OK;
   if (vocab <= 0 || !(temperature > 0.f) || !(topp > 0.f && topp < 1.f) || !probs) return BN_ERR_BAD_ARG;
   const size_t smem = nuc_list_room(vocab) * sizeof(unsigned long long);
-  static bool granted = false;
-  if (!granted) {
-    cudaError_t e = cudaFuncSetAttribute(sample_topp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NUC_LIST * (int)sizeof(unsigned long long));
-    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
-    granted = true;
-  }
+  static BnGrant grant;
+  cudaError_t e = grant.ask((const void*)sample_topp_kernel, smem, 40 * 1024);
+  if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
   BN_LAUNCH(sample_topp_kernel, n_rows, SAMPLE_THREADS, smem, stream, logits, ld, vocab, temperature, topp, rng, index, probs,
                                                            out);
   BN_CHECK_LAUNCH();
