@@ -109,6 +109,8 @@ class Model:
         if self.embedding_norm is not None:
             fams.extend(self.embedding_norm.all_kernels())
         fams.extend(self.head_part.all_kernels())
+        if any(blk.state_request() is not None for blk in self.blocks):
+            fams.append("cache_rows")  # a new sequence's states are zeroed
         return list(dict.fromkeys(fams))
 
     def bind(self, tensors: Dict[str, torch.Tensor]) -> "Model":

@@ -123,3 +123,15 @@ def test_sizes_round_up_to_pages():
     c = make([KvRequest(1, 16)], max_tokens=100)
     assert c.max_tokens == 128 and c.groups[0].pool.n_pages == 2 and PAGE == 64
     assert c.tokens_free() == 128
+
+
+@pytest.mark.parametrize("stateful", [False, True])
+def test_the_kernel_that_zeroes_states_is_built_with_the_model(stateful):
+    """Opening a sequence of a model with states launches it: it must not be the first request that has it compiled."""
+    import rudolix_cases
+    import tiny_configs
+    from bitnet_c_b200.config import architecture_of
+    cfg = rudolix_cases.CASE_A if stateful else tiny_configs.TINY_A
+    arch = architecture_of(cfg)
+    model = bitnet_c_b200.Model(arch.to_spec(arch.read_config(cfg)), dtype="float32", device=None)
+    assert ("cache_rows" in model.kernel_families()) == stateful
