@@ -19,7 +19,7 @@
 #include "common.cuh"
 
 #define MF_MAX_EXPERTS 1024
-#define MF_MAX_ITEMS 128
+#define MF_MAX_ITEMS 128  // tokens times experts per token of one call; csrc/ops.py cuts its calls by the same numbers
 // Row groups of 8 tokens that a warp multiplies with at a time (XR) and the stages of a warp's ring: a stage is, per lane, one
 // 16-byte piece of each of the S weight streams and of each row group.  A block of 256 threads takes some 100 KB of shared memory,
 // two of them an SM's, with some 130 KB of weights in flight with the fewest tokens.
@@ -426,15 +426,12 @@ static int mf_sm_count() {
 static size_t mf_list_bytes(const MfArgs& a) { return (size_t)(3 * a.n_real + 1 + a.n_items) * sizeof(int); }
 
 #define MF_SMEM_MAX (180 * 1024)
-// The most items (tokens times experts per token) of one call.
-extern "C" int bn_moe_few_max_items() { return MF_MAX_ITEMS; }
-
 // out [n_tokens, width] float32 from h [n_tokens, width], ids and weights [n_tokens, top]: both products of every chosen expert, with
 // y [n_tokens * top, ff] between them.  w_gate (null: the square of relu(up)) and w_up: row j of expert e lies at e * expert_stride +
 // j * width; w_down [experts, width, ff].  act < 0: the clamped unit with `limit` and `slope`; else act(gate) * up.  The weights
 // multiply the experts' input (scale_input) or output.  add [n_tokens, width] of add_dtype (or null), its rows times add_scale
 // [n_tokens] (or null).  Ids from n_real on are identity experts, whose output is the token's row of h.  width and ff are multiples of
-// 8, matrices and rows of bfloat16 16-byte aligned, n_tokens * top at most bn_moe_few_max_items().
+// 8, matrices and rows of bfloat16 16-byte aligned, n_tokens * top at most MF_MAX_ITEMS.
 extern "C" int bn_moe_few(const void* h, int n_tokens, int width, const int* ids, const float* weights, int scale_input, const void* w_gate,
                           const void* w_up, long long expert_stride, int ff, int top, float limit, float slope, int act, int n_real, void* y,
                           const void* w_down, const void* add, int add_dtype, const float* add_scale, float* out, cudaStream_t stream) {

@@ -2232,7 +2232,7 @@ def moe_experts_few(h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w
     y = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
     out = torch.empty((T, width), dtype=torch.float32, device=h.device)
     per_call = min(MOE_FEW_TOKENS, MOE_FEW_ITEMS // top)
-    if (read_once and h.dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and E <= 1024 and per_call > 0
+    if (read_once and h.dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and E <= MOE_FEW_EXPERTS and per_call > 0
             and moe_once_pays(width, ff, E, top, T * top, -(-T // per_call))
             and (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0):
         for t0 in range(0, T, per_call):
@@ -2268,6 +2268,7 @@ def moe_once_pays(width: int, ff: int, experts: int, top: int, items: int, launc
 
 
 MOE_FEW_ITEMS = 128  # (token, expert) items one launch of moe_few.cu takes (MF_MAX_ITEMS)
+MOE_FEW_EXPERTS = 1024  # and experts (MF_MAX_EXPERTS)
 MOE_FEW_TOKENS = 64  # and tokens: an expert's rows are then read once for all of them
 
 

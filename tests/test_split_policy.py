@@ -72,3 +72,14 @@ def test_work_lists_for_unequal_lengths():
     assert all(z == [0] for z in _check_list([30] * 8, 2, items).values())
     for g in (1, 2, 3, 4):
         _check_list(pages, g, decode_items(pages, 40, group=g, capacity=g * 8)[1])
+
+
+def test_calls_for_experts_of_few_tokens_are_cut_as_the_kernel_takes_them():
+    import os
+    import re
+    from bitnet_c_b200.csrc import build, ops
+    with open(os.path.join(os.path.dirname(build.__file__), "moe_few.cu")) as f:
+        source = f.read()
+    limit = lambda name: int(re.search(rf"#define {name} (\d+)", source).group(1))
+    assert ops.MOE_FEW_ITEMS == limit("MF_MAX_ITEMS") and ops.MOE_FEW_EXPERTS == limit("MF_MAX_EXPERTS")
+    assert ops.MOE_FEW_ITEMS <= limit("MF_THREADS")  # an item per thread lists them
