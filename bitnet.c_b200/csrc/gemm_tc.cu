@@ -63,10 +63,15 @@ struct GmArgs {
 };
 
 // The order of the tiles: bands of `band` tiles of rows, and within a band the tiles of one column of W side by side.  The rows of a
-// band stay in the L2 while all of W passes by.  Without bands every column of W passed all rows of x, which with 71,344 rows of
-// 2,048 (292 MB) came from memory again for each of 64 columns: 4682 us against 3937 with bands of 8 (gate and up, 16,384 rows of W,
-// back to back under the power limit).  A band is GM_BAND_BYTES of x, at least 8 tiles: all of x where it fits (4,096 rows of 4,096
-// in bands of 8 pass W twice: 768 us, in one 752).
+// band stay in the L2 while all of W passes by; without bands every column of W passed all rows of x, which came from memory
+// again each time.  Bands of (least) 8 tiles, 17, 26, 34, 43, 51, 68, 102 MB and all of x, us, back to back under the power limit:
+//   71,344 x 2,048, W 16,384   4035  4011  3974  3970  3987  4070  4136  4522  5072
+//   16,384 x 4,096, W 28,672   3035  3073  3021  3004  3032  3051  3267  3464  3755
+//    7,541 x 5,120, W 27,648   1712  1704  1692  1702  1693  1728  1836  1837  1838
+//   16,384 x 14,336, W 4,096   1560  1572  1573  1582  1580  1584  1581  1589  1870
+//    4,096 x 4,096, W 28,672    747   773   769   754   754   755   756   753   751
+// So a band is about a quarter of the L2 (126 MB) in bytes of x: any size from 17 to 51 MB is within 2.5 % of the best, beside it there
+// must be room for the slices of W and the results.  At least 8 tiles, which rows of more than 8,704 numbers need.
 #define GM_BAND_BYTES (34 << 20)
 static int gm_band_tiles(int rows_per_tile, int K) {
   const long long n = (long long)GM_BAND_BYTES / ((long long)rows_per_tile * K * 2);

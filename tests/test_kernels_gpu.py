@@ -693,6 +693,13 @@ def test_gemm_tc_store_swiglu_and_norm_epilogues(cuda_device, pairs, M, N, K):
     ops.gemm_pairs(True)
 
 
+@pytest.mark.parametrize("M,N,K", [(2300, 1032, 8712), (4500, 600, 8712)])
+@pytest.mark.parametrize("pairs", [True, False])
+def test_gemm_tc_bands_of_rows(cuda_device, pairs, M, N, K):
+    """More rows than one band of tiles holds, a last band of fewer tiles and a last tile that is not full, several columns of tiles."""
+    test_gemm_tc_store_swiglu_and_norm_epilogues(cuda_device, pairs, M, N, K)
+
+
 def test_linear_takes_the_own_gemm_when_asked(cuda_device, monkeypatch):
     g = torch.Generator().manual_seed(41)
     x = torch.randn(100, 512, generator=g).to(torch.bfloat16).to(cuda_device)
