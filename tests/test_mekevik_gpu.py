@@ -207,9 +207,9 @@ def test_norms_over_whole_projections_the_blend_and_the_cache_in_one_launch(cuda
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("tokens,H,G,d,dv", [(2, 4, 2, 16, 24), (256, 9, 1, 512, 8), (257, 9, 3, 512, 40)])
-def test_norms_in_whole_pieces_are_those_number_by_number(cuda_device, dtype, tokens, H, G, d, dv):
-    """Rows whose slices lie at 16-byte boundaries, a block per slice or one for all three, slices longer than a thread keeps:
-    the same numbers as rows that lie elsewhere."""
+def test_norms_of_long_slices_at_any_place(cuda_device, dtype, tokens, H, G, d, dv):
+    """Slices of up to 4,608 numbers of many tokens, in rows that begin at 16-byte boundaries or do not, against 64 bits: the rows and
+    what the cache got of them."""
     from bitnet_c_b200.csrc import ops
     g = torch.Generator(device="cuda").manual_seed(tokens + d)
     t = DT[dtype]
@@ -217,15 +217,20 @@ def test_norms_in_whole_pieces_are_those_number_by_number(cuda_device, dtype, to
     x = torch.randn((tokens, nq + nk + nv), device="cuda", generator=g).to(t) * 3
     wq, wk = (1 + 0.3 * torch.randn(n, device="cuda", generator=g).to(t) for n in (nq, nk))
     other = torch.randn((tokens, nv), device="cuda", generator=g).to(t)
-    got = []
+    normed = lambda a, w: a.double() / torch.sqrt(a.double().square().mean(1, keepdim=True) + 1e-5) * w.double()
+    q, k = normed(x[:, :nq], wq), normed(x[:, nq: nq + nk], wk)
+    v = 0.75 * x[:, nq + nk:].double() + 0.25 * other.double()
+    # float32: up to 4,608 squares, 18 in a row per thread, a division, a root and two products; bfloat16: the result's rounding
+    near = lambda a, b: bool(((a.double() - b).abs() <= (2e-6 if dtype == "float32" else 2.0 ** -8 + 2e-6) * b.abs() + 1e-30).all())
     for pad in (0, 1):
         rows = torch.cat([x, torch.zeros((tokens, pad), dtype=t, device="cuda")], dim=1).contiguous()
         kc, vc = (torch.full((-(-tokens // 64), G, 64, n), 9.0, dtype=t, device="cuda") for n in (d, dv))
         ops.slice_norm_append(rows, nq, wq, nq, wk, nq + nk, G, d, dv, 1e-5, v_other=other, blend=0.25, tok_seq=ints([0] * tokens),
                               tok_pos=ints(range(tokens)), slots=ints([0]), page_table=ints(range(-(-tokens // 64)))[None].contiguous(), k_cache=kc, v_cache=vc)
-        got.append((rows[:, : nq + nk + nv].float(), kc.float(), vc.float()))
-    for a, b in zip(*got):  # the sums of squares differ in their order
-        assert bool(((a - b).abs() <= (1e-5 if dtype == "float32" else 2.0 ** -7) * b.abs() + 1e-6).all())
+        assert near(rows[:, :nq], q) and near(rows[:, nq: nq + nk], k)
+        assert bool(((rows[:, nq + nk: nq + nk + nv].double() - v).abs() <= 2.0 ** (-22 if dtype == "float32" else -8) * (v.abs() + 4)).all())
+        for cache, at, n in ((kc, nq, nk), (vc, nq + nk, nv)):
+            assert torch.equal(cache.transpose(1, 2).reshape(-1, n)[:tokens], rows[:, at: at + n]) and (cache.transpose(1, 2).reshape(-1, n)[tokens:] == 9).all()
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
