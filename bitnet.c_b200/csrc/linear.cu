@@ -143,8 +143,7 @@ __device__ __forceinline__ float warp_sums_of_32(float* a, int lane) {
   return a[0];
 }
 
-// FOURS: a piece's four products are added before they go to the sum, which so takes 16 additions per part instead of 64.
-template <int MT, int COLS, bool FOURS>  // rows of x and columns at a time
+template <int MT, int COLS>  // rows of x and columns at a time
 __global__ void __launch_bounds__(SF_THREADS, 2)
 linear_stream_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, void* __restrict__ out, int out_dtype, int M, int N, int K,
                          int ldo, float* __restrict__ partial, const float* __restrict__ bias) {
@@ -205,21 +204,17 @@ linear_stream_f32_kernel(const float* __restrict__ x, const float* __restrict__ 
                        : "=f"(v[c].x), "=f"(v[c].y), "=f"(v[c].z), "=f"(v[c].w) : "r"(ring + src * STAGE + c * SLOT) : "memory");
         src = src + 1 == D ? 0 : src + 1;
         const int k = p * 128 + lane * 4;
-        auto add_rows = [&](auto rows) {
+        if (k < kn) {
 #pragma unroll
-          for (int i = 0; i < decltype(rows)::value; ++i) {
+          for (int i = 0; i < MT; ++i) {
             const float4 u = *reinterpret_cast<const float4*>(xs + i * SF_KC + k);
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
-              float t = FOURS ? v[c].x * u.x : fmaf(v[c].x, u.x, acc[i * COLS + c]);
-              t = fmaf(v[c].y, u.y, t); t = fmaf(v[c].z, u.z, t); t = fmaf(v[c].w, u.w, t);
-              acc[i * COLS + c] = FOURS ? acc[i * COLS + c] + t : t;
+              float t = acc[i * COLS + c];
+              t = fmaf(v[c].x, u.x, t); t = fmaf(v[c].y, u.y, t); t = fmaf(v[c].z, u.z, t); t = fmaf(v[c].w, u.w, t);
+              acc[i * COLS + c] = t;
             }
           }
-        };
-        if (k < kn) {  // half of the rows where there are no more: the last ones of 9 to 12
-          if (MT == 8 && mt <= 4) add_rows(std::integral_constant<int, MT / 2>());
-          else add_rows(std::integral_constant<int, MT>());
         }
       }
       float v;
@@ -300,35 +295,24 @@ extern "C" int bn_linear_skinny(const void* x, const void* w, int dtype, void* o
     if (most < 1) most = 1;
     grid.x = columns < most ? columns : most;
     const int per_warp = (N + (int)(grid.x * SF_WARPS) - 1) / (int)(grid.x * SF_WARPS);
-    // Matrices of up to 16 rows per block and four blocks an SM are those whose inner dimension the kernel named above shared out in
-    // parts of 1,024.  Their longer parts made the error against 64 bits larger (8 rows, relative: 4096 x 4096 1.27e-7 / 1.58e-7,
-    // 1024 x 14336 1.39e-7 / 1.64e-7); with the products in fours it is 1.09e-7 and 1.18e-7, for 3 % of the time (20.0 / 20.7 us).
-    // With more rows the error fell with the parts (28672 x 4096 2.11e-7 / 1.58e-7), and fours cost 5 % (92.7 / 97.2 us).
-    const bool fours = K > SF_KC / 2 && (N + 15) / 16 <= 4 * sk_sm_count();
-#define SF_LAUNCH(MT, COLS, FOURS)                                                                                            \
+#define SF_LAUNCH(MT, COLS)                                                                                                   \
   do {                                                                                                                        \
     static BnGrant grant;                                                                                                     \
-    cudaError_t e = grant.ask((const void*)linear_stream_f32_kernel<MT, COLS, FOURS>, sf_smem(MT), 0);                        \
+    cudaError_t e = grant.ask((const void*)linear_stream_f32_kernel<MT, COLS>, sf_smem(MT), 0);                               \
     if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;                                                                      \
-    BN_LAUNCH((linear_stream_f32_kernel<MT, COLS, FOURS>), grid, SF_THREADS, sf_smem(MT), stream, (const float*)x, (const float*)w,  \
+    BN_LAUNCH((linear_stream_f32_kernel<MT, COLS>), grid, SF_THREADS, sf_smem(MT), stream, (const float*)x, (const float*)w,  \
               out, out_dtype, M, N, K, ldo, partial, bias);                                                                   \
   } while (0)
-#define SF_ORDER(MT, COLS)                \
-  do {                                    \
-    if (fours) SF_LAUNCH(MT, COLS, true); \
-    else SF_LAUNCH(MT, COLS, false);      \
-  } while (0)
-#define SF_COLUMNS(MT)                                                         \
-  do {                                                                         \
-    if (per_warp == 1) SF_ORDER(MT, 1);                                        \
-    else if (per_warp == 2 || per_warp == 5 || per_warp == 6) SF_ORDER(MT, 2); \
-    else SF_ORDER(MT, 4);                                                      \
+#define SF_COLUMNS(MT)                                                          \
+  do {                                                                          \
+    if (per_warp == 1) SF_LAUNCH(MT, 1);                                        \
+    else if (per_warp == 2 || per_warp == 5 || per_warp == 6) SF_LAUNCH(MT, 2); \
+    else SF_LAUNCH(MT, 4);                                                      \
   } while (0)
     if (M <= 2) SF_COLUMNS(2);
     else if (M <= 4) SF_COLUMNS(4);
     else SF_COLUMNS(8);
 #undef SF_COLUMNS
-#undef SF_ORDER
 #undef SF_LAUNCH
   } else if (dtype == BN_BF16)
     BN_LAUNCH((linear_skinny_kernel<__nv_bfloat16>), grid, SK_WARPS * 32, 0, stream,

@@ -871,28 +871,6 @@ def test_attention_of_few_tokens_is_as_exact_as_float32(cuda_device, H, KV, hd, 
     assert err[0] <= 1.2 * err[1]  # (a fifth for chance: the orders of the sums differ)
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 1024, 4096), (8, 1024, 4096), (8, 256, 14336), (16, 9000, 2048)])
-def test_linear_stream_float32_is_as_exact_as_shorter_parts(cuda_device, M, N, K):
-    """No further from 64 bits than sums in parts of 1,024 elements, 32 in a row per lane, then the lanes' tree and the parts one after
-    another, which are reckoned here (products and sums in 64 bits, rounded to float32 after each: as a fused multiply-add does)."""
-    g = torch.Generator(device="cuda").manual_seed(K + N)
-    x, w = torch.randn((M, K), device="cuda", generator=g), torch.randn((N, K), device="cuda", generator=g) * K ** -0.5
-    some = torch.arange(0, N, max(1, N // 256), device="cuda")
-    ref = x.double() @ w[some].double().t()
-    a = (x[:, None].double() * w[some][None].double()).view(M, len(some), K // 1024, 8, 32, 4)
-    lanes = torch.zeros(a.shape[:3] + (32,), device="cuda")
-    for piece in range(8):
-        for e in range(4):
-            lanes = (lanes.double() + a[:, :, :, piece, :, e]).float()
-    for o in (16, 8, 4, 2, 1):
-        lanes = lanes[..., :o] + lanes[..., o: 2 * o]
-    short = torch.zeros((M, len(some)), device="cuda")
-    for part in range(K // 1024):
-        short = short + lanes[:, :, part, 0]
-    err = [float((o.double() - ref).norm()) for o in (ops.linear(x, w)[:, some], short)]
-    assert err[0] <= 1.1 * err[1]
-
-
 def _few_tokens(n_keys, KV, hd, dv, seed):
     """Caches and tables of sequences of n_keys keys with one new token each."""
     g = torch.Generator(device="cuda").manual_seed(seed)
