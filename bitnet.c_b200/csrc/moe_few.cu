@@ -4,8 +4,9 @@
 //   bn_moe_few_gate_up  y[t * top + k] = act(W_gate[e] x, W_up[e] x), x = h[t] (times the weight, when it scales the input), e = ids[t][k]
 //   bn_moe_few_down     out[t] = sum_k (weight) W_down[e] y[t * top + k] (+ what a shared expert gave), float32
 //
-// The products are bound by the experts' bytes.  Streaming them per (token, expert) item (moe.cu, which stays for float32 and for
-// sizes that are not whole 16-byte pieces) read an expert as often as tokens chose it: eight tokens with two of eight experts of
+// The products are bound by the experts' bytes.  Streaming them per (token, expert) item (moe.cu, which stays for float32, for
+// sizes that are not whole 16-byte pieces, and where ops.moe_once_pays finds it faster) read an expert as often as tokens chose it:
+// eight tokens with two of eight experts of
 // 14336 + 7168 rows of 4096 took 393 us a layer (0.9 GB of different bytes, 135 us at the memory's rate).
 // Here a warp multiplies 8 weight rows with up to 16 tokens at a time on the tensor cores (mma.sync m16n8k16, tokens as the 16
 // rows): a lane's 16-byte piece of a weight row is at once its operand of two such instructions, because the order of the inner

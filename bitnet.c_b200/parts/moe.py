@@ -26,7 +26,7 @@ class Moe(FeedForward):
     the input itself; ``activation`` "relu2": down(max(up x, 0)^2), no gate; ``shared_gate``: the shared expert's output times the
     logistic function of one number per token, a row of the router's product.
 
-    Few rows (a decode step): two kernels stream the chosen experts (``read_once``: in bfloat16 once for all the tokens that chose them) from
+    Few rows (a decode step): two kernels stream the chosen experts (``read_once``: in bfloat16, where that gains, once for all the tokens that chose them) from
     device memory alone.  Many rows: the (token, expert) items are sorted by expert, and in bfloat16 all experts run as one
     grouped product each way, which reads the experts' row counts on the device.  Otherwise (float32, odd sizes) every
     expert's rows go through the ordinary products; the host then needs the counts, one copy per call."""
