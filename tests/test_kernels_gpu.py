@@ -288,8 +288,8 @@ def test_sample_topp_follows_the_reference_nucleus(cuda_device, V, topp, temp):
 @pytest.mark.parametrize("candidates", [1, 2, 1025, 16383, 16384, 16385])
 @pytest.mark.parametrize("levels", [0, 40])
 def test_sample_topp_lists_of_candidates(cuda_device, candidates, levels):
-    """Around the number of candidates that the kernel keeps in shared memory (16384), with distinct logits and with ties (``levels``
-    different ones), a vocabulary of more than one window, rows that are not 16-byte aligned, against sums in 64 bits: the token drawn
+    """Few candidates, which the kernel keeps in shared memory, and about as many as fit there (16384), with distinct logits and with
+    ties (``levels`` different ones), a vocabulary of more than one window, rows that are not 16-byte aligned, against sums in 64 bits: the token drawn
     is the first in falling order, lower ids first, whose running sum exceeds the draw."""
     V, rows = 140001, 4
     g = torch.Generator().manual_seed(candidates + levels)
