@@ -40,6 +40,7 @@ SOURCES: Dict[str, str] = {
     "attention_prefill": "attention_prefill.cu",
     "attention_prefill_tc": "attention_prefill_tc.cu",
     "linear": "linear.cu",
+    "linear_resident": "linear_resident.cu",
     "linear_mma": "linear_mma.cu",
     "linear_tc": "linear_tc.cu",
     "gemm_tc": "gemm_tc.cu",

@@ -1210,7 +1210,8 @@ ACTIVATIONS = {"silu": ACT_SILU, "gelu_tanh": ACT_GELU_TANH}
 def linear_tc(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: bool = False,
               cluster: int = 0, sink: Optional[NormSink] = None, _checked: bool = False, act: int = 0,
               bias: Optional[torch.Tensor] = None):
-    """x[M, K] . w[N, K]^T for M <= 64 in bfloat16 on tcgen05 tensor cores with TMA-fed operands.
+    """x[M, K] . w[N, K]^T for M <= 64 in bfloat16 on tcgen05 tensor cores with TMA-fed operands (small matrices, where the number of
+    blocks is not given: linear_resident.cu).
     ``cluster`` blocks (1 to 8) share the inner dimension of each 128-row tile of w and add their
     parts up through distributed shared memory (0: chosen from the number of tiles).  ``x`` may be
     ``RowScaled``.  With ``sink`` the product is added to ``sink.residual`` in place and the result
@@ -1227,8 +1228,9 @@ def linear_tc(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swigl
         _need(w, "w", torch.bfloat16, 2)
         if w.shape[1] != K or M > TC_MAX_ROWS or K % 8 or (swiglu and N % 16) or not 0 <= cluster <= 8:
             raise KernelError(f"linear_tc: x {tuple(x.shape)}, w {tuple(w.shape)}, cluster {cluster} not supported")
-    fn = _fn("linear_tc", "bn_linear_tc_ex")
     dev = x.device
+    resident = cluster == 0 and linear_resident_pays(M, N, K, n_sms(dev)) and (x.data_ptr() | w.data_ptr()) % 16 == 0
+    fn = _fn("linear_resident", "bn_linear_resident") if resident else _fn("linear_tc", "bn_linear_tc_ex")
     if scaled is not None:
         ss_rows = scaled.ss
         _need(ss_rows, "ss", torch.float32, 2)
@@ -1244,10 +1246,16 @@ def linear_tc(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swigl
         if swiglu or tuple(res.shape) != (M, N) or sink.weight.shape[0] != N or sink.weight.dtype not in _DT:
             raise KernelError(f"linear_tc: residual {tuple(res.shape)} / norm weight {tuple(sink.weight.shape)} do not fit "
                               f"a product [{M}, {N}]")
+        xg = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
+        if resident:
+            ss = torch.empty(((N + 15) // 16, M), dtype=torch.float32, device=dev)
+            _check(fn(c_void_p(x.data_ptr()), c_void_p(w.data_ptr()), c_void_p(res.data_ptr()), 0, M, N, K, N, 3, *row,
+                      c_void_p(sink.weight.data_ptr()), _DT[sink.weight.dtype], c_void_p(xg.data_ptr()), c_void_p(ss.data_ptr()), M,
+                      _stream()), "linear_resident")
+            return RowScaled(xg, ss, N, sink.eps)
         if cluster == 0:
             cluster = _auto_cluster(N, K)
         tiles = (N + 127) // 128
-        xg = torch.empty((M, N), dtype=torch.bfloat16, device=dev)
         ss = torch.empty((tiles * cluster, M), dtype=torch.float32, device=dev)
         _check(fn(c_void_p(x.data_ptr()), c_void_p(w.data_ptr()), c_void_p(res.data_ptr()), 0, M, N, K, N, 3,
                   cluster, *row, c_void_p(sink.weight.data_ptr()), _DT[sink.weight.dtype], c_void_p(xg.data_ptr()),
@@ -1256,10 +1264,26 @@ def linear_tc(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swigl
     out_dtype = out_dtype or x.dtype
     cols = N // 2 if swiglu else N
     out = torch.empty((M, cols), dtype=out_dtype, device=dev)
+    if resident:
+        _check(fn(c_void_p(x.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), _DT[out_dtype], M, N, K, cols,
+                  (2 | act << 8) if swiglu else (act << 8 if act == ACT_RELU2 else 0), *row,
+                  _NULL if bias is None else c_void_p(bias.data_ptr()), 0, _NULL, _NULL, 0, _stream()), "linear_resident")
+        return out
     _check(fn(c_void_p(x.data_ptr()), c_void_p(w.data_ptr()), c_void_p(out.data_ptr()), _DT[out_dtype], M, N, K, cols,
               (2 | act << 8) if swiglu else (act << 8 if act == ACT_RELU2 else 0), cluster, *row,
               _NULL if bias is None else c_void_p(bias.data_ptr()), 0, _NULL, _NULL, 0, _tc_status_arg(dev), _stream()), "linear_tc")
     return out
+
+
+def linear_resident_pays(M: int, N: int, K: int, sms: int) -> bool:
+    """Whether a product of few rows goes to ``linear_resident.cu``: where all its blocks (16 rows of w each) run at once.  By shared memory an SM
+    takes as many as hold their rows there, by registers three, or two with more than 8 rows of x.  Saved per product in a chain of dependent
+    ones, against linear_tc.cu: 8 rows of x, 2.0 to 3.4 us on this side of the line (1.2 to 1.7 at 6144 x 1024 and less), 0.1 to -2.1 beyond
+    it; 16 rows, 1.5 to 2.9 us up to K = 2048, 0.5 to 1.2 up to 4096, none at 6144, -0.1 to -6.4 beyond the line."""
+    if M > 16 or K > (6144 if M <= 8 else 4096):
+        return False
+    per_sm = min(3 if M <= 8 else 2, (227 * 1024) // (-(-K // 256) * 8192 + 11 * 1024))
+    return -(-N // 16) <= per_sm * sms
 
 
 _auto_clusters = {}  # (N, K) -> how many blocks share a tile's inner dimension (a property of the sizes and the device)
