@@ -41,6 +41,7 @@ SOURCES: Dict[str, str] = {
     "attention_prefill_tc": "attention_prefill_tc.cu",
     "linear": "linear.cu",
     "linear_resident": "linear_resident.cu",
+    "linear_split": "linear_split.cu",
     "linear_mma": "linear_mma.cu",
     "linear_tc": "linear_tc.cu",
     "gemm_tc": "gemm_tc.cu",

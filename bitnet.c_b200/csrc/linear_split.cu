@@ -1,0 +1,419 @@
+// out[M, N] = x[M, K] . W[N, K]^T (+ a bias) in float32 for many rows, on the 5th-generation tensor cores (tcgen05).
+//
+// A float32 number is the sum of three bfloat16 numbers, exactly: its leading eight bits, the next eight, and what is left (rounded or cut off,
+// the rest has at most eight bits).  Of the nine products of two such sums six are kept (high x high, the two of high x middle,
+// middle x middle, the two of high x low); the other three are below 2^-24 of the product.  The tensor cores multiply them exactly and add
+// them up in their accumulator, which cuts off where an addition rounds, so a sum stays there for 32 numbers of the inner dimension only (small
+// products first) and is then added in float32: the error against 64 bits is a third to a sixth of the float32 library product's
+// (520 rows, 4096 x 4096: 2.2e-7 against 1.1e-6 of the result's norm; 1024 x 14336: 3.9e-7 against 2.2e-6).
+//
+// The float32 units reach 72 TFLOP/s at most, the library's product 54; six bfloat16 products per float32 product are 230 TFLOP/s at the tensor
+// cores' rate.  520 rows: 28672 x 4096 705 us (library 2291), 6144 x 4096 149 (541), 4096 x 4096 133 (324), 4096 x 14336 424 (1126).
+//
+// A tile is 128 rows of W times up to 192 rows of x: D[128 rows of W, NT rows of x], so that few and odd numbers of rows of x waste
+// little (NT is a multiple of 16, chosen so that the tiles fill the SMs).  x is split once, by a kernel of its own, into three
+// planes of bfloat16 in memory (it is small, and every tile column of W reads it again).  W is split on the way: its float32 tiles arrive by
+// TMA, four warps turn a row each thread into three bfloat16 operands in tensor memory, from where the MMA takes its A operand; in
+// shared memory they would cost more of its bandwidth than there is (the MMAs read 5.6 KB of x's planes in 88 cycles each).
+//
+// A persistent block of 16 warps per SM:
+//   warp 0      requests float32 tiles of W (128 rows x 32 numbers)
+//   warp 1      requests tiles of x's three planes (NT rows x 32 numbers each, 64-byte swizzle)
+//   warp 2      allocates tensor memory; one thread issues twelve MMAs per 32 numbers, into one of two accumulators
+//   warps 4-7   split W: shared memory -> registers -> tensor memory, two buffers in turn
+//   warps 8-15  add the accumulators up in registers (a row of W each thread, two warps share a row's columns) and store
+//
+// Numbers that are not finite, or round to infinity in bfloat16, do not split.  Rows that have one are marked (of x by the kernel that
+// splits it, of W by the warps that do); outputs of marked rows are computed again in plain float32.
+//
+// Every wait on an mbarrier is bounded in time; a wait that gives up records code 8 in *status, every role leaves its loops, and the
+// block frees its tensor memory and returns.
+//
+// Reference: y = W x with float32 accumulation (src/quant/f32_scalar.c:4-32); the reference's CUDA prefill calls cublasSgemm
+// (src/gpu_cuda.cu:11788-11879).
+#include "tma.cuh"
+#include "umma.cuh"
+
+#define LS_BM 128        // rows of W per tile (UMMA M)
+#define LS_BK 32         // numbers of the inner dimension per stage and per sum in the tensor cores
+#define LS_NT_MAX 192    // rows of x per tile at most
+#define LS_THREADS 512
+#define LS_W_STAGES 4
+#define LS_W_BYTES (LS_BM * LS_BK * 4)
+#define LS_X_STAGES_MAX 8
+#define LS_A_COLS 48     // columns of tensor memory per buffer of W's three operands (two numbers a column)
+#define LS_ACC_COLS LS_NT_MAX
+#define LS_SMEM_MAX (224 * 1024)
+#define LS_ERR_WAIT 8
+
+struct LsArgs {
+  float* out;
+  const float *x, *w, *bias;
+  const int* x_marked;  // [M]
+  int M, N, K, ldo, k_blocks;
+  int nt, m_tiles, n_tiles, x_stages;
+  int* status;
+};
+
+// Two numbers as three pairs of bfloat16, rounded
+__device__ __forceinline__ void ls_split(float a, float b, unsigned& high, unsigned& mid, unsigned& low) {
+  high = pack_bf16x2(a, b);
+  const float ra = a - __uint_as_float(high << 16), rb = b - __uint_as_float(high & 0xffff0000u);
+  mid = pack_bf16x2(ra, rb);
+  low = pack_bf16x2(ra - __uint_as_float(mid << 16), rb - __uint_as_float(mid & 0xffff0000u));
+}
+// The same cut off instead of rounded, which takes no conversions.  The parts left out of the products have random signs all the same, since
+// x's parts are rounded.
+__device__ __forceinline__ void ls_cut(float a, float b, unsigned& high, unsigned& mid, unsigned& low) {
+  const unsigned ua = __float_as_uint(a), ub = __float_as_uint(b);
+  high = __byte_perm(ua, ub, 0x7632);
+  const float ra = a - __uint_as_float(ua & 0xffff0000u), rb = b - __uint_as_float(ub & 0xffff0000u);
+  const unsigned va = __float_as_uint(ra), vb = __float_as_uint(rb);
+  mid = __byte_perm(va, vb, 0x7632);
+  low = __byte_perm(__float_as_uint(ra - __uint_as_float(va & 0xffff0000u)), __float_as_uint(rb - __uint_as_float(vb & 0xffff0000u)), 0x7632);
+}
+// No split: infinities, what is not a number, and what a rounding to bfloat16 may make infinite
+__device__ __forceinline__ unsigned ls_size(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+#define LS_TOO_LARGE 0x7f000000u
+
+// planes [3][M][pitch] bfloat16 and the marks of x [M, K]; a block per row
+__global__ void __launch_bounds__(256) linear_split_rows_kernel(const float* __restrict__ x, int M, int K, int pitch, __nv_bfloat16* __restrict__ planes,
+                                                                 int* __restrict__ marked) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int m = blockIdx.x;
+  const float* row = x + (size_t)m * K;
+  const size_t plane = (size_t)M * pitch;
+  __nv_bfloat16* to = planes + (size_t)m * pitch;
+  unsigned most = 0;
+  for (int k = threadIdx.x * 4; k < K; k += 1024) {  // K is a multiple of 4
+    const float4 v = *reinterpret_cast<const float4*>(row + k);
+    most = max(max(most, max(ls_size(v.x), ls_size(v.y))), max(ls_size(v.z), ls_size(v.w)));
+    uint2 h, i, l;
+    ls_split(v.x, v.y, h.x, i.x, l.x);
+    ls_split(v.z, v.w, h.y, i.y, l.y);
+    *reinterpret_cast<uint2*>(to + k) = h;
+    *reinterpret_cast<uint2*>(to + plane + k) = i;
+    *reinterpret_cast<uint2*>(to + 2 * plane + k) = l;
+  }
+  const int any = __syncthreads_or(most >= LS_TOO_LARGE);
+  if (threadIdx.x == 0) marked[m] = any;
+}
+
+// K-major tile with rows of 64 bytes, 64-byte swizzled: groups of 8 rows 512 bytes apart
+__device__ __forceinline__ unsigned long long ls_desc(unsigned addr) {
+  return (unsigned long long)((addr >> 4) & 0x3FFF) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
+}
+// An output of a marked row, in plain float32
+__device__ __noinline__ float ls_plain(const float* x, const float* w, int K) {
+  float s = 0.f;
+  for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
+  return s;
+}
+
+template <int CH>  // an adding warp takes 16 CH columns, the tile has up to 32 CH
+__global__ void __launch_bounds__(LS_THREADS, 1)
+linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ LsArgs a) {
+  pdl_launch_dependents();
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const unsigned plane_bytes = a.nt * LS_BK * 2, x_bytes = 3 * plane_bytes;  // nt is a multiple of 16: whole 1024 bytes
+  unsigned char* x_ring = base + LS_W_STAGES * LS_W_BYTES;
+  __shared__ unsigned long long bars[2 * LS_W_STAGES + 2 * LS_X_STAGES_MAX + 7];
+  __shared__ unsigned tmem_slot;
+  __shared__ int s_failed;
+  __shared__ int w_marked[LS_BM];
+  volatile int* failed = &s_failed;
+  const unsigned w_full = smem_u32(bars), w_free = w_full + 8 * LS_W_STAGES, x_full = w_free + 8 * LS_W_STAGES, x_free = x_full + 8 * LS_X_STAGES_MAX,
+                 a_full = x_free + 8 * LS_X_STAGES_MAX, acc_full = a_full + 16, acc_free = acc_full + 16, marks = acc_free + 16;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    s_failed = 0;
+    tma_prefetch_map(&map_w);
+    tma_prefetch_map(&map_x);
+    for (int s = 0; s < LS_W_STAGES; ++s) {
+      mbar_init(w_full + 8 * s, 1);
+      mbar_init(w_free + 8 * s, 4);
+    }
+    for (int s = 0; s < LS_X_STAGES_MAX; ++s) {
+      mbar_init(x_full + 8 * s, 1);
+      mbar_init(x_free + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(a_full + 8 * b, 4);
+      mbar_init(acc_full + 8 * b, 1);
+      mbar_init(acc_free + 8 * b, 8);
+    }
+    mbar_init(marks, 4);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem = tmem_slot;  // accumulators at 0 and LS_ACC_COLS, W's operands behind them
+  const unsigned tmem_a = tmem + 2 * LS_ACC_COLS;
+  const int tiles = a.m_tiles * a.n_tiles;
+  // tile t: rows of W from (t / m_tiles) * 128, rows of x from (t % m_tiles) * nt (the blocks that run at once share rows of W)
+  auto wait = [&](unsigned bar, unsigned parity) {
+    if (!mbar_wait(bar, parity & 1u, a.status, LS_ERR_WAIT) || *failed) {
+      *failed = 1;
+      return false;
+    }
+    return true;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int s = 0, round = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x)
+        for (int kb = 0; kb < a.k_blocks; ++kb) {
+          if (round > 0 && !(ok = wait(w_free + 8 * s, round - 1))) break;
+          mbar_expect_tx(w_full + 8 * s, LS_W_BYTES);
+          tma_load_2d(smem_u32(base + s * LS_W_BYTES), &map_w, w_full + 8 * s, kb * LS_BK, t / a.m_tiles * LS_BM);
+          if (++s == LS_W_STAGES) { s = 0; ++round; }
+        }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      pdl_wait();
+      int s = 0, round = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x)
+        for (int kb = 0; kb < a.k_blocks; ++kb) {
+          if (round > 0 && !(ok = wait(x_free + 8 * s, round - 1))) break;
+          mbar_expect_tx(x_full + 8 * s, x_bytes);
+          for (int p = 0; p < 3; ++p)  // rows behind x's last are another plane's, or zeros: their results are not stored
+            tma_load_2d(smem_u32(x_ring + s * x_bytes + p * plane_bytes), &map_x, x_full + 8 * s, kb * LS_BK, p * a.M + t % a.m_tiles * a.nt);
+          if (++s == a.x_stages) { s = 0; ++round; }
+        }
+    }
+  } else if (warp == 2) {
+    if (lane == 0) {
+      // D float32, A and B bfloat16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24
+      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(a.nt >> 3) << 17) | ((LS_BM >> 4) << 24);
+      int s = 0, round = 0, it = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x)
+        for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
+          const int b = it & 1, use = it >> 1;
+          if (!(ok = wait(a_full + 8 * b, use) && (use == 0 || wait(acc_free + 8 * b, use - 1)) && wait(x_full + 8 * s, round))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const unsigned acc = tmem + b * LS_ACC_COLS, wa = tmem_a + b * LS_A_COLS, xs = smem_u32(x_ring + s * x_bytes);
+          // planes of W and x (0 high, 1 middle, 2 low), the smallest products first
+          constexpr int PW[6] = {2, 1, 0, 1, 0, 0}, PX[6] = {0, 1, 2, 0, 1, 0};
+#pragma unroll
+          for (int i = 0; i < 6; ++i)
+#pragma unroll
+            for (int kk = 0; kk < LS_BK / 16; ++kk)
+              umma_mma_ts(acc, wa + PW[i] * 16 + kk * 8, ls_desc(xs + PX[i] * plane_bytes + kk * 32), idesc, (i | kk) ? 1u : 0u);
+          umma_commit(x_free + 8 * s);   // arrives when these MMAs have read the stage
+          umma_commit(acc_full + 8 * b);  // and W's operands, and the sums are complete
+          if (++s == a.x_stages) { s = 0; ++round; }
+        }
+    }
+  } else if (warp >= 4 && warp < 8) {
+    const int row = (warp & 3) * 32 + lane;
+    const unsigned to0 = tmem_a + ((unsigned)((warp & 3) * 32) << 16);
+    int s = 0, round = 0, it = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
+      float none = 0.f;
+      for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
+        const int b = it & 1, use = it >> 1;
+        ok = __all_sync(0xffffffffu, wait(w_full + 8 * s, round));
+        if (!ok) break;
+        const unsigned char* from = base + s * LS_W_BYTES + row * 128;
+        float4 v[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) v[c] = *reinterpret_cast<const float4*>(from + ((c ^ (row & 7)) << 4));
+        unsigned high[16], mid[16], low[16];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          ls_cut(v[c].x, v[c].y, high[2 * c], mid[2 * c], low[2 * c]);
+          ls_cut(v[c].z, v[c].w, high[2 * c + 1], mid[2 * c + 1], low[2 * c + 1]);
+          // zero, or not a number once a number is not finite
+          none = fmaf(v[c].x, 0.f, fmaf(v[c].y, 0.f, fmaf(v[c].z, 0.f, fmaf(v[c].w, 0.f, none))));
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(w_free + 8 * s);
+        if (use > 0) {  // the MMAs that read this buffer two turns ago are done
+          ok = __all_sync(0xffffffffu, wait(acc_full + 8 * b, use - 1));
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        const unsigned to = to0 + b * LS_A_COLS;
+        tmem_st16(to, reinterpret_cast<const float*>(high));
+        tmem_st16(to + 16, reinterpret_cast<const float*>(mid));
+        tmem_st16(to + 32, reinterpret_cast<const float*>(low));
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (kb + 1 == a.k_blocks) w_marked[row] = none != 0.f;  // (the adding warps have read the tile's before: k_blocks >= 4)
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(a_full + 8 * b);
+          if (kb + 1 == a.k_blocks) mbar_arrive(marks);
+        }
+        if (++s == LS_W_STAGES) { s = 0; ++round; }
+      }
+    }
+  } else if (warp >= 8) {
+    const int quad = warp & 3, row = quad * 32 + lane, c0 = ((warp - 8) >> 2) * 16 * CH;
+    const unsigned from0 = tmem + ((unsigned)(quad * 32) << 16) + c0;
+    int it = 0, tile_i = 0;
+    bool ok = true, waited = false;
+    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, ++tile_i) {
+      float acc[16 * CH];
+#pragma unroll
+      for (int c = 0; c < 16 * CH; ++c) acc[c] = 0.f;
+      int row_marked = 0;
+      for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
+        const int b = it & 1, use = it >> 1;
+        ok = __all_sync(0xffffffffu, wait(acc_full + 8 * b, use));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < CH; ++j)
+          if (c0 + j * 16 < a.nt) {
+            float v[16];
+            tmem_ld16(from0 + b * LS_ACC_COLS + j * 16, v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < 16; ++c) acc[j * 16 + c] += v[c];
+          }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (kb + 1 == a.k_blocks) {
+          ok = __all_sync(0xffffffffu, wait(marks, tile_i));
+          if (!ok) break;
+          row_marked = w_marked[row];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_free + 8 * b);
+      }
+      if (!ok) break;
+      if (!waited) {
+        pdl_wait();
+        waited = true;
+      }
+      const int n = t / a.m_tiles * LS_BM + row, m0 = t % a.m_tiles * a.nt + c0;
+      if (n < a.N) {
+        const float bias = a.bias != nullptr ? a.bias[n] : 0.f;
+        const int m_end = min(a.M, t % a.m_tiles * a.nt + a.nt);
+#pragma unroll
+        for (int c = 0; c < 16 * CH; ++c) {
+          const int m = m0 + c;
+          if (m < m_end) {
+            float v = acc[c];
+            if (row_marked | a.x_marked[m]) v = ls_plain(a.x + (size_t)m * a.K, a.w + (size_t)n * a.K, a.K);
+            a.out[(size_t)m * a.ldo + n] = v + bias;
+          }
+        }
+      }
+      __syncwarp();
+    }
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*failed) {
+    // a wait gave up: loads that were requested may still be landing in this block's shared memory
+    unsigned long long t0 = global_timer();
+    while (global_timer() - t0 < 200000ull) __nanosleep(1000);
+    __syncthreads();
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+static int ls_sm_count() {
+  static int n = 0;
+  if (!n) {
+    int dev = 0, v = 0;
+    n = cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0 ? v : 148;
+  }
+  return n;
+}
+
+// A matrix [rows, cols] whose rows lie row_bytes apart, loaded in boxes of box_rows rows of 32 numbers (zeros outside).  Kind 3: float32,
+// 128-byte swizzle; kind 4: bfloat16, 64-byte swizzle.
+static bool ls_map(CUtensorMap* map, int kind, const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long row_bytes,
+                   int box_rows) {
+  if (tma_map_lookup(kind, ptr, rows, cols, row_bytes, box_rows, map)) return true;
+  PFN_cuTensorMapEncodeTiled enc = tma_encoder();
+  if (!enc) return false;
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)row_bytes};
+  cuuint32_t box[2] = {LS_BK, (cuuint32_t)box_rows}, estr[2] = {1, 1};
+  if (enc(map, kind == 3 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+          CU_TENSOR_MAP_INTERLEAVE_NONE, kind == 3 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return false;
+  tma_map_keep(kind, ptr, rows, cols, row_bytes, box_rows, map);
+  return true;
+}
+
+// Rows of x per tile: the number of tiles of rows for which the last wave costs least.  A tile costs its rows plus LS_TILE_COST.
+#define LS_TILE_COST 24
+static int ls_choose_nt(int M, int n_tiles, int sms) {
+  const int least = (M + LS_NT_MAX - 1) / LS_NT_MAX;
+  int best_nt = 0;
+  long long best = 0;
+  for (int mt = least; mt < least + 6; ++mt) {
+    const int nt = ((M + mt - 1) / mt + 15) / 16 * 16;
+    const long long tiles = (long long)n_tiles * ((M + nt - 1) / nt), cost = (tiles + sms - 1) / sms * (nt + LS_TILE_COST);
+    if (best_nt == 0 || cost < best) { best = cost; best_nt = nt; }
+    if (nt == 16) break;
+  }
+  return best_nt;
+}
+
+// Bytes of working space for M rows of K numbers: three planes of bfloat16 and a mark per row.
+extern "C" long long bn_linear_split_scratch(int M, int K) { return 6ll * M * ((K + 7) / 8 * 8) + 4ll * M; }
+
+// x [M, K], w [N, K], out [M, ldo] float32, all 16-byte aligned with K a multiple of 4 and at least 128; bias [N] or null; scratch as above.
+extern "C" int bn_linear_split(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldo, void* scratch,
+                               int* status, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return BN_OK;
+  if (!x || !w || !out || !scratch || !status || K < 4 * LS_BK || K % 4 || ldo < N || ((uintptr_t)x | (uintptr_t)w | (uintptr_t)scratch) & 15 ||
+      M > (1 << 28))
+    return BN_ERR_BAD_ARG;
+  const int pitch = (K + 7) / 8 * 8;
+  __nv_bfloat16* planes = (__nv_bfloat16*)scratch;
+  int* marked = (int*)((unsigned char*)scratch + 6ll * M * pitch);
+  LsArgs a = {};
+  a.out = out; a.x = x; a.w = w; a.bias = bias; a.x_marked = marked;
+  a.M = M; a.N = N; a.K = K; a.ldo = ldo; a.k_blocks = (K + LS_BK - 1) / LS_BK; a.status = status;
+  a.n_tiles = (N + LS_BM - 1) / LS_BM;
+  a.nt = ls_choose_nt(M, a.n_tiles, ls_sm_count());
+  a.m_tiles = (M + a.nt - 1) / a.nt;
+  if ((long long)a.n_tiles * a.m_tiles > 0x3fffffff) return BN_ERR_BAD_ARG;
+  const int x_bytes = 3 * a.nt * LS_BK * 2, room = LS_SMEM_MAX - 1024 - LS_W_STAGES * LS_W_BYTES;
+  a.x_stages = room / x_bytes < LS_X_STAGES_MAX ? room / x_bytes : LS_X_STAGES_MAX;
+  CUtensorMap mw, mx;
+  if (!ls_map(&mw, 3, w, N, K, 4ull * K, LS_BM) || !ls_map(&mx, 4, planes, 3ull * M, K, 2ull * pitch, a.nt)) return BN_ERR_BAD_ARG;
+  BN_LAUNCH(linear_split_rows_kernel, M, 256, 0, stream, x, M, K, pitch, planes, marked);
+  const size_t smem = 1024 + LS_W_STAGES * LS_W_BYTES + (size_t)a.x_stages * x_bytes;
+  const int tiles = a.n_tiles * a.m_tiles, grid = tiles < ls_sm_count() ? tiles : ls_sm_count();
+#define LS_RUN(CH)                                                                                       \
+  do {                                                                                                   \
+    static BnGrant grant;                                                                                \
+    cudaError_t e = grant.ask((const void*)linear_split_kernel<CH>, smem, 1024);                         \
+    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;                                                 \
+    BN_LAUNCH((linear_split_kernel<CH>), grid, LS_THREADS, smem, stream, mw, mx, a);                     \
+  } while (0)
+  switch ((a.nt + 31) / 32) {
+    case 1: LS_RUN(1); break;
+    case 2: LS_RUN(2); break;
+    case 3: LS_RUN(3); break;
+    case 4: LS_RUN(4); break;
+    case 5: LS_RUN(5); break;
+    default: LS_RUN(6); break;
+  }
+  BN_CHECK_LAUNCH();
+  return BN_OK;
+}

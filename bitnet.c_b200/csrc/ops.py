@@ -1545,7 +1545,10 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: 
         if w.dtype == torch.float32:
             if torch.backends.cuda.matmul.allow_tf32:
                 raise KernelError("float32 products need torch.backends.cuda.matmul.allow_tf32 = False")
-            product = lambda: torch.matmul(x, w.t()) if bias is None else torch.addmm(bias, x, w.t())
+            if K % 4 == 0 and (x.data_ptr() | w.data_ptr()) % 16 == 0 and linear_split_pays(M, N, K):
+                product = lambda: linear_split(x, w, bias)
+            else:
+                product = lambda: torch.matmul(x, w.t()) if bias is None else torch.addmm(bias, x, w.t())
         elif out_dtype == torch.float32:
             product = lambda: torch.mm(x, w.t(), out_dtype=torch.float32) if bias is None else torch.mm(x, w.t(), out_dtype=torch.float32).add_(bias)
         else:  # (biases that come from the file in the compute type lose nothing by going back to it)
@@ -1557,6 +1560,40 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: 
     if swiglu:
         res = torch.empty((M, N // 2), dtype=out.dtype, device=x.device)
         return glu_mul(out, res, act)
+    return out
+
+
+def linear_split_pays(M: int, N: int, K: int) -> bool:
+    """Whether a float32 product goes to ``linear_split.cu``: with many outputs, or wide matrices and not too few rows.  The library product's
+    time over that kernel's: 520 to 2,048 rows 1.3 to 3.7 with a million outputs and more (1.05 to 1.1 right at the line), 0.5 to 0.9 with half as
+    many unless N is 3,072 and more; 48 to 128 rows 1.1 to 2.4 for N of 4,096 to 28,672, 0.4 to 1.0 for narrower ones; 17 to 32 rows 0.7 to
+    1.1.  Short inner dimensions leave it its start: 4,000 x 256 x 256 0.6."""
+    if M * N >= 1 << 20 and M >= 48 and M * N * K >= 1 << 30:
+        return True
+    return N >= 4096 and M >= 48 and M * N >= 280000 and K >= 1024
+
+
+def linear_split(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """x[M, K] . w[N, K]^T + bias in float32 on the tensor cores, from operands split into three bfloat16 numbers each
+    (linear_split.cu): as exact as float32 sums.  K a multiple of 4 and at least 128."""
+    _need(x, "x", torch.float32, 2)
+    _need(w, "w", torch.float32, 2)
+    M, K = x.shape
+    N = w.shape[0]
+    if w.shape[1] != K:
+        raise KernelError(f"linear_split: x {tuple(x.shape)} and w {tuple(w.shape)} do not share the inner size")
+    if bias is not None:
+        _need(bias, "bias", torch.float32, 1)
+        if bias.shape[0] != N:
+            raise KernelError(f"linear_split: {bias.shape[0]} biases for {N} rows")
+    out = torch.empty((M, N), dtype=torch.float32, device=x.device)
+    size = build.library("linear_split").bn_linear_split_scratch
+    size.restype = ctypes.c_longlong
+    scratch = torch.empty(size(int(M), int(K)), dtype=torch.uint8, device=x.device)
+    _check(_fn("linear_split", "bn_linear_split")(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), int(M), int(N), int(K), int(N), _ptr(scratch),
+                                                  _ptr(tc_status(x.device)), _stream()), "linear_split")
+    global LAUNCHES
+    LAUNCHES += 1  # two kernels
     return out
 
 

@@ -102,7 +102,7 @@ class Model:
         return max((b.decode_blocks_per_sequence() for b in self.blocks), default=0)
 
     def kernel_families(self) -> List[str]:
-        fams = ["embed", "linear", "linear_resident"]
+        fams = ["embed", "linear", "linear_resident" if self.dtype == torch.bfloat16 else "linear_split"]
         for blk in self.blocks:
             fams.extend(blk.all_kernels())
         fams.extend(self.final_norm.all_kernels())

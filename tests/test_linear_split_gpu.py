@@ -1,0 +1,74 @@
+"""Float32 products of many rows from split operands (csrc/linear_split.cu), against 64 bits and plain float32."""
+import pytest
+import torch
+
+from bitnet_c_b200.csrc import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _pair(M, N, K, seed, spread=0.0):
+    g = torch.Generator().manual_seed(seed)
+    x, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g) * K ** -0.5
+    if spread:  # columns of very different sizes: the small ones are the low parts' business
+        x = x * torch.exp(spread * torch.randn(K, generator=g))
+    return x.cuda(), w.cuda()
+
+
+@pytest.mark.parametrize("M,N,K,spread", [
+    (17, 128, 128, 0.0),     # the fewest rows, one tile, the smallest inner dimension
+    (17, 130, 132, 0.0),     # a tile of two rows of w; an inner dimension that ends within a stage
+    (192, 256, 512, 0.0),    # one full tile of rows of x
+    (193, 72, 1000, 0.0),    # two of them, the second nearly empty
+    (520, 1000, 516, 0.0),
+    (33, 8, 2048, 0.0),
+    (1000, 64, 192, 0.0),    # more tiles of rows than SMs have tiles of w
+    (400, 20000, 160, 0.0),  # several tiles per block
+    (300, 384, 4096, 3.0),
+])
+@pytest.mark.parametrize("with_bias", [False, True])
+def test_linear_split(M, N, K, spread, with_bias):
+    x, w = _pair(M, N, K, M + N + K, spread)
+    b = torch.randn(N, device="cuda") if with_bias else None
+    got = ops.linear_split(x, w, b)
+    ops.check_tc_status(x.device)
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    if with_bias:
+        want, size = want + b.double(), size + b.double().abs()
+    # A sum of 32 numbers in the tensor cores is cut off some twelve times at 2^-23 of its size at most, the sums of those are rounded at
+    # 2^-24 each, and what the split leaves out is below 2^-23 of each product.
+    bound = (12 + K / 64 + 1) * 2.0 ** -23 * size
+    assert ((got.double() - want).abs() <= bound).all()
+    plain = torch.matmul(x, w.t()) if b is None else torch.addmm(b, x, w.t())
+    err = lambda y: float((y.double() - want).norm() / want.norm())
+    assert err(got) <= max(1.05 * err(plain), 1.5e-7)  # no less exact than float32 sums (below, both are at one rounding of the result)
+
+
+def test_linear_split_what_does_not_split():
+    """Infinities and what is not a number come out as float32 sums give them, numbers near the largest one stay finite, and other rows are
+    not touched."""
+    x, w = _pair(40, 200, 256, 3)
+    clean = ops.linear_split(x, w)
+    x[3, 7], x[5, 9], x[6, 1], x[8, 2], w[100, 5], w[7, 7] = float("inf"), float("nan"), 3.39e38, 1e-39, -float("inf"), 0.0
+    got, want = ops.linear_split(x, w), torch.matmul(x.double(), w.double().t())
+    finite = want.isfinite() & (want.abs() < 3.4e38)
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf() & want.isinf(), want.isinf()) and torch.equal(got[want.isinf()].sign().double(), want[want.isinf()].sign())
+    assert got[finite].isfinite().all()
+    assert ((got.double() - want).abs()[finite] <= 1e-5 * (x.double().abs() @ w.double().abs().t())[finite]).all()
+    rows, cols = [m for m in range(40) if m not in (3, 5, 6, 8)], [n for n in range(200) if n not in (7, 100)]
+    assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
+
+
+def test_float32_products_go_by_one_rule(monkeypatch):
+    """``linear`` takes whichever kernel the sizes choose, refuses TF32 on both, and both agree."""
+    x, w = _pair(70, 256, 512, 9)
+    out = {}
+    for chosen in (True, False):
+        monkeypatch.setattr(ops, "linear_split_pays", lambda *a: chosen)
+        out[chosen] = ops.linear(x, w)
+        monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", True)
+        with pytest.raises(ops.KernelError):
+            ops.linear(x, w)
+        monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", False)
+    assert (out[True] - out[False]).norm() <= 3e-6 * out[False].norm()
