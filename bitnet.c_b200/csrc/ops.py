@@ -1568,6 +1568,8 @@ def linear_split_pays(M: int, N: int, K: int) -> bool:
     time over that kernel's: 520 to 2,048 rows 1.3 to 3.7 with a million outputs and more (1.05 to 1.1 right at the line), 0.5 to 0.9 with half as
     many unless N is 3,072 and more; 48 to 128 rows 1.1 to 2.4 for N of 4,096 to 28,672, 0.4 to 1.0 for narrower ones; 17 to 32 rows 0.7 to
     1.1.  Short inner dimensions leave it its start: 4,000 x 256 x 256 0.6."""
+    if K < 128:  # the kernel's least
+        return False
     if M * N >= 1 << 20 and M >= 48 and M * N * K >= 1 << 30:
         return True
     return N >= 4096 and M >= 48 and M * N >= 280000 and K >= 1024
