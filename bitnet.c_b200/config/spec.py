@@ -372,8 +372,8 @@ class MoeSpec:
     keep_groups: int = 1  # ... and are chosen among those of the so many groups whose best choice score is largest
     identity: int = 0  # the router's last so many outputs are experts whose output is the input itself
     shared_gate: bool = False  # the shared expert's output times the logistic function of one number per token
-    # few bfloat16 tokens: each expert read once for all tokens that chose it (False: once per token and expert, whose sums have
-    # another order)
+    # few bfloat16 tokens: each expert read once for all tokens that chose it on the tensor cores (False: on the float32 units, with the sums of
+    # the kernels that read an expert once per token, which have another order)
     read_once: bool = True
     kind: str = "moe"
 

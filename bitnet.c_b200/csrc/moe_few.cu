@@ -495,3 +495,415 @@ extern "C" int bn_moe_few(const void* h, int n_tokens, int width, const int* ids
   BN_CHECK_LAUNCH();
   return BN_OK;
 }
+
+// ---- the same products with the sums of moe.cu ------------------------------------------------------------------------------------
+//
+//   bn_moe_few_in_order  out[t] as bn_moe_gate_up_ex and bn_moe_down of moe.cu give it, bit for bit
+//
+// For designs whose next token would fall to another order of summation (MoeSpec.read_once = False): a lane takes pieces of eight
+// numbers, 256 apart, multiplies and adds them one after another in float32, and the 32 lanes' sums meet in a butterfly.  The tensor
+// cores have no such order; the float32 units have time for it as long as an expert has few tokens.
+//
+// One block per SM.  A block keeps the rows of x of the tokens that chose an expert in shared memory (as many as fit: `cap`; an expert
+// with more is passed over again); a warp takes a run of all experts' rows and streams 8 of them at a time (4 of each matrix, where
+// there are two; half of that where no more are left) through slots of its lanes' own, copied D - 1 stages ahead.  Runs are cut at any
+// row, and a row counts MR_ROW_COST + its tokens: with equal runs the blocks of the expert that most tokens chose were the last by far.
+// A piece of x serves eight rows, two of them with each instruction (fma.rn.f32x2: two float32 multiply-adds, each rounded as one alone).
+#define MR_WARPS 8
+#define MR_THREADS (32 * MR_WARPS)
+#define MR_S 8       // rows of weights a warp multiplies with at a time
+#define MR_TOKENS 8  // tokens a pass takes at most
+#ifndef MR_ROW_COST
+#define MR_ROW_COST 3
+#endif
+#define MR_SMEM_MAX (226 * 1024)
+__host__ __device__ constexpr int mr_ring_bytes(int D) { return MR_WARPS * D * MR_S * 512; }
+
+struct MrArgs {
+  MfArgs m;
+  int cap;   // tokens of an expert that one pass takes
+  float* d;  // the last product (else null): [items, rows] every item's product
+};
+
+__device__ __forceinline__ float mr_low(unsigned v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float mr_high(unsigned v) { return __uint_as_float(v & 0xffff0000u); }
+__device__ __forceinline__ unsigned long long mr_pair(float a, float b) {
+  unsigned long long v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b));
+  return v;
+}
+// The sums over the warp's lanes of v[0 .. C - 1], each by the additions of warp_sum: lane l meets l ^ O.  Where there is an even number of
+// them left, a lane goes on with half: v[0 ..] are then the numbers from mr_fold_first(C, lane) on.
+template <int C, int O>
+__device__ __forceinline__ void mr_fold(float* v, int lane) {
+  if constexpr (O > 0 && C % 2 == 0) {
+    const bool upper = lane & O;
+#pragma unroll
+    for (int i = 0; i < C / 2; ++i) {
+      const float send = upper ? v[i] : v[i + C / 2], keep = upper ? v[i + C / 2] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+    }
+    mr_fold<C / 2, O / 2>(v, lane);
+  } else if constexpr (O > 0) {
+#pragma unroll
+    for (int i = 0; i < C; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], O);
+    mr_fold<C, O / 2>(v, lane);
+  }
+}
+__host__ __device__ constexpr int mr_fold_left(int c) {  // how many numbers a lane ends with
+  for (int o = 16; o > 0; o >>= 1)
+    if (c % 2 == 0) c /= 2;
+  return c;
+}
+__device__ __forceinline__ int mr_fold_first(int c, int lane) {
+  int first = 0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    if (c % 2 == 0) {
+      c /= 2;
+      if (lane & o) first += c;
+    }
+  return first;
+}
+
+// The passes over experts: seg_expert[s] and the first of its tokens seg_m0[s]; returns how many there are (at most n_items).
+// seg_cost[s]: what a row of every pass before s costs, seg_cost[passes] a row of all.
+__device__ int mr_passes(const MfArgs& a, const MfLists& l, int used, int cap, int* seg_expert, int* seg_m0, int* seg_cost) {
+  __shared__ int s_passes;
+  // The items of an expert in their order: every block has to cut them into the same passes (mf_lists leaves them as they come).
+  int e = -1, place = 0;
+  if (threadIdx.x < a.n_items) {
+    e = a.ids[threadIdx.x];
+    if (e < 0 || e >= a.n_real) e = -1;
+    else for (int i = l.off[e]; i < l.off[e + 1]; ++i) place += l.list[i] < (int)threadIdx.x;
+  }
+  __syncthreads();
+  if (e >= 0) l.list[l.off[e] + place] = threadIdx.x;
+  constexpr int PER = MF_MAX_ITEMS / 32;  // used experts, and passes, a lane takes
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int n[PER], mine = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int u = lane * PER + i;
+      n[i] = u < used ? (l.off[l.used[u] + 1] - l.off[l.used[u]] + cap - 1) / cap : 0;
+      mine += n[i];
+    }
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    int at = upto - mine;
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      for (int p = 0; p < n[i]; ++p) {
+        seg_expert[at] = l.used[lane * PER + i];
+        seg_m0[at++] = p * cap;
+      }
+    if (lane == 31) s_passes = upto;
+    __syncwarp();
+    const int passes = __shfl_sync(0xffffffffu, upto, 31);
+    int cost[PER], sum = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int s = lane * PER + i;
+      cost[i] = 0;
+      if (s < passes) {
+        const int x = seg_expert[s];
+        cost[i] = MR_ROW_COST + min(cap, l.off[x + 1] - l.off[x] - seg_m0[s]);
+      }
+      sum += cost[i];
+    }
+    upto = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    at = upto - sum;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int s = lane * PER + i;
+      if (s <= passes) seg_cost[s] = at;
+      at += cost[i];
+    }
+    if (lane == 31 && passes == MF_MAX_ITEMS) seg_cost[passes] = at;
+  }
+  __syncthreads();
+  return s_passes;
+}
+
+// What a warp streams in one pass: rows 0 .. n_rows - 1 behind w (and w_up), pieces of 256 numbers.
+struct MrStream {
+  const __nv_bfloat16 *w, *w_up;  // this lane's first number of its first row
+  int n_rows, pieces, K, in_row;  // in_row: numbers of a row from this lane's first on
+  unsigned ring;                  // this lane's first slot
+  int fj, fk, f_stage, stage;     // asked for: rows from fj on, piece fk, into f_stage; read next: stage
+};
+// Rows of each matrix in the unit that begins with `left` rows left
+template <int G>
+__device__ __forceinline__ int mr_unit(int left) { return left > MR_S / G / 2 ? MR_S / G : MR_S / G / 2; }
+
+template <int G, int D>
+__device__ __forceinline__ void mr_fetch(MrStream& q) {
+  const int left = q.n_rows - q.fj;
+  if (left > 0) {
+    const int unit = mr_unit<G>(left);
+    if (q.fk * 256 < q.in_row) {
+      const size_t at = (size_t)q.fj * q.K + q.fk * 256;
+      const unsigned dst = q.ring + q.f_stage * (MR_S * 512);
+#pragma unroll
+      for (int r = 0; r < MR_S / G; ++r)
+        if (r < left) {  // (never more than a unit: what is left of a smaller one is at most its size)
+          mf_copy_weights(dst + r * 512, q.w + at + (size_t)r * q.K, true);
+          if (G == 2) mf_copy_weights(dst + (unit + r) * 512, q.w_up + at + (size_t)r * q.K, true);
+        }
+    }
+    if (++q.fk == q.pieces) {
+      q.fk = 0;
+      q.fj += unit;
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  q.f_stage = q.f_stage + 1 == D ? 0 : q.f_stage + 1;
+}
+
+// One unit: R rows (of all matrices together) times N tokens, whose rows begin at x; the sums go to out [N][R].
+template <int G, int D, int N, int R>
+__device__ __forceinline__ void mr_rows(MrStream& q, const __nv_bfloat16* x, float* out, int lane) {
+  unsigned long long acc[N][R / 2];
+#pragma unroll
+  for (int t = 0; t < N; ++t)
+#pragma unroll
+    for (int r = 0; r < R / 2; ++r) acc[t][r] = 0ull;
+#pragma unroll 1
+  for (int k = 0; k < q.pieces; ++k) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(D - 2) : "memory");  // the oldest stage has landed
+    unsigned w[R][4], xs[N][4];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint4 v = mf_slot(q.ring + (q.stage * MR_S + r) * 512);
+      w[r][0] = v.x; w[r][1] = v.y; w[r][2] = v.z; w[r][3] = v.w;
+    }
+    q.stage = q.stage + 1 == D ? 0 : q.stage + 1;
+    const bool live = k * 256 < q.in_row;
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (live) v = *reinterpret_cast<const uint4*>(x + (size_t)t * q.K + k * 256);
+      xs[t][0] = v.x; xs[t][1] = v.y; xs[t][2] = v.z; xs[t][3] = v.w;
+    }
+    mr_fetch<G, D>(q);  // into the stage that was read one turn ago
+    if (live) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        unsigned long long wp[R / 2];
+#pragma unroll
+        for (int r = 0; r < R / 2; ++r)
+          wp[r] = i & 1 ? mr_pair(mr_high(w[2 * r][i / 2]), mr_high(w[2 * r + 1][i / 2])) : mr_pair(mr_low(w[2 * r][i / 2]), mr_low(w[2 * r + 1][i / 2]));
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+          const float v = i & 1 ? mr_high(xs[t][i / 2]) : mr_low(xs[t][i / 2]);
+          const unsigned long long xx = mr_pair(v, v);
+#pragma unroll
+          for (int r = 0; r < R / 2; ++r) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[t][r]) : "l"(xx), "l"(wp[r]));
+        }
+      }
+    }
+  }
+  float v[N * R];
+#pragma unroll
+  for (int t = 0; t < N; ++t)
+#pragma unroll
+    for (int r = 0; r < R / 2; ++r) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[t * R + 2 * r]), "=f"(v[t * R + 2 * r + 1]) : "l"(acc[t][r]));
+  mr_fold<N * R, 16>(v, lane);
+  const int first = mr_fold_first(N * R, lane);
+#pragma unroll
+  for (int i = 0; i < mr_fold_left(N * R); ++i) out[first + i] = v[i];
+}
+
+// G matrices: 2, gate and up; 1, up alone, or the last product's
+template <int G, int D>
+__global__ void __launch_bounds__(MR_THREADS, 1) moe_in_order_kernel(MrArgs p) {
+  const MfArgs& a = p.m;
+  const bool down = p.d != nullptr;
+  if (!down) pdl_wait();
+  pdl_launch_dependents();  // (gate and up: not before, the last product's blocks rely on the ids being there)
+  extern __shared__ __align__(16) unsigned char mr_smem[];
+  __shared__ float s_sums[MR_WARPS][MR_TOKENS * MR_S];
+  __nv_bfloat16* xs = (__nv_bfloat16*)(mr_smem + mr_ring_bytes(D));  // [cap][K]
+  const MfLists l = mf_place_lists((int*)(xs + (size_t)p.cap * a.K), a);
+  int *seg_expert = l.list + a.n_items, *seg_m0 = seg_expert + a.n_items, *seg_cost = seg_m0 + a.n_items;  // (the last: one number more)
+  const int used = mf_lists(l, a);
+  const int passes = mr_passes(a, l, used, p.cap, seg_expert, seg_m0, seg_cost);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // The run of warp w: rows whose cost lies in [w, w + 1) of so many equal shares.  cut(w): a pass and a row in it.
+  const long long total = (long long)seg_cost[passes] * a.rows, share = (long long)gridDim.x * MR_WARPS;
+  auto cut = [&](int w, int& row) {
+    const long long at = total * w / share;
+    int seg = 0;
+    while (seg < passes && (long long)seg_cost[seg + 1] * a.rows <= at) ++seg;
+    row = seg < passes ? (int)((at - (long long)seg_cost[seg] * a.rows) / (seg_cost[seg + 1] - seg_cost[seg])) : 0;
+    return seg;
+  };
+  const int w0 = blockIdx.x * MR_WARPS;
+  int row0, row1, ignored;
+  const int seg0 = cut(w0 + warp, row0), seg1 = cut(w0 + warp + 1, row1);  // this warp's rows: from row0 of pass seg0 to before row1 of seg1
+  const int block0 = cut(w0, ignored), block1 = cut(w0 + MR_WARPS, ignored);
+  MrStream q;
+  q.K = a.K;
+  q.pieces = (a.K + 255) / 256;
+  q.in_row = a.K - lane * 8;
+  q.ring = (unsigned)__cvta_generic_to_shared(mr_smem) + warp * (D * MR_S * 512) + lane * 16;
+  bool waited = !down;
+
+  for (int seg = block0; seg < passes && seg <= block1; ++seg) {
+    const int j0 = seg < seg0 ? a.rows : seg == seg0 ? row0 : 0, j1 = seg < seg1 ? a.rows : seg == seg1 ? row1 : 0;
+    const int e = seg_expert[seg], first = l.off[e] + seg_m0[seg];
+    const int n = min(p.cap, l.off[e + 1] - first);
+    const size_t at = (size_t)e * a.expert_stride + (size_t)j0 * a.K + lane * 8;
+    q.w = (G == 2 ? a.w : a.w_up) + at;
+    q.w_up = a.w_up + at;
+    q.n_rows = j1 > j0 ? j1 - j0 : 0;
+    q.fj = q.fk = q.f_stage = q.stage = 0;
+#pragma unroll 1
+    for (int i = 0; i < D - 1; ++i) mr_fetch<G, D>(q);
+    if (!waited) {
+      pdl_wait();
+      waited = true;
+    }
+    __syncthreads();  // nobody reads the rows of the pass before any more
+    for (int t = 0; t < n; ++t) {  // the rows of x
+      const int item = l.list[first + t];
+      const __nv_bfloat16* src = a.x + (size_t)(down ? item : item / a.top) * a.K;
+      __nv_bfloat16* dst = xs + (size_t)t * a.K;
+      if (!down && a.scale_input) {
+        const float s = a.weights[item];
+#pragma unroll 4
+        for (int c = tid * 8; c < a.K; c += MR_THREADS * 8) *reinterpret_cast<uint4*>(dst + c) = mf_scaled(*reinterpret_cast<const uint4*>(src + c), s);
+      } else {
+        for (int c = tid * 8; c < a.K; c += MR_THREADS * 8) mf_copy_weights((unsigned)__cvta_generic_to_shared(dst + c), src + c, true);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const __nv_bfloat16* x = xs + lane * 8;
+    float* sums = s_sums[warp];
+    for (int j = 0; j < q.n_rows;) {
+      const int unit = mr_unit<G>(q.n_rows - j);
+#define MR_CASE(N)                                                             \
+  case N:                                                                      \
+    if (unit == MR_S / G) mr_rows<G, D, N, MR_S>(q, x, sums, lane);            \
+    else mr_rows<G, D, N, MR_S / 2>(q, x, sums, lane);                         \
+    break
+      switch (n) {
+        MR_CASE(1); MR_CASE(2); MR_CASE(3); MR_CASE(4); MR_CASE(5); MR_CASE(6); MR_CASE(7); MR_CASE(8);
+      }
+#undef MR_CASE
+      __syncwarp();
+      const int rows = min(unit, q.n_rows - j);
+      for (int o = lane; o < n * unit; o += 32) {
+        const int t = o / unit, r = o - t * unit;
+        if (r >= rows) continue;
+        const int item = l.list[first + t];
+        const size_t to = (size_t)item * a.rows + j0 + j + r;
+        const float last = sums[t * unit * G + (G - 1) * unit + r];
+        if (down) {
+          p.d[to] = last;
+          continue;
+        }
+        // the products' results pass through bfloat16, as they do on the sorted path
+        const float up = to_f32<__nv_bfloat16>(from_f32<__nv_bfloat16>(last));
+        float v;
+        if (G == 1) {
+          v = relu_squared(up);
+        } else {
+          const float gate = to_f32<__nv_bfloat16>(from_f32<__nv_bfloat16>(sums[t * unit * G + r]));
+          if (a.act >= 0) {
+            v = glu_activation(gate, a.act) * up;
+          } else {
+            const float gl = fminf(gate, a.limit);
+            v = gl / (1.0f + expf(-a.slope * gl)) * (fminf(fmaxf(up, -a.limit), a.limit) + 1.0f);
+          }
+        }
+        a.y[to] = from_f32<__nv_bfloat16>(v);
+      }
+      __syncwarp();
+      j += unit;
+    }
+  }
+  if (!waited) pdl_wait();  // a block without rows ends no sooner than the kernel before this one
+}
+
+// Every token's items, in their order; identity experts hand on the token's row; what a shared expert gave comes last.
+__global__ void moe_in_order_sum_kernel(MrArgs p) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const MfArgs& a = p.m;
+  const int t = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
+  if (c >= a.rows) return;
+  float total = 0.f;
+  for (int k = 0; k < a.top; ++k) {
+    const int item = t * a.top + k, e = a.ids[item];
+    float d = 0.f;
+    if (e >= a.n_real) d = to_f32<__nv_bfloat16>(a.h[(size_t)t * a.rows + c]);
+    else if (e >= 0) d = p.d[(size_t)item * a.rows + c];
+    const float wt = a.scale_output ? a.weights[item] : 1.0f;
+    total += d * wt;
+  }
+  if (a.add) total += load_as_f32(a.add, a.add_dtype, (size_t)t * a.rows + c) * (a.add_scale ? a.add_scale[t] : 1.0f);
+  a.out[(size_t)t * a.rows + c] = total;
+}
+
+// Rows of K numbers that fit beside a ring of D stages
+static int mr_room(int D, int K, size_t lists) { return (int)((MR_SMEM_MAX - 4096 - mr_ring_bytes(D) - lists) / (2 * (size_t)K)); }
+
+// bn_moe_few with the sums of moe.cu, for the same arguments: d [n_tokens * top, width] float32 is working space.  No row of x may be
+// larger than the shared memory beside a ring (width and ff up to 40,960 numbers).
+extern "C" int bn_moe_few_in_order(const void* h, int n_tokens, int width, const int* ids, const float* weights, int scale_input, const void* w_gate,
+                                   const void* w_up, long long expert_stride, int ff, int top, float limit, float slope, int act, int n_real,
+                                   void* y, const void* w_down, const void* add, int add_dtype, const float* add_scale, float* d, float* out,
+                                   cudaStream_t stream) {
+  if (n_tokens <= 0) return BN_OK;
+  if (!h || !ids || !weights || !w_up || !w_down || !y || !d || !out || top <= 0 || top > MF_MAX_ITEMS || n_tokens > MF_MAX_ITEMS / top ||
+      n_real <= 0 || n_real > MF_MAX_EXPERTS || width <= 0 || width % 8 || ff <= 0 || ff % 8 || expert_stride % 8 || width > 40960 || ff > 40960 ||
+      (((uintptr_t)h | (uintptr_t)w_gate | (uintptr_t)w_up | (uintptr_t)w_down | (uintptr_t)y) & 15))
+    return BN_ERR_BAD_ARG;
+  MrArgs p = {};
+  MfArgs& a = p.m;
+  a.x = (const __nv_bfloat16*)h; a.ids = ids; a.weights = weights; a.n_items = n_tokens * top; a.top = top; a.n_real = n_real;
+  a.K = width; a.rows = ff; a.w = (const __nv_bfloat16*)w_gate; a.w_up = (const __nv_bfloat16*)w_up; a.expert_stride = (size_t)expert_stride;
+  a.scale_input = scale_input; a.limit = limit; a.slope = slope; a.act = act; a.y = (__nv_bfloat16*)y;
+  const size_t lists = mf_list_bytes(a) + (3 * a.n_items + 1) * sizeof(int);
+  // Stages: four where the tokens' rows leave room for them, else three.
+#define MR_RUN(G, D)                                                                                                            \
+  do {                                                                                                                          \
+    p.cap = most < mr_room(D, a.K, lists) ? most : mr_room(D, a.K, lists);                                                      \
+    if (p.cap < 1) return BN_ERR_BAD_ARG;                                                                                       \
+    const size_t smem = mr_ring_bytes(D) + (size_t)p.cap * a.K * 2 + lists;                                                     \
+    static BnGrant grant;                                                                                                       \
+    cudaError_t e = grant.ask((const void*)moe_in_order_kernel<G, D>, smem, 4096);                                              \
+    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;                                                                        \
+    BN_LAUNCH((moe_in_order_kernel<G, D>), (unsigned)mf_sm_count(), MR_THREADS, smem, stream, p);                               \
+  } while (0)
+  const int most = n_tokens < MR_TOKENS ? n_tokens : MR_TOKENS;
+  if (w_gate) {
+    if (mr_room(4, a.K, lists) >= most) MR_RUN(2, 4);
+    else MR_RUN(2, 3);
+  } else {
+    if (mr_room(4, a.K, lists) >= most) MR_RUN(1, 4);
+    else MR_RUN(1, 3);
+  }
+  a.x = (const __nv_bfloat16*)y;
+  a.K = ff; a.rows = width; a.w = nullptr; a.w_up = (const __nv_bfloat16*)w_down; a.expert_stride = (size_t)width * ff;
+  a.scale_output = !scale_input; a.add = add; a.add_dtype = add_dtype; a.add_scale = add_scale; a.h = (const __nv_bfloat16*)h; a.out = out;
+  p.d = d;
+  if (mr_room(4, a.K, lists) >= most) MR_RUN(1, 4);
+  else MR_RUN(1, 3);
+  BN_LAUNCH(moe_in_order_sum_kernel, dim3(n_tokens, (width + 255) / 256), 256, 0, stream, p);
+  BN_CHECK_LAUNCH();
+  return BN_OK;
+}

@@ -2301,8 +2301,9 @@ def moe_experts_few(h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w
                     w_down: torch.Tensor, limit: float, slope: float, scale_input: bool,
                     add: Optional[torch.Tensor] = None, act: int = -1, add_scale: Optional[torch.Tensor] = None,
                     read_once: bool = True) -> torch.Tensor:
-    """The chosen experts of every token (with ``read_once``, in bfloat16, each expert is read once for all tokens that chose it; else, and where rows
-    are not whole 16-byte pieces, once per (token, expert)): float32 ``[T, width]``, the sum over
+    """The chosen experts of every token (with ``read_once``, in bfloat16, each expert is read once for all tokens that chose it; without, the
+    sums have the order of the kernels that read an expert once per (token, expert), which run where rows are not whole 16-byte pieces, in
+    float32, and where it does not pay to read an expert once): float32 ``[T, width]``, the sum over
     a token's experts plus ``add``.  The weight multiplies the expert's input (``scale_input``) or its output.
     ``act`` < 0: the clamped unit with ``limit`` and ``slope``; ACT_SILU / ACT_GELU_TANH: act(gate) * up; ACT_RELU2: no gate,
     the square of relu(up), and ``w_gate_up`` is ``[experts, ff, width]``.  Ids from the number of experts on are identity experts:
@@ -2339,6 +2340,14 @@ def moe_experts_few(h: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor, w
             _moe_few_tokens(h, ids, weights, w_gate_up, w_down, limit, slope, scale_input, add, act, add_scale, y, out, t0,
                             min(per_call, T - t0))
         return out
+    if (not read_once and h.dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0 and E <= MOE_FEW_EXPERTS and per_call > 0
+            and max(width, ff) <= MOE_IN_ORDER_ROW and moe_in_order_pays(width, ff, T * top)
+            and (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0):
+        products = torch.empty((min(per_call, T) * top, width), dtype=torch.float32, device=h.device)
+        for t0 in range(0, T, per_call):
+            _moe_few_tokens(h, ids, weights, w_gate_up, w_down, limit, slope, scale_input, add, act, add_scale, y, out, t0,
+                            min(per_call, T - t0), products)
+        return out
     w_up = w_gate_up[:, ff:] if per == 2 else w_gate_up
     _check(_fn("moe", "bn_moe_gate_up_ex")(_ptr(h), int(_code(h)), int(T), int(width), _ptr(ids), _ptr(weights),
                                            int(bool(scale_input)), _ptr(w_gate_up if per == 2 else None), c_void_p(w_up.data_ptr()),
@@ -2367,24 +2376,38 @@ def moe_once_pays(width: int, ff: int, experts: int, top: int, items: int, launc
     return items <= 32
 
 
+MOE_IN_ORDER_ROW = 40960  # numbers of a row of x that the kernels of the other order hold beside their ring (moe_few.cu)
+
+
+def moe_in_order_pays(width: int, ff: int, items: int) -> bool:
+    """Whether few bfloat16 tokens whose sums must keep their order gain from reading each chosen expert once.  The time of the kernels
+    that read an expert per item over theirs: experts of 4096 x 7168 1.36 to 1.93, 2048 x 4096 1.28 to 2.4, 1024 x 2048 1.19 to 1.96 (8 experts,
+    2 to 128 items), 64 of 2048 x 1408 1.0 to 2.1 (6 to 384 items); 128 of 2048 x 768 1.0 to 1.4 up to 128 items, 0.84 to 0.98 beyond; 32 of
+    1024 x 512 1.05 to 1.3 up to 16 items, 0.78 to 1.06 beyond; 512 x 256 0.45 to 0.6."""
+    return width * ff >= 1 << 21 or (width * ff >= 1 << 20 and items <= 128) or (width * ff >= 1 << 19 and items <= 16)
+
+
 MOE_FEW_ITEMS = 128  # (token, expert) items one launch of moe_few.cu takes (MF_MAX_ITEMS)
 MOE_FEW_EXPERTS = 1024  # and experts (MF_MAX_EXPERTS)
 MOE_FEW_TOKENS = 64  # and tokens: an expert's rows are then read once for all of them
 
 
-def _moe_few_tokens(h, ids, weights, w_gate_up, w_down, limit, slope, scale_input, add, act, add_scale, y, out, t0: int, n: int) -> None:
-    """``moe_experts_few`` for the tokens ``t0 .. t0 + n``: every chosen expert read once for all of them (bfloat16)."""
+def _moe_few_tokens(h, ids, weights, w_gate_up, w_down, limit, slope, scale_input, add, act, add_scale, y, out, t0: int, n: int,
+                    products: Optional[torch.Tensor] = None) -> None:
+    """``moe_experts_few`` for the tokens ``t0 .. t0 + n``: every chosen expert read once for all of them (bfloat16).  With
+    ``products`` (float32, a row per item) the sums are added up in the order of the kernels that read an expert per item."""
     width, top, E, ff = h.shape[1], ids.shape[1], w_gate_up.shape[0], w_down.shape[2]
     per = w_gate_up.shape[1] // ff
     at = lambda t, rows: c_void_p(t.data_ptr() + rows * t.stride(0) * t.element_size() if t is not None else 0)
     gate = w_gate_up.data_ptr()
-    _check(_fn("moe_few", "bn_moe_few")(
+    between = () if products is None else (_ptr(products),)
+    _check(_fn("moe_few", "bn_moe_few" if products is None else "bn_moe_few_in_order")(
         at(h, t0), int(n), int(width), at(ids, t0), at(weights, t0), int(bool(scale_input)), c_void_p(gate if per == 2 else 0),
         c_void_p(gate + (per - 1) * ff * width * 2), ctypes.c_longlong(per * ff * width), int(ff), int(top), c_float(limit), c_float(slope),
         int(act), int(E), at(y, t0 * top), _ptr(w_down), at(add, t0), int(_code(add) if add is not None else 0), at(add_scale, t0),
-        at(out, t0), _stream()), "moe_few")
+        *between, at(out, t0), _stream()), "moe_few")
     global LAUNCHES
-    LAUNCHES += 1  # two kernels
+    LAUNCHES += 1 if products is None else 2  # two kernels, three with the sums of a token's items
 
 
 def moe_count(ids: torch.Tensor, n_experts: int) -> torch.Tensor:

@@ -122,3 +122,28 @@ def test_moe_experts_few_on_both_sides_of_the_choice(monkeypatch, tokens, width,
         assert ((run().double() - want).abs() <= (4 * 2.0 ** -8) * size + 1e-6).all()  # as above
     monkeypatch.undo()
     assert torch.equal(run(), got)
+
+
+@pytest.mark.parametrize("tokens,width,ff,experts,top,act,scale_input,identity", [
+    (1, 64, 64, 3, 2, 0, False, 0),
+    (5, 72, 200, 4, 2, 0, False, 0),      # lanes without a last piece; runs that end within a unit of rows
+    (3, 4104, 264, 2, 1, 1, False, 0),
+    (33, 128, 2048, 4, 3, ops.ACT_RELU2, False, 0),  # experts passed over several times
+    (64, 520, 264, 6, 2, -1, True, 0),    # the most items of one launch; weights on the input
+    (64, 264, 128, 1, 1, 0, True, 0),     # one expert for all
+    (8, 128, 40, 12, 16, 0, False, 4),    # identity experts
+    (9, 128, 64, 40, 32, 0, False, 0),    # several launches
+    (3, 40960, 64, 4, 2, 0, False, 0),    # the longest rows: few beside the ring
+    (12, 64, 40960, 3, 1, 0, False, 0),
+])
+@pytest.mark.parametrize("with_add", [False, True])
+def test_moe_experts_few_in_order(monkeypatch, tokens, width, ff, experts, top, act, scale_input, identity, with_add):
+    """Without ``read_once`` the sums are those of the kernels that read an expert per item, bit for bit, whichever kernels run."""
+    h, ids, weights, up, down = _case(tokens, width, ff, experts, top, act, identity, seed=tokens * 1000 + ff)
+    add = torch.randn(tokens, width, device="cuda") if with_add else None
+    add_scale = torch.rand(tokens, device="cuda") if with_add and act == 0 else None
+    out = []
+    for once in (True, False):
+        monkeypatch.setattr(ops, "moe_in_order_pays", lambda *a: once)
+        out.append(ops.moe_experts_few(h, ids, weights, up, down, 3.0, 1.5, scale_input, add=add, act=act, add_scale=add_scale, read_once=False))
+    assert torch.equal(*out)
