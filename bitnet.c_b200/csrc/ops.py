@@ -888,43 +888,6 @@ def latent_pages(keys: torch.Tensor, values: torch.Tensor, k_cache: torch.Tensor
                                             _ptr(scratch_table), int(scratch_table.shape[1]), _ptr(k_pages), _ptr(v_pages), _stream()), "latent_pages")
 
 
-LATENT_FEW_TOKENS = 64
-
-
-def latent_few(tokens: int, q: torch.Tensor, w_uk: torch.Tensor, w_uv: torch.Tensor) -> bool:
-    """Whether ``latent_queries`` and ``latent_values`` take these: few bfloat16 tokens, rows of whole 16-byte pieces, a block's share of a
-    head's weights in its registers (latent.cu: LT_DIM_MAX, LT_PIECES)."""
-    return (tokens <= LATENT_FEW_TOKENS and q.dtype == w_uk.dtype == w_uv.dtype == torch.bfloat16 and q.stride(1) == 1 and w_uk.shape[1] <= 256
-            and w_uk.shape[2] % 8 == 0 and w_uk.shape[2] <= 512 and (w_uk.data_ptr() | w_uv.data_ptr()) % 16 == 0)
-
-
-def latent_queries(q: torch.Tensor, w_uk: torch.Tensor, rot: int) -> torch.Tensor:
-    """``[tokens, heads, rank + rot]``: every head's first numbers times its ``w_uk`` ``[heads, dim, rank]``, its rotated ones behind them.
-    ``q`` ``[tokens, heads * (dim + rot)]``, a view with unit inner stride."""
-    _need_rows(q, "q", torch.bfloat16)
-    _need(w_uk, "w_uk", torch.bfloat16, 3)
-    H, dim, rank = w_uk.shape
-    if q.shape[1] != H * (dim + rot):
-        raise KernelError(f"latent_queries: q {tuple(q.shape)} does not hold {H} heads of {dim} + {rot}")
-    out = torch.empty((q.shape[0], H, rank + rot), dtype=q.dtype, device=q.device)
-    _check(_fn("latent", "bn_latent_queries")(_ptr(q), ctypes.c_longlong(q.stride(0)), int(dim + rot), _ptr(w_uk), int(q.shape[0]), int(H), int(dim),
-                                              int(rot), int(rank), _ptr(out), _stream()), "latent_queries")
-    return out
-
-
-def latent_values(x: torch.Tensor, w_uv: torch.Tensor) -> torch.Tensor:
-    """``[tokens, heads * vdim]``: every head's ``rank`` numbers of x ``[tokens, heads * rank]`` times its ``w_uv`` ``[heads, vdim, rank]``."""
-    _need(x, "x", torch.bfloat16, 2)
-    _need(w_uv, "w_uv", torch.bfloat16, 3)
-    H, vdim, rank = w_uv.shape
-    if x.shape[1] != H * rank:
-        raise KernelError(f"latent_values: x {tuple(x.shape)} does not hold {H} heads of {rank}")
-    out = torch.empty((x.shape[0], H * vdim), dtype=x.dtype, device=x.device)
-    _check(_fn("latent", "bn_latent_values")(_ptr(x), _ptr(w_uv), int(x.shape[0]), int(H), int(rank), int(vdim), _ptr(out), _stream()),
-           "latent_values")
-    return out
-
-
 DECODE_CHUNK = 128  # positions per block of the decode attention; must equal DEC_CHUNK in attention_decode.cu
 
 

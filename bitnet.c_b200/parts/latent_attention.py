@@ -153,14 +153,10 @@ class LatentAttention(Mixer):
                 and (not in_latent_space or self.on_tcgen05 and sum(ctx.host_pos0) <= (self.SEEN_PER_NEW - 1) * ctx.n_tokens)):
             return self._per_head_keys(q, gate, ctx, kv, egate)
         # queries in the latent space: [W_uk^T q_plain | q_rot] per head
-        few = ops.latent_few(n, q, self.w_uk, self.w_uv)
-        if few:
-            ql = ops.latent_queries(q, self.w_uk, dr)
-        else:
-            q3 = q.unflatten(1, (H, d + dr))
-            ql = torch.empty((n, H, row), dtype=q.dtype, device=q.device)
-            torch.bmm(q3[:, :, :d].transpose(0, 1), self.w_uk.to(q.dtype), out=ql[:, :, :rank].transpose(0, 1))
-            ql[:, :, rank:] = q3[:, :, d:]
+        q3 = q.unflatten(1, (H, d + dr))
+        ql = torch.empty((n, H, row), dtype=q.dtype, device=q.device)
+        torch.bmm(q3[:, :, :d].transpose(0, 1), self.w_uk.to(q.dtype), out=ql[:, :, :rank].transpose(0, 1))
+        ql[:, :, rank:] = q3[:, :, d:]
         if ctx.diag is not None:
             ctx.tap("attn_q", lambda: ql.view(n, H * row))
         out = torch.empty((n, H * rank), dtype=dt, device=h.device)
@@ -176,12 +172,9 @@ class LatentAttention(Mixer):
                                   max_keys=min(ctx.max_len, s.window) if s.window > 0 else ctx.max_len, sink=self.sink)
         ctx.tap("attn_out", out)
         # back from the latent space: W_uv per head, heads side by side
-        if few:
-            o = ops.latent_values(out, self.w_uv)
-        else:
-            o = torch.empty((n, H, s.v_head_dim), dtype=dt, device=h.device)
-            torch.bmm(out.view(n, H, rank).transpose(0, 1), self.w_uv.to(dt).transpose(1, 2), out=o.transpose(0, 1))
-            o = o.view(n, H * s.v_head_dim)
+        o = torch.empty((n, H, s.v_head_dim), dtype=dt, device=h.device)
+        torch.bmm(out.view(n, H, rank).transpose(0, 1), self.w_uv.to(dt).transpose(1, 2), out=o.transpose(0, 1))
+        o = o.view(n, H * s.v_head_dim)
         if egate is not None:
             ops.gate_rows(o, egate)
         return ops.linear(o, self.w_o, out_dtype=torch.float32)
