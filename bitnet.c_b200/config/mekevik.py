@@ -131,7 +131,7 @@ class MekevikConfig:
         experts, top = _int(router, "experts", where + ".router"), _int(router, "top", where + ".router")
         if top > experts:
             raise ConfigError(f"config.json: {where}.router.top={top} exceeds its {experts} experts")
-        # read_once is the faster path with several tokens, but behind prompts of 1,100 tokens and more the two largest logits of this
+        # read_once sums on the tensor cores, which is faster with several tokens, but behind prompts of 1,100 tokens and more the two largest logits of this
         # design often lie 0.1 to 2 % of the logits' deviation apart: with sums in another order up to 13 % of a batch's tokens
         # became others
         return MoeSpec(width=self.width, n_experts=experts, top=top, expert_ff=_int(expert, "ff", where + ".expert"),
@@ -152,7 +152,9 @@ class MekevikConfig:
                                             # without a feed-forward the second norm's gain may or may not be in the file
                                             ffn_norm=norm if ffn is not None else RmsNormSpec(width=self.width, eps=eps, optional=True)))
             schedule.append(ScheduleEntry(block=i))
-        spec = ModelSpec(vocab_size=self.vocab, width=self.width, blocks=tuple(blocks), schedule=tuple(schedule),
+        # the products of few rows keep the order of their sums too: with others 2 to 10 % of the tokens behind prompts of 1,900 became others at
+        # widths 1024 and 2048
+        spec = ModelSpec(vocab_size=self.vocab, width=self.width, blocks=tuple(blocks), schedule=tuple(schedule), resident=False,
                          final_norm=norm, max_positions=self.max_positions, embedding_scale=float(d["embedding"]["scale"]),
                          head=LinearHeadSpec(scale=float(d["logit_scale"])))
         spec.validate()

@@ -540,6 +540,9 @@ class ModelSpec:
     stop_ids: Tuple[int, ...] = field(default_factory=tuple)
     head: Any = field(default_factory=LinearHeadSpec)  # a head spec; its part turns normed rows into logits
     streams: int = 1  # the residual holds so many streams of ``width`` side by side, which start alike (the embedding row)
+    # few rows times a small matrix: the kernel that holds the whole matrix on the chip (False: only the one for matrices of any size, whose
+    # sums have another order)
+    resident: bool = True
 
     def validate(self) -> None:
         if self.vocab_size <= 0 or self.width <= 0 or self.max_positions <= 0:

@@ -1209,9 +1209,9 @@ ACTIVATIONS = {"silu": ACT_SILU, "gelu_tanh": ACT_GELU_TANH}
 
 def linear_tc(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: bool = False,
               cluster: int = 0, sink: Optional[NormSink] = None, _checked: bool = False, act: int = 0,
-              bias: Optional[torch.Tensor] = None):
+              bias: Optional[torch.Tensor] = None, resident: bool = True):
     """x[M, K] . w[N, K]^T for M <= 64 in bfloat16 on tcgen05 tensor cores with TMA-fed operands (small matrices, where the number of
-    blocks is not given: linear_resident.cu).
+    blocks is not given and unless ``resident`` is False: linear_resident.cu).
     ``cluster`` blocks (1 to 8) share the inner dimension of each 128-row tile of w and add their
     parts up through distributed shared memory (0: chosen from the number of tiles).  ``x`` may be
     ``RowScaled``.  With ``sink`` the product is added to ``sink.residual`` in place and the result
@@ -1229,7 +1229,7 @@ def linear_tc(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swigl
         if w.shape[1] != K or M > TC_MAX_ROWS or K % 8 or (swiglu and N % 16) or not 0 <= cluster <= 8:
             raise KernelError(f"linear_tc: x {tuple(x.shape)}, w {tuple(w.shape)}, cluster {cluster} not supported")
     dev = x.device
-    resident = cluster == 0 and linear_resident_pays(M, N, K, n_sms(dev)) and (x.data_ptr() | w.data_ptr()) % 16 == 0
+    resident = resident and cluster == 0 and linear_resident_pays(M, N, K, n_sms(dev)) and (x.data_ptr() | w.data_ptr()) % 16 == 0
     fn = _fn("linear_resident", "bn_linear_resident") if resident else _fn("linear_tc", "bn_linear_tc_ex")
     if scaled is not None:
         ss_rows = scaled.ss
@@ -1417,7 +1417,8 @@ def _own_gemm_fits(x, w: torch.Tensor, swiglu: bool, out_dtype, kind: str) -> bo
 
 
 def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: bool = False,
-           partial_sums: bool = False, sink: Optional[NormSink] = None, act: int = 0, bias: Optional[torch.Tensor] = None):
+           partial_sums: bool = False, sink: Optional[NormSink] = None, act: int = 0, bias: Optional[torch.Tensor] = None,
+           resident: bool = True):
     """x[M, K] . w[N, K]^T.  A weight kept in float32 makes the product float32 whatever x is.
 
     ``x`` may be ``RowScaled`` (the output of a norm that a product's epilogue prepared).  With
@@ -1429,7 +1430,8 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: 
     act(gate) * up, ``[M, N / 2]`` (``act``: ACT_SILU or ACT_GELU_TANH).  ``partial_sums``: return the float32 partial sums
     ``[parts, M, N]`` of a product that split its inner dimension instead of their sum
     (``add_rmsnorm`` can add them up); by default the product sums them itself.  ``bias``: float32 ``[N]``, added to a
-    plain product's rows before they are rounded; ``act`` ACT_RELU2 then takes the square of their positive part.
+    plain product's rows before they are rounded; ``act`` ACT_RELU2 then takes the square of their positive part.  ``resident`` False:
+    few rows times a small matrix keep to the kernel for matrices of any size.
     """
     _need(w, "w", dims=2)
     if x.shape[1] != w.shape[1] or len(x.shape) != 2:
@@ -1449,16 +1451,16 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: 
     fast = streams and x.dtype == torch.bfloat16
     if sink is not None:
         if fast and USE_FUSED_NORM and not swiglu and tuple(sink.residual.shape) == (M, N):
-            return linear_tc(x, w, sink=sink, _checked=True)
+            return linear_tc(x, w, sink=sink, _checked=True, resident=resident)
         if (not swiglu and not isinstance(x, RowScaled) and tuple(sink.residual.shape) == (M, N)
                 and _own_gemm_fits(x, w, False, None, "sink") and not partial_sums):
             return gemm_tc(x, w, sink=sink)
-        delta = linear(x, w, out_dtype=out_dtype, swiglu=swiglu, act=act)
+        delta = linear(x, w, out_dtype=out_dtype, swiglu=swiglu, act=act, resident=resident)
         normed = torch.empty((M, sink.residual.shape[1]), dtype=delta.dtype, device=delta.device)
         return add_rmsnorm(sink.residual, delta, sink.weight, sink.eps, normed)
     if isinstance(x, RowScaled):
         if fast:
-            return linear_tc(x, w, out_dtype=out_dtype or x.dtype, swiglu=swiglu, _checked=True, act=act, bias=bias)
+            return linear_tc(x, w, out_dtype=out_dtype or x.dtype, swiglu=swiglu, _checked=True, act=act, bias=bias, resident=resident)
         if _own_gemm_fits(x.x, w, swiglu, out_dtype, "scaled") and not partial_sums and bias is None:
             return gemm_tc(x, w, out_dtype=out_dtype or x.dtype, swiglu=swiglu, act=act)
         x = x.dense()
@@ -1467,7 +1469,7 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: 
     if x.dtype != w.dtype:
         x = x.to(w.dtype)
     if streams:
-        return linear_tc(x, w, out_dtype=out_dtype, swiglu=swiglu, _checked=True, act=act, bias=bias)
+        return linear_tc(x, w, out_dtype=out_dtype, swiglu=swiglu, _checked=True, act=act, bias=bias, resident=resident)
     if _own_gemm_fits(x, w, swiglu, out_dtype, "swiglu" if swiglu or squared else "plain") and not partial_sums and bias is None:
         return gemm_tc(x, w, out_dtype=out_dtype, swiglu=swiglu, act=act)
     if small:

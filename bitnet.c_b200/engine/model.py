@@ -53,7 +53,7 @@ class Model:
         self.spec, self.arch, self.config = spec, arch, config
         self.dtype = resolve_dtype(dtype)
         self.device = torch.device(device) if device is not None else None
-        b = BuildContext(dtype=self.dtype, device=self.device)
+        b = BuildContext(dtype=self.dtype, device=self.device, resident=getattr(spec, "resident", True))
         self.blocks = [build_part("block", bs, b) for bs in spec.blocks]
         self.final_norm = build_part("norm", spec.final_norm, b)
         en = getattr(spec, "embedding_norm", None)

@@ -57,6 +57,7 @@ class ParamSpec:
 class BuildContext:
     dtype: torch.dtype  # compute type: torch.bfloat16 or torch.float32
     device: Any
+    resident: bool = True  # products of small matrices may take linear_resident.cu (False: the sums of linear_tc.cu throughout)
 
 
 @dataclass(frozen=True)

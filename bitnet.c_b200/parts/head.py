@@ -19,7 +19,7 @@ class LinearHead(Head):
     kernels = ("linear", "linear_mma", "linear_tc", "gemm_tc", "act")
 
     def forward(self, h, table, ctx):
-        logits = ops.linear(h, table, out_dtype=torch.float32)
+        logits = ops.linear(h, table, out_dtype=torch.float32, resident=self.build.resident)
         s = self.spec
         if s.scale != 1.0 or s.softcap != 0.0:
             ops.scale_softcap(logits, s.scale, s.softcap)

@@ -47,9 +47,9 @@ class GatedMlp(FeedForward):
         self.w_down = down
 
     def forward(self, h, ctx, sink=None):
-        act = ops.linear(h, self.w_gate_up, out_dtype=self.build.dtype, swiglu=True, act=self.act)
+        act = ops.linear(h, self.w_gate_up, out_dtype=self.build.dtype, swiglu=True, act=self.act, resident=self.build.resident)
         out_dtype = torch.float32 if getattr(self.spec, "wide_output", False) else self.build.dtype
-        return ops.linear(act, self.w_down, out_dtype=out_dtype, sink=sink)
+        return ops.linear(act, self.w_down, out_dtype=out_dtype, sink=sink, resident=self.build.resident)
 
 
 @register_ffn("limited_mlp")
@@ -80,10 +80,10 @@ class LimitedMlp(FeedForward):
 
     def forward(self, h, ctx):
         s = self.spec
-        gu = ops.linear(h, self.w_gate_up, out_dtype=self.build.dtype)
+        gu = ops.linear(h, self.w_gate_up, out_dtype=self.build.dtype, resident=self.build.resident)
         act = torch.empty((h.shape[0], self.inter), dtype=gu.dtype, device=gu.device)
         ops.glu_limited(gu, act, s.limit, s.slope)
-        return ops.linear(act, self.w_down, out_dtype=torch.float32)
+        return ops.linear(act, self.w_down, out_dtype=torch.float32, resident=self.build.resident)
 
 
 @register_ffn("poly_mlp")
@@ -110,6 +110,6 @@ class PolyMlp(FeedForward):
 
     def forward(self, h, ctx):
         s = self.spec
-        z = ops.linear(h, self.w_up, out_dtype=torch.float32)
+        z = ops.linear(h, self.w_up, out_dtype=torch.float32, resident=self.build.resident)
         act = ops.poly_norm(z, self.coef, s.eps, self.build.dtype, length=s.intermediate)
-        return ops.linear(act, self.w_down, out_dtype=torch.float32)
+        return ops.linear(act, self.w_down, out_dtype=torch.float32, resident=self.build.resident)

@@ -122,8 +122,8 @@ class Moe(FeedForward):
 
     def _expert(self, x, w_gate_up, w_down, limit, out_dtype):
         if not self.gated:
-            return ops.linear(ops.linear(x, w_gate_up, out_dtype=self.build.dtype, act=ops.ACT_RELU2), w_down, out_dtype=out_dtype)
-        return ops.linear(self._activate(ops.linear(x, w_gate_up, out_dtype=self.build.dtype), limit), w_down, out_dtype=out_dtype)
+            return ops.linear(ops.linear(x, w_gate_up, out_dtype=self.build.dtype, act=ops.ACT_RELU2, resident=self.build.resident), w_down, out_dtype=out_dtype, resident=self.build.resident)
+        return ops.linear(self._activate(ops.linear(x, w_gate_up, out_dtype=self.build.dtype, resident=self.build.resident), limit), w_down, out_dtype=out_dtype, resident=self.build.resident)
 
     def forward(self, h, ctx):
         s = self.spec
@@ -138,7 +138,7 @@ class Moe(FeedForward):
             ids, weights = ctx.memo[key]
         else:
             # the logits are a product of the library's own for few rows; only then the choice is made
-            logits = ops.linear(h, self.w_router, out_dtype=torch.float32)
+            logits = ops.linear(h, self.w_router, out_dtype=torch.float32, resident=self.build.resident)
             ids, weights, *gate = ops.moe_choose(
                 logits, self.outputs, s.top, s.renormalise, softmax=self.softmax, weight_scale=s.weight_scale, sum_eps=s.renormalise_eps,
                 bias=self.b_router, correction=self.correction, groups=s.groups, keep=s.keep_groups, gate=s.shared_gate)

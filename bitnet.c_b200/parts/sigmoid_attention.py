@@ -118,7 +118,7 @@ class SigmoidAttention(Mixer):
     def forward(self, h, ctx, kv, state):
         s = self.spec
         n = h.shape[0]
-        proj = ops.linear(h, self.w_in, out_dtype=self.build.dtype)
+        proj = ops.linear(h, self.w_in, out_dtype=self.build.dtype, resident=self.build.resident)
         key = ("value_mix_source", s.value_group)
         other = None
         if s.value_mix == "blend":
@@ -145,18 +145,18 @@ class SigmoidAttention(Mixer):
                                           kv.page_table, kv.k, kv.v, rel=self.rel, mix=self.mix, gate=gate, gate_stride=self.row,
                                           splits=splits)
             ctx.tap("attn_out", out)
-            return ops.linear(out, self.w_o, out_dtype=torch.float32)
+            return ops.linear(out, self.w_o, out_dtype=torch.float32, resident=self.build.resident)
         if (self.tiled_fits and not ctx.decode and ctx.tile_seq is not None and ctx.max_new >= self.TILED_MIN_TOKENS):
             ops.sigmoid_attention_prefill(proj, self.row, out, s.n_heads, s.n_kv_heads, s.head_dim, s.scale, s.window, ctx.tile_seq,
                                           ctx.tile_row0, ctx.seq_start, ctx.seq_pos0, ctx.slots, kv.page_table, kv.k, kv.v,
                                           rel=self.rel, mix=self.mix, gate=gate, gate_stride=self.row)
             ctx.tap("attn_out", out)
-            return ops.linear(out, self.w_o, out_dtype=torch.float32)
+            return ops.linear(out, self.w_o, out_dtype=torch.float32, resident=self.build.resident)
         ops.sigmoid_attention(proj, self.row, out, n, s.n_heads, s.n_kv_heads, s.head_dim, s.scale, s.window, ctx.tok_seq,
                               ctx.tok_pos, ctx.slots, kv.page_table, kv.k, kv.v, rel=self.rel, mix=self.mix, gate=gate,
                               gate_stride=self.row, max_keys=min(ctx.max_len, s.window) if s.window > 0 else ctx.max_len)
         ctx.tap("attn_out", out)
-        return ops.linear(out, self.w_o, out_dtype=torch.float32)
+        return ops.linear(out, self.w_o, out_dtype=torch.float32, resident=self.build.resident)
 
 
 def bias_buckets(n_buckets: int, max_distance: int) -> torch.Tensor:
