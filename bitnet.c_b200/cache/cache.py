@@ -293,6 +293,13 @@ class Cache:
                       head_dim=g.request.head_dim, window=g.request.window, owner=owner,
                       v_head_dim=g.request.v_head_dim)
 
+    def plane(self, entry: int):
+        """Addresses of the entry's own keys and values, their page table and number of pages (for a launch; kept by nobody)."""
+        gi, plane = self._plane[entry]
+        g = self.groups[gi]
+        return (g.k.data_ptr() + plane * g.k.stride(0) * g.k.element_size(), g.v.data_ptr() + plane * g.v.stride(0) * g.v.element_size(),
+                g.page_table, g.k.shape[1])
+
     def state(self, entry: int):
         """The entry's state tensor, or a dict of them by name if it keeps several, or None."""
         named = self._named.get(entry)

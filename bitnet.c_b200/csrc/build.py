@@ -42,6 +42,7 @@ SOURCES: Dict[str, str] = {
     "linear": "linear.cu",
     "linear_resident": "linear_resident.cu",
     "linear_split": "linear_split.cu",
+    "few_layers": "few_layers.cu",
     "linear_mma": "linear_mma.cu",
     "linear_tc": "linear_tc.cu",
     "gemm_tc": "gemm_tc.cu",

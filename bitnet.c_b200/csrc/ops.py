@@ -1528,6 +1528,14 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: 
     return out
 
 
+def few_layers(step, launches: int) -> None:
+    """All layers of a Llama-style model for few tokens (few_layers.cu): ``step`` is the native structure that engine/few_layers.py fills in,
+    ``launches`` how many kernels it comes to."""
+    global LAUNCHES
+    _check(_fn("few_layers", "bn_few_layers")(ctypes.byref(step), _stream()), "few_layers")
+    LAUNCHES += launches - 1
+
+
 def linear_split_pays(M: int, N: int, K: int) -> bool:
     """Whether a float32 product goes to ``linear_split.cu``: with many outputs, or wide matrices and not too few rows.  The library product's
     time over that kernel's: 520 to 2,048 rows 1.3 to 3.7 with a million outputs and more (1.05 to 1.1 right at the line), 0.5 to 0.9 with half as

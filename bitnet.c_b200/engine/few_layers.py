@@ -1,0 +1,140 @@
+"""All layers of a Llama-style model for few tokens in bfloat16, launched from one native call (csrc/few_layers.cu)."""
+from __future__ import annotations
+
+import ctypes
+from ctypes import c_float, c_int, c_void_p
+from typing import Optional
+
+import torch
+
+from ..csrc import build, ops
+from ..parts.attention import Attention
+from ..parts.base import Normed
+from ..parts.block import PreNormBlock
+from ..parts.mlp import GatedMlp
+from ..parts.norm import RmsNorm
+from ..parts.position import Rotary
+
+
+class _Layer(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("w_qkv", "w_o", "w_gate_up", "w_down", "gain_ffn", "gain_next", "k_cache", "v_cache", "page_table")] + \
+               [(n, c_int) for n in ("gain_ffn_dtype", "gain_next_dtype", "pt_stride", "n_cache_pages")] + [("eps_ffn", c_float), ("eps_next", c_float)]
+
+
+class _Step(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in (
+        "layers", "linear_tc", "resident", "rope", "decode", "decode_items", "prefill", "x", "h", "qkv", "attn", "act", "mid", "next", "delta", "mid_ss",
+        "next_ss", "tok_pos", "tok_seq", "slots", "tile_seq", "tile_row0", "seq_start", "seq_pos0", "items", "part_o", "part_ml", "tickets", "status")] + \
+        [(n, c_int) for n in (
+            "n_layers", "M", "n_seqs", "width", "inter", "n_heads", "n_kv_heads", "head_dim", "act_code", "rotary_dims", "window", "decoding", "n_splits",
+            "pages_per_block", "n_tickets", "n_items", "item_group", "n_tiles", "res_qkv", "res_o", "res_gate_up", "res_down", "cluster_o",
+            "cluster_down")] + [("scale", c_float), ("theta_scale", c_float)]
+
+
+class FewLayers:
+    """The layers of ``model`` if they are all alike and of the kinds that ``bn_few_layers`` knows (``FewLayers.of``)."""
+
+    @staticmethod
+    def of(model) -> Optional["FewLayers"]:
+        """Called when all parameters are bound; None for every other model."""
+        runs = [model.blocks[e.block] for e in model.spec.schedule]
+        if model.dtype != torch.bfloat16 or model.embedding_norm is not None or getattr(model.spec, "streams", 1) != 1 or type(model.final_norm) is not RmsNorm:
+            return None
+        if any(e.cache_of is not None for e in model.spec.schedule):
+            return None
+        for b in runs:
+            if not (type(b) is PreNormBlock and type(b.mixer) is Attention and type(b.ffn) is GatedMlp and type(b.mixer_norm) is RmsNorm
+                    and type(b.ffn_norm) is RmsNorm and type(b.mixer.position) is Rotary and b.build.resident
+                    and not getattr(b.ffn.spec, "wide_output", False)):
+                return None
+            a, f, first = b.mixer, b.ffn, runs[0]
+            weights = (a.w_qkv, a.w_o, f.w_gate_up, f.w_down)
+            if [w.shape for w in weights] != [w.shape for w in (first.mixer.w_qkv, first.mixer.w_o, first.ffn.w_gate_up, first.ffn.w_down)]:
+                return None
+            if any(w.dtype != torch.bfloat16 or not w.is_cuda or not w.is_contiguous() or w.data_ptr() % 16 or w.shape[1] % 8 for w in weights):
+                return None
+            if a.spec != first.mixer.spec or f.act != first.ffn.act or a.spec.head_dim > 128 or a.w_qkv.shape[0] % 8:
+                return None
+            if any(n.weight.dtype not in ops._DT or not n.weight.is_contiguous() for n in (b.mixer_norm, b.ffn_norm, model.final_norm)):
+                return None
+        return FewLayers(model, runs)
+
+    def __init__(self, model, runs):
+        self.model, self.runs = model, runs
+        a, f = runs[0].mixer, runs[0].ffn
+        self.shapes = [tuple(w.shape) for w in (a.w_qkv, a.w_o, f.w_gate_up, f.w_down)]
+        self.entries = None
+
+    def _entry_points(self):
+        if self.entries is None:
+            names = (("linear_tc", "bn_linear_tc_ex"), ("linear_resident", "bn_linear_resident"), ("rope", "bn_rope_append"),
+                     ("attention_decode_tc", "bn_attention_decode_tc"), ("attention_decode_tc", "bn_attention_decode_tc_items"),
+                     ("attention_prefill_tc", "bn_attention_prefill_tc"))
+            self.entries = [ctypes.cast(getattr(build.library(lib), name), c_void_p).value for lib, name in names]
+        return self.entries
+
+    def takes(self, ctx) -> bool:
+        """Whether a step of these tokens goes this way; every switch that sends a part elsewhere sends the step there too."""
+        return (ctx.n_tokens <= ops.TC_MAX_ROWS and ctx.diag is None and ops.PROFILE is None and ops.USE_TCGEN05 and ops.USE_FUSED_NORM
+                and not ops._FORCE_SPLITS and (ctx.decode or (ctx.wide_tile_seq is not None and ops.USE_TCGEN05_ATTENTION)))
+
+    def run(self, x, h, cache, ctx, last_norm):
+        """The layers on the residual x [T, width] from the first one's normed rows h; ``last_norm``: the norm behind the last
+        layer, if that layer's product is to prepare it.  Returns what is pending (as the last block would)."""
+        spec, T, width, dev = self.runs[0].mixer.spec, x.shape[0], self.shapes[1][0], x.device
+        (n_qkv, _), (_, q_dim), (n_gu, _), (_, inter) = self.shapes
+        s = _Step()
+        s.linear_tc, s.resident, s.rope, s.decode, s.decode_items, s.prefill = self._entry_points()
+        sms = ops.n_sms(dev)
+        s.res_qkv, s.res_o, s.res_gate_up, s.res_down = (int(ops.linear_resident_pays(T, n, k, sms)) for n, k in self.shapes)
+        s.cluster_o, s.cluster_down = ops._auto_cluster(width, q_dim), ops._auto_cluster(width, inter)
+        tiles = (width + 127) // 128
+        mid_parts = (width + 15) // 16 if s.res_o else tiles * s.cluster_o
+        next_parts = (width + 15) // 16 if s.res_down else tiles * s.cluster_down
+        part_o = part_ml = 0
+        if ctx.decode:
+            if ctx.decode_items is not None:
+                s.items, s.n_items, s.item_group = ctx.decode_items.data_ptr(), ctx.decode_items.shape[0], ctx.decode_item_group
+                splits = ctx.decode_item_group
+            else:
+                pages = max(1, (ctx.max_len + ops.PAGE - 1) // ops.PAGE)
+                want = ops.decode_splits(pages, T * spec.n_kv_heads * ((spec.n_heads // spec.n_kv_heads + 15) // 16))
+                s.pages_per_block = (pages + want - 1) // want
+                splits = s.n_splits = (pages + s.pages_per_block - 1) // s.pages_per_block
+            part_o, part_ml = T * spec.n_heads * splits * spec.head_dim * 4, T * spec.n_heads * splits * 8
+            counters = ops._split_scratch(dev)[1]
+            s.tickets, s.n_tickets, s.decoding = counters.data_ptr(), counters.numel(), 1
+        else:
+            s.tok_seq, s.tile_seq, s.tile_row0 = ctx.tok_seq.data_ptr(), ctx.wide_tile_seq.data_ptr(), ctx.wide_tile_row0.data_ptr()
+            s.seq_start, s.seq_pos0, s.n_tiles = ctx.seq_start.data_ptr(), ctx.seq_pos0.data_ptr(), ctx.wide_tile_seq.shape[0]
+        # everything between the kernels from one allocation, pieces on 256-byte borders
+        sizes = {"qkv": 2 * T * n_qkv, "attn": 2 * T * q_dim, "act": 2 * T * inter, "mid": 2 * T * width, "mid_ss": 4 * T * mid_parts, "part_o": part_o,
+                 "part_ml": part_ml}
+        room = torch.empty(sum((n + 255) & ~255 for n in sizes.values()), dtype=torch.uint8, device=dev)
+        at = room.data_ptr()
+        for name, n in sizes.items():
+            setattr(s, name, at)
+            at += (n + 255) & ~255
+        nxt = torch.empty((T, width), dtype=torch.bfloat16, device=dev)  # rows for the next layer, or the last product itself
+        ss = torch.empty((next_parts, T), dtype=torch.float32, device=dev)
+        delta = torch.empty((T, width), dtype=torch.bfloat16, device=dev) if last_norm is None else None
+        layers = (_Layer * len(self.runs))()
+        for i, (l, b) in enumerate(zip(layers, self.runs)):
+            a, f = b.mixer, b.ffn
+            l.w_qkv, l.w_o, l.w_gate_up, l.w_down = a.w_qkv.data_ptr(), a.w_o.data_ptr(), f.w_gate_up.data_ptr(), f.w_down.data_ptr()
+            l.gain_ffn, l.gain_ffn_dtype, l.eps_ffn = b.ffn_norm.weight.data_ptr(), ops._DT[b.ffn_norm.weight.dtype], b.ffn_norm.spec.eps
+            norm = self.runs[i + 1].mixer_norm if i + 1 < len(self.runs) else last_norm
+            if norm is not None:
+                l.gain_next, l.gain_next_dtype, l.eps_next = norm.weight.data_ptr(), ops._DT[norm.weight.dtype], norm.spec.eps
+            l.k_cache, l.v_cache, table, l.n_cache_pages = cache.plane(i)
+            l.page_table, l.pt_stride = table.data_ptr(), table.shape[1]
+        s.layers = ctypes.addressof(layers)
+        s.x, s.h, s.next, s.next_ss, s.delta = x.data_ptr(), h.data_ptr(), nxt.data_ptr(), ss.data_ptr(), delta.data_ptr() if delta is not None else None
+        s.tok_pos, s.slots, s.status = ctx.tok_pos.data_ptr(), ctx.slots.data_ptr(), ops.tc_status(dev).data_ptr()
+        s.n_layers, s.M, s.n_seqs, s.width, s.inter, s.n_heads, s.n_kv_heads = len(self.runs), T, ctx.n_seqs, width, inter, spec.n_heads, spec.n_kv_heads
+        s.head_dim, s.act_code, s.window, s.scale = spec.head_dim, self.runs[0].ffn.act, spec.window, spec.softmax_scale
+        s.rotary_dims, s.theta_scale = self.runs[0].mixer.position.rotary_params()
+        ops.few_layers(s, len(self.runs) * (5 if ctx.decode else 6))
+        if delta is not None:
+            return delta
+        return Normed(ops.RowScaled(nxt, ss, width, last_norm.spec.eps))

@@ -21,6 +21,7 @@ from ..csrc import ops
 from ..parts import BuildContext, ParamSpec, Part, build_part
 from ..parts.base import Cast, Normed, StreamDelta
 from .batch import SeqStep, StepContext, pack_step
+from .few_layers import FewLayers
 
 _DTYPES = {"bfloat16": torch.bfloat16, "bf16": torch.bfloat16, "float32": torch.float32, "fp32": torch.float32,
            torch.bfloat16: torch.bfloat16, torch.float32: torch.float32}
@@ -66,6 +67,7 @@ class Model:
         # them need not look again
         self._passes = itertools.count(1)
         self.last_pass = 0
+        self.few_layers: Optional[FewLayers] = None  # the layers as one native call, for models whose layers it knows
         self.diagnostics = None  # engine/diagnostics.py: tensor dumps, top logits, kernel timers
         self._owners: Dict[str, tuple] = {}
         for i, blk in enumerate(self.blocks):
@@ -141,6 +143,7 @@ class Model:
         self.embedding = tensors["embedding.table"]
         self.head = tensors["head.weight"] if not self.spec.tie_embeddings else self.embedding
         self._bad_token = torch.zeros(1, dtype=torch.int32, device=self.device)
+        self.few_layers = FewLayers.of(self)
         return self
 
     @classmethod
@@ -279,7 +282,11 @@ class Model:
         diag = ctx.diag = self.diagnostics
         ctx.layer = -1
         ctx.tap("inp", x)
-        for i, e in enumerate(sched):
+        native = self.few_layers is not None and self.few_layers.takes(ctx)
+        if native:
+            h = self.blocks[sched[0].block].mixer_norm.add_norm(x, None, ctx)
+            pending = self.few_layers.run(x, h, cache, ctx, self.final_norm if ctx.rows is not None and ctx.rows_all else None)
+        for i, e in enumerate(sched if not native else ()):
             blk = self.blocks[e.block]
             if isinstance(pending, Cast) and not getattr(blk, "accepts_cast", False):
                 pending = None  # nothing is left to add; this block reads the float32 rows itself

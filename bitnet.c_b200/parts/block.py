@@ -21,6 +21,7 @@ class PreNormBlock(Block):
 
     graph_safe = True  # as far as its parts are
     accepts_normed = True
+    kernels = ("few_layers",)
 
     def entry_norm(self):
         return self.mixer_norm

@@ -1,0 +1,55 @@
+"""A model's layers launched from one native call (csrc/few_layers.cu) against the same kernels launched part by part: the same bits."""
+import pytest
+import torch
+
+import bitnet_c_b200 as bn
+from bitnet_c_b200.engine import Model
+
+pytestmark = pytest.mark.gpu
+
+
+def _config(width, heads, kv, dim, ff, layers, tied):
+    return {"architectures": ["LlamaForCausalLM"], "model_type": "llama", "hidden_size": width, "intermediate_size": ff, "num_hidden_layers": layers,
+            "num_attention_heads": heads, "num_key_value_heads": kv, "head_dim": dim, "vocab_size": 512, "max_position_embeddings": 4096,
+            "rope_theta": 10000.0, "rms_norm_eps": 1e-5, "tie_word_embeddings": tied, "hidden_act": "silu"}
+
+
+def _logits(model, prompts, wants, steps):
+    room = sum(-(-(len(p) + steps + 1) // 64) * 64 for p in prompts)
+    cache = model.new_cache(max_tokens=room, max_seqs=len(prompts))
+    slots = [cache.open() for _ in prompts]
+    out = [model.step(cache, [bn.SeqStep(s, p, w) for s, p, w in zip(slots, prompts, wants)])]
+    for i in range(steps):
+        out.append(model.step(cache, [bn.SeqStep(s, [(7 * i + s) % 512], [0]) for s in slots]))
+    return out
+
+
+@pytest.mark.parametrize("size", [(64, 4, 2, 16, 176, 2, False), (2048, 32, 8, 64, 8192, 2, True), (512, 4, 4, 128, 1536, 3, False)])
+@pytest.mark.parametrize("lengths", [[1], [12], [64], [3, 1, 20], [1] * 17, [5] * 12])
+def test_same_bits(size, lengths):
+    model = Model.from_random(_config(*size), seed=3, matrix_std=size[0] ** -0.5)
+    assert model.few_layers is not None
+    g = torch.Generator().manual_seed(len(lengths))
+    prompts = [torch.randint(0, 512, (n,), generator=g).tolist() for n in lengths]
+    for wants in ([[n - 1] for n in lengths], [list(range(n)) for n in lengths]):  # the last rows, or all of them (the final norm is then fused)
+        native = _logits(model, prompts, wants, 3)
+        few, model.few_layers = model.few_layers, None
+        parts = _logits(model, prompts, wants, 3)
+        model.few_layers = few
+        assert all(torch.equal(a, b) for a, b in zip(native, parts))
+
+
+def test_what_stays_with_the_parts():
+    cfg = _config(64, 4, 2, 16, 176, 2, False)
+    assert Model.from_random(cfg, dtype="float32").few_layers is None
+    wide = Model.from_random(dict(cfg, head_dim=144), seed=1)  # no tcgen05 attention for prompts
+    assert wide.few_layers is None
+    model = Model.from_random(cfg, seed=1)
+    cache = model.new_cache(max_tokens=128, max_seqs=1)
+    slot = cache.open()
+    ran = []
+    run, model.few_layers.run = model.few_layers.run, lambda *a: ran.append(a) or run(*a)
+    model.step(cache, [bn.SeqStep(slot, list(range(65)), [64])])  # more rows than the products of few rows take
+    assert not ran
+    model.step(cache, [bn.SeqStep(slot, [1], [0])])
+    assert len(ran) == 1
