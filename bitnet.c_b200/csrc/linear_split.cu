@@ -8,7 +8,7 @@
 // (520 rows, 4096 x 4096: 2.2e-7 against 1.1e-6 of the result's norm; 1024 x 14336: 3.9e-7 against 2.2e-6).
 //
 // The float32 units reach 72 TFLOP/s at most, the library's product 54; six bfloat16 products per float32 product are 230 TFLOP/s at the tensor
-// cores' rate.  520 rows: 28672 x 4096 705 us (library 2291), 6144 x 4096 149 (541), 4096 x 4096 133 (324), 4096 x 14336 424 (1126).
+// cores' rate.  520 rows: 28672 x 4096 634 us (library 2288), 6144 x 4096 134 (540), 4096 x 4096 117 (324), 4096 x 14336 375 (1125).
 //
 // A tile is 128 rows of W times up to 192 rows of x: D[128 rows of W, NT rows of x], so that few and odd numbers of rows of x waste
 // little (NT is a multiple of 16, chosen so that the tiles fill the SMs).  x is split once, by a kernel of its own, into three
@@ -19,15 +19,20 @@
 // A persistent block of 16 warps per SM:
 //   warp 0      requests float32 tiles of W (128 rows x 32 numbers)
 //   warp 1      requests tiles of x's three planes (NT rows x 32 numbers each, 64-byte swizzle)
-//   warp 2      allocates tensor memory; one thread issues twelve MMAs per 32 numbers, into one of two accumulators
+//   warp 2      allocates tensor memory; issues twelve MMAs per 32 numbers, into one of two accumulators
 //   warps 4-7   split W: shared memory -> registers -> tensor memory, two buffers in turn
 //   warps 8-15  add the accumulators up in registers (a row of W each thread, two warps share a row's columns) and store
 //
 // Numbers that are not finite, or round to infinity in bfloat16, do not split.  Rows that have one are marked (of x by the kernel that
 // splits it, of W by the warps that do); outputs of marked rows are computed again in plain float32.
 //
-// Every wait on an mbarrier is bounded in time; a wait that gives up records code 8 in *status, every role leaves its loops, and the
-// block frees its tensor memory and returns.
+// The twelve MMAs of 32 numbers take 1,060 cycles for 176 rows of x; a wait for an mbarrier costs its role some 200, even if it is over.  So
+// the whole of warp 2 walks its loop, with descriptors in uniform registers, and one elected lane issues (as one thread's work a step took 1,700
+// cycles: 790 to issue, 900 for three waits); the splitting warps wait for the MMAs only, and fetch the next numbers while the operands they
+// stored are on their way (before, 1,530 to 1,700 cycles a step: 28672 x 4096 705 us, 4096 x 4096 133).
+//
+// Every wait on an mbarrier is bounded in time; a wait that gives up records code 8 in *status, every role leaves its loops (the others
+// when a wait of theirs gives up in turn), and the block frees its tensor memory and returns.
 //
 // Reference: y = W x with float32 accumulation (src/quant/f32_scalar.c:4-32); the reference's CUDA prefill calls cublasSgemm
 // (src/gpu_cuda.cu:11788-11879).
@@ -159,11 +164,9 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   const int tiles = a.m_tiles * a.n_tiles;
   // tile t: rows of W from (t / m_tiles) * 128, rows of x from (t % m_tiles) * nt (the blocks that run at once share rows of W)
   auto wait = [&](unsigned bar, unsigned parity) {
-    if (!mbar_wait(bar, parity & 1u, a.status, LS_ERR_WAIT) || *failed) {
-      *failed = 1;
-      return false;
-    }
-    return true;
+    if (mbar_wait(bar, parity & 1u, a.status, LS_ERR_WAIT)) return true;
+    *failed = 1;  // (the other roles find out when a wait of theirs gives up)
+    return false;
   };
 
   if (warp == 0) {
@@ -193,44 +196,57 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
     }
   } else if (warp == 2) {
-    if (lane == 0) {
-      // D float32, A and B bfloat16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(a.nt >> 3) << 17) | ((LS_BM >> 4) << 24);
-      int s = 0, round = 0, it = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x)
-        for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
-          const int b = it & 1, use = it >> 1;
-          if (!(ok = wait(a_full + 8 * b, use) && (use == 0 || wait(acc_free + 8 * b, use - 1)) && wait(x_full + 8 * s, round))) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const unsigned acc = tmem + b * LS_ACC_COLS, wa = tmem_a + b * LS_A_COLS, xs = smem_u32(x_ring + s * x_bytes);
+    // the whole warp walks the loop, so that addresses and descriptors are warp-uniform values
+    const bool issuer = elect_one();
+    const unsigned tbase = __shfl_sync(0xffffffffu, tmem, 0);
+    // D float32, A and B bfloat16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24
+    const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(a.nt >> 3) << 17) | ((LS_BM >> 4) << 24);
+    const unsigned long long desc0 = ls_desc(smem_u32(x_ring));
+    int s = 0, round = 0, it = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x)
+      for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
+        const int b = it & 1, use = it >> 1;
+        // what is ready first is waited for first; W's operands are the last to come
+        ok = __all_sync(0xffffffffu, (use == 0 || wait(acc_free + 8 * b, use - 1)) && wait(x_full + 8 * s, round) && wait(a_full + 8 * b, use));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (issuer) {
+          const unsigned acc = tbase + b * LS_ACC_COLS, wa = tbase + 2 * LS_ACC_COLS + b * LS_A_COLS;
+          const unsigned long long xd = desc0 + ((s * x_bytes) >> 4);
+          const unsigned plane = plane_bytes >> 4;
           // planes of W and x (0 high, 1 middle, 2 low), the smallest products first
           constexpr int PW[6] = {2, 1, 0, 1, 0, 0}, PX[6] = {0, 1, 2, 0, 1, 0};
 #pragma unroll
           for (int i = 0; i < 6; ++i)
 #pragma unroll
             for (int kk = 0; kk < LS_BK / 16; ++kk)
-              umma_mma_ts(acc, wa + PW[i] * 16 + kk * 8, ls_desc(xs + PX[i] * plane_bytes + kk * 32), idesc, (i | kk) ? 1u : 0u);
+              umma_mma_ts(acc, wa + PW[i] * 16 + kk * 8, xd + PX[i] * plane + kk * 2, idesc, (i | kk) ? 1u : 0u);
           umma_commit(x_free + 8 * s);   // arrives when these MMAs have read the stage
           umma_commit(acc_full + 8 * b);  // and W's operands, and the sums are complete
-          if (++s == a.x_stages) { s = 0; ++round; }
         }
-    }
+        __syncwarp();
+        if (++s == a.x_stages) { s = 0; ++round; }
+      }
   } else if (warp >= 4 && warp < 8) {
     const int row = (warp & 3) * 32 + lane;
     const unsigned to0 = tmem_a + ((unsigned)((warp & 3) * 32) << 16);
     int s = 0, round = 0, it = 0;
     bool ok = true;
+    float4 v[8];
+    // the next 32 numbers of the thread's row; the next stage's slot is free again
+    auto take = [&]() {
+      ok = __all_sync(0xffffffffu, wait(w_full + 8 * s, round));
+      if (!ok) return;
+      const unsigned char* from = base + s * LS_W_BYTES + row * 128;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v[c] = *reinterpret_cast<const float4*>(from + ((c ^ (row & 7)) << 4));
+    };
+    if ((int)blockIdx.x < tiles) take();
     for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
       float none = 0.f;
       for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
         const int b = it & 1, use = it >> 1;
-        ok = __all_sync(0xffffffffu, wait(w_full + 8 * s, round));
-        if (!ok) break;
-        const unsigned char* from = base + s * LS_W_BYTES + row * 128;
-        float4 v[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) v[c] = *reinterpret_cast<const float4*>(from + ((c ^ (row & 7)) << 4));
         unsigned high[16], mid[16], low[16];
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -241,6 +257,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(w_free + 8 * s);
+        if (++s == LS_W_STAGES) { s = 0; ++round; }
         if (use > 0) {  // the MMAs that read this buffer two turns ago are done
           ok = __all_sync(0xffffffffu, wait(acc_full + 8 * b, use - 1));
           if (!ok) break;
@@ -250,6 +267,8 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         tmem_st16(to, reinterpret_cast<const float*>(high));
         tmem_st16(to + 16, reinterpret_cast<const float*>(mid));
         tmem_st16(to + 32, reinterpret_cast<const float*>(low));
+        // the numbers for the next turn come while the operands are on their way
+        if (kb + 1 < a.k_blocks || t + (int)gridDim.x < tiles) take();
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         if (kb + 1 == a.k_blocks) w_marked[row] = none != 0.f;  // (the adding warps have read the tile's before: k_blocks >= 4)
@@ -258,7 +277,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           mbar_arrive(a_full + 8 * b);
           if (kb + 1 == a.k_blocks) mbar_arrive(marks);
         }
-        if (++s == LS_W_STAGES) { s = 0; ++round; }
+        if (!ok) break;
       }
     }
   } else if (warp >= 8) {
