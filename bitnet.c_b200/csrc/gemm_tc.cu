@@ -5,7 +5,7 @@
 // turn (tile t = block index + i x blocks, in the order of gm_place below: neighbouring blocks share slices of W and of x, which
 // are then found in the L2).
 // Operands arrive by TMA (boxes of 128 x 64 and 256 x 64 elements, 128-byte swizzle) through a
-// ring of four stages of 48 KB; one thread issues tcgen05.mma (M 128, N 256, K 16, four per
+// ring of four stages of 48 KB; one warp issues tcgen05.mma (M 128, N 256, K 16, four per
 // stage) into one of two accumulators of 256 columns in tensor memory; while it works on the next
 // tile's accumulator, four epilogue warps read the finished one (a thread owns a row: its TMEM
 // lane) and finish it:
@@ -20,6 +20,11 @@
 // Grouped: the rows of x belong to groups, packed one behind another (offsets on the device), and every group has a matrix of its
 // own in a stack of W: the experts of a mixture in one launch, however their rows are shared out, without asking the
 // device for the counts.  The tiles of all groups form one list; a tile's rows past its group's end are not stored.
+//
+// The four MMAs of a stage take 512 cycles, and issuing them must take less.  With the whole warp in the loop descriptors and barrier addresses
+// are warp-uniform (an elected lane issues); as one thread's loop it was the slowest role.  Pairs of blocks (below), before and now: 520 rows,
+// 4096 x 14336 83 -> 75 us, 28672 x 4096 134 -> 126; 2,048 rows, 6144 x 4096 82 -> 75, 28672 x 4096 349 -> 327; 8,192 rows, 28672 x 4096
+// 1340 -> 1221 (1.58 PFLOP/s); 128 to 8,192 rows, 2 to 13 %.
 //
 // This removes the separate passes over the activations that a library product leaves to other
 // kernels: the SwiGLU pass over [M, 2 I] and both residual + norm passes of a layer.
@@ -290,35 +295,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issue: one thread, accumulator tile_i & 1
-    if (lane == 0) {
-      int it = 0, tile_i = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; ok && t < n_tiles_total; t += gridDim.x, ++tile_i) {
-        const int buf = tile_i & 1, use = tile_i >> 1;
-        if (use > 0 && (!mbar_wait(acc_empty0 + 8 * buf, (unsigned)(use - 1) & 1u, a.status, GM_ERR_WAIT) || *failed)) {
-          *failed = 1;
-          break;
-        }
+    // ---- MMA issue, accumulator tile_i & 1: the whole warp walks the loop, so that descriptors are warp-uniform; an elected lane issues
+    const bool issuer = elect_one();
+    const unsigned tbase = __shfl_sync(0xffffffffu, tmem_base, 0);
+    int it = 0, tile_i = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; ok && t < n_tiles_total; t += gridDim.x, ++tile_i) {
+      const int buf = tile_i & 1, use = tile_i >> 1;
+      ok = __all_sync(0xffffffffu, use == 0 || mbar_wait(acc_empty0 + 8 * buf, (unsigned)(use - 1) & 1u, a.status, GM_ERR_WAIT));
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned acc = tbase + buf * GM_BN;
+      for (int kb = 0; ok && kb < a.k_blocks; ++kb, ++it) {
+        const int s = it % GM_STAGES, round = it / GM_STAGES;
+        ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, (unsigned)round & 1u, a.status, GM_ERR_WAIT));
+        if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned acc = tmem_base + buf * GM_BN;
-        for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
-          const int s = it % GM_STAGES, round = it / GM_STAGES;
-          if (!mbar_wait(full0 + 8 * s, (unsigned)round & 1u, a.status, GM_ERR_WAIT) || *failed) {
-            *failed = 1;
-            ok = false;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (issuer) {
           const unsigned sa = smem_u32(base + s * STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
           for (int kk = 0; kk < GM_BK / 16; ++kk)
             umma_mma(acc, umma_desc_k(sa + kk * 32), umma_desc_k(sb + kk * 32), IDESC, (kb | kk) ? 1u : 0u);
           umma_commit(empty0 + 8 * s);  // arrives when these MMAs have read the stage
         }
-        if (ok) umma_commit(acc_full0 + 8 * buf);  // arrives when the tile's last MMA is done
+        __syncwarp();
       }
+      if (ok && issuer) umma_commit(acc_full0 + 8 * buf);  // arrives when the tile's last MMA is done
+      __syncwarp();
     }
+    if (!ok) *failed = 1;
   } else {
     // ---- epilogue: thread <-> row of the tile <-> TMEM lane (a warp reaches the lanes of its index modulo 4)
     const int quad = warp & 3, et = tid - 64;
@@ -525,34 +529,35 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issue: the leader's thread, for both blocks
-    if (lane == 0 && leader) {
+    // ---- MMA issue: the leader's elected lane, for both blocks
+    if (leader) {
+      const bool issuer = elect_one();
+      const unsigned tbase = __shfl_sync(0xffffffffu, tmem_base, 0);
       int it = 0, tile_i = 0;
       bool ok = true;
       for (int t = pair; ok && t < n_tiles_total; t += n_pairs, ++tile_i) {
         const int buf = tile_i & 1, use = tile_i >> 1;
-        if (use > 0 && (!mbar_wait(acc_empty0 + 8 * buf, (unsigned)(use - 1) & 1u, a.status, GM_ERR_WAIT) || *failed)) {
-          *failed = 1;
-          break;
-        }
+        ok = __all_sync(0xffffffffu, use == 0 || mbar_wait(acc_empty0 + 8 * buf, (unsigned)(use - 1) & 1u, a.status, GM_ERR_WAIT));
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned acc = tmem_base + buf * GM_BN;
-        for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
+        const unsigned acc = tbase + buf * GM_BN;
+        for (int kb = 0; ok && kb < a.k_blocks; ++kb, ++it) {
           const int s = it % GM2_STAGES, round = it / GM2_STAGES;
-          if (!mbar_wait(full0 + 8 * s, (unsigned)round & 1u, a.status, GM_ERR_WAIT) || *failed) {
-            *failed = 1;
-            ok = false;
-            break;
-          }
+          ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, (unsigned)round & 1u, a.status, GM_ERR_WAIT));
+          if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const unsigned sa = smem_u32(base + s * STAGE_BYTES), sb = sa + A_BYTES;
+          if (issuer) {
+            const unsigned sa = smem_u32(base + s * STAGE_BYTES), sb = sa + A_BYTES;
 #pragma unroll
-          for (int kk = 0; kk < GM_BK / 16; ++kk)
-            gm_mma_pair(acc, umma_desc_k(sa + kk * 32), umma_desc_k(sb + kk * 32), IDESC, (kb | kk) ? 1u : 0u);
-          gm_commit_pair(empty0 + 8 * s);  // both blocks' stage is free when these MMAs have read it
+            for (int kk = 0; kk < GM_BK / 16; ++kk)
+              gm_mma_pair(acc, umma_desc_k(sa + kk * 32), umma_desc_k(sb + kk * 32), IDESC, (kb | kk) ? 1u : 0u);
+            gm_commit_pair(empty0 + 8 * s);  // both blocks' stage is free when these MMAs have read it
+          }
+          __syncwarp();
         }
-        if (ok) gm_commit_pair(acc_full0 + 8 * buf);  // both blocks' accumulator is complete
+        if (ok && issuer) gm_commit_pair(acc_full0 + 8 * buf);  // both blocks' accumulator is complete
+        __syncwarp();
       }
+      if (!ok) *failed = 1;
     }
   } else {
     // ---- epilogue: this block's 128 rows of the pair's tile
