@@ -8,28 +8,31 @@
 // (520 rows, 4096 x 4096: 2.2e-7 against 1.1e-6 of the result's norm; 1024 x 14336: 3.9e-7 against 2.2e-6).
 //
 // The float32 units reach 72 TFLOP/s at most, the library's product 54; six bfloat16 products per float32 product are 230 TFLOP/s at the tensor
-// cores' rate.  520 rows: 28672 x 4096 634 us (library 2288), 6144 x 4096 134 (540), 4096 x 4096 117 (324), 4096 x 14336 375 (1125).
+// cores' rate.  520 rows: 28672 x 4096 611 us (library 2289), 6144 x 4096 129 (540), 4096 x 4096 109 (325), 4096 x 14336 356 (1126).
 //
 // A tile is 128 rows of W times up to 192 rows of x: D[128 rows of W, NT rows of x], so that few and odd numbers of rows of x waste
 // little (NT is a multiple of 16, chosen so that the tiles fill the SMs).  x is split once, by a kernel of its own, into three
 // planes of bfloat16 in memory (it is small, and every tile column of W reads it again).  W is split on the way: its float32 tiles arrive by
-// TMA, four warps turn a row each thread into three bfloat16 operands in tensor memory, from where the MMA takes its A operand; in
+// TMA, groups of four warps turn a row each thread into three bfloat16 operands in tensor memory, from where the MMA takes its A operand; in
 // shared memory they would cost more of its bandwidth than there is (the MMAs read 5.6 KB of x's planes in 88 cycles each).
 //
-// A persistent block of 16 warps per SM:
+// A persistent block of 20 warps per SM:
 //   warp 0      requests float32 tiles of W (128 rows x 32 numbers)
 //   warp 1      requests tiles of x's three planes (NT rows x 32 numbers each, 64-byte swizzle)
 //   warp 2      allocates tensor memory; issues twelve MMAs per 32 numbers, into one of two accumulators
-//   warps 4-7   split W: shared memory -> registers -> tensor memory, two buffers in turn
-//   warps 8-15  add the accumulators up in registers (a row of W each thread, two warps share a row's columns) and store
+//   warps 4-11  split W: shared memory -> registers -> tensor memory, two groups of four warps with a buffer each take turns
+//   warps 12-19 add the accumulators up in registers (a row of W each thread, two warps share a row's columns) and store
 //
 // Numbers that are not finite, or round to infinity in bfloat16, do not split.  Rows that have one are marked (of x by the kernel that
 // splits it, of W by the warps that do); outputs of marked rows are computed again in plain float32.
 //
 // The twelve MMAs of 32 numbers take 1,060 cycles for 176 rows of x; a wait for an mbarrier costs its role some 200, even if it is over.  So
 // the whole of warp 2 walks its loop, with descriptors in uniform registers, and one elected lane issues (as one thread's work a step took 1,700
-// cycles: 790 to issue, 900 for three waits); the splitting warps wait for the MMAs only, and fetch the next numbers while the operands they
-// stored are on their way (before, 1,530 to 1,700 cycles a step: 28672 x 4096 705 us, 4096 x 4096 133).
+// cycles: 790 to issue, 900 for three waits).  Splitting 32 numbers of a row, which is a chain of waits, loads and stores, takes a warp 1,400: so
+// two groups take turns (with one 4096 x 4096 117 us, 128 rows of 6144 x 4096 108 instead of 73; before both 133 and 28672 x 4096 705).
+//
+// The adding warps keep 96 sums a thread in registers.  The block starts with 96 registers for each of 640 threads, and its warps share them
+// anew: 4 x 40 + 8 x 88 + 8 x 128 = 1,888 of 20 x 96 = 1,920 per lane, so that nobody waits for registers.
 //
 // Every wait on an mbarrier is bounded in time; a wait that gives up records code 8 in *status, every role leaves its loops (the others
 // when a wait of theirs gives up in turn), and the block frees its tensor memory and returns.
@@ -42,7 +45,7 @@
 #define LS_BM 128        // rows of W per tile (UMMA M)
 #define LS_BK 32         // numbers of the inner dimension per stage and per sum in the tensor cores
 #define LS_NT_MAX 192    // rows of x per tile at most
-#define LS_THREADS 512
+#define LS_THREADS 640   // five warpgroups
 #define LS_W_STAGES 4
 #define LS_W_BYTES (LS_BM * LS_BK * 4)
 #define LS_X_STAGES_MAX 8
@@ -127,7 +130,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   __shared__ unsigned long long bars[2 * LS_W_STAGES + 2 * LS_X_STAGES_MAX + 7];
   __shared__ unsigned tmem_slot;
   __shared__ int s_failed;
-  __shared__ int w_marked[LS_BM];
+  __shared__ unsigned char w_marked[2][2][LS_BM];  // by turn of the tile, group of splitting warps, row
   volatile int* failed = &s_failed;
   const unsigned w_full = smem_u32(bars), w_free = w_full + 8 * LS_W_STAGES, x_full = w_free + 8 * LS_W_STAGES, x_free = x_full + 8 * LS_X_STAGES_MAX,
                  a_full = x_free + 8 * LS_X_STAGES_MAX, acc_full = a_full + 16, acc_free = acc_full + 16, marks = acc_free + 16;
@@ -149,7 +152,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       mbar_init(acc_full + 8 * b, 1);
       mbar_init(acc_free + 8 * b, 8);
     }
-    mbar_init(marks, 4);
+    mbar_init(marks, 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
@@ -169,6 +172,9 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     return false;
   };
 
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+  }
   if (warp == 0) {
     if (lane == 0) {
       int s = 0, round = 0;
@@ -228,60 +234,62 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         __syncwarp();
         if (++s == a.x_stages) { s = 0; ++round; }
       }
-  } else if (warp >= 4 && warp < 8) {
-    const int row = (warp & 3) * 32 + lane;
-    const unsigned to0 = tmem_a + ((unsigned)((warp & 3) * 32) << 16);
-    int s = 0, round = 0, it = 0;
+  } else if (warp >= 4 && warp < 12) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    // group 0 splits the even steps' numbers into buffer 0, group 1 the odd steps' into buffer 1
+    const int group = (warp - 4) >> 2, row = (warp & 3) * 32 + lane;
+    const unsigned to = tmem_a + ((unsigned)((warp & 3) * 32) << 16) + group * LS_A_COLS;
+    int kb = group, tile_i = 0, it = group;
     bool ok = true;
-    float4 v[8];
-    // the next 32 numbers of the thread's row; the next stage's slot is free again
-    auto take = [&]() {
-      ok = __all_sync(0xffffffffu, wait(w_full + 8 * s, round));
-      if (!ok) return;
+    float none = 0.f;
+    for (int t = blockIdx.x; ok && t < tiles;) {
+      const int s = it % LS_W_STAGES, use = it >> 1;
+      ok = __all_sync(0xffffffffu, wait(w_full + 8 * s, it / LS_W_STAGES));
+      if (!ok) break;
       const unsigned char* from = base + s * LS_W_BYTES + row * 128;
+      float4 v[8];
 #pragma unroll
       for (int c = 0; c < 8; ++c) v[c] = *reinterpret_cast<const float4*>(from + ((c ^ (row & 7)) << 4));
-    };
-    if ((int)blockIdx.x < tiles) take();
-    for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
-      float none = 0.f;
-      for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
-        const int b = it & 1, use = it >> 1;
-        unsigned high[16], mid[16], low[16];
+      unsigned high[16], mid[16], low[16];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          ls_cut(v[c].x, v[c].y, high[2 * c], mid[2 * c], low[2 * c]);
-          ls_cut(v[c].z, v[c].w, high[2 * c + 1], mid[2 * c + 1], low[2 * c + 1]);
-          // zero, or not a number once a number is not finite
-          none = fmaf(v[c].x, 0.f, fmaf(v[c].y, 0.f, fmaf(v[c].z, 0.f, fmaf(v[c].w, 0.f, none))));
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(w_free + 8 * s);
-        if (++s == LS_W_STAGES) { s = 0; ++round; }
-        if (use > 0) {  // the MMAs that read this buffer two turns ago are done
-          ok = __all_sync(0xffffffffu, wait(acc_full + 8 * b, use - 1));
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        }
-        const unsigned to = to0 + b * LS_A_COLS;
-        tmem_st16(to, reinterpret_cast<const float*>(high));
-        tmem_st16(to + 16, reinterpret_cast<const float*>(mid));
-        tmem_st16(to + 32, reinterpret_cast<const float*>(low));
-        // the numbers for the next turn come while the operands are on their way
-        if (kb + 1 < a.k_blocks || t + (int)gridDim.x < tiles) take();
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        if (kb + 1 == a.k_blocks) w_marked[row] = none != 0.f;  // (the adding warps have read the tile's before: k_blocks >= 4)
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(a_full + 8 * b);
-          if (kb + 1 == a.k_blocks) mbar_arrive(marks);
-        }
+      for (int c = 0; c < 8; ++c) {
+        ls_cut(v[c].x, v[c].y, high[2 * c], mid[2 * c], low[2 * c]);
+        ls_cut(v[c].z, v[c].w, high[2 * c + 1], mid[2 * c + 1], low[2 * c + 1]);
+        // zero, or not a number once a number is not finite
+        none = fmaf(v[c].x, 0.f, fmaf(v[c].y, 0.f, fmaf(v[c].z, 0.f, fmaf(v[c].w, 0.f, none))));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(w_free + 8 * s);
+      if (use > 0) {  // the MMAs that read this buffer two steps ago are done
+        ok = __all_sync(0xffffffffu, wait(acc_full + 8 * group, use - 1));
         if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      }
+      tmem_st16(to, reinterpret_cast<const float*>(high));
+      tmem_st16(to + 16, reinterpret_cast<const float*>(mid));
+      tmem_st16(to + 32, reinterpret_cast<const float*>(low));
+      const bool last = kb + 2 >= a.k_blocks;  // this group's last step of the tile
+      // (the adding warps have read the marks of two tiles before: a tile has at least four steps)
+      if (last) w_marked[tile_i & 1][group][row] = none != 0.f;
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        if (last) mbar_arrive(marks);
+        mbar_arrive(a_full + 8 * group);
+      }
+      it += 2;
+      kb += 2;
+      if (last) {
+        kb -= a.k_blocks;
+        t += gridDim.x;
+        ++tile_i;
+        none = 0.f;
       }
     }
-  } else if (warp >= 8) {
-    const int quad = warp & 3, row = quad * 32 + lane, c0 = ((warp - 8) >> 2) * 16 * CH;
+  } else if (warp >= 12) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
+    const int quad = warp & 3, row = quad * 32 + lane, c0 = ((warp - 12) >> 2) * 16 * CH;
     const unsigned from0 = tmem + ((unsigned)(quad * 32) << 16) + c0;
     int it = 0, tile_i = 0;
     bool ok = true, waited = false;
@@ -308,7 +316,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         if (kb + 1 == a.k_blocks) {
           ok = __all_sync(0xffffffffu, wait(marks, tile_i));
           if (!ok) break;
-          row_marked = w_marked[row];
+          row_marked = w_marked[tile_i & 1][0][row] | w_marked[tile_i & 1][1][row];
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(acc_free + 8 * b);
