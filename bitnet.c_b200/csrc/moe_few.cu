@@ -505,17 +505,18 @@ extern "C" int bn_moe_few(const void* h, int n_tokens, int width, const int* ids
 // cores have no such order; the float32 units have time for it as long as an expert has few tokens.
 //
 // One block per SM.  A block keeps the rows of x of the tokens that chose an expert in shared memory (as many as fit: `cap`; an expert
-// with more is passed over again); a warp takes a run of all experts' rows and streams 8 of them at a time (4 of each matrix, where
-// there are two; half of that where no more are left) through slots of its lanes' own, copied D - 1 stages ahead.  Runs are cut at any
-// row, and a row counts MR_ROW_COST + its tokens: with equal runs the blocks of the expert that most tokens chose were the last by far.
+// with more is passed over again); it takes a run of all experts' rows, whose part of each expert its warps share in half units, and a warp
+// streams 8 rows at a time (4 of each matrix, where there are two; half of that where no more are left) through slots of its lanes' own,
+// copied D - 1 stages ahead.  Runs are cut at any row, and a row counts MR_ROW_COST + its tokens: with equal runs the blocks of the expert
+// that most tokens chose were the last by far.  (With a run for every warp of its own, cut from all rows alike, half of a block's warps
+// waited for the others wherever a block's run went from one expert to the next: 8 experts of 4096 x 7168, 8 tokens 280 -> 185 us, 16 tokens
+// 398 -> 263, 64 tokens 1270 -> 730; 64 of 2048 x 1408, 16 tokens 124.)
 // A piece of x serves eight rows, two of them with each instruction (fma.rn.f32x2: two float32 multiply-adds, each rounded as one alone).
 #define MR_WARPS 8
 #define MR_THREADS (32 * MR_WARPS)
 #define MR_S 8       // rows of weights a warp multiplies with at a time
 #define MR_TOKENS 8  // tokens a pass takes at most
-#ifndef MR_ROW_COST
-#define MR_ROW_COST 3
-#endif
+#define MR_ROW_COST 4
 #define MR_SMEM_MAX (226 * 1024)
 __host__ __device__ constexpr int mr_ring_bytes(int D) { return MR_WARPS * D * MR_S * 512; }
 
@@ -739,19 +740,17 @@ __global__ void __launch_bounds__(MR_THREADS, 1) moe_in_order_kernel(MrArgs p) {
   const int used = mf_lists(l, a);
   const int passes = mr_passes(a, l, used, p.cap, seg_expert, seg_m0, seg_cost);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // The run of warp w: rows whose cost lies in [w, w + 1) of so many equal shares.  cut(w): a pass and a row in it.
-  const long long total = (long long)seg_cost[passes] * a.rows, share = (long long)gridDim.x * MR_WARPS;
-  auto cut = [&](int w, int& row) {
-    const long long at = total * w / share;
+  // The run of block b: rows whose cost lies in [b, b + 1) of gridDim.x equal shares.  cut(b): a pass and a row in it.
+  const long long total = (long long)seg_cost[passes] * a.rows;
+  auto cut = [&](int b, int& row) {
+    const long long at = total * b / gridDim.x;
     int seg = 0;
     while (seg < passes && (long long)seg_cost[seg + 1] * a.rows <= at) ++seg;
     row = seg < passes ? (int)((at - (long long)seg_cost[seg] * a.rows) / (seg_cost[seg + 1] - seg_cost[seg])) : 0;
     return seg;
   };
-  const int w0 = blockIdx.x * MR_WARPS;
-  int row0, row1, ignored;
-  const int seg0 = cut(w0 + warp, row0), seg1 = cut(w0 + warp + 1, row1);  // this warp's rows: from row0 of pass seg0 to before row1 of seg1
-  const int block0 = cut(w0, ignored), block1 = cut(w0 + MR_WARPS, ignored);
+  int row0, row1;
+  const int seg0 = cut(blockIdx.x, row0), seg1 = cut(blockIdx.x + 1, row1);  // from row0 of pass seg0 to before row1 of pass seg1
   MrStream q;
   q.K = a.K;
   q.pieces = (a.K + 255) / 256;
@@ -759,8 +758,11 @@ __global__ void __launch_bounds__(MR_THREADS, 1) moe_in_order_kernel(MrArgs p) {
   q.ring = (unsigned)__cvta_generic_to_shared(mr_smem) + warp * (D * MR_S * 512) + lane * 16;
   bool waited = !down;
 
-  for (int seg = block0; seg < passes && seg <= block1; ++seg) {
-    const int j0 = seg < seg0 ? a.rows : seg == seg0 ? row0 : 0, j1 = seg < seg1 ? a.rows : seg == seg1 ? row1 : 0;
+  for (int seg = seg0; seg < passes && seg <= seg1; ++seg) {
+    // the warps share the block's rows of this pass, in half units
+    const int b0 = seg == seg0 ? row0 : 0, b1 = seg < seg1 ? a.rows : row1, halves = (b1 - b0 + MR_S / G / 2 - 1) / (MR_S / G / 2);
+    if (halves <= 0) continue;
+    const int j0 = b0 + halves * warp / MR_WARPS * (MR_S / G / 2), j1 = min(b1, b0 + halves * (warp + 1) / MR_WARPS * (MR_S / G / 2));
     const int e = seg_expert[seg], first = l.off[e] + seg_m0[seg];
     const int n = min(p.cap, l.off[e + 1] - first);
     const size_t at = (size_t)e * a.expert_stride + (size_t)j0 * a.K + lane * 8;

@@ -1537,15 +1537,18 @@ def few_layers(step, launches: int) -> None:
 
 
 def linear_split_pays(M: int, N: int, K: int) -> bool:
-    """Whether a float32 product goes to ``linear_split.cu``: with many outputs, or wide matrices and not too few rows.  The library product's
-    time over that kernel's: 520 to 2,048 rows 1.3 to 3.7 with a million outputs and more (1.05 to 1.1 right at the line), 0.5 to 0.9 with half as
-    many unless N is 3,072 and more; 48 to 128 rows 1.1 to 2.4 for N of 4,096 to 28,672, 0.4 to 1.0 for narrower ones; 17 to 32 rows 0.7 to
-    1.1.  Short inner dimensions leave it its start: 4,000 x 256 x 256 0.6."""
+    """Whether a float32 product goes to ``linear_split.cu``.  The library product's time over that kernel's: 520 to 2,048 rows 1.3 to 4.2 with a
+    million outputs and more (1.05 to 1.1 right at the line); 17 and more rows of matrices of 2,048 rows and more 1.2 to 1.95 (2048 x 1024, 8192 x 512 and
+    16384 x 256 to 28672 x 4096), unless the inner dimension is so long that the library splits it (2048 x 8192 0.76 to 1.26, 4096 x 14336 1.27);
+    100 and more rows of 1,024 x 2,048, 1,536 x 4,096, 1024 x 14336 1.2 to 2.1.  A matrix of fewer rows leaves most SMs idle: 17 rows 1024 x 4096
+    0.5, 512 x 2048 0.54.  Short inner dimensions leave it its start: 4,000 x 256 x 256 0.6."""
     if K < 128:  # the kernel's least
         return False
     if M * N >= 1 << 20 and M >= 48 and M * N * K >= 1 << 30:
         return True
-    return N >= 4096 and M >= 48 and M * N >= 280000 and K >= 1024
+    if N >= 4096 and M >= 48 and M * N >= 280000 and K >= 1024:
+        return True
+    return N * K >= 1 << 21 and K >= 256 and (N >= 2048 and M >= 17 and K <= 2 * N or N >= 1024 and M >= 96)
 
 
 def linear_split(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -2354,10 +2357,10 @@ MOE_IN_ORDER_ROW = 40960  # numbers of a row of x that the kernels of the other 
 
 def moe_in_order_pays(width: int, ff: int, items: int) -> bool:
     """Whether few bfloat16 tokens whose sums must keep their order gain from reading each chosen expert once.  The time of the kernels
-    that read an expert per item over theirs: experts of 4096 x 7168 1.36 to 1.93, 2048 x 4096 1.28 to 2.4, 1024 x 2048 1.19 to 1.96 (8 experts,
-    2 to 128 items), 64 of 2048 x 1408 1.0 to 2.1 (6 to 384 items); 128 of 2048 x 768 1.0 to 1.4 up to 128 items, 0.84 to 0.98 beyond; 32 of
-    1024 x 512 1.05 to 1.3 up to 16 items, 0.78 to 1.06 beyond; 512 x 256 0.45 to 0.6."""
-    return width * ff >= 1 << 21 or (width * ff >= 1 << 20 and items <= 128) or (width * ff >= 1 << 19 and items <= 16)
+    that read an expert per item over theirs: experts of 4096 x 7168 1.76 to 2.85, 2048 x 4096 1.74 to 2.7, 1024 x 2048 1.28 to 2.1 (8 experts,
+    2 to 128 items), 64 of 2048 x 1408 1.39 to 2.28 (6 to 384 items), 128 of 2048 x 768 1.1 to 1.65 (8 to 512 items); 32 of
+    1024 x 512 1.12 to 1.34 up to 16 items, 0.93 to 1.29 beyond; 512 x 256 0.43 to 0.6."""
+    return width * ff >= 3 << 19 or (width * ff >= 1 << 20 and items <= 128) or (width * ff >= 1 << 19 and items <= 16)
 
 
 MOE_FEW_ITEMS = 128  # (token, expert) items one launch of moe_few.cu takes (MF_MAX_ITEMS)
