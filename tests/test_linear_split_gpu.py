@@ -25,6 +25,8 @@ def _pair(M, N, K, seed, spread=0.0):
     (1000, 64, 192, 0.0),    # more tiles of rows than SMs have tiles of w
     (400, 20000, 160, 0.0),  # several tiles per block
     (300, 384, 4096, 3.0),
+    (17, 2048, 288, 0.0),    # nine steps a tile: the groups that split w change places from tile to tile
+    (100, 19100, 160, 0.0),  # the same with several tiles per block, and the fewest steps but one
 ])
 @pytest.mark.parametrize("with_bias", [False, True])
 def test_linear_split(M, N, K, spread, with_bias):
