@@ -1300,10 +1300,11 @@ def _auto_cluster(N: int, K: int) -> int:
 
 # Many-row bfloat16 products on this library's tcgen05 kernel (gemm_tc.cu) instead of the library product
 # followed by separate kernels.  "fused": where the kernel's epilogue replaces a pass over the activations
-# and that saves more than its main loop loses against the library's (measured on a B200 at widths 4096
-# and 14336: the SwiGLU epilogue from 1,024 rows on, 0.88 to 0.98 of the library product + activation
-# kernel; the residual + norm epilogue from 2,048 rows on for inner sizes up to 8192, 0.85 to 0.95 of the
-# library product + norm kernel; plain products are 1.09 to 1.16 of the library's and stay there).
+# and that saves more than its main loop loses against the library's (measured on a B200 at widths of 2048 to
+# 5120: the SwiGLU epilogue from 1,024 rows on, 0.85 to 0.985 of the library product + activation kernel, with 512
+# rows 0.94 to 1.18; the residual + norm epilogue from 2,048 rows on for inner sizes up to 8192, 0.64 to 0.985 of the
+# library product + norm kernel, with 1,024 rows 0.96 to 1.63, inner sizes of 13,824 and 14,336 0.99 to 1.09 up to
+# 4,096 rows; plain products are 0.99 to 1.33 of the library's with 2,048 and 4,096 rows, 0.86 to 1.06 with 8,192, and stay there).
 # True: every product that fits.  False: none.
 USE_OWN_GEMM = "fused"
 GEMM_MIN_ROWS = 65            # True: from so many rows on
