@@ -399,6 +399,16 @@ static int ls_choose_nt(int M, int n_tiles, int sms) {
   return best_nt;
 }
 
+// Whether a block starts with as many registers as its warps share out (else a warp would wait for some that nobody gives back)
+template <int CH>
+static bool ls_registers() {
+  static const bool enough = [] {
+    cudaFuncAttributes f;
+    return cudaFuncGetAttributes(&f, linear_split_kernel<CH>) == cudaSuccess && f.numRegs * (LS_THREADS / 32) >= 4 * 40 + 8 * 88 + 8 * 128;
+  }();
+  return enough;
+}
+
 // Bytes of working space for M rows of K numbers: three planes of bfloat16 and a mark per row.
 extern "C" long long bn_linear_split_scratch(int M, int K) { return 6ll * M * ((K + 7) / 8 * 8) + 4ll * M; }
 
@@ -429,6 +439,7 @@ extern "C" int bn_linear_split(const float* x, const float* w, const float* bias
 #define LS_RUN(CH)                                                                                       \
   do {                                                                                                   \
     static BnGrant grant;                                                                                \
+    if (!ls_registers<CH>()) return BN_ERR_BAD_ARG;                                                      \
     cudaError_t e = grant.ask((const void*)linear_split_kernel<CH>, smem, 1024);                         \
     if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;                                                 \
     BN_LAUNCH((linear_split_kernel<CH>), grid, LS_THREADS, smem, stream, mw, mx, a);                     \

@@ -19,7 +19,7 @@
 // A block of 192 threads (320 with the wider accumulators):
 //   warp 0     one thread issues the TMA loads of W and x tiles into a ring of stages and arms each
 //              stage's "full" mbarrier with the bytes to expect;
-//   warp 1     allocates tensor memory; one thread waits for "full", issues four MMAs per stage,
+//   warp 1     allocates tensor memory; waits for "full", issues four MMAs per stage (one elected lane),
 //              commits them to the stage's "empty" mbarrier and at the end to "accumulator full";
 //   warps 2-5  wait for the accumulator, move it from tensor memory to shared memory
 //              (tcgen05.ld, one weight row per thread), send and receive the slices, add them up
