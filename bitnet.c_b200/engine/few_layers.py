@@ -76,7 +76,7 @@ class FewLayers:
     def takes(self, ctx) -> bool:
         """Whether a step of these tokens goes this way; every switch that sends a part elsewhere sends the step there too."""
         return (ctx.n_tokens <= ops.TC_MAX_ROWS and ctx.diag is None and ops.PROFILE is None and ops.USE_TCGEN05 and ops.USE_FUSED_NORM
-                and not ops._FORCE_SPLITS and (ctx.decode or (ctx.wide_tile_seq is not None and ops.USE_TCGEN05_ATTENTION)))
+                and not ops._FORCE_SPLITS and not ops._FORCE_ITEM_GROUP and (ctx.decode or (ctx.wide_tile_seq is not None and ops.USE_TCGEN05_ATTENTION)))
 
     def run(self, x, h, cache, ctx, last_norm):
         """The layers on the residual x [T, width] from the first one's normed rows h; ``last_norm``: the norm behind the last
