@@ -863,6 +863,25 @@ __global__ void moe_in_order_sum_kernel(MrArgs p) {
 // Rows of K numbers that fit beside a ring of D stages
 static int mr_room(int D, int K, size_t lists) { return (int)((MR_SMEM_MAX - 4096 - mr_ring_bytes(D) - lists) / (2 * (size_t)K)); }
 
+// One product (the launch of an instantiation stands in one place, so that it has one grant): at most `most` tokens of an expert a pass
+template <int G, int D>
+static int mr_launch(MrArgs& p, int most, size_t lists, cudaStream_t stream) {
+  const int room = mr_room(D, p.m.K, lists);
+  p.cap = most < room ? most : room;
+  if (p.cap < 1) return BN_ERR_BAD_ARG;
+  const size_t smem = mr_ring_bytes(D) + (size_t)p.cap * p.m.K * 2 + lists;
+  static BnGrant grant;
+  cudaError_t e = grant.ask((const void*)moe_in_order_kernel<G, D>, smem, 4096);
+  if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
+  BN_LAUNCH((moe_in_order_kernel<G, D>), (unsigned)mf_sm_count(), MR_THREADS, smem, stream, p);
+  return BN_OK;
+}
+// Stages: four where the tokens' rows leave room for them, else three.
+template <int G>
+static int mr_product(MrArgs& p, int most, size_t lists, cudaStream_t stream) {
+  return mr_room(4, p.m.K, lists) >= most ? mr_launch<G, 4>(p, most, lists, stream) : mr_launch<G, 3>(p, most, lists, stream);
+}
+
 // bn_moe_few with the sums of moe.cu, for the same arguments: d [n_tokens * top, width] float32 is working space.  No row of x may be
 // larger than the shared memory beside a ring (width and ff up to 40,960 numbers).
 extern "C" int bn_moe_few_in_order(const void* h, int n_tokens, int width, const int* ids, const float* weights, int scale_input, const void* w_gate,
@@ -880,31 +899,15 @@ extern "C" int bn_moe_few_in_order(const void* h, int n_tokens, int width, const
   a.K = width; a.rows = ff; a.w = (const __nv_bfloat16*)w_gate; a.w_up = (const __nv_bfloat16*)w_up; a.expert_stride = (size_t)expert_stride;
   a.scale_input = scale_input; a.limit = limit; a.slope = slope; a.act = act; a.y = (__nv_bfloat16*)y;
   const size_t lists = mf_list_bytes(a) + (3 * a.n_items + 1) * sizeof(int);
-  // Stages: four where the tokens' rows leave room for them, else three.
-#define MR_RUN(G, D)                                                                                                            \
-  do {                                                                                                                          \
-    p.cap = most < mr_room(D, a.K, lists) ? most : mr_room(D, a.K, lists);                                                      \
-    if (p.cap < 1) return BN_ERR_BAD_ARG;                                                                                       \
-    const size_t smem = mr_ring_bytes(D) + (size_t)p.cap * a.K * 2 + lists;                                                     \
-    static BnGrant grant;                                                                                                       \
-    cudaError_t e = grant.ask((const void*)moe_in_order_kernel<G, D>, smem, 4096);                                              \
-    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;                                                                        \
-    BN_LAUNCH((moe_in_order_kernel<G, D>), (unsigned)mf_sm_count(), MR_THREADS, smem, stream, p);                               \
-  } while (0)
   const int most = n_tokens < MR_TOKENS ? n_tokens : MR_TOKENS;
-  if (w_gate) {
-    if (mr_room(4, a.K, lists) >= most) MR_RUN(2, 4);
-    else MR_RUN(2, 3);
-  } else {
-    if (mr_room(4, a.K, lists) >= most) MR_RUN(1, 4);
-    else MR_RUN(1, 3);
-  }
+  int rc = w_gate ? mr_product<2>(p, most, lists, stream) : mr_product<1>(p, most, lists, stream);
+  if (rc != BN_OK) return rc;
   a.x = (const __nv_bfloat16*)y;
   a.K = ff; a.rows = width; a.w = nullptr; a.w_up = (const __nv_bfloat16*)w_down; a.expert_stride = (size_t)width * ff;
   a.scale_output = !scale_input; a.add = add; a.add_dtype = add_dtype; a.add_scale = add_scale; a.h = (const __nv_bfloat16*)h; a.out = out;
   p.d = d;
-  if (mr_room(4, a.K, lists) >= most) MR_RUN(1, 4);
-  else MR_RUN(1, 3);
+  rc = mr_product<1>(p, most, lists, stream);
+  if (rc != BN_OK) return rc;
   BN_LAUNCH(moe_in_order_sum_kernel, dim3(n_tokens, (width + 255) / 256), 256, 0, stream, p);
   BN_CHECK_LAUNCH();
   return BN_OK;

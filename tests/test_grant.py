@@ -1,5 +1,6 @@
 """Grants of shared memory (csrc/grant.h) against a runtime that only counts: compiled for the host, no GPU and no CUDA library."""
 import os
+import re
 import subprocess
 
 import pytest
@@ -66,3 +67,24 @@ def test_kernels_that_once_needed_no_grant_ask_per_device(family):
     without any grant; one flag for all devices left their kernels without it there."""
     with open(os.path.join(os.path.dirname(build.__file__), build.SOURCES[family])) as f:
         assert "static bool granted" not in f.read()
+
+
+@pytest.mark.parametrize("family", sorted(build.SOURCES))
+def test_no_kernel_has_two_grants(family):
+    """A macro with a grant of its own that is written out twice for the same kernel leaves it with two, of which one lowers what the other
+    relies on."""
+    with open(os.path.join(os.path.dirname(build.__file__), build.SOURCES[family])) as f:
+        text = f.read().replace("\\\n", " ")
+    for name in re.findall(r"#define (\w+)\([^)]*\)[^\n]*static BnGrant", text):
+        for line in re.findall(r"#define (\w+)\(([^)]*)\)([^\n]*)", text):
+            if name + "(" in line[2]:  # written out by another macro: count that one's arguments through
+                outer, params, body = line
+                inner = re.findall(rf"\b{name}\(([^)]*)\)", body)
+                text += "\n" + "\n".join(f"{name}({_put(i, params, args)})" for args in re.findall(rf"(?<!define )\b{outer}\(([^)]*)\)", text) for i in inner)
+        made = [a for line in text.split("\n") if "#define" not in line for a in re.findall(rf"\b{name}\(([^)]*)\)", line)]
+        assert made and len(made) == len(set(made)), (name, sorted(made))
+
+
+def _put(args, params, values):
+    given = dict(zip((p.strip() for p in params.split(",")), (v.strip() for v in values.split(","))))
+    return ", ".join(given.get(a.strip(), a.strip()) for a in args.split(","))

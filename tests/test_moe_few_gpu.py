@@ -147,3 +147,15 @@ def test_moe_experts_few_in_order(monkeypatch, tokens, width, ff, experts, top, 
         monkeypatch.setattr(ops, "moe_in_order_pays", lambda *a: once)
         out.append(ops.moe_experts_few(h, ids, weights, up, down, 3.0, 1.5, scale_input, add=add, act=act, add_scale=add_scale, read_once=False))
     assert torch.equal(*out)
+
+
+def test_moe_experts_few_in_order_again_and_again(monkeypatch):
+    """Experts without a gate run one kernel for both products: the larger shared memory of the one is still granted when the other has asked for
+    less, in every later call."""
+    wide, narrow = (_case(8, w, f, 8, 2, ops.ACT_RELU2, 0, seed=w) for w, f in ((4096, 1024), (1024, 4096)))
+    for case in (wide, narrow, wide, wide):
+        out = []
+        for once in (True, False):
+            monkeypatch.setattr(ops, "moe_in_order_pays", lambda *a: once)
+            out.append(ops.moe_experts_few(*case, 3.0, 1.5, False, act=ops.ACT_RELU2, read_once=False))
+        assert torch.equal(*out)
