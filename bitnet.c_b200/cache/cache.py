@@ -293,12 +293,24 @@ class Cache:
                       head_dim=g.request.head_dim, window=g.request.window, owner=owner,
                       v_head_dim=g.request.v_head_dim)
 
-    def plane(self, entry: int):
-        """Addresses of the entry's own keys and values, their page table and number of pages (for a launch; kept by nobody)."""
-        gi, plane = self._plane[entry]
-        g = self.groups[gi]
-        return (g.k.data_ptr() + plane * g.k.stride(0) * g.k.element_size(), g.v.data_ptr() + plane * g.v.stride(0) * g.v.element_size(),
-                g.page_table, g.k.shape[1])
+    def own_planes(self, entries: int, n_kv_heads: int, head_dim: int, dtype: torch.dtype, device):
+        """For a launch that covers schedule entries 0 .. ``entries`` - 1: of each the addresses of its own keys, values and page table, the page table's
+        row length and the number of pages.  None unless every one has keys and values ``[pages, n_kv_heads, PAGE, head_dim]`` of ``dtype`` on ``device``."""
+        found, out = {}, []
+        for entry in range(entries):
+            at = self._plane.get(entry)
+            if at is None:
+                return None
+            g = found.get(at[0])
+            if g is None:
+                group = self.groups[at[0]]
+                k, v, table = group.k, group.v, group.page_table
+                if (k is None or v is None or k.shape[2:] != (n_kv_heads, PAGE, head_dim) or v.shape != k.shape or k.dtype is not dtype
+                        or v.dtype is not dtype or table.dtype is not torch.int32 or any(t.device != device or not t.is_contiguous() for t in (k, v, table))):
+                    return None
+                g = found[at[0]] = (k.data_ptr(), v.data_ptr(), k.stride(0) * k.element_size(), table.data_ptr(), table.shape[1], k.shape[1])
+            out.append((g[0] + at[1] * g[2], g[1] + at[1] * g[2], *g[3:]))
+        return out
 
     def state(self, entry: int):
         """The entry's state tensor, or a dict of them by name if it keeps several, or None."""

@@ -73,16 +73,27 @@ class FewLayers:
             self.entries = [ctypes.cast(getattr(build.library(lib), name), c_void_p).value for lib, name in names]
         return self.entries
 
-    def takes(self, ctx) -> bool:
-        """Whether a step of these tokens goes this way; every switch that sends a part elsewhere sends the step there too."""
-        return (ctx.n_tokens <= ops.TC_MAX_ROWS and ctx.diag is None and ops.PROFILE is None and ops.USE_TCGEN05 and ops.USE_FUSED_NORM
-                and not ops._FORCE_SPLITS and not ops._FORCE_ITEM_GROUP and (ctx.decode or (ctx.wide_tile_seq is not None and ops.USE_TCGEN05_ATTENTION)))
+    def takes(self, cache, ctx):
+        """What ``run`` needs of the cache for a step of these tokens: where each layer's keys and values lie.  None if the step does not go this way;
+        every switch that sends a part elsewhere sends the step there too, and a cache of another shape or type than the layers' goes there to be
+        refused."""
+        if not (ctx.n_tokens <= ops.TC_MAX_ROWS and ctx.diag is None and ops.PROFILE is None and ops.USE_TCGEN05 and ops.USE_FUSED_NORM
+                and not ops._FORCE_SPLITS and not ops._FORCE_ITEM_GROUP
+                and (ctx.decode or (ctx.wide_tile_seq is not None and ops.USE_TCGEN05_ATTENTION))):
+            return None
+        mixer = self.runs[0].mixer
+        return cache.own_planes(len(self.runs), mixer.spec.n_kv_heads, mixer.spec.head_dim, torch.bfloat16, mixer.w_qkv.device)
 
-    def run(self, x, h, cache, ctx, last_norm):
-        """The layers on the residual x [T, width] from the first one's normed rows h; ``last_norm``: the norm behind the last
-        layer, if that layer's product is to prepare it.  Returns what is pending (as the last block would)."""
+    def run(self, planes, x, h, ctx, last_norm):
+        """The layers on the residual x [T, width] from the first one's normed rows h; ``planes`` is what ``takes`` answered, ``last_norm`` the norm
+        behind the last layer, if that layer's product is to prepare it.  Returns what is pending (as the last block would)."""
         spec, T, width, dev = self.runs[0].mixer.spec, x.shape[0], self.shapes[1][0], x.device
         (n_qkv, _), (_, q_dim), (n_gu, _), (_, inter) = self.shapes
+        steps = ("tok_pos", "slots") if ctx.decode else ("tok_pos", "slots", "tok_seq", "wide_tile_seq", "wide_tile_row0", "seq_start", "seq_pos0")
+        for name in steps:
+            ops._need(getattr(ctx, name), name, torch.int32, 1)
+        if ctx.tok_pos.shape[0] < T or ctx.slots.shape[0] < ctx.n_seqs:
+            raise ops.KernelError(f"few_layers: {ctx.tok_pos.shape[0]} positions and {ctx.slots.shape[0]} slots do not fit {T} tokens of {ctx.n_seqs} sequences")
         s = _Step()
         s.linear_tc, s.resident, s.rope, s.decode, s.decode_items, s.prefill = self._entry_points()
         sms = ops.n_sms(dev)
@@ -94,6 +105,9 @@ class FewLayers:
         part_o = part_ml = 0
         if ctx.decode:
             if ctx.decode_items is not None:
+                ops._need(ctx.decode_items, "items", torch.int32, 1)
+                if not 1 <= ctx.decode_item_group <= 8 or ctx.decode_items.shape[0] % ctx.decode_item_group or ctx.decode_items.shape[0] == 0:
+                    raise ops.KernelError(f"few_layers: {ctx.decode_items.shape[0]} items in groups of {ctx.decode_item_group}")
                 s.items, s.n_items, s.item_group = ctx.decode_items.data_ptr(), ctx.decode_items.shape[0], ctx.decode_item_group
                 splits = ctx.decode_item_group
             else:
@@ -126,8 +140,7 @@ class FewLayers:
             norm = self.runs[i + 1].mixer_norm if i + 1 < len(self.runs) else last_norm
             if norm is not None:
                 l.gain_next, l.gain_next_dtype, l.eps_next = norm.weight.data_ptr(), ops._DT[norm.weight.dtype], norm.spec.eps
-            l.k_cache, l.v_cache, table, l.n_cache_pages = cache.plane(i)
-            l.page_table, l.pt_stride = table.data_ptr(), table.shape[1]
+            l.k_cache, l.v_cache, l.page_table, l.pt_stride, l.n_cache_pages = planes[i]
         s.layers = ctypes.addressof(layers)
         s.x, s.h, s.next, s.next_ss, s.delta = x.data_ptr(), h.data_ptr(), nxt.data_ptr(), ss.data_ptr(), delta.data_ptr() if delta is not None else None
         s.tok_pos, s.slots, s.status = ctx.tok_pos.data_ptr(), ctx.slots.data_ptr(), ops.tc_status(dev).data_ptr()

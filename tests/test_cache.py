@@ -135,3 +135,28 @@ def test_the_kernel_that_zeroes_states_is_built_with_the_model(stateful):
     arch = architecture_of(cfg)
     model = bitnet_c_b200.Model(arch.to_spec(arch.read_config(cfg)), dtype="float32", device=None)
     assert ("cache_rows" in model.kernel_families()) == stateful
+
+
+def test_own_planes_are_what_the_views_show_or_none():
+    """Addresses for a launch over several entries: those of the views, and none at all unless every entry is as it is asked for."""
+    kv, cpu = KvRequest(2, 16), torch.device("cpu")
+
+    def cache(requests, cache_of=None, dtype=torch.bfloat16):
+        return Cache(requests, cache_of or [None] * len(requests), [None] * len(requests), 640, 512, dtype, cpu, max_seqs=4)
+
+    mixed = [kv, KvRequest(2, 16, window=128), kv]  # two groups
+    c = cache(mixed)
+    got = c.own_planes(3, 2, 16, torch.bfloat16, cpu)
+    for i, (k, v, table, row, pages) in enumerate(got):
+        view = c.view(i)
+        assert (k, v, table) == (view.k.data_ptr(), view.v.data_ptr(), view.page_table.data_ptr())
+        assert (row, pages) == (view.page_table.shape[1], view.k.shape[0])
+    assert len({k for k, *_ in got}) == 3
+    assert c.own_planes(4, 2, 16, torch.bfloat16, cpu) is None  # more entries than it has
+    assert c.own_planes(3, 1, 16, torch.bfloat16, cpu) is None and c.own_planes(3, 2, 32, torch.bfloat16, cpu) is None
+    assert c.own_planes(3, 2, 16, torch.float32, cpu) is None and c.own_planes(3, 2, 16, torch.bfloat16, torch.device("meta")) is None
+    assert cache(mixed, dtype=torch.float32).own_planes(3, 2, 16, torch.bfloat16, cpu) is None
+    assert cache([kv, kv], [None, 0]).own_planes(2, 2, 16, torch.bfloat16, cpu) is None  # an entry that reads another's
+    for other in (KvRequest(4, 16), KvRequest(2, 32), KvRequest(2, 16, v_head_dim=8), KvRequest(2, 16, values_in_keys=True), None):
+        assert cache([kv, other]).own_planes(2, 2, 16, torch.bfloat16, cpu) is None
+        assert len(cache([kv, other]).own_planes(1, 2, 16, torch.bfloat16, cpu)) == 1

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 import bitnet_c_b200 as bn
+from bitnet_c_b200.csrc import ops
 from bitnet_c_b200.engine import Model
 
 pytestmark = pytest.mark.gpu
@@ -53,3 +54,29 @@ def test_what_stays_with_the_parts():
     assert not ran
     model.step(cache, [bn.SeqStep(slot, [1], [0])])
     assert len(ran) == 1
+
+
+@pytest.fixture
+def native_calls(monkeypatch):
+    """The native call's structures, as often as it is made."""
+    made, run = [], ops.few_layers
+    monkeypatch.setattr(ops, "few_layers", lambda step, launches: (made.append(step), run(step, launches))[1])
+    return made
+
+
+@pytest.mark.parametrize("other", [dict(head_dim=32), dict(num_key_value_heads=1), dict(num_key_value_heads=4), "float32"])
+@pytest.mark.parametrize("tokens", [1, 20])
+def test_a_cache_that_does_not_fit_is_refused(native_calls, other, tokens):
+    """A cache of another head size, number of heads or type: the parts' error, and the native call is not made."""
+    cfg = _config(64, 4, 2, 16, 176, 2, False)
+    model = Model.from_random(cfg, seed=1)
+    owner = Model.from_random(cfg, seed=1, dtype="float32") if other == "float32" else Model.from_random(dict(cfg, **other), seed=1)
+    cache = owner.new_cache(max_tokens=128, max_seqs=1)
+    slot = cache.open()
+    with pytest.raises(ops.KernelError):
+        model.step(cache, [bn.SeqStep(slot, list(range(tokens)), [0])])
+    assert not native_calls
+    assert cache.length(slot) == 0
+    fitting = model.new_cache(max_tokens=128, max_seqs=1)
+    model.step(fitting, [bn.SeqStep(fitting.open(), list(range(tokens)), [0])])
+    assert len(native_calls) == 1
