@@ -31,38 +31,64 @@ class _Step(ctypes.Structure):
             "cluster_down")] + [("scale", c_float), ("theta_scale", c_float)]
 
 
+def _layers(model):
+    """The blocks of ``model`` in the order they run, of each the addresses of its matrices (QKV, O, gate and up, down), and of all norms (the mixers' and the
+    feed-forwards' in turn, then the last one) address, type and eps; None unless all blocks are alike and of the kinds that ``bn_few_layers`` knows, with
+    parameters of the types and shapes that its kernels read without another look."""
+    spec = model.spec
+    if (model.dtype is not torch.bfloat16 or not spec.schedule or model.embedding_norm is not None or getattr(spec, "streams", 1) != 1
+            or type(model.final_norm) is not RmsNorm):
+        return None
+    runs, matrices, norms, blocks, bf16, gains = [], [], [], model.blocks, torch.bfloat16, (spec.width,)
+    s = None
+    for e in spec.schedule:
+        b = blocks[e.block]
+        if e.cache_of is not None or type(b) is not PreNormBlock:
+            return None
+        m, f = b.mixer, b.ffn
+        n1, n2 = b.mixer_norm, b.ffn_norm
+        if type(m) is not Attention or type(f) is not GatedMlp or type(n1) is not RmsNorm or type(n2) is not RmsNorm:
+            return None
+        qkv, o, gate_up, down = m.w_qkv, m.w_o, f.w_gate_up, f.w_down
+        if s is None:
+            s, act, inter = m.spec, f.act, down.shape[1]
+            if s.head_dim > 128 or type(m.position) is not Rotary or (s.q_dim | s.kv_dim | spec.width | inter) % 8:
+                return None
+            shapes = ((s.q_dim + 2 * s.kv_dim, spec.width), (spec.width, s.q_dim), (2 * inter, spec.width), (spec.width, inter))
+        if (m.spec is not s and m.spec != s) or f.act != act or not b.build.resident or getattr(f.spec, "wide_output", False):
+            return None
+        if (qkv.shape, o.shape, gate_up.shape, down.shape) != shapes:
+            return None
+        at = []
+        for w in (qkv, o, gate_up, down):
+            if w.dtype is not bf16 or not w.is_cuda or not w.is_contiguous():
+                return None
+            at.append(w.data_ptr())
+        if (at[0] | at[1] | at[2] | at[3]) & 15:
+            return None
+        runs.append(b)
+        matrices.append(at)
+        norms += (n1, n2)
+    norms.append(model.final_norm)
+    for i, n in enumerate(norms):
+        w = n.weight
+        code = ops._DT.get(w.dtype) if w is not None else None
+        if code is None or w.shape != gains or not w.is_cuda or not w.is_contiguous():
+            return None
+        norms[i] = (w.data_ptr(), code, n.spec.eps)
+    return runs, matrices, norms
+
+
 class FewLayers:
-    """The layers of ``model`` if they are all alike and of the kinds that ``bn_few_layers`` knows (``FewLayers.of``)."""
+    """Runs the layers of a model from one native call.  It keeps nothing of the model, and what the kernels rely on is looked at for every step: a
+    weight set anew or a cache of another shape goes the way of the parts, which take it or refuse it."""
 
     @staticmethod
     def of(model) -> Optional["FewLayers"]:
-        """Called when all parameters are bound; None for every other model."""
-        runs = [model.blocks[e.block] for e in model.spec.schedule]
-        if model.dtype != torch.bfloat16 or model.embedding_norm is not None or getattr(model.spec, "streams", 1) != 1 or type(model.final_norm) is not RmsNorm:
-            return None
-        if any(e.cache_of is not None for e in model.spec.schedule):
-            return None
-        for b in runs:
-            if not (type(b) is PreNormBlock and type(b.mixer) is Attention and type(b.ffn) is GatedMlp and type(b.mixer_norm) is RmsNorm
-                    and type(b.ffn_norm) is RmsNorm and type(b.mixer.position) is Rotary and b.build.resident
-                    and not getattr(b.ffn.spec, "wide_output", False)):
-                return None
-            a, f, first = b.mixer, b.ffn, runs[0]
-            weights = (a.w_qkv, a.w_o, f.w_gate_up, f.w_down)
-            if [w.shape for w in weights] != [w.shape for w in (first.mixer.w_qkv, first.mixer.w_o, first.ffn.w_gate_up, first.ffn.w_down)]:
-                return None
-            if any(w.dtype != torch.bfloat16 or not w.is_cuda or not w.is_contiguous() or w.data_ptr() % 16 or w.shape[1] % 8 for w in weights):
-                return None
-            if a.spec != first.mixer.spec or f.act != first.ffn.act or a.spec.head_dim > 128 or a.w_qkv.shape[0] % 8:
-                return None
-            if any(n.weight.dtype not in ops._DT or not n.weight.is_contiguous() for n in (b.mixer_norm, b.ffn_norm, model.final_norm)):
-                return None
-        return FewLayers(model, runs)
+        """Called when all parameters are bound; None for a model whose layers are not of this kind."""
+        return FewLayers() if _layers(model) is not None else None
 
-    def __init__(self, model, runs):
-        self.model, self.runs = model, runs
-        a, f = runs[0].mixer, runs[0].ffn
-        self.shapes = [tuple(w.shape) for w in (a.w_qkv, a.w_o, f.w_gate_up, f.w_down)]
+    def __init__(self):
         self.entries = None
 
     def _entry_points(self):
@@ -73,22 +99,28 @@ class FewLayers:
             self.entries = [ctypes.cast(getattr(build.library(lib), name), c_void_p).value for lib, name in names]
         return self.entries
 
-    def takes(self, cache, ctx):
-        """What ``run`` needs of the cache for a step of these tokens: where each layer's keys and values lie.  None if the step does not go this way;
-        every switch that sends a part elsewhere sends the step there too, and a cache of another shape or type than the layers' goes there to be
-        refused."""
+    def takes(self, model, cache, ctx):
+        """What ``run`` needs for a step of these tokens: the layers, where their matrices lie, and where their keys and values lie.  None if the step does not go this
+        way; every switch that sends a part elsewhere sends the step there too."""
         if not (ctx.n_tokens <= ops.TC_MAX_ROWS and ctx.diag is None and ops.PROFILE is None and ops.USE_TCGEN05 and ops.USE_FUSED_NORM
                 and not ops._FORCE_SPLITS and not ops._FORCE_ITEM_GROUP
                 and (ctx.decode or (ctx.wide_tile_seq is not None and ops.USE_TCGEN05_ATTENTION))):
             return None
-        mixer = self.runs[0].mixer
-        return cache.own_planes(len(self.runs), mixer.spec.n_kv_heads, mixer.spec.head_dim, torch.bfloat16, mixer.w_qkv.device)
+        layers = _layers(model)
+        if layers is None:
+            return None
+        m = layers[0][0].mixer
+        planes = cache.own_planes(len(layers[0]), m.spec.n_kv_heads, m.spec.head_dim, torch.bfloat16, m.w_qkv.device)
+        return (*layers, planes) if planes is not None else None
 
-    def run(self, planes, x, h, ctx, last_norm):
-        """The layers on the residual x [T, width] from the first one's normed rows h; ``planes`` is what ``takes`` answered, ``last_norm`` the norm
+    def run(self, taken, x, h, ctx, last_norm):
+        """The layers on the residual x [T, width] from the first one's normed rows h; ``taken`` is what ``takes`` answered, ``last_norm`` the norm
         behind the last layer, if that layer's product is to prepare it.  Returns what is pending (as the last block would)."""
-        spec, T, width, dev = self.runs[0].mixer.spec, x.shape[0], self.shapes[1][0], x.device
-        (n_qkv, _), (_, q_dim), (n_gu, _), (_, inter) = self.shapes
+        runs, matrices, norms, planes = taken
+        attention, ffn = runs[0].mixer, runs[0].ffn
+        spec, T, dev = attention.spec, x.shape[0], x.device
+        shapes = [tuple(w.shape) for w in (attention.w_qkv, attention.w_o, ffn.w_gate_up, ffn.w_down)]
+        (n_qkv, _), (width, q_dim), (n_gu, _), (_, inter) = shapes
         steps = ("tok_pos", "slots") if ctx.decode else ("tok_pos", "slots", "tok_seq", "wide_tile_seq", "wide_tile_row0", "seq_start", "seq_pos0")
         for name in steps:
             ops._need(getattr(ctx, name), name, torch.int32, 1)
@@ -97,7 +129,7 @@ class FewLayers:
         s = _Step()
         s.linear_tc, s.resident, s.rope, s.decode, s.decode_items, s.prefill = self._entry_points()
         sms = ops.n_sms(dev)
-        s.res_qkv, s.res_o, s.res_gate_up, s.res_down = (int(ops.linear_resident_pays(T, n, k, sms)) for n, k in self.shapes)
+        s.res_qkv, s.res_o, s.res_gate_up, s.res_down = (int(ops.linear_resident_pays(T, n, k, sms)) for n, k in shapes)
         s.cluster_o, s.cluster_down = ops._auto_cluster(width, q_dim), ops._auto_cluster(width, inter)
         tiles = (width + 127) // 128
         mid_parts = (width + 15) // 16 if s.res_o else tiles * s.cluster_o
@@ -132,22 +164,17 @@ class FewLayers:
         nxt = torch.empty((T, width), dtype=torch.bfloat16, device=dev)  # rows for the next layer, or the last product itself
         ss = torch.empty((next_parts, T), dtype=torch.float32, device=dev)
         delta = torch.empty((T, width), dtype=torch.bfloat16, device=dev) if last_norm is None else None
-        layers = (_Layer * len(self.runs))()
-        for i, (l, b) in enumerate(zip(layers, self.runs)):
-            a, f = b.mixer, b.ffn
-            l.w_qkv, l.w_o, l.w_gate_up, l.w_down = a.w_qkv.data_ptr(), a.w_o.data_ptr(), f.w_gate_up.data_ptr(), f.w_down.data_ptr()
-            l.gain_ffn, l.gain_ffn_dtype, l.eps_ffn = b.ffn_norm.weight.data_ptr(), ops._DT[b.ffn_norm.weight.dtype], b.ffn_norm.spec.eps
-            norm = self.runs[i + 1].mixer_norm if i + 1 < len(self.runs) else last_norm
-            if norm is not None:
-                l.gain_next, l.gain_next_dtype, l.eps_next = norm.weight.data_ptr(), ops._DT[norm.weight.dtype], norm.spec.eps
-            l.k_cache, l.v_cache, l.page_table, l.pt_stride, l.n_cache_pages = planes[i]
+        behind = norms[2::2] if last_norm is not None else norms[2:-1:2] + [(None, 0, 0.0)]
+        layers = (_Layer * len(runs))(*[
+            (*w, gain, gain_next, k, v, table, dtype, dtype_next, row, pages, eps, eps_next)
+            for w, (gain, dtype, eps), (gain_next, dtype_next, eps_next), (k, v, table, row, pages) in zip(matrices, norms[1::2], behind, planes)])
         s.layers = ctypes.addressof(layers)
         s.x, s.h, s.next, s.next_ss, s.delta = x.data_ptr(), h.data_ptr(), nxt.data_ptr(), ss.data_ptr(), delta.data_ptr() if delta is not None else None
         s.tok_pos, s.slots, s.status = ctx.tok_pos.data_ptr(), ctx.slots.data_ptr(), ops.tc_status(dev).data_ptr()
-        s.n_layers, s.M, s.n_seqs, s.width, s.inter, s.n_heads, s.n_kv_heads = len(self.runs), T, ctx.n_seqs, width, inter, spec.n_heads, spec.n_kv_heads
-        s.head_dim, s.act_code, s.window, s.scale = spec.head_dim, self.runs[0].ffn.act, spec.window, spec.softmax_scale
-        s.rotary_dims, s.theta_scale = self.runs[0].mixer.position.rotary_params()
-        ops.few_layers(s, len(self.runs) * (5 if ctx.decode else 6))
+        s.n_layers, s.M, s.n_seqs, s.width, s.inter, s.n_heads, s.n_kv_heads = len(runs), T, ctx.n_seqs, width, inter, spec.n_heads, spec.n_kv_heads
+        s.head_dim, s.act_code, s.window, s.scale = spec.head_dim, ffn.act, spec.window, spec.softmax_scale
+        s.rotary_dims, s.theta_scale = attention.position.rotary_params()
+        ops.few_layers(s, len(runs) * (5 if ctx.decode else 6))
         if delta is not None:
             return delta
         return Normed(ops.RowScaled(nxt, ss, width, last_norm.spec.eps))

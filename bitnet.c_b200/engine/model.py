@@ -282,11 +282,11 @@ class Model:
         diag = ctx.diag = self.diagnostics
         ctx.layer = -1
         ctx.tap("inp", x)
-        planes = self.few_layers.takes(cache, ctx) if self.few_layers is not None else None
-        if planes is not None:
+        native = self.few_layers.takes(self, cache, ctx) if self.few_layers is not None else None
+        if native is not None:
             h = self.blocks[sched[0].block].mixer_norm.add_norm(x, None, ctx)
-            pending = self.few_layers.run(planes, x, h, ctx, self.final_norm if ctx.rows is not None and ctx.rows_all else None)
-        for i, e in enumerate(sched if planes is None else ()):
+            pending = self.few_layers.run(native, x, h, ctx, self.final_norm if ctx.rows is not None and ctx.rows_all else None)
+        for i, e in enumerate(sched if native is None else ()):
             blk = self.blocks[e.block]
             if isinstance(pending, Cast) and not getattr(blk, "accepts_cast", False):
                 pending = None  # nothing is left to add; this block reads the float32 rows itself

@@ -1,4 +1,7 @@
 """A model's layers launched from one native call (csrc/few_layers.cu) against the same kernels launched part by part: the same bits."""
+import gc
+import weakref
+
 import pytest
 import torch
 
@@ -80,3 +83,34 @@ def test_a_cache_that_does_not_fit_is_refused(native_calls, other, tokens):
     fitting = model.new_cache(max_tokens=128, max_seqs=1)
     model.step(fitting, [bn.SeqStep(fitting.open(), list(range(tokens)), [0])])
     assert len(native_calls) == 1
+
+
+def test_a_weight_set_anew_is_looked_at(native_calls):
+    """Weights of another type or layout than those bound are what the parts make of them, not bits read as bfloat16."""
+    model = Model.from_random(_config(64, 4, 2, 16, 176, 2, False), seed=3, matrix_std=0.125)
+    few = model.few_layers
+    for part, name in ((model.blocks[1].ffn, "w_down"), (model.blocks[0].mixer, "w_qkv"), (model.blocks[1].mixer, "w_o")):
+        old = getattr(part, name)
+        setattr(part, name, old.float())
+        native = _logits(model, [[5, 9, 11]], [[2]], 2)
+        model.few_layers = None
+        parts = _logits(model, [[5, 9, 11]], [[2]], 2)
+        model.few_layers = few
+        assert all(torch.equal(a, b) for a, b in zip(native, parts))
+        setattr(part, name, old)
+    assert not native_calls
+    _logits(model, [[5, 9, 11]], [[2]], 2)
+    assert len(native_calls) == 3
+
+
+def test_a_dropped_model_is_gone():
+    """Nothing of a model refers back to it: its weights are free when the last reference goes, not when the collector runs."""
+    model = Model.from_random(_config(64, 4, 2, 16, 176, 2, False), seed=1)
+    assert model.few_layers is not None
+    gone = weakref.ref(model)
+    gc.disable()
+    try:
+        del model
+        assert gone() is None
+    finally:
+        gc.enable()
