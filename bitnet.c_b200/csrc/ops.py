@@ -954,6 +954,16 @@ def decode_splits(pages: int, blocks_per_split: int) -> int:
     return best
 
 
+def decode_grid(max_len: int, n_seqs: int, n_heads: int, n_kv_heads: int):
+    """(blocks per sequence, cache pages per block) of ``attention_decode_fused`` without a work list."""
+    pages = max(1, (max_len + PAGE - 1) // PAGE)
+    want = decode_splits(pages, n_seqs * n_kv_heads * ((n_heads // n_kv_heads + 15) // 16))
+    if _FORCE_SPLITS:
+        want = max(1, min(pages, _FORCE_SPLITS))
+    pages_per_block = (pages + want - 1) // want
+    return (pages + pages_per_block - 1) // pages_per_block, pages_per_block
+
+
 DECODE_ITEM_BLOCKS = 450  # a work list may come to so many blocks (three per SM run at once)
 _FORCE_ITEM_GROUP = 0  # tests: a work list in groups of this many whatever the batch
 
@@ -1056,13 +1066,7 @@ def attention_decode_fused(qkv: torch.Tensor, k_off: int, v_off: int, out: torch
             _ptr(v_cache), int(k_cache.shape[0]), _ptr(tc_status(qkv.device)), _ptr(part_o), _ptr(part_ml), _ptr(counters),
             int(counters.numel()), _ptr(items), int(items.shape[0]), int(item_group), _stream()), "attention_decode_fused")
         return out
-    pages = max(1, (max_len + PAGE - 1) // PAGE)
-    blocks_per_split = n_seqs * n_kv_heads * ((n_heads // n_kv_heads + 15) // 16)
-    want_splits = decode_splits(pages, blocks_per_split)
-    if _FORCE_SPLITS:
-        want_splits = max(1, min(pages, _FORCE_SPLITS))
-    pages_per_block = (pages + want_splits - 1) // want_splits
-    n_splits = (pages + pages_per_block - 1) // pages_per_block
+    n_splits, pages_per_block = decode_grid(max_len, n_seqs, n_heads, n_kv_heads)
     part_o = torch.empty((n_seqs * n_heads * n_splits * head_dim,), dtype=torch.float32, device=qkv.device)
     part_ml = torch.empty((n_seqs * n_heads * n_splits * 2,), dtype=torch.float32, device=qkv.device)
     _scr, counters = _split_scratch(qkv.device)

@@ -103,7 +103,6 @@ class FewLayers:
         """What ``run`` needs for a step of these tokens: the layers, where their matrices lie, and where their keys and values lie.  None if the step does not go this
         way; every switch that sends a part elsewhere sends the step there too."""
         if not (ctx.n_tokens <= ops.TC_MAX_ROWS and ctx.diag is None and ops.PROFILE is None and ops.USE_TCGEN05 and ops.USE_FUSED_NORM
-                and not ops._FORCE_SPLITS and not ops._FORCE_ITEM_GROUP
                 and (ctx.decode or (ctx.wide_tile_seq is not None and ops.USE_TCGEN05_ATTENTION))):
             return None
         layers = _layers(model)
@@ -143,10 +142,8 @@ class FewLayers:
                 s.items, s.n_items, s.item_group = ctx.decode_items.data_ptr(), ctx.decode_items.shape[0], ctx.decode_item_group
                 splits = ctx.decode_item_group
             else:
-                pages = max(1, (ctx.max_len + ops.PAGE - 1) // ops.PAGE)
-                want = ops.decode_splits(pages, T * spec.n_kv_heads * ((spec.n_heads // spec.n_kv_heads + 15) // 16))
-                s.pages_per_block = (pages + want - 1) // want
-                splits = s.n_splits = (pages + s.pages_per_block - 1) // s.pages_per_block
+                s.n_splits, s.pages_per_block = ops.decode_grid(ctx.max_len, T, spec.n_heads, spec.n_kv_heads)
+                splits = s.n_splits
             part_o, part_ml = T * spec.n_heads * splits * spec.head_dim * 4, T * spec.n_heads * splits * 8
             counters = ops._split_scratch(dev)[1]
             s.tickets, s.n_tickets, s.decoding = counters.data_ptr(), counters.numel(), 1

@@ -1,4 +1,5 @@
 """A model's layers launched from one native call (csrc/few_layers.cu) against the same kernels launched part by part: the same bits."""
+import dataclasses
 import gc
 import weakref
 
@@ -6,8 +7,11 @@ import pytest
 import torch
 
 import bitnet_c_b200 as bn
+from bitnet_c_b200.cache import PAGE
 from bitnet_c_b200.csrc import ops
 from bitnet_c_b200.engine import Model
+from bitnet_c_b200.engine.batch import pack_step
+from bitnet_c_b200.weights import random_parameters
 
 pytestmark = pytest.mark.gpu
 
@@ -114,3 +118,71 @@ def test_a_dropped_model_is_gone():
         assert gone() is None
     finally:
         gc.enable()
+
+
+def _step_of(model, cache, slots, tokens, group):
+    """One token for every sequence; ``group``: with the work list that a recorded step of these lengths would have."""
+    lengths = [cache.length(s) for s in slots]
+    seqs = [bn.SeqStep(s, [t], [0]) for s, t in zip(slots, tokens)]
+    ctx = pack_step(seqs, lengths, model.device)
+    if group:
+        ctx.decode_item_group, items = ops.decode_items([n // PAGE + 1 for n in lengths], model.decode_blocks_per_sequence(),
+                                                        group=None if group < 0 else group)
+        ctx.decode_items = torch.tensor(items, dtype=torch.int32, device=model.device)
+    for s in slots:
+        cache.reserve(s, 1)
+    cache.sync()
+    logits = model.forward(cache, ctx)
+    for s in slots:
+        cache.advance(s, 1)
+    return logits
+
+
+@pytest.mark.parametrize("group", [-1, 1, 2, 3, 0])  # -1: the group that the batch itself asks for; 0: no list
+def test_unequal_lengths_same_bits(native_calls, group):
+    """Steps of a batch of unequal lengths, with a work list and without one."""
+    model = Model.from_random(_config(256, 16, 16, 16, 704, 2, False), seed=5, matrix_std=0.06)
+    lengths = [900, 70, 130, 10, 65, 64, 63, 200, 5, 77]
+    g = torch.Generator().manual_seed(1)
+    prompts = [torch.randint(0, 512, (n,), generator=g).tolist() for n in lengths]
+    out = {}
+    for few in (model.few_layers, None):
+        model.few_layers = few
+        cache = model.new_cache(max_tokens=sum(-(-(n + 4) // 64) * 64 for n in lengths), max_seqs=len(lengths))
+        slots = [cache.open() for _ in lengths]
+        for s, p in zip(slots, prompts):
+            model.step(cache, [bn.SeqStep(s, p, ())])
+        del native_calls[:]
+        out[few] = [_step_of(model, cache, slots, [(7 * i + s) % 512 for s in range(len(slots))], group) for i in range(3)]
+        assert len(native_calls) == (3 if few is not None else 0)
+        assert all(bool(c.items) == bool(group) for c in native_calls)
+    a, b = out.values()
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("forced", [0, 12])  # 12: more blocks a sequence than one cluster has, merged through global memory
+@pytest.mark.parametrize("window", [0, 100])
+def test_split_sequences_and_windows_same_bits(native_calls, monkeypatch, forced, window):
+    """Long sequences, whose pages several blocks share, and layers that see the last ``window`` keys only."""
+    base = Model.from_random(_config(64, 4, 2, 16, 176, 2, False), seed=3, matrix_std=0.125)
+    blocks = tuple(dataclasses.replace(b, mixer=dataclasses.replace(b.mixer, window=window)) for b in base.spec.blocks)
+    model = Model(dataclasses.replace(base.spec, blocks=blocks), arch=base.arch, config=base.config)
+    model.bind({path: t for path, _name, t in random_parameters(model.spec, base.arch.tensor_name, 3, model.dtype, 0.125, 0.1, model.device)})
+    few = model.few_layers
+    assert few is not None
+    monkeypatch.setattr(ops, "_FORCE_SPLITS", forced)
+    g = torch.Generator().manual_seed(1)
+    pieces = [torch.randint(0, 512, (n,), generator=g).tolist() for n in (1500, 40, 64)]  # the last two: prompts of few tokens behind a long one
+    out = {}
+    for f in (few, None):
+        model.few_layers = f
+        cache = model.new_cache(max_tokens=1664, max_seqs=1)
+        slot = cache.open()
+        del native_calls[:]
+        got = [model.step(cache, [bn.SeqStep(slot, p, [len(p) - 1])]) for p in pieces]
+        got += [model.step(cache, [bn.SeqStep(slot, [i], [0])]) for i in range(3)]
+        out[f] = got
+        assert len(native_calls) == (5 if f is not None else 0)
+        assert all(c.window == window for c in native_calls) and all(c.n_splits > 1 for c in native_calls[2:])
+    a, b = out.values()
+    assert all(torch.equal(x, y) for x, y in zip(a, b))

@@ -274,9 +274,9 @@ def test_a_work_list_for_unequal_lengths_changes_no_tokens(tmp_path, cuda_device
     base = bn.generate(model, prompts, max_new_tokens=new, stop_ids=[])
     assert _tokens_that_are_the_plain_choice(pcfg, w, prompts, base, "bfloat16") >= 0.9 * sum(new)
     monkeypatch.setattr(ops, "_FORCE_ITEM_GROUP", group)
-    calls = []
-    real = ops.attention_decode_fused
-    monkeypatch.setattr(ops, "attention_decode_fused", lambda *a, **k: (calls.append(k.get("item_group", 0)), real(*a, **k))[1])
+    calls = []  # the layers' native calls
+    real = ops.few_layers
+    monkeypatch.setattr(ops, "few_layers", lambda step, launches: (calls.append(step.item_group), real(step, launches))[1])
     got = bn.generate(model, prompts, max_new_tokens=new, stop_ids=[])
     assert group in calls  # the recorded steps were made with the list
     assert [len(g.tokens) for g in got] == new
