@@ -1162,7 +1162,8 @@ def check_tc_status(device) -> None:
                 4: "attention_decode_tc: a cache page never arrived (TMA load)",
                 5: "attention_prefill_tc: a wait inside the kernel gave up",
                 6: "linear_tc: a slice of partial sums from another block of the cluster never arrived",
-                7: "gemm_tc: a wait inside the kernel gave up"}.get(code, f"code {code}")
+                7: "gemm_tc: a wait inside the kernel gave up",
+                8: "linear_split: a wait inside the kernel gave up"}.get(code, f"code {code}")
         raise KernelError(f"{what}; the result of that launch is not valid")
 
 
