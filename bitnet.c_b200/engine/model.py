@@ -104,7 +104,8 @@ class Model:
         return max((b.decode_blocks_per_sequence() for b in self.blocks), default=0)
 
     def kernel_families(self) -> List[str]:
-        fams = ["embed", "linear", "linear_resident" if self.dtype == torch.bfloat16 else "linear_split"]
+        # (a model in bfloat16 may have parameters that stay float32: their products of many rows are linear_split's)
+        fams = ["embed", "linear", "linear_split"] + (["linear_resident"] if self.dtype == torch.bfloat16 else [])
         for blk in self.blocks:
             fams.extend(blk.all_kernels())
         fams.extend(self.final_norm.all_kernels())

@@ -100,3 +100,11 @@ def test_schedule_validation():
         with_schedule([ScheduleEntry(0, cache_of=0)]).validate()
     with pytest.raises(ConfigError, match="owns none"):
         with_schedule([ScheduleEntry(0), ScheduleEntry(1, cache_of=0), ScheduleEntry(1, cache_of=1)]).validate()
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_a_model_lists_the_kernels_of_products_in_float32(dtype):
+    """They are compiled when the model is made and not during a request: a model in bfloat16 may have parameters that its file keeps in float32."""
+    from bitnet_c_b200.engine import Model
+    families = Model(LlamaConfig.from_dict(TINY_A).to_spec(), dtype=dtype, device=None).kernel_families()
+    assert {"linear", "linear_split"} <= set(families) and ("linear_resident" in families) == (dtype == "bfloat16")
