@@ -1517,14 +1517,15 @@ def linear(x, w: torch.Tensor, out_dtype: Optional[torch.dtype] = None, swiglu: 
             if torch.backends.cuda.matmul.allow_tf32:
                 raise KernelError("float32 products need torch.backends.cuda.matmul.allow_tf32 = False")
             if K % 4 == 0 and (x.data_ptr() | w.data_ptr()) % 16 == 0 and linear_split_pays(M, N, K):
-                product = lambda: linear_split(x, w, bias)
+                out, product = linear_split(x, w, bias), None
             else:
                 product = lambda: torch.matmul(x, w.t()) if bias is None else torch.addmm(bias, x, w.t())
         elif out_dtype == torch.float32:
             product = lambda: torch.mm(x, w.t(), out_dtype=torch.float32) if bias is None else torch.mm(x, w.t(), out_dtype=torch.float32).add_(bias)
         else:  # (biases that come from the file in the compute type lose nothing by going back to it)
             product = lambda: torch.matmul(x, w.t()) if bias is None else torch.addmm(bias.to(w.dtype), x, w.t())
-        out = product() if PROFILE is None else _timed("library.matmul", product)
+        if product is not None:
+            out = product() if PROFILE is None else _timed("library.matmul", product)
         out = out if out.dtype == out_dtype else out.to(out_dtype)
     if squared:
         return relu_squared(out)

@@ -74,3 +74,13 @@ def test_float32_products_go_by_one_rule(monkeypatch):
             ops.linear(x, w)
         monkeypatch.setattr(torch.backends.cuda.matmul, "allow_tf32", False)
     assert (out[True] - out[False]).norm() <= 3e-6 * out[False].norm()
+
+
+def test_profile_counts_a_product_once(monkeypatch):
+    """While kernel classes are timed, a float32 product stands under the kernel that ran it and nowhere else."""
+    x, w = _pair(70, 256, 512, 9)
+    for chosen, key in ((True, "linear_split.bn_linear_split"), (False, "library.matmul")):
+        monkeypatch.setattr(ops, "linear_split_pays", lambda *a: chosen)
+        monkeypatch.setattr(ops, "PROFILE", {})
+        ops.linear(x, w)
+        assert {k: len(v) for k, v in ops.PROFILE.items()} == {key: 1}
