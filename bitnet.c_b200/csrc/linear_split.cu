@@ -308,7 +308,6 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
           if (c0 + j * 16 < a.nt) {
             float v[16];
             tmem_ld16(from0 + b * LS_ACC_COLS + j * 16, v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int c = 0; c < 16; ++c) acc[j * 16 + c] += v[c];
           }

@@ -298,9 +298,10 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const int c0 = ((warp - 2) >> 2) * COLS;
     float v[COLS];
     if (s_acc_ok) {
-#pragma unroll
-      for (int c = 0; c < COLS; c += 16) tmem_ld16(tmem_base + ((unsigned)(quad * 32) << 16) + c0 + c, v + c);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      const unsigned from = tmem_base + ((unsigned)(quad * 32) << 16) + c0;
+      static_assert(COLS == 16 || COLS == 32, "a load is as wide as the thread's columns");
+      if constexpr (COLS == 32) tmem_ld32(from, v);
+      else tmem_ld16(from, v);
     } else {
 #pragma unroll
       for (int c = 0; c < COLS; ++c) v[c] = 0.f;

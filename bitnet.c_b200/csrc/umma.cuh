@@ -39,6 +39,7 @@ __device__ __forceinline__ void umma_mma_ts(unsigned tmem_d, unsigned tmem_a, un
 __device__ __forceinline__ void umma_commit(unsigned bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// Loads of tensor memory: the wait is part of the same statement, so that nothing that uses the registers can be scheduled in front of it.
 // 32 consecutive columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld32(unsigned addr, float* v) {
   unsigned r[32];
@@ -54,8 +55,7 @@ __device__ __forceinline__ void tmem_ld32(unsigned addr, float* v) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
-// 64 consecutive columns of this thread's TMEM lane; the wait is part of the same statement so that
-// nothing that uses the registers can be scheduled in front of it
+// 64 consecutive columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld64(unsigned addr, float* v) {
   unsigned r[64];
   asm volatile(
@@ -112,15 +112,15 @@ __device__ __forceinline__ unsigned pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<unsigned*>(&v);
 }
-// 16 consecutive columns of this thread's TMEM lane (the wait is the caller's: several loads may be in flight)
+// 16 consecutive columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld16(unsigned addr, float* v) {
   unsigned r[16];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(addr));
+      : "r"(addr) : "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-

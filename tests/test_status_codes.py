@@ -32,3 +32,15 @@ def test_every_code_names_its_kernel(monkeypatch, family, name, code):
     with pytest.raises(ops.KernelError, match=rf"^{family}: "):
         ops.check_tc_status(cpu)
     ops.check_tc_status(cpu)  # reported once
+
+
+def test_loads_of_tensor_memory_wait_in_their_own_statement():
+    """A load's registers are valid behind its wait only, and nothing ties a use of them to a wait in a statement of its own."""
+    seen = 0
+    for path in sorted(glob.glob(os.path.join(os.path.dirname(build.__file__), "*.cu*"))):
+        with open(path) as f:
+            for statement in re.findall(r"asm volatile\((.*?)\);", f.read(), re.S):
+                if "tcgen05.ld" in statement or "tcgen05.wait::ld" in statement:
+                    seen += 1
+                    assert "tcgen05.ld" in statement and "tcgen05.wait::ld" in statement, (os.path.basename(path), statement[:80])
+    assert seen >= 3
