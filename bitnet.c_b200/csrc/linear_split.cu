@@ -87,8 +87,8 @@ __device__ __forceinline__ unsigned ls_size(float v) { return __float_as_uint(v)
 // planes [3][M][pitch] bfloat16 and the marks of x [M, K]; a block per row
 __global__ void __launch_bounds__(256) linear_split_rows_kernel(const float* __restrict__ x, int M, int K, int pitch, __nv_bfloat16* __restrict__ planes,
                                                                  int* __restrict__ marked) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();  // (not before: the product's blocks read W without a wait of their own, and the kernel in front may have written it)
   const int m = blockIdx.x;
   const float* row = x + (size_t)m * K;
   const size_t plane = (size_t)M * pitch;

@@ -84,3 +84,15 @@ def test_profile_counts_a_product_once(monkeypatch):
         monkeypatch.setattr(ops, "PROFILE", {})
         ops.linear(x, w)
         assert {k: len(v) for k, v in ops.PROFILE.items()} == {key: 1}
+
+
+def test_linear_split_of_a_matrix_that_was_just_written():
+    """W, like x, may be what the kernel in front of the product writes."""
+    x, w = _pair(64, 8192, 2048, 4)
+    clean = ops.linear_split(x, w)
+    for i in range(1, 21):
+        w1 = w.clone()
+        torch.cuda.synchronize()
+        ops.scale_softcap(w1, 2.0 ** i, 0.0)  # a kernel of the library, which lets the next one start early
+        got = ops.linear_split(x, w1)
+        assert torch.equal(got, clean * 2.0 ** i)
