@@ -23,8 +23,11 @@
 //   warps 4-11  split W: shared memory -> registers -> tensor memory, two groups of four warps with a buffer each take turns
 //   warps 12-19 add the accumulators up in registers (a row of W each thread, two warps share a row's columns) and store
 //
-// Numbers that are not finite, or round to infinity in bfloat16, do not split.  Rows that have one are marked (of x by the kernel that
-// splits it, of W by the warps that do); outputs of marked rows are computed again in plain float32.
+// Three bfloat16 numbers hold a float32 only while the last of them is no subnormal number (below 2^-109 bits were lost), so both operands are
+// scaled by 2^24 first, which takes float32's smallest numbers there, and the sums are scaled back.  Products and sums stay finite while
+// numbers are below 2^30; a row of x with a larger one has a smaller scale of its own.  What does not split (rows of x with numbers that are not
+// finite, or so far apart that the smallest lose bits; rows of W with a number of 2^30 or more, or not finite) is marked, of x by the kernel
+// that splits it, of W by the warps that do, and outputs of marked rows are computed again in plain float32.
 //
 // The twelve MMAs of 32 numbers take 1,060 cycles for 176 rows of x; a wait for an mbarrier costs its role some 200, even if it is over.  So
 // the whole of warp 2 walks its loop, with descriptors in uniform registers, and one elected lane issues (as one thread's work a step took 1,700
@@ -57,7 +60,7 @@
 struct LsArgs {
   float* out;
   const float *x, *w, *bias;
-  const int* x_marked;  // [M]
+  const float* x_unscale;  // [M] what takes a sum back to x's and W's own scale; 0: a marked row
   int M, N, K, ldo, k_blocks;
   int nt, m_tiles, n_tiles, x_stages;
   int* status;
@@ -80,32 +83,65 @@ __device__ __forceinline__ void ls_cut(float a, float b, unsigned& high, unsigne
   mid = __byte_perm(va, vb, 0x7632);
   low = __byte_perm(__float_as_uint(ra - __uint_as_float(va & 0xffff0000u)), __float_as_uint(rb - __uint_as_float(vb & 0xffff0000u)), 0x7632);
 }
-// No split: infinities, what is not a number, and what a rounding to bfloat16 may make infinite
-__device__ __forceinline__ unsigned ls_size(float v) { return __float_as_uint(v) & 0x7fffffffu; }
-#define LS_TOO_LARGE 0x7f000000u
+#define LS_SCALE 16777216.0f  // 2^24
+#define LS_LARGE 1073741824.0f  // 2^30
+#define LS_MARK 316912650057057350374175801344.0f  // 2^98: LS_LARGE times it is infinite
+#define LS_MAX_K (1 << 18)  // products below 2^54 2^54, so many of them below 2^127
+__device__ __forceinline__ float ls_power(int e) { return __uint_as_float((unsigned)(e + 127) << 23); }  // 2^e, a normal number
 
-// planes [3][M][pitch] bfloat16 and the marks of x [M, K]; a block per row
+// planes [3][M][pitch] bfloat16 and the scales of x [M, K]; a block per row
 __global__ void __launch_bounds__(256) linear_split_rows_kernel(const float* __restrict__ x, int M, int K, int pitch, __nv_bfloat16* __restrict__ planes,
-                                                                 int* __restrict__ marked) {
+                                                                 float* __restrict__ unscale) {
   pdl_wait();
   pdl_launch_dependents();  // (not before: the product's blocks read W without a wait of their own, and the kernel in front may have written it)
+  __shared__ unsigned s_most[8];
   const int m = blockIdx.x;
   const float* row = x + (size_t)m * K;
   const size_t plane = (size_t)M * pitch;
   __nv_bfloat16* to = planes + (size_t)m * pitch;
-  unsigned most = 0;
-  for (int k = threadIdx.x * 4; k < K; k += 1024) {  // K is a multiple of 4
-    const float4 v = *reinterpret_cast<const float4*>(row + k);
-    most = max(max(most, max(ls_size(v.x), ls_size(v.y))), max(ls_size(v.z), ls_size(v.w)));
-    uint2 h, i, l;
-    ls_split(v.x, v.y, h.x, i.x, l.x);
-    ls_split(v.z, v.w, h.y, i.y, l.y);
-    *reinterpret_cast<uint2*>(to + k) = h;
-    *reinterpret_cast<uint2*>(to + plane + k) = i;
-    *reinterpret_cast<uint2*>(to + 2 * plane + k) = l;
+  unsigned most = 0;  // (sizes of numbers are in the order of their bits, behind them infinities and what is not a number)
+  bool lost = false;
+  auto rows = [&](float scale, auto look) {
+    for (int k = threadIdx.x * 4; k < K; k += 1024) {  // K is a multiple of 4
+      const float4 v = *reinterpret_cast<const float4*>(row + k);
+      const float a = v.x * scale, b = v.y * scale, c = v.z * scale, d = v.w * scale;
+      uint2 h, i, l;
+      ls_split(a, b, h.x, i.x, l.x);
+      ls_split(c, d, h.y, i.y, l.y);
+      *reinterpret_cast<uint2*>(to + k) = h;
+      *reinterpret_cast<uint2*>(to + plane + k) = i;
+      *reinterpret_cast<uint2*>(to + 2 * plane + k) = l;
+      look(v, h, i, l);
+    }
+  };
+  rows(LS_SCALE, [&](float4 v, uint2, uint2, uint2) {
+    const unsigned ab = max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu);
+    most = max(max(most, ab), max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu));
+  });
+  if (!__syncthreads_or(most >= __float_as_uint(LS_LARGE))) {
+    if (threadIdx.x == 0) unscale[m] = 1.0f / (LS_SCALE * LS_SCALE);
+    return;
   }
-  const int any = __syncthreads_or(most >= LS_TOO_LARGE);
-  if (threadIdx.x == 0) marked[m] = any;
+  // a row with large numbers: its largest goes to [2^53, 2^54)
+  most = __reduce_max_sync(0xffffffffu, most);
+  if ((threadIdx.x & 31) == 0) s_most[threadIdx.x >> 5] = most;
+  __syncthreads();
+  for (int i = 0; i < 8; ++i) most = max(most, s_most[i]);
+  if (most >= 0x7f800000u) {
+    if (threadIdx.x == 0) unscale[m] = 0.f;
+    return;
+  }
+  const int e = 53 - ((int)(most >> 23) - 127);
+  const float back = ls_power(-e);
+  rows(ls_power(e), [&](float4 v, uint2 h, uint2 i, uint2 l) {
+    auto whole = [&](float one, unsigned high, unsigned mid, unsigned low, bool upper) {  // whether the parts add up to the number
+      auto part = [&](unsigned p) { return __uint_as_float(upper ? p & 0xffff0000u : p << 16); };
+      return ((part(high) + part(mid)) + part(low)) * back == one;
+    };
+    lost |= !(whole(v.x, h.x, i.x, l.x, false) & whole(v.y, h.x, i.x, l.x, true) & whole(v.z, h.y, i.y, l.y, false) & whole(v.w, h.y, i.y, l.y, true));
+  });
+  lost = __syncthreads_or(lost);
+  if (threadIdx.x == 0) unscale[m] = lost ? 0.f : back * (1.0f / LS_SCALE);
 }
 
 // K-major tile with rows of 64 bytes, 64-byte swizzled: groups of 8 rows 512 bytes apart
@@ -253,10 +289,10 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       unsigned high[16], mid[16], low[16];
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        ls_cut(v[c].x, v[c].y, high[2 * c], mid[2 * c], low[2 * c]);
-        ls_cut(v[c].z, v[c].w, high[2 * c + 1], mid[2 * c + 1], low[2 * c + 1]);
-        // zero, or not a number once a number is not finite
-        none = fmaf(v[c].x, 0.f, fmaf(v[c].y, 0.f, fmaf(v[c].z, 0.f, fmaf(v[c].w, 0.f, none))));
+        ls_cut(v[c].x * LS_SCALE, v[c].y * LS_SCALE, high[2 * c], mid[2 * c], low[2 * c]);
+        ls_cut(v[c].z * LS_SCALE, v[c].w * LS_SCALE, high[2 * c + 1], mid[2 * c + 1], low[2 * c + 1]);
+        // finite, until a number is 2^30 or more, or not finite (or their sum is: such a row is marked without need)
+        none = fmaf(v[c].x, LS_MARK, fmaf(v[c].y, LS_MARK, fmaf(v[c].z, LS_MARK, fmaf(v[c].w, LS_MARK, none))));
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(w_free + 8 * s);
@@ -270,7 +306,7 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       tmem_st16(to + 32, reinterpret_cast<const float*>(low));
       const bool last = kb + 2 >= a.k_blocks;  // this group's last step of the tile
       // (the adding warps have read the marks of two tiles before: a tile has at least four steps)
-      if (last) w_marked[tile_i & 1][group][row] = none != 0.f;
+      if (last) w_marked[tile_i & 1][group][row] = !(fabsf(none) <= 3.402823466e38f);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -333,8 +369,9 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         for (int c = 0; c < 16 * CH; ++c) {
           const int m = m0 + c;
           if (m < m_end) {
-            float v = acc[c];
-            if (row_marked | a.x_marked[m]) v = ls_plain(a.x + (size_t)m * a.K, a.w + (size_t)n * a.K, a.K);
+            const float back = a.x_unscale[m];
+            float v = acc[c] * back;
+            if (row_marked | (back == 0.f)) v = ls_plain(a.x + (size_t)m * a.K, a.w + (size_t)n * a.K, a.K);
             a.out[(size_t)m * a.ldo + n] = v + bias;
           }
         }
@@ -408,21 +445,21 @@ static bool ls_registers() {
   return enough;
 }
 
-// Bytes of working space for M rows of K numbers: three planes of bfloat16 and a mark per row.
+// Bytes of working space for M rows of K numbers: three planes of bfloat16 and a scale per row.
 extern "C" long long bn_linear_split_scratch(int M, int K) { return 6ll * M * ((K + 7) / 8 * 8) + 4ll * M; }
 
-// x [M, K], w [N, K], out [M, ldo] float32, all 16-byte aligned with K a multiple of 4 and at least 128; bias [N] or null; scratch as above.
+// x [M, K], w [N, K], out [M, ldo] float32, all 16-byte aligned with K a multiple of 4, 128 to 262,144; bias [N] or null; scratch as above.
 extern "C" int bn_linear_split(const float* x, const float* w, const float* bias, float* out, int M, int N, int K, int ldo, void* scratch,
                                int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return BN_OK;
-  if (!x || !w || !out || !scratch || !status || K < 4 * LS_BK || K % 4 || ldo < N || ((uintptr_t)x | (uintptr_t)w | (uintptr_t)scratch) & 15 ||
+  if (!x || !w || !out || !scratch || !status || K < 4 * LS_BK || K % 4 || K > LS_MAX_K || ldo < N || ((uintptr_t)x | (uintptr_t)w | (uintptr_t)scratch) & 15 ||
       M > (1 << 28))
     return BN_ERR_BAD_ARG;
   const int pitch = (K + 7) / 8 * 8;
   __nv_bfloat16* planes = (__nv_bfloat16*)scratch;
-  int* marked = (int*)((unsigned char*)scratch + 6ll * M * pitch);
+  float* unscale = (float*)((unsigned char*)scratch + 6ll * M * pitch);
   LsArgs a = {};
-  a.out = out; a.x = x; a.w = w; a.bias = bias; a.x_marked = marked;
+  a.out = out; a.x = x; a.w = w; a.bias = bias; a.x_unscale = unscale;
   a.M = M; a.N = N; a.K = K; a.ldo = ldo; a.k_blocks = (K + LS_BK - 1) / LS_BK; a.status = status;
   a.n_tiles = (N + LS_BM - 1) / LS_BM;
   a.nt = ls_choose_nt(M, a.n_tiles, ls_sm_count());
@@ -432,7 +469,7 @@ extern "C" int bn_linear_split(const float* x, const float* w, const float* bias
   a.x_stages = room / x_bytes < LS_X_STAGES_MAX ? room / x_bytes : LS_X_STAGES_MAX;
   CUtensorMap mw, mx;
   if (!ls_map(&mw, 3, w, N, K, 4ull * K, LS_BM) || !ls_map(&mx, 4, planes, 3ull * M, K, 2ull * pitch, a.nt)) return BN_ERR_BAD_ARG;
-  BN_LAUNCH(linear_split_rows_kernel, M, 256, 0, stream, x, M, K, pitch, planes, marked);
+  BN_LAUNCH(linear_split_rows_kernel, M, 256, 0, stream, x, M, K, pitch, planes, unscale);
   const size_t smem = 1024 + LS_W_STAGES * LS_W_BYTES + (size_t)a.x_stages * x_bytes;
   const int tiles = a.n_tiles * a.m_tiles, grid = tiles < ls_sm_count() ? tiles : ls_sm_count();
 #define LS_RUN(CH)                                                                                       \

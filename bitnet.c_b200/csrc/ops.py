@@ -1549,7 +1549,7 @@ def linear_split_pays(M: int, N: int, K: int) -> bool:
     16384 x 256 to 28672 x 4096), unless the inner dimension is so long that the library splits it (2048 x 8192 0.76 to 1.26, 4096 x 14336 1.27);
     100 and more rows of 1,024 x 2,048, 1,536 x 4,096, 1024 x 14336 1.2 to 2.1.  A matrix of fewer rows leaves most SMs idle: 17 rows 1024 x 4096
     0.5, 512 x 2048 0.54.  Short inner dimensions leave it its start: 4,000 x 256 x 256 0.6."""
-    if K < 128:  # the kernel's least
+    if not 128 <= K <= 1 << 18:  # the kernel's least and most
         return False
     if M * N >= 1 << 20 and M >= 48 and M * N * K >= 1 << 30:
         return True
@@ -1560,7 +1560,7 @@ def linear_split_pays(M: int, N: int, K: int) -> bool:
 
 def linear_split(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """x[M, K] . w[N, K]^T + bias in float32 on the tensor cores, from operands split into three bfloat16 numbers each
-    (linear_split.cu): as exact as float32 sums.  K a multiple of 4 and at least 128."""
+    (linear_split.cu): as exact as float32 sums.  K a multiple of 4, 128 to 262,144."""
     _need(x, "x", torch.float32, 2)
     _need(w, "w", torch.float32, 2)
     M, K = x.shape

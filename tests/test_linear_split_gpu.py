@@ -96,3 +96,42 @@ def test_linear_split_of_a_matrix_that_was_just_written():
         ops.scale_softcap(w1, 2.0 ** i, 0.0)  # a kernel of the library, which lets the next one start early
         got = ops.linear_split(x, w1)
         assert torch.equal(got, clean * 2.0 ** i)
+
+
+def _as_exact_as_float32(x, w, K):
+    """``linear_split`` against 64 bits: within its bound (numbers below the smallest normal one are rounded at 2^-149), and no less exact than the
+    float32 product."""
+    got, plain = ops.linear_split(x, w), torch.matmul(x, w.t())
+    ops.check_tc_status(x.device)
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert ((got.double() - want).abs() <= (12 + K / 64 + 2) * 2.0 ** -23 * size + 2.0 ** -149).all()
+    err = lambda y: float((y.double() - want).norm() / want.norm())
+    assert err(got) <= max(1.05 * err(plain), 1.5e-7)
+
+
+@pytest.mark.parametrize("x_scale,w_scale", [(1e-33, 1.0), (1e-34, 1.0), (1e-35, 30.0), (1.0, 1e-34), (1.0, 1e-35), (3e6, 1e-38), (1e-19, 1e-15),
+                                             (1e9, 1.0), (1e20, 1e-20), (1e37, 1e-3), (1e30, 1e-38), (1.0, 1e8)])
+def test_linear_split_of_very_small_and_large_numbers(x_scale, w_scale):
+    """Operands far below and above one keep all their bits."""
+    x, w = _pair(40, 200, 256, 6)
+    _as_exact_as_float32(x * x_scale, w * w_scale, 256)
+
+
+def test_linear_split_of_rows_of_all_sizes():
+    """Rows, and numbers within a row, of very different sizes; where the large ones of x meet zeros, the small ones alone make the result."""
+    x, w = _pair(48, 200, 256, 7)
+    x[::3] *= 1e-35
+    x[1::6] *= 1e25
+    w[::2] *= 1e-34
+    got, want = ops.linear_split(x, w).double(), x.double() @ w.double().t()
+    size = x.double().abs() @ w.double().abs().t()
+    assert ((got - want).abs() <= (12 + 4 + 2) * 2.0 ** -23 * size + 2.0 ** -149).all()
+    for large in (1.0, 1e12, 1e30):  # 1e30 beside 1e-35: too far apart to be split
+        x, w = _pair(40, 200, 256, 8)
+        x[:, :128] *= large
+        x[:, 128:] *= 1e-35
+        w[:, :128] = 0
+        _as_exact_as_float32(x, w, 256)
+    x, w = _pair(40, 200, 256, 8)
+    w[5, 9], w[7, 3] = 3e9, -1e30  # weights that are not split
+    _as_exact_as_float32(x, w, 256)
