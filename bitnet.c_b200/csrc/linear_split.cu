@@ -27,7 +27,10 @@
 // scaled by 2^24 first, which takes float32's smallest numbers there, and the sums are scaled back.  Products and sums stay finite while
 // numbers are below 2^30; a row of x with a larger one has a smaller scale of its own.  What does not split (rows of x with numbers that are not
 // finite, or so far apart that the smallest lose bits; rows of W with a number of 2^30 or more, or not finite) is marked, of x by the kernel
-// that splits it, of W by the warps that do, and outputs of marked rows are computed again in plain float32.
+// that splits it, of W by the warps that do, and outputs of marked rows are computed again in plain float32 by the warps that add, four rows of W times four of x at a
+// time (520 rows, 4096 x 4096, 131 us: with one marked row of W 582, of x 283, with all rows marked 2,660; a thread per output took 14,700, 600 and
+// 69,000.  The other warps wait meanwhile: a tile whose rows are all marked takes 2 ms at K = 4,096 and less than a tenth of their limit at
+// the largest K).
 //
 // The twelve MMAs of 32 numbers take 1,060 cycles for 176 rows of x; a wait for an mbarrier costs its role some 200, even if it is over.  So
 // the whole of warp 2 walks its loop, with descriptors in uniform registers, and one elected lane issues (as one thread's work a step took 1,700
@@ -148,11 +151,48 @@ __global__ void __launch_bounds__(256) linear_split_rows_kernel(const float* __r
 __device__ __forceinline__ unsigned long long ls_desc(unsigned addr) {
   return (unsigned long long)((addr >> 4) & 0x3FFF) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
 }
-// An output of a marked row, in plain float32
-__device__ __noinline__ float ls_plain(const float* x, const float* w, int K) {
-  float s = 0.f;
-  for (int k = 0; k < K; ++k) s = fmaf(x[k], w[k], s);
-  return s;
+// The outputs of marked rows among rows n0 .. n0 + 31 of W (bit i of `rows`: n0 + i is marked) and m0 .. m_end - 1 of x, in plain float32: a warp takes
+// four by four at a time, its lanes share the inner dimension.
+__device__ __noinline__ void ls_plain(const LsArgs& a, unsigned rows, int n0, int m0, int m_end, int lane) {
+  for (int m = m0; m < m_end; m += 4) {
+    unsigned cols = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (m + j < m_end && a.x_unscale[m + j] == 0.f) cols |= 1u << j;
+    for (int i0 = 0; i0 < 32 && n0 + i0 < a.N; i0 += 4) {
+      const unsigned some = (rows >> i0) & 15u;
+      if ((some | cols) == 0) continue;
+      const float *w[4], *x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        w[i] = a.w + (size_t)min(n0 + i0 + i, a.N - 1) * a.K;
+        x[i] = a.x + (size_t)min(m + i, m_end - 1) * a.K;
+      }
+      float sum[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sum[i] = 0.f;
+      for (int k = lane * 4; k < a.K; k += 128) {
+        float4 wv[4], xv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          wv[i] = *reinterpret_cast<const float4*>(w[i] + k);
+          xv[i] = *reinterpret_cast<const float4*>(x[i] + k);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          sum[i] = fmaf(wv[i >> 2].x, xv[i & 3].x, fmaf(wv[i >> 2].y, xv[i & 3].y, fmaf(wv[i >> 2].z, xv[i & 3].z, fmaf(wv[i >> 2].w, xv[i & 3].w, sum[i]))));
+      }
+      float mine = 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float s = warp_sum(sum[i]);
+        if (lane == i) mine = s;
+      }
+      const int i = lane >> 2, j = lane & 3, n = n0 + i0 + i;
+      if (lane < 16 && ((some >> i | cols >> j) & 1u) && n < a.N && m + j < m_end)
+        a.out[(size_t)(m + j) * a.ldo + n] = mine + (a.bias != nullptr ? a.bias[n] : 0.f);
+    }
+  }
 }
 
 template <int CH>  // an adding warp takes 16 CH columns, the tile has up to 32 CH
@@ -361,22 +401,20 @@ linear_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         pdl_wait();
         waited = true;
       }
-      const int n = t / a.m_tiles * LS_BM + row, m0 = t % a.m_tiles * a.nt + c0;
-      if (n < a.N) {
-        const float bias = a.bias != nullptr ? a.bias[n] : 0.f;
-        const int m_end = min(a.M, t % a.m_tiles * a.nt + a.nt);
+      const int n = t / a.m_tiles * LS_BM + row, m0 = t % a.m_tiles * a.nt + c0, m_end = min(a.M, t % a.m_tiles * a.nt + a.nt);
+      const float bias = n < a.N && a.bias != nullptr ? a.bias[n] : 0.f;
+      bool plain = row_marked && n < a.N;
 #pragma unroll
-        for (int c = 0; c < 16 * CH; ++c) {
-          const int m = m0 + c;
-          if (m < m_end) {
-            const float back = a.x_unscale[m];
-            float v = acc[c] * back;
-            if (row_marked | (back == 0.f)) v = ls_plain(a.x + (size_t)m * a.K, a.w + (size_t)n * a.K, a.K);
-            a.out[(size_t)m * a.ldo + n] = v + bias;
-          }
+      for (int c = 0; c < 16 * CH; ++c) {
+        const int m = m0 + c;
+        if (m < m_end) {
+          const float back = a.x_unscale[m];
+          plain |= back == 0.f;
+          if (n < a.N) a.out[(size_t)m * a.ldo + n] = fmaf(acc[c], back, bias);
         }
       }
-      __syncwarp();
+      __syncwarp();  // (of two stores to one place the second one stays)
+      if (__any_sync(0xffffffffu, plain)) ls_plain(a, __ballot_sync(0xffffffffu, row_marked), n - lane, m0, min(m_end, m0 + 16 * CH), lane);
     }
   }
 

@@ -135,3 +135,26 @@ def test_linear_split_of_rows_of_all_sizes():
     x, w = _pair(40, 200, 256, 8)
     w[5, 9], w[7, 3] = 3e9, -1e30  # weights that are not split
     _as_exact_as_float32(x, w, 256)
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 130, 132), (193, 300, 1000), (100, 19100, 160)])
+@pytest.mark.parametrize("of_x,of_w", [([0], []), ([], [0]), ([3, 16], [5, 129]), (slice(None), []), ([], slice(None))])
+def test_linear_split_marked_rows(M, N, K, of_x, of_w):
+    """Rows that do not split, at the edges of tiles and all at once: what float32 sums give, and the others' bits untouched."""
+    x, w = _pair(M, N, K, M)
+    b = torch.randn(N, device="cuda")
+    clean = ops.linear_split(x, w, b)
+    x1, w1 = x.clone(), w.clone()
+    x1[of_x, K // 2] = 3e38
+    x1[of_x, K // 3] = 1e-38  # too far apart
+    w1[of_w, K - 1] = 2e9
+    got, want = ops.linear_split(x1, w1, b).double(), torch.addmm(b.double(), x1.double(), w1.double().t())
+    size = x1.double().abs() @ w1.double().abs().t() + b.double().abs()
+    fits = size < 3e38  # (sums may become infinite on the way, in any order)
+    assert ((got - want).abs()[fits] <= (K / 32 + 8) * 2.0 ** -23 * size[fits]).all()
+    x1[of_x, 1], w1[of_w, 2] = float("nan"), float("inf")
+    got = ops.linear_split(x1, w1, b)
+    rows, cols = torch.ones(M, dtype=torch.bool, device="cuda"), torch.ones(N, dtype=torch.bool, device="cuda")
+    rows[of_x], cols[of_w] = False, False
+    assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
+    assert got[~rows].isnan().all() and not got[rows][:, ~cols].isfinite().any()
