@@ -1,11 +1,12 @@
 // out[M, N] = x[M, K] . W[N, K]^T (+ a bias) in float32 for many rows, on the 5th-generation tensor cores (tcgen05).
 //
-// A float32 number is the sum of three bfloat16 numbers, exactly: its leading eight bits, the next eight, and what is left (rounded or cut off,
-// the rest has at most eight bits).  Of the nine products of two such sums six are kept (high x high, the two of high x middle,
-// middle x middle, the two of high x low); the other three are below 2^-24 of the product.  The tensor cores multiply them exactly and add
-// them up in their accumulator, which cuts off where an addition rounds, so a sum stays there for 32 numbers of the inner dimension only (small
-// products first) and is then added in float32: the error against 64 bits is a third to a sixth of the float32 library product's
-// (520 rows, 4096 x 4096: 2.2e-7 against 1.1e-6 of the result's norm; 1024 x 14336: 3.9e-7 against 2.2e-6).
+// A float32 number is the sum of three bfloat16 numbers, exactly: its leading eight bits, the next eight, and what is left, at most eight bits.
+// x's are rounded, W's cut off: beside the power of two at or below a number, x's middle and low parts are at most 2^-8 and 2^-17, W's less than
+// 2^-7 and 2^-15.  Of the nine products of two such sums six are kept (high x high, the two of high x middle, middle x middle, the two of
+// high x low); the other three come to less than 2^-24 + 2^-23 + 2^-32 of the product, with signs of their own.  The tensor cores multiply
+// exactly and add up in their accumulator, which cuts off where an addition rounds, so a sum stays there for 32 numbers of the inner
+// dimension only (small products first) and is then added in float32: the error against 64 bits is a third to a sixth of the float32 library
+// product's (520 rows, 4096 x 4096: 2.2e-7 against 1.1e-6 of the result's norm; 1024 x 14336: 3.9e-7 against 2.2e-6).
 //
 // The float32 units reach 72 TFLOP/s at most, the library's product 54; six bfloat16 products per float32 product are 230 TFLOP/s at the tensor
 // cores' rate.  520 rows: 28672 x 4096 611 us (library 2289), 6144 x 4096 129 (540), 4096 x 4096 109 (325), 4096 x 14336 356 (1126).
@@ -29,8 +30,7 @@
 // finite, or so far apart that the smallest lose bits; rows of W with a number of 2^30 or more, or not finite) is marked, of x by the kernel
 // that splits it, of W by the warps that do, and outputs of marked rows are computed again in plain float32 by the warps that add, four rows of W times four of x at a
 // time (520 rows, 4096 x 4096, 131 us: with one marked row of W 582, of x 283, with all rows marked 2,660; a thread per output took 14,700, 600 and
-// 69,000.  The other warps wait meanwhile: a tile whose rows are all marked takes 2 ms at K = 4,096 and less than a tenth of their limit at
-// the largest K).
+// 69,000.  The other warps wait meanwhile: for a tile whose rows are all marked some 3 ms at K = 4,096, 0.2 s of their limit of 2 s at the largest K).
 //
 // The twelve MMAs of 32 numbers take 1,060 cycles for 176 rows of x; a wait for an mbarrier costs its role some 200, even if it is over.  So
 // the whole of warp 2 walks its loop, with descriptors in uniform registers, and one elected lane issues (as one thread's work a step took 1,700
@@ -76,8 +76,8 @@ __device__ __forceinline__ void ls_split(float a, float b, unsigned& high, unsig
   mid = pack_bf16x2(ra, rb);
   low = pack_bf16x2(ra - __uint_as_float(mid << 16), rb - __uint_as_float(mid & 0xffff0000u));
 }
-// The same cut off instead of rounded, which takes no conversions.  The parts left out of the products have random signs all the same, since
-// x's parts are rounded.
+// The same cut off instead of rounded, which takes no conversions.  The signs of what the products leave out follow x's parts, which are
+// rounded to either side.
 __device__ __forceinline__ void ls_cut(float a, float b, unsigned& high, unsigned& mid, unsigned& low) {
   const unsigned ua = __float_as_uint(a), ub = __float_as_uint(b);
   high = __byte_perm(ua, ub, 0x7632);

@@ -38,8 +38,8 @@ def test_linear_split(M, N, K, spread, with_bias):
     if with_bias:
         want, size = want + b.double(), size + b.double().abs()
     # A sum of 32 numbers in the tensor cores is cut off some twelve times at 2^-23 of its size at most, the sums of those are rounded at
-    # 2^-24 each, and what the split leaves out is below 2^-23 of each product.
-    bound = (12 + K / 64 + 1) * 2.0 ** -23 * size
+    # 2^-24 each, and the three products that the split leaves out are below 2^-24 + 2^-23 + 2^-32 < 2 * 2^-23 of each product.
+    bound = (12 + K / 64 + 2) * 2.0 ** -23 * size
     assert ((got.double() - want).abs() <= bound).all()
     plain = torch.matmul(x, w.t()) if b is None else torch.addmm(b, x, w.t())
     err = lambda y: float((y.double() - want).norm() / want.norm())
@@ -158,3 +158,15 @@ def test_linear_split_marked_rows(M, N, K, of_x, of_w):
     rows[of_x], cols[of_w] = False, False
     assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
     assert got[~rows].isnan().all() and not got[rows][:, ~cols].isfinite().any()
+
+
+@pytest.mark.parametrize("numbers", [1, 128])
+def test_linear_split_leaves_out_no_more_than_it_says(numbers):
+    """The significands whose products lose most to the split, of one sign, so that nothing cancels."""
+    x, w = torch.zeros(17, 128, device="cuda"), torch.zeros(128, 128, device="cuda")
+    x[:, :numbers] = torch.tensor(0x3f807f40, dtype=torch.int32).view(torch.float32)
+    w[:, :numbers] = torch.tensor(0x3f80ffff, dtype=torch.int32).view(torch.float32)
+    got, want = ops.linear_split(x, w).double(), x.double() @ w.double().t()
+    # of one product: its six kept parts are added up with five cuts at 2^-23; of 128, as above
+    cuts = 5 if numbers == 1 else 12 + 128 / 64
+    assert ((got - want).abs() <= (cuts + 1.51) * 2.0 ** -23 * want).all()
