@@ -1571,6 +1571,8 @@ def linear_split(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] 
         _need(bias, "bias", torch.float32, 1)
         if bias.shape[0] != N:
             raise KernelError(f"linear_split: {bias.shape[0]} biases for {N} rows")
+    if w.device != x.device or (bias is not None and bias.device != x.device):
+        raise KernelError(f"linear_split: x on {x.device}, w on {w.device}" + (f", bias on {bias.device}" if bias is not None else ""))
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     size = build.library("linear_split").bn_linear_split_scratch
     size.restype = ctypes.c_longlong
