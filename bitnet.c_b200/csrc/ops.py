@@ -1576,12 +1576,18 @@ def linear_split(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] 
     out = torch.empty((M, N), dtype=torch.float32, device=x.device)
     size = build.library("linear_split").bn_linear_split_scratch
     size.restype = ctypes.c_longlong
-    scratch = torch.empty(size(int(M), int(K)), dtype=torch.uint8, device=x.device)
-    _check(_fn("linear_split", "bn_linear_split")(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), int(M), int(N), int(K), int(N), _ptr(scratch),
-                                                  _ptr(tc_status(x.device)), _stream()), "linear_split")
+    # x's parts take half as much again as x: bands of rows, where that would be more than LINEAR_SPLIT_SCRATCH
+    band = max(1, min(M, LINEAR_SPLIT_SCRATCH // size(1, K)))
+    scratch = torch.empty(size(band, K), dtype=torch.uint8, device=x.device)
     global LAUNCHES
-    LAUNCHES += 1  # two kernels
+    for m0 in range(0, M, band):
+        _check(_fn("linear_split", "bn_linear_split")(c_void_p(x.data_ptr() + m0 * K * 4), _ptr(w), _ptr(bias), c_void_p(out.data_ptr() + m0 * N * 4),
+                                                      min(band, M - m0), N, K, N, _ptr(scratch), _ptr(tc_status(x.device)), _stream()), "linear_split")
+        LAUNCHES += 1  # two kernels
     return out
+
+
+LINEAR_SPLIT_SCRATCH = 1 << 29  # bytes of working space of one product: 21,800 rows of 4,096 numbers, 6,200 of 14,336
 
 
 # ---- state --------------------------------------------------------------------------------

@@ -160,6 +160,23 @@ def test_linear_split_marked_rows(M, N, K, of_x, of_w):
     assert got[~rows].isnan().all() and not got[rows][:, ~cols].isfinite().any()
 
 
+
+@pytest.mark.parametrize("rows", [1, 192, 299, 300])
+def test_linear_split_in_bands(monkeypatch, rows):
+    """Working space for so many rows only: the same bits, and no more space is asked for."""
+    x, w = _pair(300, 200, 516, 5)
+    b = torch.randn(200, device="cuda")
+    whole = ops.linear_split(x, w, b)
+    most = rows * (6 * 520 + 4)
+    monkeypatch.setattr(ops, "LINEAR_SPLIT_SCRATCH", most)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    got = ops.linear_split(x, w, b)
+    assert torch.cuda.max_memory_allocated() - before <= most + 300 * 200 * 4 + 2 * 512  # (sizes are rounded up to 512 bytes)
+    assert torch.equal(got, whole)
+
+
 @pytest.mark.parametrize("numbers", [1, 128])
 def test_linear_split_leaves_out_no_more_than_it_says(numbers):
     """The significands whose products lose most to the split, of one sign, so that nothing cancels."""
