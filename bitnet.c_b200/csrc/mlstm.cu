@@ -63,14 +63,43 @@ extern "C" int bn_mlstm_gates(const void* h, int h_dtype, int n_tokens, int widt
   return BN_OK;
 }
 
+// The blocks of one (sequence, head) all start from the n and m that are in memory, and one of them puts the new ones there: not before the
+// others have read, and they need not run at the same time (the chunked form has one block on an SM; 64 sequences of 8 heads with 256
+// columns are 4,096 blocks).  Up to ML_CLUSTER blocks are a cluster, whose barrier they pass behind their reads (nobody waits for it before
+// the end).  More of them, or such as would leave SMs empty as clusters, take tickets when they are done (tickets [sequences][heads], zero):
+// the last one writes, all have the same numbers.
+#define ML_CLUSTER 8
+__device__ __forceinline__ void ml_has_read(const int* tickets) {
+  if (tickets == nullptr && gridDim.z > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+}
+// Whether this block writes n and m; every thread of every block calls it once, behind ml_has_read
+__device__ __forceinline__ bool ml_writes(int* tickets) {
+  if (gridDim.z == 1) return true;
+  if (tickets == nullptr) {
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    return blockIdx.z == 0;
+  }
+  __shared__ int ticket;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) ticket = atomicAdd(tickets + blockIdx.x * gridDim.y + blockIdx.y, 1);
+  __syncthreads();
+  return ticket == (int)gridDim.z - 1;
+}
+template <typename... KArgs, typename... Args>
+static cudaError_t ml_launch(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const int* tickets, Args&&... args) {
+  if (tickets == nullptr && grid.z > 1) return bn_launch_cluster(kernel, grid, dim3(threads), smem, stream, dim3(1, 1, grid.z), std::forward<Args>(args)...);
+  return bn_launch(kernel, grid, dim3(threads), smem, stream, std::forward<Args>(args)...);
+}
+
 // One block per (sequence, head, chunk of value columns); thread c owns column c0 + c of S, which
 // lies in shared memory as S[d][c].  Every block of a head keeps n and m itself (the same numbers
-// in the same order in each), the block of chunk 0 writes them back.
+// in the same order in each), one of them writes them back.
 template <typename T>
 __global__ void mlstm_recurrence_kernel(const T* __restrict__ qkv, int row_stride, int k_off, int v_off,
                                         const float* __restrict__ gates, float* __restrict__ state,
                                         const int* __restrict__ seq_start, const int* __restrict__ slots, int n_heads,
-                                        int dim, int vdim, int cols, float q_scale, float* __restrict__ out) {
+                                        int dim, int vdim, int cols, float q_scale, float* __restrict__ out, int* __restrict__ tickets) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ float sm[];
@@ -88,6 +117,7 @@ __global__ void mlstm_recurrence_kernel(const T* __restrict__ qkv, int row_strid
     for (int d = 0; d < dim; ++d) S[d * cols + c] = st[(size_t)d * vdim + c0 + c];
   for (int d = threadIdx.x; d < dim; d += blockDim.x) sn[d] = st_n[d];
   float m = st_n[dim];
+  ml_has_read(tickets);
   const int t0 = seq_start[seq], t1 = seq_start[seq + 1];
   for (int t = t0; t < t1; ++t) {
     const T* row = qkv + (size_t)t * row_stride;
@@ -121,7 +151,7 @@ __global__ void mlstm_recurrence_kernel(const T* __restrict__ qkv, int row_strid
   if (has_col)
     for (int d = 0; d < dim; ++d) st[(size_t)d * vdim + c0 + c] = S[d * cols + c];
   __syncthreads();
-  if (blockIdx.z == 0) {
+  if (ml_writes(tickets)) {
     for (int d = threadIdx.x; d < dim; d += blockDim.x) st_n[d] = sn[d];
     if (threadIdx.x == 0) st_n[dim] = m;
   }
@@ -137,7 +167,7 @@ template <typename T, int D>
 __global__ void __launch_bounds__(128) mlstm_recurrence_warp_kernel(
     const T* __restrict__ qkv, int row_stride, int k_off, int v_off, const float* __restrict__ gates,
     float* __restrict__ state, const int* __restrict__ seq_start, const int* __restrict__ slots, int n_heads, int dim,
-    int vdim, float q_scale, float* __restrict__ out) {
+    int vdim, float q_scale, float* __restrict__ out, int* __restrict__ tickets) {
   pdl_launch_dependents();
   pdl_wait();
   constexpr int DW = D / 4;  // rows of S per warp: 8, 16 or 32
@@ -157,6 +187,7 @@ __global__ void __launch_bounds__(128) mlstm_recurrence_warp_kernel(
   for (int r = 0; r < DW; ++r) S[r] = (has_col && d0 + r < dim) ? st[(size_t)(d0 + r) * vdim + c] : 0.f;
   float n = has_row ? st_n[my_d] : 0.f;
   float m = st_n[dim];
+  ml_has_read(tickets);
   const int t0 = seq_start[seq], t1 = seq_start[seq + 1];
   float qn = 0.f, kn = 0.f, vn = 0.f, gi_n = 0.f, gf_n = 0.f;
   auto fetch = [&](int t) {
@@ -204,7 +235,7 @@ __global__ void __launch_bounds__(128) mlstm_recurrence_warp_kernel(
     for (int r = 0; r < DW; ++r)
       if (d0 + r < dim) st[(size_t)(d0 + r) * vdim + c] = S[r];
   }
-  if (blockIdx.z == 0) {
+  if (ml_writes(tickets)) {
     if (has_row) st_n[my_d] = n;
     if (threadIdx.x == 0) st_n[dim] = m;
   }
@@ -213,31 +244,33 @@ __global__ void __launch_bounds__(128) mlstm_recurrence_warp_kernel(
 template <typename T>
 static cudaError_t launch_mlstm_warp(const void* qkv, int row_stride, int k_off, int v_off, const float* gates, float* state,
                                      const int* seq_start, const int* slots, int n_seqs, int n_heads, int dim, int vdim,
-                                     float q_scale, float* out, cudaStream_t stream) {
+                                     float q_scale, float* out, int* tickets, cudaStream_t stream) {
   dim3 grid(n_seqs, n_heads, (vdim + 31) / 32);
   if (dim <= 32)
-    return bn_launch(mlstm_recurrence_warp_kernel<T, 32>, grid, dim3(128), 0, stream, (const T*)qkv, row_stride, k_off, v_off,
-                     gates, state, seq_start, slots, n_heads, dim, vdim, q_scale, out);
+    return ml_launch(mlstm_recurrence_warp_kernel<T, 32>, grid, 128, 0, stream, tickets, (const T*)qkv, row_stride, k_off, v_off,
+                     gates, state, seq_start, slots, n_heads, dim, vdim, q_scale, out, tickets);
   if (dim <= 64)
-    return bn_launch(mlstm_recurrence_warp_kernel<T, 64>, grid, dim3(128), 0, stream, (const T*)qkv, row_stride, k_off, v_off,
-                     gates, state, seq_start, slots, n_heads, dim, vdim, q_scale, out);
-  return bn_launch(mlstm_recurrence_warp_kernel<T, 128>, grid, dim3(128), 0, stream, (const T*)qkv, row_stride, k_off, v_off,
-                   gates, state, seq_start, slots, n_heads, dim, vdim, q_scale, out);
+    return ml_launch(mlstm_recurrence_warp_kernel<T, 64>, grid, 128, 0, stream, tickets, (const T*)qkv, row_stride, k_off, v_off,
+                     gates, state, seq_start, slots, n_heads, dim, vdim, q_scale, out, tickets);
+  return ml_launch(mlstm_recurrence_warp_kernel<T, 128>, grid, 128, 0, stream, tickets, (const T*)qkv, row_stride, k_off, v_off,
+                   gates, state, seq_start, slots, n_heads, dim, vdim, q_scale, out, tickets);
 }
 
 // qkv: rows of the new tokens with the query heads at element 0, key heads at k_off, value heads at
-// v_off; gates [n_tokens, 2 * heads]; state [slots, heads, dim * vdim + dim + 1]; out [n_tokens, heads * vdim] float32.
+// v_off; gates [n_tokens, 2 * heads]; state [slots, heads, dim * vdim + dim + 1]; out [n_tokens, heads * vdim] float32.  tickets [n_seqs, heads], zero,
+// or null where vdim is at most 32 * ML_CLUSTER.
 extern "C" int bn_mlstm_recurrence(const void* qkv, int dtype, int row_stride, int k_off, int v_off, const float* gates,
                                    float* state, const int* seq_start, const int* slots, int n_seqs, int n_heads, int dim,
-                                   int vdim, float q_scale, float* out, cudaStream_t stream) {
+                                   int vdim, float q_scale, float* out, int* tickets, cudaStream_t stream) {
   if (n_seqs <= 0) return BN_OK;
   if (!qkv || !gates || !state || !out || n_heads <= 0 || dim <= 0 || vdim <= 0 || n_heads > 65535) return BN_ERR_BAD_ARG;
+  if (!tickets && (vdim + 31) / 32 > ML_CLUSTER) return BN_ERR_BAD_ARG;
   if (dim <= 128 && (vdim + 31) / 32 <= 65535 && (dtype == BN_F32 || dtype == BN_BF16)) {
     cudaError_t e = dtype == BN_F32
         ? launch_mlstm_warp<float>(qkv, row_stride, k_off, v_off, gates, state, seq_start, slots, n_seqs, n_heads, dim, vdim,
-                                   q_scale, out, stream)
+                                   q_scale, out, tickets, stream)
         : launch_mlstm_warp<__nv_bfloat16>(qkv, row_stride, k_off, v_off, gates, state, seq_start, slots, n_seqs, n_heads, dim,
-                                           vdim, q_scale, out, stream);
+                                           vdim, q_scale, out, tickets, stream);
     if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
     BN_CHECK_LAUNCH();
     return BN_OK;
@@ -256,16 +289,18 @@ extern "C" int bn_mlstm_recurrence(const void* qkv, int dtype, int row_stride, i
       if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
       granted_f = smem;
     }
-    BN_LAUNCH(mlstm_recurrence_kernel<float>, grid, cols, smem, stream, (const float*)qkv, row_stride, k_off, v_off, gates,
-              state, seq_start, slots, n_heads, dim, vdim, cols, q_scale, out);
+    cudaError_t e = ml_launch(mlstm_recurrence_kernel<float>, grid, cols, smem, stream, tickets, (const float*)qkv, row_stride, k_off, v_off, gates, state,
+                              seq_start, slots, n_heads, dim, vdim, cols, q_scale, out, tickets);
+    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
   } else if (dtype == BN_BF16) {
     if (smem > 48 * 1024 && smem > granted_b) {
       cudaError_t e = cudaFuncSetAttribute(mlstm_recurrence_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
       granted_b = smem;
     }
-    BN_LAUNCH(mlstm_recurrence_kernel<__nv_bfloat16>, grid, cols, smem, stream, (const __nv_bfloat16*)qkv, row_stride,
-              k_off, v_off, gates, state, seq_start, slots, n_heads, dim, vdim, cols, q_scale, out);
+    cudaError_t e = ml_launch(mlstm_recurrence_kernel<__nv_bfloat16>, grid, cols, smem, stream, tickets, (const __nv_bfloat16*)qkv, row_stride, k_off, v_off,
+                              gates, state, seq_start, slots, n_heads, dim, vdim, cols, q_scale, out, tickets);
+    if (e != cudaSuccess) return BN_ERR_LAUNCH + (int)e;
   } else {
     return BN_ERR_BAD_ARG;
   }
@@ -294,7 +329,7 @@ template <typename T>
 __global__ void __launch_bounds__(MLC_THREADS) mlstm_chunk_kernel(
     const T* __restrict__ qkv, int row_stride, int k_off, int v_off, const float* __restrict__ gates,
     float* __restrict__ state, const int* __restrict__ seq_start, const int* __restrict__ slots, int n_heads, int dim,
-    int vdim, float q_scale, float* __restrict__ out) {
+    int vdim, float q_scale, float* __restrict__ out, int* __restrict__ tickets) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
@@ -320,6 +355,7 @@ __global__ void __launch_bounds__(MLC_THREADS) mlstm_chunk_kernel(
   }
   for (int d = tid; d < dim; d += MLC_THREADS) sn[d] = st_n[d];
   float m0 = st_n[dim];
+  ml_has_read(tickets);
   const int t0 = seq_start[seq], t1 = seq_start[seq + 1];
   // Rows of whole 16-byte pieces (the usual case) are read in such pieces, and a chunk's q and k rows are
   // requested into registers while the chunk before is worked on; other sizes go number by number.
@@ -519,18 +555,19 @@ __global__ void __launch_bounds__(MLC_THREADS) mlstm_chunk_kernel(
     int d = i >> 5, cc = i & 31;
     if (c0 + cc < vdim) st[(size_t)d * vdim + c0 + cc] = sS[i];
   }
-  if (blockIdx.z == 0) {
+  if (ml_writes(tickets)) {
     for (int d = tid; d < dim; d += MLC_THREADS) st_n[d] = sn[d];
     if (tid == 0) st_n[dim] = m0;
   }
 }
 
-// As bn_mlstm_recurrence, by chunks of 32 tokens (for steps that bring runs of many tokens).
+// As bn_mlstm_recurrence, by chunks of 32 tokens (for steps that bring runs of many tokens).  tickets [n_seqs, heads], zero: a block fills an SM, and
+// of 148 SMs clusters of eight such blocks would leave some empty.
 extern "C" int bn_mlstm_chunks(const void* qkv, int dtype, int row_stride, int k_off, int v_off, const float* gates,
                                float* state, const int* seq_start, const int* slots, int n_seqs, int n_heads, int dim,
-                               int vdim, float q_scale, float* out, cudaStream_t stream) {
+                               int vdim, float q_scale, float* out, int* tickets, cudaStream_t stream) {
   if (n_seqs <= 0) return BN_OK;
-  if (!qkv || !gates || !state || !out || n_heads <= 0 || dim <= 0 || dim % 4 || vdim <= 0 || n_heads > 65535 ||
+  if (!qkv || !gates || !state || !out || !tickets || n_heads <= 0 || dim <= 0 || dim % 4 || vdim <= 0 || n_heads > 65535 ||
       (vdim + 31) / 32 > 65535)
     return BN_ERR_BAD_ARG;
   size_t floats = 2 * (size_t)MLC_L * (dim + 4) + (size_t)dim * 32 + MLC_L * 32 + MLC_L * (MLC_L + 1) + dim + 2 * MLC_L;
@@ -545,7 +582,7 @@ extern "C" int bn_mlstm_chunks(const void* qkv, int dtype, int row_stride, int k
       granted_f = smem;
     }
     BN_LAUNCH(mlstm_chunk_kernel<float>, grid, MLC_THREADS, smem, stream, (const float*)qkv, row_stride, k_off, v_off, gates,
-              state, seq_start, slots, n_heads, dim, vdim, q_scale, out);
+              state, seq_start, slots, n_heads, dim, vdim, q_scale, out, tickets);
   } else if (dtype == BN_BF16) {
     if (smem > 48 * 1024 && smem > granted_b) {
       cudaError_t e = cudaFuncSetAttribute(mlstm_chunk_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -553,7 +590,7 @@ extern "C" int bn_mlstm_chunks(const void* qkv, int dtype, int row_stride, int k
       granted_b = smem;
     }
     BN_LAUNCH(mlstm_chunk_kernel<__nv_bfloat16>, grid, MLC_THREADS, smem, stream, (const __nv_bfloat16*)qkv, row_stride, k_off,
-              v_off, gates, state, seq_start, slots, n_heads, dim, vdim, q_scale, out);
+              v_off, gates, state, seq_start, slots, n_heads, dim, vdim, q_scale, out, tickets);
   } else {
     return BN_ERR_BAD_ARG;
   }

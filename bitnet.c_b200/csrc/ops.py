@@ -1628,6 +1628,9 @@ def mlstm_state_floats(dim: int, vdim: int) -> int:
     return dim * vdim + dim + 1
 
 
+MLSTM_CLUSTER = 8  # blocks of 32 value columns that run as one cluster (ML_CLUSTER in mlstm.cu)
+
+
 def mlstm_recurrence(qkv: torch.Tensor, k_off: int, v_off: int, gates: torch.Tensor, state: torch.Tensor,
                      seq_start: torch.Tensor, slots: torch.Tensor, n_seqs: int, n_heads: int, dim: int, vdim: int,
                      q_scale: float, chunks: bool = False) -> torch.Tensor:
@@ -1648,9 +1651,11 @@ def mlstm_recurrence(qkv: torch.Tensor, k_off: int, v_off: int, gates: torch.Ten
         raise KernelError("mlstm_recurrence: sizes do not fit")
     out = torch.empty((T, n_heads * vdim), dtype=torch.float32, device=qkv.device)
     entry = "bn_mlstm_chunks" if chunks and dim % 4 == 0 and (2 * 32 * (dim + 4) + 33 * dim + 2200) * 4 <= 200 * 1024 else "bn_mlstm_recurrence"
+    # blocks of one head that cannot be a cluster take tickets when they are done: the last one writes what they share (mlstm.cu)
+    tickets = torch.zeros(n_seqs * n_heads, dtype=torch.int32, device=qkv.device) if entry == "bn_mlstm_chunks" or vdim > 32 * MLSTM_CLUSTER else None
     _check(_fn("mlstm", entry)(_ptr(qkv), int(_code(qkv)), int(qkv.shape[1]), int(k_off), int(v_off),
                                                _ptr(gates), _ptr(state), _ptr(seq_start), _ptr(slots), int(n_seqs),
-                                               int(n_heads), int(dim), int(vdim), c_float(q_scale), _ptr(out), _stream()),
+                                               int(n_heads), int(dim), int(vdim), c_float(q_scale), _ptr(out), _ptr(tickets), _stream()),
            "mlstm_recurrence")
     return out
 

@@ -301,3 +301,42 @@ def test_the_command_line_writes_a_random_model_of_the_design_and_generates_from
     assert p2.returncode == 0, p2.stderr[-2000:]
     assert [l for l in p2.stderr.splitlines() if l.startswith("token_id=")] == \
            [l for l in p.stderr.splitlines() if l.startswith("token_id=")]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("d,vd,lens,chunks", [
+    (128, 256, [2, 500, 1, 64, 3, 300, 33, 5, 31, 32], True),   # a block of the chunked form fills an SM: short sequences are long done when the last ones begin
+    (64, 40, [1, 70, 2, 40] * 20, True),
+    (128, 256, [1] * 64, False),                                 # a token each: 4,096 blocks
+    (128, 256, [3, 1, 9, 2] * 8, False),
+    (32, 320, [1] * 70, False),                                  # more blocks per head than a cluster has
+    (160, 256, [1, 5] * 40, False),                              # heads too large for registers
+    (24, 32, [1, 4] * 8, False),                                 # one block per head
+])
+def test_mlstm_of_many_sequences_is_that_of_each_alone(cuda_device, dtype, d, vd, lens, chunks):
+    """The blocks of a head start from the same n and m, however many of them run at once."""
+    from bitnet_c_b200.csrc import ops
+    H, n = 8, len(lens)
+    g = torch.Generator(device="cuda").manual_seed(d + vd)
+    T = sum(lens)
+    rows = torch.randn(T, 2 * H * d + H * vd, generator=g, device="cuda").to(dtype)
+    gates = torch.randn(T, 2 * H, generator=g, device="cuda")
+    gates[:, H:] = torch.nn.functional.logsigmoid(gates[:, H:] + 2)
+    start = torch.randn(n, H, ops.mlstm_state_floats(d, vd), generator=g, device="cuda") * 0.1
+    slots = torch.arange(n, dtype=torch.int32, device="cuda")
+    at = [0]
+    for l in lens:
+        at.append(at[-1] + l)
+
+    def run(rows_of, gates_of, starts, of):
+        state = start.clone()
+        o = ops.mlstm_recurrence(rows_of.contiguous(), H * d, 2 * H * d, gates_of.contiguous(), state, torch.tensor(starts, dtype=torch.int32, device="cuda"),
+                                 slots[of].contiguous(), len(starts) - 1, H, d, vd, d ** -0.5, chunks=chunks)
+        return o, state
+
+    for _ in range(3):
+        whole, state = run(rows, gates, at, slice(0, n))
+        for i in range(n):
+            a, b = at[i], at[i + 1]
+            o, alone = run(rows[a:b], gates[a:b], [0, b - a], slice(i, i + 1))
+            assert torch.equal(whole[a:b], o) and torch.equal(state[i], alone[i]), i
