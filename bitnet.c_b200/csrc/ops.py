@@ -1544,18 +1544,19 @@ def few_layers(step, launches: int) -> None:
 
 
 def linear_split_pays(M: int, N: int, K: int) -> bool:
-    """Whether a float32 product goes to ``linear_split.cu``.  The library product's time over that kernel's: 520 to 2,048 rows 1.3 to 4.2 with a
-    million outputs and more (1.05 to 1.1 right at the line); 17 and more rows of matrices of 2,048 rows and more 1.2 to 1.95 (2048 x 1024, 8192 x 512 and
-    16384 x 256 to 28672 x 4096), unless the inner dimension is so long that the library splits it (2048 x 8192 0.76 to 1.26, 4096 x 14336 1.27);
-    100 and more rows of 1,024 x 2,048, 1,536 x 4,096, 1024 x 14336 1.2 to 2.1.  A matrix of fewer rows leaves most SMs idle: 17 rows 1024 x 4096
-    0.5, 512 x 2048 0.54.  Short inner dimensions leave it its start: 4,000 x 256 x 256 0.6."""
+    """Whether a float32 product goes to ``linear_split.cu``.  The library product's time over that kernel's, calls behind a flush of the L2:
+    many rows and outputs (the first rule) 1.5 to 4.0; matrices of 2,048 rows and more with 17 to 128 rows of x 1.13 to 2.0 while the inner dimension is no
+    more than twice the rows (8192 x 256 with 17 rows 0.93), beyond that, where the library splits it, from 4,096 rows on and with 40 rows of x 1.36 to
+    2.4; matrices of 1,024 and 1,536 rows with 96 and more 1.2 to 1.9 (1024 x 14336 with 96 rows 0.95).  Left to the library: long inner dimensions with
+    fewer rows of x (4096 x 9000 to 8192 x 28672 1.0 to 1.7, 2048 x 8192 0.75 to 1.26, 3072 x 8192 0.88 to 1.04), matrices of 1,024 rows with up to 72
+    (0.47 to 1.0; 1024 x 2048 with 48 to 88 1.2 to 1.5), which leave most SMs idle, 512 x 2048 (0.59 to 0.73 with up to 96), and short inner dimensions
+    (2048 x 512 1.05 to 1.2; 4,000 x 256 x 256 0.6)."""
     if not 128 <= K <= 1 << 18:  # the kernel's least and most
         return False
-    if M * N >= 1 << 20 and M >= 48 and M * N * K >= 1 << 30:
+    if M >= 48 and M * N >= 1 << 20 and M * N * K >= 1 << 30:
         return True
-    if N >= 4096 and M >= 48 and M * N >= 280000 and K >= 1024:
-        return True
-    return N * K >= 1 << 21 and K >= 256 and (N >= 2048 and M >= 17 and K <= 2 * N or N >= 1024 and M >= 96)
+    few = 17 if K <= 2 * N else 40 if N >= 4096 else 96  # the least rows of x
+    return K >= 256 and N * K >= 1 << 21 and M >= (few if N >= 2048 else 96) and N >= 1024
 
 
 def linear_split(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
