@@ -9,7 +9,8 @@
 // product's (520 rows, 4096 x 4096: 2.2e-7 against 1.1e-6 of the result's norm; 1024 x 14336: 3.9e-7 against 2.2e-6).
 //
 // The float32 units reach 72 TFLOP/s at most, the library's product 54; six bfloat16 products per float32 product are 230 TFLOP/s at the tensor
-// cores' rate.  520 rows: 28672 x 4096 611 us (library 2289), 6144 x 4096 129 (540), 4096 x 4096 109 (325), 4096 x 14336 356 (1126).
+// cores' rate.  520 rows: 28672 x 4096 611 us (library 2289), 6144 x 4096 129 (540), 4096 x 4096 109 (325), 4096 x 14336 356 (1126); scaling W on the way
+// (below) takes 0 to 2 % of that: 28672 x 4096 behind a flush of the L2 617 -> 620.
 //
 // A tile is 128 rows of W times up to 192 rows of x: D[128 rows of W, NT rows of x], so that few and odd numbers of rows of x waste
 // little (NT is a multiple of 16, chosen so that the tiles fill the SMs).  x is split once, by a kernel of its own, into three
